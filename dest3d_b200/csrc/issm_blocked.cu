@@ -1,0 +1,1080 @@
+// Blocked fp32 kernels of the ISSM scan: float32 arithmetic in register-tiled contractions.  They serve every call that
+// the tensor-core kernels do not (float32 activations, other state counts and head widths) up to headdim 128 or what
+// shared memory holds; wider heads stay on the per-pair kernels of issm_simt.cu.
+//
+// A warp owns 32 states of one (batch, head) stream and walks the sequence in blocks of 32 rows; its operand tiles live
+// in its own part of shared memory.  With a = in-block cumsum of dt*A in log2 units and a_last its value at the block end
+//   Cd[n,l] = C[l,n] 2^a[l,n]          Bd[n,s] = B[s,n] dt[s,n] 2^-a[s,n]
+//   M[l,s]  = sum_n Cd Bd,  Y[l,p] = sum_n Cd[n,l] S[n,p] + sum_{s<=l} M[l,s] x[s,p],  S <- 2^a_last (S + sum_s Bd x)
+// (the reference's chunk stages, issm_triton/issm_combined.py:57-179, with the state carried on chip).  Per block and
+// warp that is 115 k multiply-adds forward and 250 k backward at headdim 36; the per-pair kernels spent an exponential on
+// every (row, row, state) triple.  The bound is the fp32 pipe (FFMA2 pairs); the elementwise part is ~1/4 of it.
+// Measured against the per-pair kernels: 2 layers x 2 directions forward, b16 x 4096 points x 512 states float32 148 -> 21.8 ms;
+// both directions forward + backward, b2 x 1024 x 256 float32 16.3 -> 2.75 ms.
+//
+// Range: every factor stays finite while |a| <= 100 over a block.  A block outside that is computed from non-positive
+// differences only: Bd is built relative to the block END, and M (and the in-block parts of the backward) come from a
+// per-pair routine (slow_*).  The vote is block-wide, so no second launch is needed.
+//
+// Work split: grid = (batch x heads) x (slices of NW warps = 32 NW states) x (segments of the sequence).  Slices give
+// partial output rows that a combine kernel adds (M is linear in the states).  Segments are used when the streams alone
+// leave the chip idle: a states-only walk gives each segment's local end state, k_blk_chain chains them, and the full walk
+// then starts every segment from the state entering it.
+#include "issm_common.cuh"
+
+namespace issm {
+namespace {
+
+constexpr int R = 32;            // rows per block
+constexpr int LDT = 36;          // row stride of the [state][row] tiles: 16-byte aligned, 4 banks apart
+constexpr float kLog2e = 1.4426950408889634f;
+constexpr float kRange = 100.f;  // largest |a| of the factored form
+
+struct BArgs {
+  int b, L, H, P, N, G, hpg, rev, softplus, dt_bf16, has_D, D_has_hdim, want_final, vec4;
+  int nblk, nseg, seg_blk, nslice, nw, nch, SP;     // SP: row stride of the state tiles (floats)
+  float dtmin, dtmax;
+  const void *x, *B, *C, *z, *dout, *y;
+  int64_t x_sb, x_sl, x_sh, B_sb, B_sl, B_sg, C_sb, C_sl, C_sg, z_sb, z_sl, z_sh, g_sb, g_sl, g_sh, o_sb, o_sl, o_sh;
+  const void* dt; int64_t dt_sb, dt_sl, dt_sh;
+  const float *A, *bias, *D;
+  const float* enter;     // (b*H, nseg, N, PW) state entering (forward) / gradient leaving (backward) every segment
+  const void* init;       // (b, H, P, N), first segment when `enter` is not used
+  const float* dfinal;    // (b, H, P, N), last segment of the backward when `enter` is not used
+  float* seg_out;         // states-only walk: (b*H, nseg, N, PW) local end state
+  float* seg_sum;         //                   (b*H, nseg, N) summed a
+  float* saved;           // (b*H, nblk + 1, N, PW) state entering every block
+  void *out, *out_x;
+  float* part;            // (nslice, b, L, H, P) partial output rows (forward y, backward dx) when nslice > 1
+  float* final_states;
+  void *dx, *dz, *dinit, *ddt, *dB, *dC;
+  float *dBh, *dCh;       // (b, L, H, N)
+  float *dApart, *dbpart; // (b*H*nseg, N)
+  float* dDpart;          // (b*H*nseg) or (b*H*nseg, P)
+};
+
+__device__ __forceinline__ int brow(const BArgs& a, int t) { return a.rev ? a.L - 1 - t : t; }
+__device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float4 ld4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) { *(float4*)p = make_float4(a, b, c, d); }
+__device__ __forceinline__ float f4get(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+
+// dt of one row as the scan uses it: bias, softplus (reference threshold), clamp
+__device__ __forceinline__ float dt_value(const BArgs& a, float raw, float bias) {
+  float v = raw + bias;
+  if (a.softplus) v = softplus_thr(v);
+  return fminf(fmaxf(v, a.dtmin), a.dtmax);
+}
+
+// this lane's state column of the 32 rows of a block: raw dt (all loads in flight together)
+__device__ __forceinline__ void load_dt(const BArgs& a, int bi, int h, int n, bool act, int row0, int rows, float* raw) {
+  const int64_t base = bi * a.dt_sb + h * a.dt_sh + n;
+  if (a.dt_bf16) {
+    const bf16* __restrict__ p = (const bf16*)a.dt + base;
+#pragma unroll
+    for (int r = 0; r < R; ++r) raw[r] = act ? ldf(p + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.dt_sl) : 0.f;
+  } else {
+    const float* __restrict__ p = (const float*)a.dt + base;
+#pragma unroll
+    for (int r = 0; r < R; ++r) raw[r] = act ? ldf(p + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.dt_sl) : 0.f;
+  }
+}
+
+// rows [lg*8, +8) x the columns {cg*4.., 32 + cg} of a state tile chunk: += sum_k A[k][row] * S[k][col]
+template <int PC, bool kM>
+__device__ __forceinline__ void gemm_y(const float* A, const float* Bm, const float* S, int SP, int lg, int cg, float2 (&m)[8][2],
+                                       float2 (&y)[8][2], float2 (&y4)[4]) {
+#pragma unroll 4
+  for (int k = 0; k < R; ++k) {
+    const float4 a0 = ld4(A + k * LDT + lg * 8), a1 = ld4(A + k * LDT + lg * 8 + 4), sv = ld4(S + k * SP + cg * 4);
+    const float av[8] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w};
+    float4 bv;
+    if (kM) bv = ld4(Bm + k * LDT + cg * 4);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float2 d = dup(av[i]);
+      if (kM) {
+        m[i][0] = __ffma2_rn(d, make_float2(bv.x, bv.y), m[i][0]);
+        m[i][1] = __ffma2_rn(d, make_float2(bv.z, bv.w), m[i][1]);
+      }
+      y[i][0] = __ffma2_rn(d, make_float2(sv.x, sv.y), y[i][0]);
+      y[i][1] = __ffma2_rn(d, make_float2(sv.z, sv.w), y[i][1]);
+    }
+    if (PC == 5) {
+      const float2 s4 = dup(S[k * SP + 32 + cg]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y4[i] = __ffma2_rn(make_float2(av[2 * i], av[2 * i + 1]), s4, y4[i]);
+    }
+  }
+}
+// states {lg + 4 i} x 4 columns (cg*4): += sum_k A[n][k] * Bm[k][col]   (A state-major with row stride lda, `kn` k's, % 4 == 0)
+__device__ __forceinline__ void gemm_n(const float* A, int lda, const float* Bm, int ldb, int kn, int lg, int cg, float2 (&acc)[8][2]) {
+#pragma unroll 2
+  for (int k = 0; k < kn; k += 4) {
+    float4 b[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) b[q] = ld4(Bm + (k + q) * ldb + cg * 4);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 av = ld4(A + (lg + 4 * i) * lda + k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 d = dup(f4get(av, q));
+        acc[i][0] = __ffma2_rn(d, make_float2(b[q].x, b[q].y), acc[i][0]);
+        acc[i][1] = __ffma2_rn(d, make_float2(b[q].z, b[q].w), acc[i][1]);
+      }
+    }
+  }
+}
+// state update: T[n][p] <- post[n] * (pre[n] * T[n][p] + sum_r Op[n][r] * src[r][p]) over one chunk of columns; optionally
+// copies the OLD tile to `keep` (global, row stride PW)
+template <int PC>
+__device__ __forceinline__ void update_state(float* T, int SP, const float* Op, const float* src, int lg, int cg, float pre, float post) {
+  float2 acc[8][2];
+  float a4[8], po[8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const float pr = __shfl_sync(0xffffffffu, pre, lg + 4 * i);
+    po[i] = __shfl_sync(0xffffffffu, post, lg + 4 * i);
+    const float4 v = ld4(T + (lg + 4 * i) * SP + cg * 4);
+    acc[i][0] = make_float2(v.x * pr, v.y * pr);
+    acc[i][1] = make_float2(v.z * pr, v.w * pr);
+    a4[i] = PC == 5 ? T[(lg + 4 * i) * SP + 32 + cg] * pr : 0.f;
+  }
+#pragma unroll 2
+  for (int k = 0; k < R; k += 4) {
+    float4 b[4];
+    float b4[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      b[q] = ld4(src + (k + q) * SP + cg * 4);
+      b4[q] = PC == 5 ? src[(k + q) * SP + 32 + cg] : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const float4 av = ld4(Op + (lg + 4 * i) * LDT + k);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float2 d = dup(f4get(av, q));
+        acc[i][0] = __ffma2_rn(d, make_float2(b[q].x, b[q].y), acc[i][0]);
+        acc[i][1] = __ffma2_rn(d, make_float2(b[q].z, b[q].w), acc[i][1]);
+        if (PC == 5) a4[i] = fmaf(d.x, b4[q], a4[i]);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    st4(T + (lg + 4 * i) * SP + cg * 4, acc[i][0].x * po[i], acc[i][0].y * po[i], acc[i][1].x * po[i], acc[i][1].y * po[i]);
+    if (PC == 5) T[(lg + 4 * i) * SP + 32 + cg] = a4[i] * po[i];
+  }
+}
+
+// ---- blocks outside the range of the factored form (rare, kept out of line) -----------------------------------------
+template <typename TIO>
+struct Lane { float v[R], a[R], c[R], b[R]; };
+template <typename TIO>
+__device__ __noinline__ void slow_lane(const BArgs& p, int bi, int h, int n, bool act, int row0, int rows, float A2, float bias, Lane<TIO>& s) {
+  const int g = h / p.hpg;
+  load_dt(p, bi, h, n, act, row0, rows, s.v);
+  float acc = 0.f;
+  for (int r = 0; r < R; ++r) {
+    const bool in = act && r < rows;
+    const int mr = brow(p, row0 + min(r, rows - 1));
+    s.v[r] = in ? dt_value(p, s.v[r], bias) : 0.f;
+    acc = fmaf(s.v[r], A2, acc);
+    s.a[r] = acc;
+    s.c[r] = in ? ldf((const TIO*)p.C + bi * p.C_sb + (int64_t)mr * p.C_sl + g * p.C_sg + n) : 0.f;
+    s.b[r] = in ? ldf((const TIO*)p.B + bi * p.B_sb + (int64_t)mr * p.B_sl + g * p.B_sg + n) * s.v[r] : 0.f;
+  }
+}
+// this warp's part of M[l][s] = sum_n C B dt 2^(a_l - a_s), s <= l, to out[l * ldo + s] (or transposed)
+template <typename TIO>
+__device__ __noinline__ void slow_M(const BArgs& p, int bi, int h, int n, bool act, int row0, int rows, float A2, float bias, float* out,
+                                    int ldo, bool transposed) {
+  Lane<TIO> s;
+  slow_lane<TIO>(p, bi, h, n, act, row0, rows, A2, bias, s);
+  for (int l = 0; l < R; ++l)
+    for (int q = 0; q <= l; ++q) {
+      const float m = warp_sum(s.c[l] * s.b[q] * exp2f(s.a[l] - s.a[q]));
+      if ((threadIdx.x & 31) == 0) out[transposed ? q * ldo + l : l * ldo + q] = m;
+    }
+  __syncwarp();
+}
+// this lane's rows of CD and BD, complete with their decays:
+//   CD[l] <- 2^a_l CD[l] + sum_{s<=l} B dt 2^(a_l - a_s) dM[l][s]
+//   BD[s] <- 2^(a_last - a_s) BD[s] + sum_{l>=s} C 2^(a_l - a_s) dM[l][s]
+template <typename TIO>
+__device__ __noinline__ void slow_grads(const BArgs& p, int bi, int h, int n, bool act, int row0, int rows, float A2, float bias,
+                                        const float* dM, float* CD, float* BD) {
+  Lane<TIO> s;
+  slow_lane<TIO>(p, bi, h, n, act, row0, rows, A2, bias, s);
+  for (int l = 0; l < R; ++l) {
+    float acc = exp2f(s.a[l]) * CD[l];
+    for (int q = 0; q <= l; ++q) acc = fmaf(s.b[q] * exp2f(s.a[l] - s.a[q]), dM[l * LDT + q], acc);
+    CD[l] = acc;
+    acc = exp2f(s.a[R - 1] - s.a[l]) * BD[l];
+    for (int q = l; q < R; ++q) acc = fmaf(s.c[q] * exp2f(s.a[q] - s.a[l]), dM[q * LDT + l], acc);
+    BD[l] = acc;
+  }
+}
+
+// one element of dy = dout * z * sigmoid(z) (dout without a gate) at memory row mr; dz as issm_chunk_scan.py:351-360
+template <typename TIO>
+__device__ __forceinline__ float dy_value(const BArgs& a, int bi, int h, int mr, int p, bool write_dz) {
+  const float go = ldf((const TIO*)a.dout + bi * a.g_sb + (int64_t)mr * a.g_sl + h * a.g_sh + p);
+  if (!a.z) return go;
+  const float zv = ldf((const TIO*)a.z + bi * a.z_sb + (int64_t)mr * a.z_sl + h * a.z_sh + p);
+  const float sg = sigmoidf_(zv);
+  if (write_dz) {
+    const float yv = ldf((const TIO*)a.y + bi * a.o_sb + (int64_t)mr * a.o_sl + h * a.o_sh + p);
+    stf((TIO*)a.dz + (((size_t)bi * a.L + mr) * a.H + h) * a.P + p, go * yv * sg * (1.f + zv * (1.f - sg)));
+  }
+  return go * zv * sg;
+}
+
+// ---- states-only walk ------------------------------------------------------------------------------------------------
+// kBwd = false: S <- 2^a_last S + sum_s B dt 2^(a_last - a_s) x_s in scan order, the state entering every block to `saved`
+// (when asked for); kBwd = true: G <- 2^a_last G + sum_l C 2^a_l dy_l against the scan order.  Local end states and the
+// summed decay of every segment go to seg_out / seg_sum.  Exponents are non-positive: no range rule.
+template <int PC, typename TIO, bool kBwd>
+__global__ void __launch_bounds__(128) k_blk_states(const __grid_constant__ BArgs a) {
+  constexpr int W = 8 * PC;
+  extern __shared__ float4 sm4[];
+  float* sm = (float*)sm4;
+  const int SP = a.SP, PW = a.nch * W;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lg = lane >> 3, cg = lane & 7, nt = blockDim.x;
+  float* src = sm;                                        // [32][SP] x or dy rows
+  float* Op = sm + R * SP + warp * (R * LDT + R * SP);    // [n][row]
+  float* T = Op + R * LDT;                                // [n][SP]
+  const int seg = blockIdx.z, stream = blockIdx.x, bi = stream / a.H, h = stream % a.H, g = h / a.hpg;
+  const int n = (blockIdx.y * a.nw + warp) * 32 + lane;
+  const bool act = n < a.N;
+  const float A2 = act ? a.A[h * a.N + n] * kLog2e : 0.f, bias = (act && a.bias) ? a.bias[h * a.N + n] : 0.f;
+  for (int i = tid; i < R * SP; i += nt) src[i] = 0.f;
+  for (int p = 0; p < SP; ++p) T[lane * SP + p] = 0.f;
+  if (!kBwd && act && a.nseg == 1 && a.init)
+    for (int p = 0; p < a.P; ++p) T[lane * SP + p] = ldf((const TIO*)a.init + ((size_t)stream * a.P + p) * a.N + n);
+  if (!kBwd && act && a.enter)
+    for (int p = 0; p < a.P; ++p) T[lane * SP + p] = a.enter[(((size_t)stream * a.nseg + seg) * a.N + n) * PW + p];
+  const int j0 = seg * a.seg_blk, j1 = min(a.nblk, j0 + a.seg_blk);
+  float asum = 0.f;
+  auto keep = [&](int j) {                                // the tile to saved[j], 16 bytes per lane
+    for (int i = lane; i < R * (PW / 4); i += 32) {
+      const int r = i / (PW / 4), c = i % (PW / 4), nn = n - lane + r;
+      if (nn < a.N) *(float4*)(a.saved + (((size_t)stream * (a.nblk + 1) + j) * a.N + nn) * PW + c * 4) = ld4(T + r * SP + c * 4);
+    }
+  };
+  for (int jj = j0; jj < j1; ++jj) {
+    const int j = kBwd ? j1 - 1 - (jj - j0) : jj;
+    const int row0 = j * R, rows = min(R, a.L - row0);
+    float raw[R];
+    load_dt(a, bi, h, n, act, row0, rows, raw);
+    __syncthreads();
+    for (int i = tid; i < R * a.P; i += nt) {
+      const int r = i / a.P, p = i - r * a.P, mr = brow(a, row0 + min(r, rows - 1));
+      float v;
+      if (kBwd) v = dy_value<TIO>(a, bi, h, mr, p, false);
+      else v = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh + p);
+      src[r * SP + p] = r < rows ? v : 0.f;
+    }
+    float acc = 0.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      raw[r] = (act && r < rows) ? dt_value(a, raw[r], bias) : 0.f;
+      acc = fmaf(raw[r], A2, acc);
+    }
+    const float alast = acc;
+    asum += alast;
+    const TIO* __restrict__ bc = kBwd ? (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + n : (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + n;
+    const int64_t bsl = kBwd ? a.C_sl : a.B_sl;
+    acc = 0.f;
+    if (!kBwd && a.saved) keep(j);
+#pragma unroll
+    for (int r0 = 0; r0 < R; r0 += 8) {
+      float cv[8], o[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) cv[q] = act ? ldf(bc + (int64_t)brow(a, row0 + min(r0 + q, rows - 1)) * bsl) : 0.f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        acc = fmaf(raw[r0 + q], A2, acc);
+        o[q] = kBwd ? cv[q] * exp2f(acc) : cv[q] * raw[r0 + q] * exp2f(alast - acc);
+        if (r0 + q >= rows) o[q] = 0.f;
+      }
+      st4(Op + lane * LDT + r0, o[0], o[1], o[2], o[3]);
+      st4(Op + lane * LDT + r0 + 4, o[4], o[5], o[6], o[7]);
+    }
+    __syncthreads();
+    const float el = exp2f(alast);
+    for (int c = 0; c < a.nch; ++c) update_state<PC>(T + c * W, SP, Op, src + c * W, lg, cg, el, 1.f);
+    __syncwarp();
+  }
+  if (!kBwd && a.saved && j1 == a.nblk) keep(a.nblk);
+  if (a.seg_out && act) {
+    float* o = a.seg_out + (((size_t)stream * a.nseg + seg) * a.N + n) * PW;
+    for (int p = 0; p < PW; p += 4) *(float4*)(o + p) = ld4(T + lane * SP + p);
+    a.seg_sum[((size_t)stream * a.nseg + seg) * a.N + n] = asum;
+  }
+}
+
+// Chains the segments: state entering (reverse = 0) or gradient leaving (reverse = 1) every segment, in place of the local
+// end states; one thread per (stream, state, channel).  The last state goes to fin (b, H, P, N) when given.
+template <typename TIO>
+__global__ void k_blk_chain(const __grid_constant__ BArgs a, int PW, int reverse, float* fin, TIO* fin_io) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (size_t)a.b * a.H * a.N * PW) return;
+  const int p = (int)(i % PW), n = (int)(i / PW % a.N);
+  const size_t stream = i / ((size_t)PW * a.N);
+  const size_t e = (stream * a.P + p) * a.N + n;
+  float run = 0.f;
+  if (p < a.P) {
+    if (reverse) run = a.dfinal ? a.dfinal[e] : 0.f;
+    else run = a.init ? ldf((const TIO*)a.init + e) : 0.f;
+  }
+  for (int k = 0; k < a.nseg; ++k) {
+    const int s = reverse ? a.nseg - 1 - k : k;
+    const size_t at = (stream * a.nseg + s) * a.N + n;
+    const float local = a.seg_out[at * PW + p];
+    a.seg_out[at * PW + p] = run;
+    run = fmaf(exp2f(a.seg_sum[at]), run, local);
+  }
+  if (p < a.P && fin) fin[e] = run;
+  if (p < a.P && fin_io) stf(fin_io + e, run);
+}
+
+// Reduces the warps' partial [M | ...] tiles: masked M to Ms[row][col] (mask: col <= row, or col >= row when transposed)
+__device__ __forceinline__ void reduce_M(const float* red, size_t warp_stride, int nw, int RW, float* Ms, bool transposed) {
+  for (int i = threadIdx.x; i < R * (R / 4); i += blockDim.x) {
+    const int r = i >> 3, c = (i & 7) * 4;
+    float4 v = ld4(red + r * RW + c);
+    for (int w = 1; w < nw; ++w) {
+      const float4 u = ld4(red + w * warp_stride + r * RW + c);
+      v.x += u.x; v.y += u.y; v.z += u.z; v.w += u.w;
+    }
+    const bool t = transposed;
+    st4(Ms + r * LDT + c, (t ? c >= r : c <= r) ? v.x : 0.f, (t ? c + 1 >= r : c + 1 <= r) ? v.y : 0.f,
+        (t ? c + 2 >= r : c + 2 <= r) ? v.z : 0.f, (t ? c + 3 >= r : c + 3 <= r) ? v.w : 0.f);
+  }
+}
+// stores the lane's tile of one chunk of [M | Y] to the warp's partial tile
+template <int PC>
+__device__ __forceinline__ void store_y(float* red, int RW, int col, int lg, int cg, const float2 (&y)[8][2], const float2 (&y4)[4]) {
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    float* o = red + (lg * 8 + i) * RW + col;
+    st4(o + cg * 4, y[i][0].x, y[i][0].y, y[i][1].x, y[i][1].y);
+    if (PC == 5) o[32 + cg] = i & 1 ? y4[i >> 1].y : y4[i >> 1].x;
+  }
+}
+// rows {l0, l0 + 4} (l0 = base + lg) of one chunk: partial sums of the warps + sum_k Ms[l][k] src[k][col]
+template <int PC>
+__device__ __forceinline__ void final_rows(const float* red, size_t warp_stride, int nw, int RW, int col, const float* Ms, const float* src,
+                                           int SP, int l0, int cg, float (&y)[2][PC]) {
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    const float* q = red + (l0 + 4 * u) * RW + col;
+#pragma unroll
+    for (int c = 0; c < PC; ++c) y[u][c] = 0.f;
+    for (int w = 0; w < nw; ++w, q += warp_stride) {
+      const float4 v = ld4(q + cg * 4);
+      y[u][0] += v.x; y[u][1] += v.y; y[u][2] += v.z; y[u][3] += v.w;
+      if (PC == 5) y[u][4] += q[32 + cg];
+    }
+  }
+#pragma unroll 2
+  for (int k = 0; k < R; k += 4) {
+    const float4 m0 = ld4(Ms + l0 * LDT + k), m1 = ld4(Ms + (l0 + 4) * LDT + k);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 v = ld4(src + (k + q) * SP + cg * 4);
+      const float a0 = f4get(m0, q), a1 = f4get(m1, q);
+      y[0][0] = fmaf(a0, v.x, y[0][0]); y[0][1] = fmaf(a0, v.y, y[0][1]); y[0][2] = fmaf(a0, v.z, y[0][2]); y[0][3] = fmaf(a0, v.w, y[0][3]);
+      y[1][0] = fmaf(a1, v.x, y[1][0]); y[1][1] = fmaf(a1, v.y, y[1][1]); y[1][2] = fmaf(a1, v.z, y[1][2]); y[1][3] = fmaf(a1, v.w, y[1][3]);
+      if (PC == 5) {
+        const float s4 = src[(k + q) * SP + 32 + cg];
+        y[0][4] = fmaf(a0, s4, y[0][4]); y[1][4] = fmaf(a1, s4, y[1][4]);
+      }
+    }
+  }
+}
+
+// out = (y + D x) * silu(z) for one element; pre-gate value to out_x when gated
+template <typename TIO>
+__device__ __forceinline__ void finish_out(const BArgs& a, int bi, int h, int mr, int p, float y, float xv) {
+  if (a.has_D) y = fmaf(a.D_has_hdim ? __ldg(a.D + h * a.P + p) : __ldg(a.D + h), xv, y);
+  const int64_t o = bi * a.o_sb + (int64_t)mr * a.o_sl + h * a.o_sh + p;
+  if (a.z) {
+    stf((TIO*)a.out_x + o, y);
+    const float zv = ldf((const TIO*)a.z + bi * a.z_sb + (int64_t)mr * a.z_sl + h * a.z_sh + p);
+    y *= zv * sigmoidf_(zv);
+  }
+  stf((TIO*)a.out + o, y);
+}
+
+// ---- forward ---------------------------------------------------------------------------------------------------------
+template <int PC, typename TIO>
+__global__ void __launch_bounds__(128) k_blk_fwd(const __grid_constant__ BArgs a) {
+  constexpr int W = 8 * PC;
+  extern __shared__ float4 sm4[];
+  float* sm = (float*)sm4;
+  const int SP = a.SP, PW = a.nch * W, RW = R + PW;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lg = lane >> 3, cg = lane & 7, nt = blockDim.x;
+  float* xs = sm;                                         // [32][SP]
+  float* Ms = xs + R * SP;                                // [32][LDT]
+  const size_t wstride = 2 * R * LDT + R * SP + R * RW;
+  float* red0 = Ms + R * LDT;                             // per warp: partial [M | Y], Cd, Bd, S
+  float* red = red0 + warp * wstride;
+  float* Cd = red + R * RW;
+  float* Bd = Cd + R * LDT;
+  float* S = Bd + R * LDT;
+  const int seg = blockIdx.z, stream = blockIdx.x, bi = stream / a.H, h = stream % a.H, g = h / a.hpg;
+  const int n = (blockIdx.y * a.nw + warp) * 32 + lane;
+  const bool act = n < a.N;
+  const float A2 = act ? a.A[h * a.N + n] * kLog2e : 0.f, bias = (act && a.bias) ? a.bias[h * a.N + n] : 0.f;
+  for (int i = tid; i < R * SP; i += nt) xs[i] = 0.f;
+  for (int p = 0; p < SP; ++p) S[lane * SP + p] = 0.f;
+  if (act && a.enter)
+    for (int p = 0; p < a.P; ++p) S[lane * SP + p] = a.enter[(((size_t)stream * a.nseg + seg) * a.N + n) * PW + p];
+  else if (act && a.init)
+    for (int p = 0; p < a.P; ++p) S[lane * SP + p] = ldf((const TIO*)a.init + ((size_t)stream * a.P + p) * a.N + n);
+  const TIO* __restrict__ Bp = (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + n;
+  const TIO* __restrict__ Cp = (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + n;
+  const int j0 = seg * a.seg_blk, j1 = min(a.nblk, j0 + a.seg_blk);
+  __syncthreads();
+  for (int j = j0; j < j1; ++j) {
+    const int row0 = j * R, rows = min(R, a.L - row0);
+    float raw[R];
+    load_dt(a, bi, h, n, act, row0, rows, raw);
+    for (int i = tid; i < R * a.P; i += nt) {
+      const int r = i / a.P, p = i - r * a.P;
+      const float v = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.x_sl + h * a.x_sh + p);
+      xs[r * SP + p] = r < rows ? v : 0.f;
+    }
+    float acc = 0.f, mx = 0.f;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      raw[r] = (act && r < rows) ? dt_value(a, raw[r], bias) : 0.f;
+      acc = fmaf(raw[r], A2, acc);
+      mx = fmaxf(mx, fabsf(acc));
+    }
+    const float alast = acc;
+    const bool slow = __syncthreads_or(!(mx <= kRange));
+    const float ref = slow ? alast : 0.f;
+    acc = 0.f;
+#pragma unroll
+    for (int r0 = 0; r0 < R; r0 += 8) {
+      float cv[8], bv[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int64_t mr = brow(a, row0 + min(r0 + q, rows - 1));
+        cv[q] = act ? ldf(Cp + mr * a.C_sl) : 0.f;
+        bv[q] = act ? ldf(Bp + mr * a.B_sl) : 0.f;
+      }
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        acc = fmaf(raw[r0 + q], A2, acc);
+        cv[q] *= exp2f(acc);
+        bv[q] *= raw[r0 + q] * exp2f(ref - acc);
+        if (r0 + q >= rows) { cv[q] = 0.f; bv[q] = 0.f; }
+      }
+      st4(Cd + lane * LDT + r0, cv[0], cv[1], cv[2], cv[3]);
+      st4(Cd + lane * LDT + r0 + 4, cv[4], cv[5], cv[6], cv[7]);
+      st4(Bd + lane * LDT + r0, bv[0], bv[1], bv[2], bv[3]);
+      st4(Bd + lane * LDT + r0 + 4, bv[4], bv[5], bv[6], bv[7]);
+    }
+    __syncwarp();
+    {
+      float2 m[8][2], y[8][2], y4[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m[i][0] = m[i][1] = y[i][0] = y[i][1] = dup(0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+      gemm_y<PC, true>(Cd, Bd, S, SP, lg, cg, m, y, y4);
+      if (!slow) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st4(red + (lg * 8 + i) * RW + cg * 4, m[i][0].x, m[i][0].y, m[i][1].x, m[i][1].y);
+      }
+      store_y<PC>(red, RW, R, lg, cg, y, y4);
+      for (int c = 1; c < a.nch; ++c) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i][0] = y[i][1] = dup(0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+        gemm_y<PC, false>(Cd, Bd, S + c * W, SP, lg, cg, m, y, y4);
+        store_y<PC>(red, RW, R + c * W, lg, cg, y, y4);
+      }
+    }
+    if (slow) slow_M<TIO>(a, bi, h, n, act, row0, rows, A2, bias, red, RW, false);
+    const float el = exp2f(alast);
+    __syncwarp();
+    for (int c = 0; c < a.nch; ++c) update_state<PC>(S + c * W, SP, Bd, xs + c * W, lg, cg, slow ? el : 1.f, slow ? 1.f : el);
+    __syncthreads();
+    reduce_M(red0, wstride, a.nw, RW, Ms, false);
+    __syncthreads();
+    for (int it = 0; it < 4 / a.nw; ++it) {
+      const int l0 = (warp * (4 / a.nw) + it) * 8 + lg;
+      for (int c = 0; c < a.nch; ++c) {
+        float y[2][PC];
+        final_rows<PC>(red0, wstride, a.nw, RW, R + c * W, Ms, xs + c * W, SP, l0, cg, y);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int l = l0 + 4 * u;
+          if (l >= rows) continue;
+          const int mr = brow(a, row0 + l);
+          float* part = a.part ? a.part + ((((size_t)blockIdx.y * a.b + bi) * a.L + mr) * a.H + h) * a.P : nullptr;
+          const int p0 = c * W + cg * 4;
+          if (part && a.vec4 && p0 < a.P) {
+            st4(part + p0, y[u][0], y[u][1], y[u][2], y[u][3]);
+          } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+              if (p0 + q < a.P) {
+                if (part) part[p0 + q] = y[u][q];
+                else finish_out<TIO>(a, bi, h, mr, p0 + q, y[u][q], xs[l * SP + p0 + q]);
+              }
+          }
+          const int p4 = c * W + 32 + cg;
+          if (PC == 5 && p4 < a.P) {
+            if (part) part[p4] = y[u][4];
+            else finish_out<TIO>(a, bi, h, mr, p4, y[u][PC - 1], xs[l * SP + p4]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+  if (a.want_final && a.final_states && act && j1 == a.nblk && !a.enter)
+    for (int p = 0; p < a.P; ++p) a.final_states[((size_t)stream * a.P + p) * a.N + n] = S[lane * SP + p];
+}
+
+// out = (sum of the slices' partial rows + D x) * silu(z); one thread per element
+template <typename TIO>
+__global__ void k_blk_combine_out(const __grid_constant__ BArgs a, size_t total) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  float y = 0.f;
+  for (int s = 0; s < a.nslice; ++s) y += a.part[s * total + i];
+  const int p = (int)(i % a.P), h = (int)(i / a.P % a.H), mr = (int)(i / ((size_t)a.P * a.H) % a.L), bi = (int)(i / ((size_t)a.P * a.H * a.L));
+  finish_out<TIO>(a, bi, h, mr, p, y, ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh + p));
+}
+
+// ---- backward --------------------------------------------------------------------------------------------------------
+// Blocks in reverse scan order, G[n,p] = dLoss/dS carried in shared memory (g' = 2^a_last G):
+//   dM = tril(dy x^T);  [M^T | dx] = Bd^T [Cd | g'], dx += M^T dy;  CD = Bd dM^T + S dy^T;  BD = Cd dM + g' x^T;
+//   G <- g' + Cd dy;  then per (row, state), lane = state:
+//   dC_h = 2^a CD, dB_h = dt 2^-a BD, dacs = C dC_h - B dt (2^-a BD), ddA[l] = sum_{t>=l} dacs + <S_next, G>,
+//   ddt = (ddA A + B 2^-a BD) * sigmoid(pre) where dt is not clamped, dA += ddA dt, ddt_bias += ddt.
+template <int PC, typename TIO>
+__global__ void __launch_bounds__(128) k_blk_bwd(const __grid_constant__ BArgs a) {
+  constexpr int W = 8 * PC;
+  extern __shared__ float4 sm4[];
+  float* sm = (float*)sm4;
+  const int SP = a.SP, PW = a.nch * W, RW = R + PW;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lg = lane >> 3, cg = lane & 7, nt = blockDim.x;
+  float* dys = sm;                                        // [32 rows][SP]
+  float* xT = dys + R * SP;                               // [PW][LDT]
+  float* dyT = xT + PW * LDT;                             // [PW][LDT]
+  float* dM = dyT + PW * LDT;                             // [l][s]
+  float* dMT = dM + R * LDT;                              // [s][l]
+  float* Ms = dMT + R * LDT;                              // M^T [s][l]
+  const size_t wstride = 2 * R * LDT + 2 * R * SP + R * RW;
+  float* red0 = Ms + R * LDT;
+  float* red = red0 + warp * wstride;                     // partial [M^T | dx]
+  float* Cd = red + R * RW;
+  float* Bd = Cd + R * LDT;
+  float* S = Bd + R * LDT;
+  float* G = S + R * SP;
+  const int seg = blockIdx.z, stream = blockIdx.x, bi = stream / a.H, h = stream % a.H, g = h / a.hpg;
+  const int n = (blockIdx.y * a.nw + warp) * 32 + lane;
+  const bool act = n < a.N, first_slice = blockIdx.y == 0;
+  const float An = act ? a.A[h * a.N + n] : 0.f, A2 = An * kLog2e, bias = (act && a.bias) ? a.bias[h * a.N + n] : 0.f;
+  for (int i = tid; i < R * SP + 2 * PW * LDT; i += nt) dys[i] = 0.f;
+  for (int p = 0; p < SP; ++p) { G[lane * SP + p] = 0.f; S[lane * SP + p] = 0.f; }
+  const int j0 = seg * a.seg_blk, j1 = min(a.nblk, j0 + a.seg_blk);
+  if (act && a.enter)
+    for (int p = 0; p < a.P; ++p) G[lane * SP + p] = a.enter[(((size_t)stream * a.nseg + seg) * a.N + n) * PW + p];
+  else if (act && a.dfinal)
+    for (int p = 0; p < a.P; ++p) G[lane * SP + p] = a.dfinal[((size_t)stream * a.P + p) * a.N + n];
+  auto load_S = [&](int j) {
+    for (int i = lane; i < R * (PW / 4); i += 32) {
+      const int r = i / (PW / 4), c = i % (PW / 4), nn = n - lane + r;
+      if (nn < a.N) *(float4*)(S + r * SP + c * 4) = *(const float4*)(a.saved + (((size_t)stream * (a.nblk + 1) + j) * a.N + nn) * PW + c * 4);
+    }
+  };
+  load_S(j1);
+  const TIO* __restrict__ Bp = (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + n;
+  const TIO* __restrict__ Cp = (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + n;
+  float dAacc = 0.f, dbacc = 0.f, dDacc = 0.f;
+  for (int j = j1 - 1; j >= j0; --j) {
+    const int row0 = j * R, rows = min(R, a.L - row0);
+    __syncthreads();
+    float alast, cst = 0.f;
+    bool slow;
+    {
+      float raw[R];
+      load_dt(a, bi, h, n, act, row0, rows, raw);
+      for (int p = 0; p < PW; p += 4) {                   // <state leaving the block, gradient of it>
+        const float4 s = ld4(S + lane * SP + p), q = ld4(G + lane * SP + p);
+        cst = fmaf(s.x, q.x, fmaf(s.y, q.y, fmaf(s.z, q.z, fmaf(s.w, q.w, cst))));
+      }
+      for (int i = tid; i < R * a.P; i += nt) {
+        const int r = i / a.P, p = i - r * a.P, mr = brow(a, row0 + min(r, rows - 1));
+        float xv = 0.f, dv = 0.f;
+        if (r < rows) {
+          xv = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh + p);
+          dv = dy_value<TIO>(a, bi, h, mr, p, first_slice);
+        }
+        dys[r * SP + p] = dv;
+        dyT[p * LDT + r] = dv;
+        xT[p * LDT + r] = xv;
+      }
+      float acc = 0.f, mx = 0.f;
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        raw[r] = (act && r < rows) ? dt_value(a, raw[r], bias) : 0.f;
+        acc = fmaf(raw[r], A2, acc);
+        mx = fmaxf(mx, fabsf(acc));
+      }
+      alast = acc;
+      slow = __syncthreads_or(!(mx <= kRange));
+      load_S(j);
+      const float ref = slow ? alast : 0.f;
+      acc = 0.f;
+#pragma unroll
+      for (int r0 = 0; r0 < R; r0 += 8) {
+        float cv[8], bv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int64_t mr = brow(a, row0 + min(r0 + q, rows - 1));
+          cv[q] = act ? ldf(Cp + mr * a.C_sl) : 0.f;
+          bv[q] = act ? ldf(Bp + mr * a.B_sl) : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          acc = fmaf(raw[r0 + q], A2, acc);
+          cv[q] *= exp2f(acc);
+          bv[q] *= raw[r0 + q] * exp2f(ref - acc);
+          if (r0 + q >= rows) { cv[q] = 0.f; bv[q] = 0.f; }
+        }
+        st4(Cd + lane * LDT + r0, cv[0], cv[1], cv[2], cv[3]);
+        st4(Cd + lane * LDT + r0 + 4, cv[4], cv[5], cv[6], cv[7]);
+        st4(Bd + lane * LDT + r0, bv[0], bv[1], bv[2], bv[3]);
+        st4(Bd + lane * LDT + r0 + 4, bv[4], bv[5], bv[6], bv[7]);
+      }
+      const float el = slow ? 1.f : exp2f(alast);          // g' (a block out of range keeps G and has the decay in Bd)
+      for (int p = 0; p < PW; p += 4) {
+        const float4 q = ld4(G + lane * SP + p);
+        st4(G + lane * SP + p, q.x * el, q.y * el, q.z * el, q.w * el);
+      }
+    }
+    // dM[l][s], s <= l: this warp's 32 / nw rows, two per lane and pass
+    for (int it = 0; it < 4 / a.nw; ++it) {
+      const int l = ((warp * (4 / a.nw) + it) * 4 + lg) * 2, s = cg * 4;
+      float2 d0[2] = {dup(0.f), dup(0.f)}, d1[2] = {dup(0.f), dup(0.f)};
+#pragma unroll 4
+      for (int p = 0; p < a.P; ++p) {
+        const float2 dv = *(const float2*)(dyT + p * LDT + l);
+        const float4 xv = ld4(xT + p * LDT + s);
+        d0[0] = __ffma2_rn(dup(dv.x), make_float2(xv.x, xv.y), d0[0]); d0[1] = __ffma2_rn(dup(dv.x), make_float2(xv.z, xv.w), d0[1]);
+        d1[0] = __ffma2_rn(dup(dv.y), make_float2(xv.x, xv.y), d1[0]); d1[1] = __ffma2_rn(dup(dv.y), make_float2(xv.z, xv.w), d1[1]);
+      }
+      const float v0[4] = {d0[0].x, d0[0].y, d0[1].x, d0[1].y}, v1[4] = {d1[0].x, d1[0].y, d1[1].x, d1[1].y};
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float m0 = s + q <= l ? v0[q] : 0.f, m1 = s + q <= l + 1 ? v1[q] : 0.f;
+        dM[l * LDT + s + q] = m0;
+        dM[(l + 1) * LDT + s + q] = m1;
+        *(float2*)(dMT + (s + q) * LDT + l) = make_float2(m0, m1);
+        if (s + q == l) dDacc += m0;
+        if (s + q == l + 1) dDacc += m1;
+      }
+    }
+    if (a.has_D && a.D_has_hdim && first_slice)
+      for (int p = tid; p < a.P; p += nt) {
+        float acc = 0.f;
+        for (int r = 0; r < R; ++r) acc = fmaf(dyT[p * LDT + r], xT[p * LDT + r], acc);
+        float* o = a.dDpart + ((size_t)stream * a.nseg + seg) * a.P + p;
+        *o = j == j1 - 1 ? acc : *o + acc;
+      }
+    __syncthreads();
+    {
+      float2 m[8][2], y[8][2], y4[4];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m[i][0] = m[i][1] = y[i][0] = y[i][1] = dup(0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+      gemm_y<PC, true>(Bd, Cd, G, SP, lg, cg, m, y, y4);
+      if (!slow) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) st4(red + (lg * 8 + i) * RW + cg * 4, m[i][0].x, m[i][0].y, m[i][1].x, m[i][1].y);
+      }
+      store_y<PC>(red, RW, R, lg, cg, y, y4);
+      for (int c = 1; c < a.nch; ++c) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) y[i][0] = y[i][1] = dup(0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+        gemm_y<PC, false>(Bd, Cd, G + c * W, SP, lg, cg, m, y, y4);
+        store_y<PC>(red, RW, R + c * W, lg, cg, y, y4);
+      }
+    }
+    if (slow) slow_M<TIO>(a, bi, h, n, act, row0, rows, A2, bias, red, RW, true);
+    {
+      float2 cd[8][2], bd[8][2];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) cd[i][0] = cd[i][1] = bd[i][0] = bd[i][1] = dup(0.f);
+      if (!slow) {
+        gemm_n(Bd, LDT, dMT, LDT, R, lg, cg, cd);
+        gemm_n(Cd, LDT, dM, LDT, R, lg, cg, bd);
+      }
+      gemm_n(S, SP, dyT, LDT, PW, lg, cg, cd);
+      gemm_n(G, SP, xT, LDT, PW, lg, cg, bd);
+      __syncwarp();
+      const float pre = slow ? exp2f(alast) : 1.f;
+      for (int c = 0; c < a.nch; ++c) update_state<PC>(G + c * W, SP, Cd, dys + c * W, lg, cg, pre, 1.f);
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        st4(Cd + (lg + 4 * i) * LDT + cg * 4, cd[i][0].x, cd[i][0].y, cd[i][1].x, cd[i][1].y);
+        st4(Bd + (lg + 4 * i) * LDT + cg * 4, bd[i][0].x, bd[i][0].y, bd[i][1].x, bd[i][1].y);
+      }
+      __syncwarp();
+    }
+    if (slow) slow_grads<TIO>(a, bi, h, n, act, row0, rows, A2, bias, dM, Cd + lane * LDT, Bd + lane * LDT);
+    {                                                      // per (row, state)
+      float v[R], dac[R], gd[R], sg[R];
+      load_dt(a, bi, h, n, act, row0, rows, v);
+      float acc = 0.f;
+      const size_t hn = (size_t)a.H * a.N, gn = (size_t)a.G * a.N;
+#pragma unroll
+      for (int r0 = 0; r0 < R; r0 += 8) {
+        float cv[8], bv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int64_t mr = brow(a, row0 + min(r0 + q, rows - 1));
+          cv[q] = act ? ldf(Cp + mr * a.C_sl) : 0.f;
+          bv[q] = act ? ldf(Bp + mr * a.B_sl) : 0.f;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int r = r0 + q;
+          const bool in = act && r < rows;
+          const float pre = v[r] + bias;
+          const float tv = a.softplus ? softplus_thr(pre) : pre;
+          float s = (tv < a.dtmin || tv > a.dtmax) ? 0.f : 1.f;
+          if (a.softplus && pre <= 20.f) s *= sigmoidf_(pre);
+          v[r] = in ? fminf(fmaxf(tv, a.dtmin), a.dtmax) : 0.f;
+          acc = fmaf(v[r], A2, acc);
+          const float cdv = Cd[lane * LDT + r] * (slow ? 1.f : exp2f(acc)), bdv = Bd[lane * LDT + r] * (slow ? 1.f : exp2f(-acc));
+          const float dBv = v[r] * bdv;
+          dac[r] = in ? cv[q] * cdv - bv[q] * dBv : 0.f;
+          gd[r] = bv[q] * bdv;
+          sg[r] = in ? s : 0.f;
+          if (in) {
+            const size_t bl = (size_t)bi * a.L + brow(a, row0 + r);
+            if (a.hpg == 1) {
+              stf((TIO*)a.dB + bl * gn + (size_t)g * a.N + n, dBv);
+              stf((TIO*)a.dC + bl * gn + (size_t)g * a.N + n, cdv);
+            } else {
+              a.dBh[bl * hn + (size_t)h * a.N + n] = dBv;
+              a.dCh[bl * hn + (size_t)h * a.N + n] = cdv;
+            }
+          }
+        }
+      }
+      float run = cst;
+#pragma unroll
+      for (int r = R - 1; r >= 0; --r) {
+        run += dac[r];
+        dAacc = fmaf(run, v[r], dAacc);
+        const float o = sg[r] != 0.f ? fmaf(run, An, gd[r]) * sg[r] : 0.f;
+        dbacc += o;
+        if (act && r < rows) {
+          const size_t at = ((size_t)bi * a.L + brow(a, row0 + r)) * hn + (size_t)h * a.N + n;
+          if (a.dt_bf16) stf((bf16*)a.ddt + at, o);
+          else stf((float*)a.ddt + at, o);
+        }
+      }
+    }
+    __syncthreads();
+    reduce_M(red0, wstride, a.nw, RW, Ms, true);
+    __syncthreads();
+    for (int it = 0; it < 4 / a.nw; ++it) {
+      const int l0 = (warp * (4 / a.nw) + it) * 8 + lg;
+      for (int c = 0; c < a.nch; ++c) {
+        float y[2][PC];
+        final_rows<PC>(red0, wstride, a.nw, RW, R + c * W, Ms, dys + c * W, SP, l0, cg, y);
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          const int l = l0 + 4 * u;
+          if (l >= rows) continue;
+          const size_t row = (((size_t)bi * a.L + brow(a, row0 + l)) * a.H + h) * a.P;
+          float* part = a.part ? a.part + (size_t)blockIdx.y * a.b * a.L * a.H * a.P : nullptr;
+#pragma unroll
+          for (int q = 0; q < PC; ++q) {
+            const int p = c * W + (q < 4 ? cg * 4 + q : 32 + cg);
+            if (p >= a.P) continue;
+            float o = y[u][q];
+            if (a.has_D && first_slice) o = fmaf(a.D_has_hdim ? __ldg(a.D + h * a.P + p) : __ldg(a.D + h), dys[l * SP + p], o);
+            if (part) part[row + p] = o;
+            else stf((TIO*)a.dx + row + p, o);
+          }
+        }
+      }
+    }
+  }
+  const size_t sh = (size_t)stream * a.nseg + seg;
+  if (act) {
+    a.dApart[sh * a.N + n] = dAacc;
+    a.dbpart[sh * a.N + n] = dbacc;
+    if (a.dinit && j0 == 0 && !a.enter)
+      for (int p = 0; p < a.P; ++p) stf((TIO*)a.dinit + ((size_t)stream * a.P + p) * a.N + n, G[lane * SP + p]);
+  }
+  if (a.has_D && !a.D_has_hdim && first_slice) {          // scalar dD partial of this (stream, segment)
+    __syncthreads();
+    const float s = warp_sum(dDacc);
+    if (lane == 0) Ms[warp] = s;
+    __syncthreads();
+    if (tid == 0) {
+      float t = 0.f;
+      for (int w = 0; w < a.nw; ++w) t += Ms[w];
+      a.dDpart[sh] = t;
+    }
+  }
+}
+
+// dx = sum of the slices' partial rows (the skip term is in slice 0's)
+template <typename TIO>
+__global__ void k_blk_combine_dx(const float* __restrict__ part, int nslice, size_t total, TIO* __restrict__ dx) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  float y = 0.f;
+  for (int s = 0; s < nslice; ++s) y += part[s * total + i];
+  stf(dx + i, y);
+}
+// dB, dC (b, L, G, N) from the per-head rows, fixed order
+template <typename TIO>
+__global__ void k_blk_heads(const float* __restrict__ dBh, const float* __restrict__ dCh, int hpg, int N, size_t total, TIO* __restrict__ dB,
+                            TIO* __restrict__ dC) {
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= total) return;
+  const size_t at = (i / N) * hpg * N + i % N;
+  float sb = 0.f, sc = 0.f;
+  for (int k = 0; k < hpg; ++k) { sb += dBh[at + (size_t)k * N]; sc += dCh[at + (size_t)k * N]; }
+  stf(dB + i, sb);
+  stf(dC + i, sc);
+}
+// dA, ddt_bias (H, N) and dD (H, dw) from the (batch, head, segment) partials, fixed order
+__global__ void k_blk_params(const __grid_constant__ BArgs a, int dw, float* __restrict__ dA, float* __restrict__ db, float* __restrict__ dD) {
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int hn = a.H * a.N;
+  const float* part = a.dApart;
+  float* out = dA;
+  int width = a.N;
+  if (i >= hn) { i -= hn; part = a.dbpart; out = db; }
+  if (part == a.dbpart && i >= hn) { i -= hn; part = a.dDpart; out = dD; width = dw; if (i >= a.H * dw) return; }
+  if (!out) return;
+  const int h = i / width, c = i % width;
+  float acc = 0.f;
+  for (int bi = 0; bi < a.b; ++bi)
+    for (int s = 0; s < a.nseg; ++s) acc += part[(((size_t)bi * a.H + h) * a.nseg + s) * width + c];
+  out[i] = acc;
+}
+
+// ---- host side ---------------------------------------------------------------------------------------------------------
+constexpr size_t kSmemMax = 227 * 1024;
+struct Plan { int PC, nch, PW, SP, nw, nslice, nblk, nseg, seg_blk; size_t smem; };
+
+size_t blk_smem(const Plan& q, int pass) {
+  const size_t RW = R + q.PW;
+  if (pass == 0) return 4 * (size_t)(R * q.SP + R * LDT + q.nw * (2 * R * LDT + R * q.SP + R * RW));
+  return 4 * (size_t)(R * q.SP + 2 * q.PW * LDT + 3 * R * LDT + q.nw * (2 * R * LDT + 2 * R * q.SP + R * RW));
+}
+// false: the call stays on the per-pair kernels (head too wide for the tiles)
+bool blk_plan(const issm_params& p, int pass, Plan* out) {
+  Plan q{};
+  const int w4 = (p.headdim + 31) / 32 * 32, w5 = (p.headdim + 39) / 40 * 40;    // padded head width: the smaller one
+  q.PC = w5 <= w4 ? 5 : 4;
+  q.PW = w5 <= w4 ? w5 : w4;
+  q.nch = q.PW / (8 * q.PC);
+  q.SP = q.PW + 4;                                        // rows 4 or 12 banks apart
+  const int nw32 = (p.dstate + 31) / 32;
+  // warps per block: the widest of 4, 2, 1 that leaves at most one warp without states and fits
+  q.nw = 0;
+  for (int w = 4; w >= 1; w /= 2) {
+    const Plan t = [&] { Plan t = q; t.nw = w; return t; }();
+    if (blk_smem(t, pass) > kSmemMax) continue;
+    if (w > 1 && ((nw32 + w - 1) / w * w - nw32 > 1)) continue;
+    q.nw = w;
+    break;
+  }
+  if (!q.nw) return false;
+  q.smem = blk_smem(q, pass);
+  q.nslice = (nw32 + q.nw - 1) / q.nw;
+  q.nblk = (p.seqlen + R - 1) / R;
+  // segments only when the streams leave most of the chip idle: the extra states-only walk costs about half a pass.
+  // 148 SMs x 6 warps; a segment keeps at least 4 blocks
+  const long warps = (long)p.batch * p.nheads * q.nslice * q.nw;
+  long want = (148L * 6) / warps;
+  if (want > q.nblk / 4) want = q.nblk / 4;
+  if (want < 2) want = 1;
+  q.seg_blk = (q.nblk + (int)want - 1) / (int)want;
+  q.nseg = (q.nblk + q.seg_blk - 1) / q.seg_blk;
+  if (q.nseg > 65535) { q.nseg = 1; q.seg_blk = q.nblk; }
+  *out = q;
+  return true;
+}
+
+struct Ws { float *seg_out, *seg_sum, *part, *saved, *dBh, *dCh, *dApart, *dbpart, *dDpart; };
+Ws blk_carve(const issm_params& p, const Plan& q, int pass, size_t* total) {
+  Carver c(p.workspace);
+  Ws w{};
+  const size_t bh = (size_t)p.batch * p.nheads, N = p.dstate, L = p.seqlen;
+  if (q.nseg > 1) {
+    w.seg_out = c.take<float>(bh * q.nseg * N * q.PW);
+    w.seg_sum = c.take<float>(bh * q.nseg * N);
+  }
+  if (q.nslice > 1) w.part = c.take<float>((size_t)q.nslice * bh * L * p.headdim);
+  if (pass == 1) {
+    w.saved = c.take<float>(bh * (q.nblk + 1) * N * q.PW);
+    if (p.nheads > p.ngroups) { w.dBh = c.take<float>(bh * L * N); w.dCh = c.take<float>(bh * L * N); }
+    w.dApart = c.take<float>(bh * q.nseg * N);
+    w.dbpart = c.take<float>(bh * q.nseg * N);
+    w.dDpart = c.take<float>(bh * q.nseg * p.headdim);
+  }
+  *total = c.off;
+  return w;
+}
+
+BArgs blk_args(const issm_params& p, const Plan& q) {
+  BArgs a{};
+  a.b = p.batch; a.L = p.seqlen; a.H = p.nheads; a.P = p.headdim; a.N = p.dstate; a.G = p.ngroups; a.hpg = p.nheads / p.ngroups;
+  a.rev = p.reverse; a.softplus = p.dt_softplus; a.dt_bf16 = p.dt_dtype == ISSM_BF16; a.has_D = p.has_D; a.D_has_hdim = p.D_has_hdim;
+  a.want_final = p.want_final; a.vec4 = p.headdim % 4 == 0;
+  a.nblk = q.nblk; a.nseg = q.nseg; a.seg_blk = q.seg_blk; a.nslice = q.nslice; a.nw = q.nw; a.nch = q.nch; a.SP = q.SP;
+  a.dtmin = p.dt_min; a.dtmax = p.dt_max;
+  a.x = p.x; a.x_sb = p.x_sb; a.x_sl = p.x_sl; a.x_sh = p.x_sh;
+  a.B = p.B; a.B_sb = p.B_sb; a.B_sl = p.B_sl; a.B_sg = p.B_sg;
+  a.C = p.C; a.C_sb = p.C_sb; a.C_sl = p.C_sl; a.C_sg = p.C_sg;
+  if (p.has_z) { a.z = p.z; a.z_sb = p.z_sb; a.z_sl = p.z_sl; a.z_sh = p.z_sh; }
+  a.dt = p.dt; a.dt_sb = p.dt_sb; a.dt_sl = p.dt_sl; a.dt_sh = p.dt_sh;
+  a.A = p.A; a.bias = p.has_dt_bias ? p.dt_bias : nullptr; a.D = p.has_D ? p.D : nullptr;
+  a.init = p.has_init ? p.initial_states : nullptr;
+  a.o_sb = p.out_sb; a.o_sl = p.out_sl; a.o_sh = p.out_sh;
+  return a;
+}
+
+template <int PC, typename TIO>
+int launch_states(const BArgs& a, bool bwd, cudaStream_t s) {
+  const size_t smem = 4 * (size_t)(R * a.SP + a.nw * (R * LDT + R * a.SP));
+  struct F {}; struct B {};
+  if (SmemAttrOnce<F>::set(k_blk_states<PC, TIO, false>, kSmemMax) != ISSM_OK || SmemAttrOnce<B>::set(k_blk_states<PC, TIO, true>, kSmemMax) != ISSM_OK)
+    return ISSM_ERR_CUDA;
+  const dim3 grid(a.b * a.H, a.nslice, a.nseg);
+  if (bwd) ISSM_LAUNCH((k_blk_states<PC, TIO, true>), grid, a.nw * 32, smem, s, a);
+  else ISSM_LAUNCH((k_blk_states<PC, TIO, false>), grid, a.nw * 32, smem, s, a);
+  return ISSM_OK;
+}
+template <typename TIO>
+int launch_chain(const BArgs& a, int PW, int reverse, float* fin, TIO* fin_io, cudaStream_t s) {
+  const size_t n = (size_t)a.b * a.H * a.N * PW;
+  ISSM_LAUNCH((k_blk_chain<TIO>), (unsigned)cdiv64(n, 256), 256, 0, s, a, PW, reverse, fin, fin_io);
+  return ISSM_OK;
+}
+
+template <int PC, typename TIO>
+int run_fwd(const issm_params& p, const Plan& q, cudaStream_t s) {
+  size_t total = 0;
+  const Ws w = blk_carve(p, q, 0, &total);
+  BArgs a = blk_args(p, q);
+  a.out = p.out; a.out_x = p.out_x; a.final_states = p.final_states; a.part = w.part;
+  int rc;
+  if (q.nseg > 1) {
+    a.seg_out = w.seg_out; a.seg_sum = w.seg_sum;
+    if ((rc = launch_states<PC, TIO>(a, false, s)) != 0) return rc;
+    if ((rc = launch_chain<TIO>(a, q.PW, 0, p.want_final ? p.final_states : nullptr, (TIO*)nullptr, s)) != 0) return rc;
+    a.enter = w.seg_out;
+  }
+  struct T {};
+  if (SmemAttrOnce<T>::set(k_blk_fwd<PC, TIO>, kSmemMax) != ISSM_OK) return ISSM_ERR_CUDA;
+  ISSM_LAUNCH((k_blk_fwd<PC, TIO>), dim3(a.b * a.H, q.nslice, q.nseg), q.nw * 32, q.smem, s, a);
+  if (w.part) {
+    const size_t n = (size_t)a.b * a.L * a.H * a.P;
+    ISSM_LAUNCH((k_blk_combine_out<TIO>), (unsigned)cdiv64(n, 256), 256, 0, s, a, n);
+  }
+  return ISSM_OK;
+}
+
+template <int PC, typename TIO>
+int run_bwd(const issm_params& p, const Plan& q, cudaStream_t s) {
+  size_t total = 0;
+  const Ws w = blk_carve(p, q, 1, &total);
+  BArgs a = blk_args(p, q);
+  a.dout = p.dout; a.g_sb = p.dout_sb; a.g_sl = p.dout_sl; a.g_sh = p.dout_sh;
+  a.y = p.out_x; a.dz = p.dz; a.dx = p.dx; a.ddt = p.ddt; a.dB = p.dB; a.dC = p.dC; a.dBh = w.dBh; a.dCh = w.dCh;
+  a.dApart = w.dApart; a.dbpart = w.dbpart; a.dDpart = w.dDpart;
+  int rc;
+  // states entering every block
+  if (q.nseg > 1) {
+    BArgs f = a;
+    f.seg_out = w.seg_out; f.seg_sum = w.seg_sum;
+    if ((rc = launch_states<PC, TIO>(f, false, s)) != 0) return rc;
+    if ((rc = launch_chain<TIO>(f, q.PW, 0, nullptr, (TIO*)nullptr, s)) != 0) return rc;
+    f.enter = w.seg_out; f.seg_out = nullptr; f.saved = w.saved;
+    if ((rc = launch_states<PC, TIO>(f, false, s)) != 0) return rc;
+  } else {
+    BArgs f = a;
+    f.saved = w.saved;
+    if ((rc = launch_states<PC, TIO>(f, false, s)) != 0) return rc;
+  }
+  a.dfinal = p.has_dfinal ? p.dfinal_states : nullptr;
+  a.dinit = p.has_init ? p.dinitial_states : nullptr;
+  if (q.nseg > 1) {
+    BArgs f = a;
+    f.seg_out = w.seg_out; f.seg_sum = w.seg_sum;
+    if ((rc = launch_states<PC, TIO>(f, true, s)) != 0) return rc;
+    if ((rc = launch_chain<TIO>(f, q.PW, 1, nullptr, (TIO*)a.dinit, s)) != 0) return rc;
+    a.enter = w.seg_out;
+  }
+  a.saved = w.saved;
+  a.part = w.part;
+  struct T {};
+  if (SmemAttrOnce<T>::set(k_blk_bwd<PC, TIO>, kSmemMax) != ISSM_OK) return ISSM_ERR_CUDA;
+  ISSM_LAUNCH((k_blk_bwd<PC, TIO>), dim3(a.b * a.H, q.nslice, q.nseg), q.nw * 32, q.smem, s, a);
+  const size_t n = (size_t)a.b * a.L * a.H * a.P;
+  if (w.part) ISSM_LAUNCH((k_blk_combine_dx<TIO>), (unsigned)cdiv64(n, 256), 256, 0, s, w.part, q.nslice, n, (TIO*)p.dx);
+  if (a.hpg > 1) {
+    const size_t t = (size_t)a.b * a.L * a.G * a.N;
+    ISSM_LAUNCH((k_blk_heads<TIO>), (unsigned)cdiv64(t, 256), 256, 0, s, w.dBh, w.dCh, a.hpg, a.N, t, (TIO*)p.dB, (TIO*)p.dC);
+  }
+  const int dw = p.D_has_hdim ? p.headdim : 1, cells = 2 * a.H * a.N + a.H * dw;
+  ISSM_LAUNCH(k_blk_params, (cells + 127) / 128, 128, 0, s, a, dw, p.dA, p.has_dt_bias ? p.ddt_bias : nullptr, p.has_D ? p.dD : nullptr);
+  return ISSM_OK;
+}
+}  // namespace
+
+size_t blocked_workspace_bytes(const issm_params& p, int pass) {
+  Plan q;
+  if (!blk_plan(p, pass, &q)) return 0;
+  issm_params z = p;
+  z.workspace = nullptr;
+  size_t total = 0;
+  blk_carve(z, q, pass, &total);
+  return total;
+}
+bool blocked_supported(const issm_params& p, int pass) {
+  Plan q;
+  return blk_plan(p, pass, &q);
+}
+int blocked_run(const issm_params& p, int pass, cudaStream_t s) {
+  Plan q;
+  if (!blk_plan(p, pass, &q)) return ISSM_ERR_UNSUPPORTED;
+  const bool f32 = p.io_dtype == ISSM_F32;
+  if (pass == 0) {
+    if (q.PC == 5) return f32 ? run_fwd<5, float>(p, q, s) : run_fwd<5, bf16>(p, q, s);
+    return f32 ? run_fwd<4, float>(p, q, s) : run_fwd<4, bf16>(p, q, s);
+  }
+  if (q.PC == 5) return f32 ? run_bwd<5, float>(p, q, s) : run_bwd<5, bf16>(p, q, s);
+  return f32 ? run_bwd<4, float>(p, q, s) : run_bwd<4, bf16>(p, q, s);
+}
+
+}  // namespace issm

@@ -98,6 +98,11 @@ size_t simt_workspace_bytes(const issm_params& p, int pass);
 int simt_fwd(const issm_params& p, cudaStream_t s);
 int simt_bwd(const issm_params& p, cudaStream_t s);
 
+// the blocked fp32 kernels (issm_blocked.cu): what simt_* run wherever the shape fits their tiles
+bool blocked_supported(const issm_params& p, int pass);
+size_t blocked_workspace_bytes(const issm_params& p, int pass);
+int blocked_run(const issm_params& p, int pass, cudaStream_t s);
+
 bool tensor_path_supported(const issm_params& p, int pass);
 size_t tensor_workspace_bytes(const issm_params& p, int pass);
 int tensor_fwd(const issm_params& p, cudaStream_t s);

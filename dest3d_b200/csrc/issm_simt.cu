@@ -70,6 +70,7 @@ static SimtWs simt_carve(const issm_params& p, const SimtLayout& l, int pass, si
 }
 
 size_t simt_workspace_bytes(const issm_params& p, int pass) {
+  if (blocked_supported(p, pass)) return blocked_workspace_bytes(p, pass);
   issm_params q = p;
   q.workspace = nullptr;
   size_t total = 0;
@@ -671,7 +672,15 @@ static int simt_bwd_t(const issm_params& p, cudaStream_t s) {
   if (p.io_dtype == ISSM_F32 && p.dt_dtype == ISSM_BF16) return fn<float, bf16>(p, s); \
   return ISSM_ERR_DTYPE;
 
-int simt_fwd(const issm_params& p, cudaStream_t s) { ISSM_DISPATCH(simt_fwd_t) }
-int simt_bwd(const issm_params& p, cudaStream_t s) { ISSM_DISPATCH(simt_bwd_t) }
+// The blocked kernels wherever their tiles fit (every head width up to 128, or what shared memory holds beyond): a row
+// pair there costs a multiply-add instead of an exponential.  The per-pair kernels below serve wider heads only.
+int simt_fwd(const issm_params& p, cudaStream_t s) {
+  if (blocked_supported(p, 0)) return blocked_run(p, 0, s);
+  ISSM_DISPATCH(simt_fwd_t)
+}
+int simt_bwd(const issm_params& p, cudaStream_t s) {
+  if (blocked_supported(p, 1)) return blocked_run(p, 1, s);
+  ISSM_DISPATCH(simt_bwd_t)
+}
 
 }  // namespace issm

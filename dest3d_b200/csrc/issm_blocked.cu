@@ -53,30 +53,122 @@ struct BArgs {
   float* dDpart;          // (b*H*nseg) or (b*H*nseg, P)
 };
 
+// shared memory of one warp in floats (pass 0 forward, 1 backward): two operand tiles, the state tile(s), the partial rows
+// of the column chunks past the first, and (backward) `a` at the quarters of a block
+__host__ __device__ __forceinline__ int blk_warp_floats(int pass, int PC, int nch, int SP) {
+  return 2 * R * LDT + (1 + pass) * R * SP + (nch - 1) * R * 8 * PC + pass * 4 * 32;
+}
 __device__ __forceinline__ int brow(const BArgs& a, int t) { return a.rev ? a.L - 1 - t : t; }
 __device__ __forceinline__ float2 dup(float v) { return make_float2(v, v); }
 __device__ __forceinline__ float4 ld4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ void st4(float* p, float a, float b, float c, float d) { *(float4*)p = make_float4(a, b, c, d); }
 __device__ __forceinline__ float f4get(const float4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
 
-// dt of one row as the scan uses it: bias, softplus (reference threshold), clamp
+__device__ __forceinline__ float ex2(float v) {
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+// softplus as max(v, 0) + log1p(t), t = e^-|v|, with log1p(t) = 2 artanh(t / (2 + t)) summed to the 13th power (the next
+// term is 1.4e-8 of the sum at t = 1); branch-free, and above the reference's threshold of 20 it equals v in float.
+// Also gives the sigmoid.  1 + t inside a logarithm would lose the small dt.
+__device__ __forceinline__ float softplus_sig(float v, float& sig) {
+  const float t = expf(-fabsf(v));
+  const float s = __fdividef(t, 2.f + t), z = s * s;
+  float q = fmaf(z, 1.f / 13.f, 1.f / 11.f);
+  q = fmaf(q, z, 1.f / 9.f);
+  q = fmaf(q, z, 1.f / 7.f);
+  q = fmaf(q, z, 1.f / 5.f);
+  q = fmaf(q, z, 1.f / 3.f);
+  q = fmaf(q, z, 1.f);
+  sig = __fdividef(v >= 0.f ? 1.f : t, 1.f + t);
+  return fmaf(2.f * s, q, fmaxf(v, 0.f));
+}
+// dt of one row as the scan uses it: bias, softplus, clamp
 __device__ __forceinline__ float dt_value(const BArgs& a, float raw, float bias) {
-  float v = raw + bias;
-  if (a.softplus) v = softplus_thr(v);
+  float v = raw + bias, sg;
+  if (a.softplus) v = softplus_sig(v, sg);
   return fminf(fmaxf(v, a.dtmin), a.dtmax);
 }
 
-// this lane's state column of the 32 rows of a block: raw dt (all loads in flight together)
-__device__ __forceinline__ void load_dt(const BArgs& a, int bi, int h, int n, bool act, int row0, int rows, float* raw) {
-  const int64_t base = bi * a.dt_sb + h * a.dt_sh + n;
-  if (a.dt_bf16) {
-    const bf16* __restrict__ p = (const bf16*)a.dt + base;
+// one state column of a block: rows r0 .. r0 + 7 (rows past the end repeat the last one), all loads in flight together
+template <typename T>
+__device__ __forceinline__ void load8(const T* __restrict__ p, int64_t step, int r0, int last, float (&v)[8]) {
 #pragma unroll
-    for (int r = 0; r < R; ++r) raw[r] = act ? ldf(p + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.dt_sl) : 0.f;
-  } else {
-    const float* __restrict__ p = (const float*)a.dt + base;
+  for (int q = 0; q < 8; ++q) v[q] = ldf(p + min(r0 + q, last) * step);
+}
+__device__ __forceinline__ void load8_dt(const BArgs& a, const char* p, int r0, int last, float (&v)[8]) {
+  const int64_t step = a.rev ? -a.dt_sl : a.dt_sl;
+  if (a.dt_bf16) load8((const bf16*)p, step, r0, last, v);
+  else load8((const float*)p, step, r0, last, v);
+}
+__device__ __forceinline__ const char* dt_ptr(const BArgs& a, int bi, int h, int n, int row0) {
+  return (const char*)a.dt + (bi * a.dt_sb + h * a.dt_sh + n + (int64_t)brow(a, row0) * a.dt_sl) * (a.dt_bf16 ? 2 : 4);
+}
+// announce one row (this lane's) of a tile of the next block to L2
+__device__ __forceinline__ void l2_row(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+__device__ __forceinline__ void announce(const BArgs& a, int bi, int h, int g, int n0, int lane, int row0, int esize) {
+  const int t = row0 + lane;
+  if (row0 < 0 || t >= a.L || n0 >= a.N) return;
+  const int64_t mr = brow(a, t);
+  l2_row((const char*)a.dt + (bi * a.dt_sb + mr * a.dt_sl + h * a.dt_sh + n0) * (a.dt_bf16 ? 2 : 4));
+  l2_row((const char*)a.B + (bi * a.B_sb + mr * a.B_sl + g * a.B_sg + n0) * esize);
+  l2_row((const char*)a.C + (bi * a.C_sb + mr * a.C_sl + g * a.C_sg + n0) * esize);
+}
+// dt of the block into this lane's row of an operand tile (it waits there for the operand pass); the summed a, its
+// largest magnitude, and a before rows 8, 16, 24 (cuts[1..3][lane]) come back
+__device__ __forceinline__ float dt_pass(const BArgs& a, const char* p, float bias, float A2, bool act, int rows, float* tile_row, float& mx,
+                                         float* cuts) {
+  float raw[8], nxt[8], acc = 0.f;
+  mx = 0.f;
+  load8_dt(a, p, 0, rows - 1, raw);
+#pragma unroll 1
+  for (int r0 = 0; r0 < R; r0 += 8) {
+    if (cuts) cuts[(r0 >> 3) * 32] = acc;
+    if (r0 + 8 < R) load8_dt(a, p, r0 + 8, rows - 1, nxt);
 #pragma unroll
-    for (int r = 0; r < R; ++r) raw[r] = act ? ldf(p + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.dt_sl) : 0.f;
+    for (int q = 0; q < 8; ++q) {
+      raw[q] = (act && r0 + q < rows) ? dt_value(a, raw[q], bias) : 0.f;
+      acc = fmaf(raw[q], A2, acc);
+      mx = fmaxf(mx, fabsf(acc));
+    }
+    st4(tile_row + r0, raw[0], raw[1], raw[2], raw[3]);
+    st4(tile_row + r0 + 4, raw[4], raw[5], raw[6], raw[7]);
+#pragma unroll
+    for (int q = 0; q < 8; ++q) raw[q] = nxt[q];
+  }
+  if (!(acc == acc)) mx = acc;                            // a NaN must not pass the range vote
+  return acc;
+}
+// this lane's row of Cd = C 2^a and Bd = B dt 2^(ref - a); dt waits in Cd's row
+template <typename T>
+__device__ __forceinline__ void operand_pass(const T* __restrict__ Cp, int64_t cstep, const T* __restrict__ Bp, int64_t bstep, float A2, bool act,
+                                             int rows, float ref, float* cd_row, float* bd_row) {
+  float acc = 0.f, cn[8], bn[8];
+  load8(Cp, cstep, 0, rows - 1, cn);
+  load8(Bp, bstep, 0, rows - 1, bn);
+#pragma unroll 1
+  for (int r0 = 0; r0 < R; r0 += 8) {
+    float cv[8], bv[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) { cv[q] = cn[q]; bv[q] = bn[q]; }
+    if (r0 + 8 < R) {
+      load8(Cp, cstep, r0 + 8, rows - 1, cn);
+      load8(Bp, bstep, r0 + 8, rows - 1, bn);
+    }
+    const float4 v0 = ld4(cd_row + r0), v1 = ld4(cd_row + r0 + 4);
+    const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      acc = fmaf(v[q], A2, acc);
+      cv[q] *= ex2(acc);
+      bv[q] *= v[q] * ex2(ref - acc);                     // rows past the end have dt = 0
+      if (!act || r0 + q >= rows) { cv[q] = 0.f; bv[q] = 0.f; }
+    }
+    st4(cd_row + r0, cv[0], cv[1], cv[2], cv[3]);
+    st4(cd_row + r0 + 4, cv[4], cv[5], cv[6], cv[7]);
+    st4(bd_row + r0, bv[0], bv[1], bv[2], bv[3]);
+    st4(bd_row + r0 + 4, bv[4], bv[5], bv[6], bv[7]);
   }
 }
 
@@ -175,12 +267,14 @@ struct Lane { float v[R], a[R], c[R], b[R]; };
 template <typename TIO>
 __device__ __noinline__ void slow_lane(const BArgs& p, int bi, int h, int n, bool act, int row0, int rows, float A2, float bias, Lane<TIO>& s) {
   const int g = h / p.hpg;
-  load_dt(p, bi, h, n, act, row0, rows, s.v);
+  const char* dp = dt_ptr(p, bi, h, n, row0);
+  const int64_t step = p.rev ? -p.dt_sl : p.dt_sl;
   float acc = 0.f;
   for (int r = 0; r < R; ++r) {
     const bool in = act && r < rows;
     const int mr = brow(p, row0 + min(r, rows - 1));
-    s.v[r] = in ? dt_value(p, s.v[r], bias) : 0.f;
+    const int64_t o = min(r, rows - 1) * step;
+    s.v[r] = in ? dt_value(p, p.dt_bf16 ? ldf((const bf16*)dp + o) : ((const float*)dp)[o], bias) : 0.f;
     acc = fmaf(s.v[r], A2, acc);
     s.a[r] = acc;
     s.c[r] = in ? ldf((const TIO*)p.C + bi * p.C_sb + (int64_t)mr * p.C_sl + g * p.C_sg + n) : 0.f;
@@ -237,7 +331,7 @@ __device__ __forceinline__ float dy_value(const BArgs& a, int bi, int h, int mr,
 // (when asked for); kBwd = true: G <- 2^a_last G + sum_l C 2^a_l dy_l against the scan order.  Local end states and the
 // summed decay of every segment go to seg_out / seg_sum.  Exponents are non-positive: no range rule.
 template <int PC, typename TIO, bool kBwd>
-__global__ void __launch_bounds__(128) k_blk_states(const __grid_constant__ BArgs a) {
+__global__ void __launch_bounds__(128, 3) k_blk_states(const __grid_constant__ BArgs a) {
   constexpr int W = 8 * PC;
   extern __shared__ float4 sm4[];
   float* sm = (float*)sm4;
@@ -247,7 +341,7 @@ __global__ void __launch_bounds__(128) k_blk_states(const __grid_constant__ BArg
   float* Op = sm + R * SP + warp * (R * LDT + R * SP);    // [n][row]
   float* T = Op + R * LDT;                                // [n][SP]
   const int seg = blockIdx.z, stream = blockIdx.x, bi = stream / a.H, h = stream % a.H, g = h / a.hpg;
-  const int n = (blockIdx.y * a.nw + warp) * 32 + lane;
+  const int n = (blockIdx.y * a.nw + warp) * 32 + lane, nl = min(n, a.N - 1);
   const bool act = n < a.N;
   const float A2 = act ? a.A[h * a.N + n] * kLog2e : 0.f, bias = (act && a.bias) ? a.bias[h * a.N + n] : 0.f;
   for (int i = tid; i < R * SP; i += nt) src[i] = 0.f;
@@ -257,6 +351,7 @@ __global__ void __launch_bounds__(128) k_blk_states(const __grid_constant__ BArg
   if (!kBwd && act && a.enter)
     for (int p = 0; p < a.P; ++p) T[lane * SP + p] = a.enter[(((size_t)stream * a.nseg + seg) * a.N + n) * PW + p];
   const int j0 = seg * a.seg_blk, j1 = min(a.nblk, j0 + a.seg_blk);
+  const int64_t bsl = (a.rev ? -1 : 1) * (kBwd ? a.C_sl : a.B_sl);
   float asum = 0.f;
   auto keep = [&](int j) {                                // the tile to saved[j], 16 bytes per lane
     for (int i = lane; i < R * (PW / 4); i += 32) {
@@ -267,44 +362,44 @@ __global__ void __launch_bounds__(128) k_blk_states(const __grid_constant__ BArg
   for (int jj = j0; jj < j1; ++jj) {
     const int j = kBwd ? j1 - 1 - (jj - j0) : jj;
     const int row0 = j * R, rows = min(R, a.L - row0);
-    float raw[R];
-    load_dt(a, bi, h, n, act, row0, rows, raw);
+    announce(a, bi, h, g, n - lane, lane, kBwd ? row0 - R : row0 + R, sizeof(TIO));
     __syncthreads();
-    for (int i = tid; i < R * a.P; i += nt) {
-      const int r = i / a.P, p = i - r * a.P, mr = brow(a, row0 + min(r, rows - 1));
-      float v;
-      if (kBwd) v = dy_value<TIO>(a, bi, h, mr, p, false);
-      else v = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh + p);
-      src[r * SP + p] = r < rows ? v : 0.f;
+    for (int r = warp; r < R; r += a.nw) {
+      const int mr = brow(a, row0 + min(r, rows - 1));
+      for (int p = lane; p < a.P; p += 32) {
+        float v;
+        if (kBwd) v = dy_value<TIO>(a, bi, h, mr, p, false);
+        else v = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh + p);
+        src[r * SP + p] = r < rows ? v : 0.f;
+      }
     }
-    float acc = 0.f;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      raw[r] = (act && r < rows) ? dt_value(a, raw[r], bias) : 0.f;
-      acc = fmaf(raw[r], A2, acc);
-    }
-    const float alast = acc;
+    float mx;
+    const float alast = dt_pass(a, dt_ptr(a, bi, h, nl, row0), bias, A2, act, rows, Op + lane * LDT, mx, nullptr);
     asum += alast;
-    const TIO* __restrict__ bc = kBwd ? (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + n : (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + n;
-    const int64_t bsl = kBwd ? a.C_sl : a.B_sl;
-    acc = 0.f;
+    const TIO* bc = (kBwd ? (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + (int64_t)brow(a, row0) * a.C_sl
+                          : (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + (int64_t)brow(a, row0) * a.B_sl) + nl;
     if (!kBwd && a.saved) keep(j);
-#pragma unroll
+    float acc = 0.f, nx[8];
+    load8(bc, bsl, 0, rows - 1, nx);
+#pragma unroll 1
     for (int r0 = 0; r0 < R; r0 += 8) {
-      float cv[8], o[8];
+      float o[8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) cv[q] = act ? ldf(bc + (int64_t)brow(a, row0 + min(r0 + q, rows - 1)) * bsl) : 0.f;
+      for (int q = 0; q < 8; ++q) o[q] = nx[q];
+      if (r0 + 8 < R) load8(bc, bsl, r0 + 8, rows - 1, nx);
+      const float4 v0 = ld4(Op + lane * LDT + r0), v1 = ld4(Op + lane * LDT + r0 + 4);
+      const float v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        acc = fmaf(raw[r0 + q], A2, acc);
-        o[q] = kBwd ? cv[q] * exp2f(acc) : cv[q] * raw[r0 + q] * exp2f(alast - acc);
-        if (r0 + q >= rows) o[q] = 0.f;
+        acc = fmaf(v[q], A2, acc);
+        o[q] *= kBwd ? ex2(acc) : v[q] * ex2(alast - acc);
+        if (!act || r0 + q >= rows) o[q] = 0.f;
       }
       st4(Op + lane * LDT + r0, o[0], o[1], o[2], o[3]);
       st4(Op + lane * LDT + r0 + 4, o[4], o[5], o[6], o[7]);
     }
     __syncthreads();
-    const float el = exp2f(alast);
+    const float el = ex2(alast);
     for (int c = 0; c < a.nch; ++c) update_state<PC>(T + c * W, SP, Op, src + c * W, lg, cg, el, 1.f);
     __syncwarp();
   }
@@ -412,22 +507,24 @@ __device__ __forceinline__ void finish_out(const BArgs& a, int bi, int h, int mr
 
 // ---- forward ---------------------------------------------------------------------------------------------------------
 template <int PC, typename TIO>
-__global__ void __launch_bounds__(128) k_blk_fwd(const __grid_constant__ BArgs a) {
-  constexpr int W = 8 * PC;
+__global__ void __launch_bounds__(128, 3) k_blk_fwd(const __grid_constant__ BArgs a) {
+  constexpr int W = 8 * PC, RW = R + W;
   extern __shared__ float4 sm4[];
   float* sm = (float*)sm4;
-  const int SP = a.SP, PW = a.nch * W, RW = R + PW;
+  const int SP = a.SP, PW = a.nch * W;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lg = lane >> 3, cg = lane & 7, nt = blockDim.x;
   float* xs = sm;                                         // [32][SP]
   float* Ms = xs + R * SP;                                // [32][LDT]
-  const size_t wstride = 2 * R * LDT + R * SP + R * RW;
-  float* red0 = Ms + R * LDT;                             // per warp: partial [M | Y], Cd, Bd, S
-  float* red = red0 + warp * wstride;
-  float* Cd = red + R * RW;
+  // per warp: Cd and Bd [32][LDT] each, S [32][SP], partial Y of the column chunks past the first.  The partial [M | Y] of
+  // the first chunk (32 x (32 + W) <= both operand tiles) takes the operands' place once they have been read.
+  const size_t wstride = blk_warp_floats(0, PC, a.nch, SP);
+  float* red0 = Ms + R * LDT;
+  float* Cd = red0 + warp * wstride;
   float* Bd = Cd + R * LDT;
   float* S = Bd + R * LDT;
+  float* redx0 = red0 + 2 * R * LDT + R * SP;
   const int seg = blockIdx.z, stream = blockIdx.x, bi = stream / a.H, h = stream % a.H, g = h / a.hpg;
-  const int n = (blockIdx.y * a.nw + warp) * 32 + lane;
+  const int n = (blockIdx.y * a.nw + warp) * 32 + lane, nl = min(n, a.N - 1);
   const bool act = n < a.N;
   const float A2 = act ? a.A[h * a.N + n] * kLog2e : 0.f, bias = (act && a.bias) ? a.bias[h * a.N + n] : 0.f;
   for (int i = tid; i < R * SP; i += nt) xs[i] = 0.f;
@@ -436,77 +533,50 @@ __global__ void __launch_bounds__(128) k_blk_fwd(const __grid_constant__ BArgs a
     for (int p = 0; p < a.P; ++p) S[lane * SP + p] = a.enter[(((size_t)stream * a.nseg + seg) * a.N + n) * PW + p];
   else if (act && a.init)
     for (int p = 0; p < a.P; ++p) S[lane * SP + p] = ldf((const TIO*)a.init + ((size_t)stream * a.P + p) * a.N + n);
-  const TIO* __restrict__ Bp = (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + n;
-  const TIO* __restrict__ Cp = (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + n;
+  const int64_t csl = a.rev ? -a.C_sl : a.C_sl, bsl = a.rev ? -a.B_sl : a.B_sl;
   const int j0 = seg * a.seg_blk, j1 = min(a.nblk, j0 + a.seg_blk);
   __syncthreads();
   for (int j = j0; j < j1; ++j) {
     const int row0 = j * R, rows = min(R, a.L - row0);
-    float raw[R];
-    load_dt(a, bi, h, n, act, row0, rows, raw);
-    for (int i = tid; i < R * a.P; i += nt) {
-      const int r = i / a.P, p = i - r * a.P;
-      const float v = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.x_sl + h * a.x_sh + p);
-      xs[r * SP + p] = r < rows ? v : 0.f;
+    announce(a, bi, h, g, n - lane, lane, row0 + R, sizeof(TIO));
+    for (int r = warp; r < R; r += a.nw) {
+      const TIO* xp = (const TIO*)a.x + bi * a.x_sb + (int64_t)brow(a, row0 + min(r, rows - 1)) * a.x_sl + h * a.x_sh;
+      for (int p = lane; p < a.P; p += 32) xs[r * SP + p] = r < rows ? ldf(xp + p) : 0.f;
     }
-    float acc = 0.f, mx = 0.f;
-#pragma unroll
-    for (int r = 0; r < R; ++r) {
-      raw[r] = (act && r < rows) ? dt_value(a, raw[r], bias) : 0.f;
-      acc = fmaf(raw[r], A2, acc);
-      mx = fmaxf(mx, fabsf(acc));
-    }
-    const float alast = acc;
+    float mx;
+    const float alast = dt_pass(a, dt_ptr(a, bi, h, nl, row0), bias, A2, act, rows, Cd + lane * LDT, mx, nullptr);
     const bool slow = __syncthreads_or(!(mx <= kRange));
-    const float ref = slow ? alast : 0.f;
-    acc = 0.f;
-#pragma unroll
-    for (int r0 = 0; r0 < R; r0 += 8) {
-      float cv[8], bv[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const int64_t mr = brow(a, row0 + min(r0 + q, rows - 1));
-        cv[q] = act ? ldf(Cp + mr * a.C_sl) : 0.f;
-        bv[q] = act ? ldf(Bp + mr * a.B_sl) : 0.f;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        acc = fmaf(raw[r0 + q], A2, acc);
-        cv[q] *= exp2f(acc);
-        bv[q] *= raw[r0 + q] * exp2f(ref - acc);
-        if (r0 + q >= rows) { cv[q] = 0.f; bv[q] = 0.f; }
-      }
-      st4(Cd + lane * LDT + r0, cv[0], cv[1], cv[2], cv[3]);
-      st4(Cd + lane * LDT + r0 + 4, cv[4], cv[5], cv[6], cv[7]);
-      st4(Bd + lane * LDT + r0, bv[0], bv[1], bv[2], bv[3]);
-      st4(Bd + lane * LDT + r0 + 4, bv[4], bv[5], bv[6], bv[7]);
-    }
+    const int64_t m0 = brow(a, row0);
+    operand_pass((const TIO*)a.C + bi * a.C_sb + g * a.C_sg + m0 * a.C_sl + nl, csl, (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + m0 * a.B_sl + nl, bsl,
+                 A2, act, rows, slow ? alast : 0.f, Cd + lane * LDT, Bd + lane * LDT);
     __syncwarp();
     {
       float2 m[8][2], y[8][2], y4[4];
+      for (int c = a.nch - 1; c >= 0; --c) {              // the first chunk last: it stays in registers over the state update
 #pragma unroll
-      for (int i = 0; i < 8; ++i) m[i][0] = m[i][1] = y[i][0] = y[i][1] = dup(0.f);
+        for (int i = 0; i < 8; ++i) y[i][0] = y[i][1] = dup(0.f);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+        for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+        if (c) {
+          gemm_y<PC, false>(Cd, Bd, S + c * W, SP, lg, cg, m, y, y4);
+          store_y<PC>(redx0 + warp * wstride + (c - 1) * (R * W), W, 0, lg, cg, y, y4);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 8; ++i) m[i][0] = m[i][1] = dup(0.f);
       gemm_y<PC, true>(Cd, Bd, S, SP, lg, cg, m, y, y4);
+      const float el = ex2(alast);
+      __syncwarp();
+      for (int c = 0; c < a.nch; ++c) update_state<PC>(S + c * W, SP, Bd, xs + c * W, lg, cg, slow ? el : 1.f, slow ? 1.f : el);
+      __syncwarp();
+      float* red = Cd;
       if (!slow) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) st4(red + (lg * 8 + i) * RW + cg * 4, m[i][0].x, m[i][0].y, m[i][1].x, m[i][1].y);
       }
       store_y<PC>(red, RW, R, lg, cg, y, y4);
-      for (int c = 1; c < a.nch; ++c) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) y[i][0] = y[i][1] = dup(0.f);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
-        gemm_y<PC, false>(Cd, Bd, S + c * W, SP, lg, cg, m, y, y4);
-        store_y<PC>(red, RW, R + c * W, lg, cg, y, y4);
-      }
     }
-    if (slow) slow_M<TIO>(a, bi, h, n, act, row0, rows, A2, bias, red, RW, false);
-    const float el = exp2f(alast);
-    __syncwarp();
-    for (int c = 0; c < a.nch; ++c) update_state<PC>(S + c * W, SP, Bd, xs + c * W, lg, cg, slow ? el : 1.f, slow ? 1.f : el);
+    if (slow) slow_M<TIO>(a, bi, h, n, act, row0, rows, A2, bias, Cd, RW, false);
     __syncthreads();
     reduce_M(red0, wstride, a.nw, RW, Ms, false);
     __syncthreads();
@@ -514,7 +584,8 @@ __global__ void __launch_bounds__(128) k_blk_fwd(const __grid_constant__ BArgs a
       const int l0 = (warp * (4 / a.nw) + it) * 8 + lg;
       for (int c = 0; c < a.nch; ++c) {
         float y[2][PC];
-        final_rows<PC>(red0, wstride, a.nw, RW, R + c * W, Ms, xs + c * W, SP, l0, cg, y);
+        if (c == 0) final_rows<PC>(red0, wstride, a.nw, RW, R, Ms, xs, SP, l0, cg, y);
+        else final_rows<PC>(redx0 + (c - 1) * (R * W), wstride, a.nw, W, 0, Ms, xs + c * W, SP, l0, cg, y);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int l = l0 + 4 * u;
@@ -564,27 +635,30 @@ __global__ void k_blk_combine_out(const __grid_constant__ BArgs a, size_t total)
 //   dC_h = 2^a CD, dB_h = dt 2^-a BD, dacs = C dC_h - B dt (2^-a BD), ddA[l] = sum_{t>=l} dacs + <S_next, G>,
 //   ddt = (ddA A + B 2^-a BD) * sigmoid(pre) where dt is not clamped, dA += ddA dt, ddt_bias += ddt.
 template <int PC, typename TIO>
-__global__ void __launch_bounds__(128) k_blk_bwd(const __grid_constant__ BArgs a) {
-  constexpr int W = 8 * PC;
+__global__ void __launch_bounds__(128, 2) k_blk_bwd(const __grid_constant__ BArgs a) {
+  constexpr int W = 8 * PC, RW = R + W;
   extern __shared__ float4 sm4[];
   float* sm = (float*)sm4;
-  const int SP = a.SP, PW = a.nch * W, RW = R + PW;
+  const int SP = a.SP, PW = a.nch * W;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, lg = lane >> 3, cg = lane & 7, nt = blockDim.x;
   float* dys = sm;                                        // [32 rows][SP]
   float* xT = dys + R * SP;                               // [PW][LDT]
   float* dyT = xT + PW * LDT;                             // [PW][LDT]
-  float* dM = dyT + PW * LDT;                             // [l][s]
+  float* dM = dyT + PW * LDT;                             // [l][s]; later M^T [s][l]
   float* dMT = dM + R * LDT;                              // [s][l]
-  float* Ms = dMT + R * LDT;                              // M^T [s][l]
-  const size_t wstride = 2 * R * LDT + 2 * R * SP + R * RW;
-  float* red0 = Ms + R * LDT;
-  float* red = red0 + warp * wstride;                     // partial [M^T | dx]
-  float* Cd = red + R * RW;
+  float* Ms = dM;
+  // per warp: Cd, Bd, S, G tiles, dx partials of the column chunks past the first, `a` before rows 0, 8, 16, 24.  CD takes
+  // the place of S, BD that of Bd; the partial [M^T | dx] of the first chunk waits in registers and then takes Cd and Bd.
+  const size_t wstride = blk_warp_floats(1, PC, a.nch, SP);
+  float* red0 = dMT + R * LDT;
+  float* Cd = red0 + warp * wstride;
   float* Bd = Cd + R * LDT;
   float* S = Bd + R * LDT;
   float* G = S + R * SP;
+  float* redx0 = red0 + 2 * R * LDT + 2 * R * SP;
+  float* cuts = redx0 + warp * wstride + (a.nch - 1) * (R * W) + lane;
   const int seg = blockIdx.z, stream = blockIdx.x, bi = stream / a.H, h = stream % a.H, g = h / a.hpg;
-  const int n = (blockIdx.y * a.nw + warp) * 32 + lane;
+  const int n = (blockIdx.y * a.nw + warp) * 32 + lane, nl = min(n, a.N - 1);
   const bool act = n < a.N, first_slice = blockIdx.y == 0;
   const float An = act ? a.A[h * a.N + n] : 0.f, A2 = An * kLog2e, bias = (act && a.bias) ? a.bias[h * a.N + n] : 0.f;
   for (int i = tid; i < R * SP + 2 * PW * LDT; i += nt) dys[i] = 0.f;
@@ -600,67 +674,43 @@ __global__ void __launch_bounds__(128) k_blk_bwd(const __grid_constant__ BArgs a
       if (nn < a.N) *(float4*)(S + r * SP + c * 4) = *(const float4*)(a.saved + (((size_t)stream * (a.nblk + 1) + j) * a.N + nn) * PW + c * 4);
     }
   };
-  load_S(j1);
-  const TIO* __restrict__ Bp = (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + n;
-  const TIO* __restrict__ Cp = (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + n;
+  const int64_t csl = a.rev ? -a.C_sl : a.C_sl, bsl = a.rev ? -a.B_sl : a.B_sl;
   float dAacc = 0.f, dbacc = 0.f, dDacc = 0.f;
   for (int j = j1 - 1; j >= j0; --j) {
     const int row0 = j * R, rows = min(R, a.L - row0);
+    announce(a, bi, h, g, n - lane, lane, row0 - R, sizeof(TIO));
     __syncthreads();
-    float alast, cst = 0.f;
-    bool slow;
-    {
-      float raw[R];
-      load_dt(a, bi, h, n, act, row0, rows, raw);
-      for (int p = 0; p < PW; p += 4) {                   // <state leaving the block, gradient of it>
-        const float4 s = ld4(S + lane * SP + p), q = ld4(G + lane * SP + p);
-        cst = fmaf(s.x, q.x, fmaf(s.y, q.y, fmaf(s.z, q.z, fmaf(s.w, q.w, cst))));
-      }
-      for (int i = tid; i < R * a.P; i += nt) {
-        const int r = i / a.P, p = i - r * a.P, mr = brow(a, row0 + min(r, rows - 1));
+    for (int r = warp; r < R; r += a.nw) {
+      const int mr = brow(a, row0 + min(r, rows - 1));
+      const TIO* xp = (const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh;
+      for (int p = lane; p < a.P; p += 32) {
         float xv = 0.f, dv = 0.f;
         if (r < rows) {
-          xv = ldf((const TIO*)a.x + bi * a.x_sb + (int64_t)mr * a.x_sl + h * a.x_sh + p);
+          xv = ldf(xp + p);
           dv = dy_value<TIO>(a, bi, h, mr, p, first_slice);
         }
         dys[r * SP + p] = dv;
         dyT[p * LDT + r] = dv;
         xT[p * LDT + r] = xv;
       }
-      float acc = 0.f, mx = 0.f;
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        raw[r] = (act && r < rows) ? dt_value(a, raw[r], bias) : 0.f;
-        acc = fmaf(raw[r], A2, acc);
-        mx = fmaxf(mx, fabsf(acc));
-      }
-      alast = acc;
-      slow = __syncthreads_or(!(mx <= kRange));
-      load_S(j);
-      const float ref = slow ? alast : 0.f;
-      acc = 0.f;
-#pragma unroll
-      for (int r0 = 0; r0 < R; r0 += 8) {
-        float cv[8], bv[8];
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int64_t mr = brow(a, row0 + min(r0 + q, rows - 1));
-          cv[q] = act ? ldf(Cp + mr * a.C_sl) : 0.f;
-          bv[q] = act ? ldf(Bp + mr * a.B_sl) : 0.f;
-        }
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          acc = fmaf(raw[r0 + q], A2, acc);
-          cv[q] *= exp2f(acc);
-          bv[q] *= raw[r0 + q] * exp2f(ref - acc);
-          if (r0 + q >= rows) { cv[q] = 0.f; bv[q] = 0.f; }
-        }
-        st4(Cd + lane * LDT + r0, cv[0], cv[1], cv[2], cv[3]);
-        st4(Cd + lane * LDT + r0 + 4, cv[4], cv[5], cv[6], cv[7]);
-        st4(Bd + lane * LDT + r0, bv[0], bv[1], bv[2], bv[3]);
-        st4(Bd + lane * LDT + r0 + 4, bv[4], bv[5], bv[6], bv[7]);
-      }
-      const float el = slow ? 1.f : exp2f(alast);          // g' (a block out of range keeps G and has the decay in Bd)
+    }
+    float mx, cst = 0.f;
+    load_S(j + 1);
+    __syncwarp();
+    for (int p = 0; p < PW; p += 4) {
+      const float4 s = ld4(S + lane * SP + p), q = ld4(G + lane * SP + p);
+      cst = fmaf(s.x, q.x, fmaf(s.y, q.y, fmaf(s.z, q.z, fmaf(s.w, q.w, cst))));
+    }
+    const char* dtp = dt_ptr(a, bi, h, nl, row0);
+    const float alast = dt_pass(a, dtp, bias, A2, act, rows, Cd + lane * LDT, mx, cuts);
+    const bool slow = __syncthreads_or(!(mx <= kRange));
+    load_S(j);
+    const int64_t m0 = brow(a, row0);
+    const TIO* Cp = (const TIO*)a.C + bi * a.C_sb + g * a.C_sg + m0 * a.C_sl + nl;
+    const TIO* Bp = (const TIO*)a.B + bi * a.B_sb + g * a.B_sg + m0 * a.B_sl + nl;
+    operand_pass(Cp, csl, Bp, bsl, A2, act, rows, slow ? alast : 0.f, Cd + lane * LDT, Bd + lane * LDT);
+    {
+      const float el = slow ? 1.f : ex2(alast);            // g' (a block out of range keeps G and has the decay in Bd)
       for (int p = 0; p < PW; p += 4) {
         const float4 q = ld4(G + lane * SP + p);
         st4(G + lane * SP + p, q.x * el, q.y * el, q.z * el, q.w * el);
@@ -696,81 +746,82 @@ __global__ void __launch_bounds__(128) k_blk_bwd(const __grid_constant__ BArgs a
         *o = j == j1 - 1 ? acc : *o + acc;
       }
     __syncthreads();
+    float2 m[8][2], y[8][2], y4[4];
     {
-      float2 m[8][2], y[8][2], y4[4];
+      float2 cd[8][2], bd[8][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) m[i][0] = m[i][1] = y[i][0] = y[i][1] = dup(0.f);
+      for (int i = 0; i < 8; ++i) cd[i][0] = cd[i][1] = dup(0.f);
+      if (!slow) gemm_n(Bd, LDT, dMT, LDT, R, lg, cg, cd);
+      gemm_n(S, SP, dyT, LDT, PW, lg, cg, cd);
+      __syncwarp();
 #pragma unroll
-      for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
-      gemm_y<PC, true>(Bd, Cd, G, SP, lg, cg, m, y, y4);
-      if (!slow) {
-#pragma unroll
-        for (int i = 0; i < 8; ++i) st4(red + (lg * 8 + i) * RW + cg * 4, m[i][0].x, m[i][0].y, m[i][1].x, m[i][1].y);
-      }
-      store_y<PC>(red, RW, R, lg, cg, y, y4);
-      for (int c = 1; c < a.nch; ++c) {
+      for (int i = 0; i < 8; ++i) st4(S + (lg + 4 * i) * SP + cg * 4, cd[i][0].x, cd[i][0].y, cd[i][1].x, cd[i][1].y);
+      for (int c = a.nch - 1; c > 0; --c) {
 #pragma unroll
         for (int i = 0; i < 8; ++i) y[i][0] = y[i][1] = dup(0.f);
 #pragma unroll
         for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
         gemm_y<PC, false>(Bd, Cd, G + c * W, SP, lg, cg, m, y, y4);
-        store_y<PC>(red, RW, R + c * W, lg, cg, y, y4);
+        store_y<PC>(redx0 + warp * wstride + (c - 1) * (R * W), W, 0, lg, cg, y, y4);
       }
-    }
-    if (slow) slow_M<TIO>(a, bi, h, n, act, row0, rows, A2, bias, red, RW, true);
-    {
-      float2 cd[8][2], bd[8][2];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) cd[i][0] = cd[i][1] = bd[i][0] = bd[i][1] = dup(0.f);
-      if (!slow) {
-        gemm_n(Bd, LDT, dMT, LDT, R, lg, cg, cd);
-        gemm_n(Cd, LDT, dM, LDT, R, lg, cg, bd);
-      }
-      gemm_n(S, SP, dyT, LDT, PW, lg, cg, cd);
+      for (int i = 0; i < 8; ++i) m[i][0] = m[i][1] = y[i][0] = y[i][1] = bd[i][0] = bd[i][1] = dup(0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) y4[i] = dup(0.f);
+      gemm_y<PC, true>(Bd, Cd, G, SP, lg, cg, m, y, y4);
+      if (!slow) gemm_n(Cd, LDT, dM, LDT, R, lg, cg, bd);
       gemm_n(G, SP, xT, LDT, PW, lg, cg, bd);
       __syncwarp();
-      const float pre = slow ? exp2f(alast) : 1.f;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) st4(Bd + (lg + 4 * i) * LDT + cg * 4, bd[i][0].x, bd[i][0].y, bd[i][1].x, bd[i][1].y);
+      const float pre = slow ? ex2(alast) : 1.f;
       for (int c = 0; c < a.nch; ++c) update_state<PC>(G + c * W, SP, Cd, dys + c * W, lg, cg, pre, 1.f);
       __syncwarp();
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        st4(Cd + (lg + 4 * i) * LDT + cg * 4, cd[i][0].x, cd[i][0].y, cd[i][1].x, cd[i][1].y);
-        st4(Bd + (lg + 4 * i) * LDT + cg * 4, bd[i][0].x, bd[i][0].y, bd[i][1].x, bd[i][1].y);
-      }
-      __syncwarp();
     }
-    if (slow) slow_grads<TIO>(a, bi, h, n, act, row0, rows, A2, bias, dM, Cd + lane * LDT, Bd + lane * LDT);
-    {                                                      // per (row, state)
-      float v[R], dac[R], gd[R], sg[R];
-      load_dt(a, bi, h, n, act, row0, rows, v);
-      float acc = 0.f;
+    if (slow) slow_grads<TIO>(a, bi, h, n, act, row0, rows, A2, bias, dM, S + lane * SP, Bd + lane * LDT);
+    {                                                      // per (row, state), eight rows at a time from the end
       const size_t hn = (size_t)a.H * a.N, gn = (size_t)a.G * a.N;
-#pragma unroll
-      for (int r0 = 0; r0 < R; r0 += 8) {
-        float cv[8], bv[8];
+      const size_t bl0 = (size_t)bi * a.L + m0;            // memory row of the block's first point
+      const int dir = a.rev ? -1 : 1;
+      float raw[8], cn[8], bn[8], run = cst;
+      load8_dt(a, dtp, R - 8, rows - 1, raw);
+      load8(Cp, csl, R - 8, rows - 1, cn);
+      load8(Bp, bsl, R - 8, rows - 1, bn);
+#pragma unroll 1
+      for (int r0 = R - 8; r0 >= 0; r0 -= 8) {
+        float v[8], sg[8], ac[8], cv[8], bv[8], o[8];
+        float acc = cuts[(r0 >> 3) * 32];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-          const int64_t mr = brow(a, row0 + min(r0 + q, rows - 1));
-          cv[q] = act ? ldf(Cp + mr * a.C_sl) : 0.f;
-          bv[q] = act ? ldf(Bp + mr * a.B_sl) : 0.f;
+          const bool in = act && r0 + q < rows;
+          const float pre = raw[q] + bias;
+          float s = 1.f, tv = pre;
+          if (a.softplus) tv = softplus_sig(pre, s);
+          sg[q] = (in && tv >= a.dtmin && tv <= a.dtmax) ? s : 0.f;
+          v[q] = in ? fminf(fmaxf(tv, a.dtmin), a.dtmax) : 0.f;
+          acc = fmaf(v[q], A2, acc);
+          ac[q] = acc;
+          cv[q] = cn[q];
+          bv[q] = bn[q];
         }
+        if (r0 > 0) {
+          load8_dt(a, dtp, r0 - 8, rows - 1, raw);
+          load8(Cp, csl, r0 - 8, rows - 1, cn);
+          load8(Bp, bsl, r0 - 8, rows - 1, bn);
+        }
+        const float4 c0 = ld4(S + lane * SP + r0), c1 = ld4(S + lane * SP + r0 + 4), b0 = ld4(Bd + lane * LDT + r0), b1 = ld4(Bd + lane * LDT + r0 + 4);
+        const float CDv[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w}, BDv[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int r = r0 + q;
-          const bool in = act && r < rows;
-          const float pre = v[r] + bias;
-          const float tv = a.softplus ? softplus_thr(pre) : pre;
-          float s = (tv < a.dtmin || tv > a.dtmax) ? 0.f : 1.f;
-          if (a.softplus && pre <= 20.f) s *= sigmoidf_(pre);
-          v[r] = in ? fminf(fmaxf(tv, a.dtmin), a.dtmax) : 0.f;
-          acc = fmaf(v[r], A2, acc);
-          const float cdv = Cd[lane * LDT + r] * (slow ? 1.f : exp2f(acc)), bdv = Bd[lane * LDT + r] * (slow ? 1.f : exp2f(-acc));
-          const float dBv = v[r] * bdv;
-          dac[r] = in ? cv[q] * cdv - bv[q] * dBv : 0.f;
-          gd[r] = bv[q] * bdv;
-          sg[r] = in ? s : 0.f;
+        for (int q = 7; q >= 0; --q) {
+          const bool in = act && r0 + q < rows;
+          const float cdv = CDv[q] * (slow ? 1.f : ex2(ac[q])), bdv = BDv[q] * (slow ? 1.f : ex2(-ac[q]));
+          const float dBv = v[q] * bdv;
+          if (in) run += cv[q] * cdv - bv[q] * dBv;
+          dAacc = fmaf(run, v[q], dAacc);
+          o[q] = sg[q] != 0.f ? fmaf(run, An, bv[q] * bdv) * sg[q] : 0.f;
+          dbacc += o[q];
           if (in) {
-            const size_t bl = (size_t)bi * a.L + brow(a, row0 + r);
+            const size_t bl = bl0 + (int64_t)(dir * (r0 + q));
             if (a.hpg == 1) {
               stf((TIO*)a.dB + bl * gn + (size_t)g * a.N + n, dBv);
               stf((TIO*)a.dC + bl * gn + (size_t)g * a.N + n, cdv);
@@ -778,22 +829,21 @@ __global__ void __launch_bounds__(128) k_blk_bwd(const __grid_constant__ BArgs a
               a.dBh[bl * hn + (size_t)h * a.N + n] = dBv;
               a.dCh[bl * hn + (size_t)h * a.N + n] = cdv;
             }
+            if (a.dt_bf16) stf((bf16*)a.ddt + bl * hn + (size_t)h * a.N + n, o[q]);
+            else stf((float*)a.ddt + bl * hn + (size_t)h * a.N + n, o[q]);
           }
         }
       }
-      float run = cst;
+    }
+    __syncwarp();
+    {
+      float* red = Cd;
+      if (!slow) {
 #pragma unroll
-      for (int r = R - 1; r >= 0; --r) {
-        run += dac[r];
-        dAacc = fmaf(run, v[r], dAacc);
-        const float o = sg[r] != 0.f ? fmaf(run, An, gd[r]) * sg[r] : 0.f;
-        dbacc += o;
-        if (act && r < rows) {
-          const size_t at = ((size_t)bi * a.L + brow(a, row0 + r)) * hn + (size_t)h * a.N + n;
-          if (a.dt_bf16) stf((bf16*)a.ddt + at, o);
-          else stf((float*)a.ddt + at, o);
-        }
+        for (int i = 0; i < 8; ++i) st4(red + (lg * 8 + i) * RW + cg * 4, m[i][0].x, m[i][0].y, m[i][1].x, m[i][1].y);
       }
+      store_y<PC>(red, RW, R, lg, cg, y, y4);
+      if (slow) slow_M<TIO>(a, bi, h, n, act, row0, rows, A2, bias, red, RW, true);
     }
     __syncthreads();
     reduce_M(red0, wstride, a.nw, RW, Ms, true);
@@ -802,7 +852,8 @@ __global__ void __launch_bounds__(128) k_blk_bwd(const __grid_constant__ BArgs a
       const int l0 = (warp * (4 / a.nw) + it) * 8 + lg;
       for (int c = 0; c < a.nch; ++c) {
         float y[2][PC];
-        final_rows<PC>(red0, wstride, a.nw, RW, R + c * W, Ms, dys + c * W, SP, l0, cg, y);
+        if (c == 0) final_rows<PC>(red0, wstride, a.nw, RW, R, Ms, dys, SP, l0, cg, y);
+        else final_rows<PC>(redx0 + (c - 1) * (R * W), wstride, a.nw, W, 0, Ms, dys + c * W, SP, l0, cg, y);
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const int l = l0 + 4 * u;
@@ -885,9 +936,9 @@ constexpr size_t kSmemMax = 227 * 1024;
 struct Plan { int PC, nch, PW, SP, nw, nslice, nblk, nseg, seg_blk; size_t smem; };
 
 size_t blk_smem(const Plan& q, int pass) {
-  const size_t RW = R + q.PW;
-  if (pass == 0) return 4 * (size_t)(R * q.SP + R * LDT + q.nw * (2 * R * LDT + R * q.SP + R * RW));
-  return 4 * (size_t)(R * q.SP + 2 * q.PW * LDT + 3 * R * LDT + q.nw * (2 * R * LDT + 2 * R * q.SP + R * RW));
+  const size_t warp = blk_warp_floats(pass, q.PC, q.nch, q.SP);
+  if (pass == 0) return 4 * (R * q.SP + R * LDT + q.nw * warp);
+  return 4 * (R * q.SP + 2 * q.PW * LDT + 2 * R * LDT + q.nw * warp);
 }
 // false: the call stays on the per-pair kernels (head too wide for the tiles)
 bool blk_plan(const issm_params& p, int pass, Plan* out) {

@@ -1110,7 +1110,7 @@ size_t blocked_workspace_bytes(const issm_params& p, int pass) {
   z.workspace = nullptr;
   size_t total = 0;
   blk_carve(z, q, pass, &total);
-  return total;
+  return total ? total : 256;
 }
 bool blocked_supported(const issm_params& p, int pass) {
   Plan q;

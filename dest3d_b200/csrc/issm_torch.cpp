@@ -6,6 +6,7 @@
 // here: this file is host-side C++ only and links against libissm_b200.so.
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/library.h>
 
@@ -124,6 +125,64 @@ void attach_workspace(Common& c, int pass) {
   c.p.workspace_bytes = (size_t)ws.numel();
 }
 
+// outputs of a forward (absent ones: 0-element tensors), attached to the parameter struct
+void attach_fwd(Common& c, bool gated, bool want_final, bool save_states, Tensor& out, Tensor& out_x, Tensor& fin, Tensor& saved) {
+  issm_params& p = c.p;
+  const auto opt = c.x.options();
+  out = at::empty(c.x.sizes(), opt);
+  out_x = gated ? at::empty(c.x.sizes(), opt) : none_like(out);
+  fin = want_final ? at::empty({p.batch, p.nheads, p.headdim, p.dstate}, opt.dtype(at::kFloat)) : none_like(out);
+  saved = none_like(out);
+  if (save_states && issm_b200_resolve_path_pass(&p, 1) == ISSM_PATH_TENSOR) {
+    // the tensor-core backward reads the state entering every 64-point block instead of recomputing it
+    saved = at::empty({p.batch, p.nheads, (p.seqlen + 63) / 64 + 1, p.dstate, 48}, opt.dtype(at::kBFloat16));
+    p.saved_states = saved.data_ptr();
+  }
+  p.out = out.data_ptr(); p.out_sb = out.stride(0); p.out_sl = out.stride(1); p.out_sh = out.stride(2);
+  p.out_x = gated ? out_x.data_ptr() : nullptr;
+  p.final_states = want_final ? fin.data_ptr<float>() : nullptr;
+  p.want_final = want_final;
+}
+
+// gradients of a backward (absent ones: 0-element tensors; A, D, bias in float32), attached to the parameter struct
+struct Grads { Tensor x, dt, A, B, C, D, z, bias, init; };
+void attach_bwd(Common& c, const Tensor& dout, const OptTensor& out_x, const OptTensor& D, const OptTensor& z, const OptTensor& dt_bias,
+                const OptTensor& initial_states, const OptTensor& dfinal_states, const OptTensor& saved_states, Grads& r) {
+  issm_params& p = c.p;
+  const auto opt = c.x.options();
+  const Tensor doutk = act(dout, c.x.scalar_type(), c.keep);
+  TORCH_CHECK(doutk.sizes() == c.x.sizes(), "issm_b200: dout must have the shape of x");
+  r.x = at::empty(c.x.sizes(), opt);
+  r.dt = at::empty(c.dt.sizes(), opt.dtype(c.dt.scalar_type()));
+  r.B = at::empty(c.B.sizes(), opt);
+  r.C = at::empty(c.C.sizes(), opt);
+  r.z = z ? at::empty(c.x.sizes(), opt) : none_like(r.x);
+  r.A = at::empty({p.nheads, p.dstate}, opt.dtype(at::kFloat));
+  r.bias = dt_bias ? at::empty({p.nheads, p.dstate}, opt.dtype(at::kFloat)) : none_like(r.A);
+  r.D = D ? at::empty(D->sizes(), opt.dtype(at::kFloat)) : none_like(r.A);
+  r.init = initial_states ? at::empty(initial_states->sizes(), opt) : none_like(r.x);
+  if (z) {
+    TORCH_CHECK(out_x.has_value() && out_x->is_contiguous() && out_x->sizes() == c.x.sizes(),
+                "issm_b200: the pre-gate output saved by the forward is required when z is given");
+    p.out_x = out_x->data_ptr();
+    p.out_sb = out_x->stride(0); p.out_sl = out_x->stride(1); p.out_sh = out_x->stride(2);
+  }
+  p.dout = doutk.data_ptr(); p.dout_sb = doutk.stride(0); p.dout_sl = doutk.stride(1); p.dout_sh = doutk.stride(2);
+  if (dfinal_states) {
+    Tensor dfin = dfinal_states->to(at::kFloat).contiguous();
+    c.keep.push_back(dfin);
+    p.has_dfinal = 1;
+    p.dfinal_states = dfin.data_ptr<float>();
+  }
+  p.dx = r.x.data_ptr(); p.ddt = r.dt.data_ptr(); p.dB = r.B.data_ptr(); p.dC = r.C.data_ptr();
+  p.dz = z ? r.z.data_ptr() : nullptr;
+  p.dA = r.A.data_ptr<float>();
+  p.ddt_bias = dt_bias ? r.bias.data_ptr<float>() : nullptr;
+  p.dD = D ? r.D.data_ptr<float>() : nullptr;
+  p.dinitial_states = initial_states ? r.init.data_ptr() : nullptr;
+  if (saved_states && saved_states->numel() > 0) p.saved_states = saved_states->data_ptr();
+}
+
 // Forward; counterpart of _issm_chunk_scan_combined_fwd (issm_combined.py:57-92).
 // Returns (out, out_x, final_states, saved_states); absent ones are 0-element tensors.
 std::tuple<Tensor, Tensor, Tensor, Tensor> fwd(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C,
@@ -133,23 +192,10 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> fwd(const Tensor& x, const Tensor& dt
   const c10::cuda::CUDAGuard guard(x.device());
   Common c;
   fill_common(c, x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, dt_softplus, dt_min, dt_max, reverse, path, status);
-  issm_params& p = c.p;
-  const auto opt = c.x.options();
-  Tensor out = at::empty(c.x.sizes(), opt);
-  Tensor out_x = z ? at::empty(c.x.sizes(), opt) : none_like(out);
-  Tensor fin = want_final ? at::empty({p.batch, p.nheads, p.headdim, p.dstate}, opt.dtype(at::kFloat)) : none_like(out);
-  Tensor saved = none_like(out);
-  if (save_states && issm_b200_resolve_path_pass(&p, 1) == ISSM_PATH_TENSOR) {
-    // the tensor-core backward reads the state entering every 64-point block instead of recomputing it
-    saved = at::empty({p.batch, p.nheads, (p.seqlen + 63) / 64 + 1, p.dstate, 48}, opt.dtype(at::kBFloat16));
-    p.saved_states = saved.data_ptr();
-  }
-  p.out = out.data_ptr(); p.out_sb = out.stride(0); p.out_sl = out.stride(1); p.out_sh = out.stride(2);
-  p.out_x = z ? out_x.data_ptr() : nullptr;
-  p.final_states = want_final ? fin.data_ptr<float>() : nullptr;
-  p.want_final = want_final;
+  Tensor out, out_x, fin, saved;
+  attach_fwd(c, z.has_value(), want_final, save_states, out, out_x, fin, saved);
   attach_workspace(c, 0);
-  check_rc(issm_b200_fwd(&p, stream_of(c.x)), "issm_b200_fwd");
+  check_rc(issm_b200_fwd(&c.p, stream_of(c.x)), "issm_b200_fwd");
   return {out, out_x, fin, saved};
 }
 
@@ -164,43 +210,126 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tenso
   const c10::cuda::CUDAGuard guard(x.device());
   Common c;
   fill_common(c, x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, dt_softplus, dt_min, dt_max, reverse, path, status);
-  issm_params& p = c.p;
-  const at::ScalarType io = c.x.scalar_type();
-  const auto opt = c.x.options();
-  const Tensor doutk = act(dout, io, c.keep);
-  TORCH_CHECK(doutk.sizes() == c.x.sizes(), "issm_b200: dout must have the shape of x");
-  Tensor dx = at::empty(c.x.sizes(), opt);
-  Tensor ddt = at::empty(c.dt.sizes(), opt.dtype(c.dt.scalar_type()));
-  Tensor dB = at::empty(c.B.sizes(), opt);
-  Tensor dC = at::empty(c.C.sizes(), opt);
-  Tensor dz = z ? at::empty(c.x.sizes(), opt) : none_like(dx);
-  Tensor dA = at::empty({p.nheads, p.dstate}, opt.dtype(at::kFloat));
-  Tensor dbias = dt_bias ? at::empty({p.nheads, p.dstate}, opt.dtype(at::kFloat)) : none_like(dA);
-  Tensor dD = D ? at::empty(D->sizes(), opt.dtype(at::kFloat)) : none_like(dA);
-  Tensor dinit = initial_states ? at::empty(initial_states->sizes(), opt) : none_like(dx);
-  if (z) {
-    TORCH_CHECK(out_x.has_value() && out_x->is_contiguous() && out_x->sizes() == c.x.sizes(),
-                "issm_b200: the pre-gate output saved by the forward is required when z is given");
-    p.out_x = out_x->data_ptr();
-    p.out_sb = out_x->stride(0); p.out_sl = out_x->stride(1); p.out_sh = out_x->stride(2);
-  }
-  p.dout = doutk.data_ptr(); p.dout_sb = doutk.stride(0); p.dout_sl = doutk.stride(1); p.dout_sh = doutk.stride(2);
-  if (dfinal_states) {
-    Tensor dfin = dfinal_states->to(at::kFloat).contiguous();
-    c.keep.push_back(dfin);
-    p.has_dfinal = 1;
-    p.dfinal_states = dfin.data_ptr<float>();
-  }
-  p.dx = dx.data_ptr(); p.ddt = ddt.data_ptr(); p.dB = dB.data_ptr(); p.dC = dC.data_ptr();
-  p.dz = z ? dz.data_ptr() : nullptr;
-  p.dA = dA.data_ptr<float>();
-  p.ddt_bias = dt_bias ? dbias.data_ptr<float>() : nullptr;
-  p.dD = D ? dD.data_ptr<float>() : nullptr;
-  p.dinitial_states = initial_states ? dinit.data_ptr() : nullptr;
-  if (saved_states && saved_states->numel() > 0) p.saved_states = saved_states->data_ptr();
+  Grads r;
+  attach_bwd(c, dout, out_x, D, z, dt_bias, initial_states, dfinal_states, saved_states, r);
   attach_workspace(c, 1);
-  check_rc(issm_b200_bwd(&p, stream_of(c.x)), "issm_b200_bwd");
-  return {dx, ddt, dA, dB, dC, dD, dz, dbias, dinit};
+  check_rc(issm_b200_bwd(&c.p, stream_of(c.x)), "issm_b200_bwd");
+  return {r.x, r.dt, r.A, r.B, r.C, r.D, r.z, r.bias, r.init};
+}
+
+// ---- both scan directions ----------------------------------------------------------------------------
+// The directions share dt, A, D, z and the entering states and are independent of each other: the second one is enqueued on
+// a side stream of this host thread, forked from and joined to the caller's stream by events (which also makes them part of
+// a graph capture).  One direction alone leaves SMs idle: a scan has one block per (sample, head).  Every buffer is
+// allocated on the caller's stream and the join comes before the call returns, so the allocator needs to know nothing.
+struct Side {
+  cudaStream_t stream = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+};
+Side& side_of(int device) {
+  thread_local std::vector<Side> sides;
+  if ((int)sides.size() <= device) sides.resize(device + 1);
+  Side& s = sides[device];
+  if (!s.stream) {
+    s.stream = c10::cuda::getStreamFromPool(false, (c10::DeviceIndex)device).stream();
+    C10_CUDA_CHECK(cudaEventCreateWithFlags(&s.fork, cudaEventDisableTiming));
+    C10_CUDA_CHECK(cudaEventCreateWithFlags(&s.join, cudaEventDisableTiming));
+  }
+  return s;
+}
+struct Fork {
+  Side& side;
+  cudaStream_t main;
+  explicit Fork(const Tensor& t) : side(side_of(t.device().index())), main((cudaStream_t)stream_of(t)) {
+    C10_CUDA_CHECK(cudaEventRecord(side.fork, main));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(side.stream, side.fork, 0));
+  }
+  void join() {
+    C10_CUDA_CHECK(cudaEventRecord(side.join, side.stream));
+    C10_CUDA_CHECK(cudaStreamWaitEvent(main, side.join, 0));
+  }
+};
+void add_item(std::vector<issm_add_item>& v, const Tensor& a, const Tensor& b, double scale) {   // a <- (a + b) * scale
+  issm_add_item it{};
+  it.a = a.data_ptr(); it.b = b.data_ptr(); it.out = a.data_ptr();
+  it.n = a.numel(); it.dtype = dtype_code(a.scalar_type()); it.scale = (float)scale;
+  v.push_back(it);
+}
+
+// what both directions take is converted once
+OptTensor once(const OptTensor& t, at::ScalarType io) {
+  if (!t) return t;
+  return t->to(io).contiguous();
+}
+OptTensor bias_2d(const OptTensor& b, const Tensor& A) {
+  if (!b) return b;
+  return (b->dim() == 2 ? *b : b->unsqueeze(1).expand({A.size(0), A.size(1)})).to(at::kFloat).contiguous();
+}
+
+// out = scale * (forward scan of (x, B, C) + reversed scan of (xb, Bb, Cb)), final states likewise (models/dest_module.py:565-575).
+// Returns (out, final, out_x forward, out_x reversed, saved forward, saved reversed).
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> bi_fwd(
+    const Tensor& x, const Tensor& xb, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& Bb, const Tensor& Cb,
+    int64_t chunk_size, const OptTensor& D, const OptTensor& z, const OptTensor& dt_bias, const OptTensor& initial_states, bool dt_softplus,
+    double dt_min, double dt_max, double scale, int64_t path, bool save_states, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  std::vector<Tensor> keep;
+  const Tensor Ak = par(A, keep);
+  const OptTensor init = once(initial_states, x.scalar_type()), bias = bias_2d(dt_bias, A);
+  Common c[2];
+  Tensor out[2], out_x[2], fin[2], saved[2];
+  for (int k = 0; k < 2; ++k) {
+    fill_common(c[k], k ? xb : x, dt, Ak, k ? Bb : B, k ? Cb : C, chunk_size, D, z, bias, init, dt_softplus, dt_min, dt_max, k == 1, path, status);
+    attach_fwd(c[k], z.has_value(), true, save_states, out[k], out_x[k], fin[k], saved[k]);
+    attach_workspace(c[k], 0);
+  }
+  Fork f(c[0].x);
+  check_rc(issm_b200_fwd(&c[0].p, f.main), "issm_b200_fwd");
+  const int rc = issm_b200_fwd(&c[1].p, f.side.stream);
+  f.join();
+  check_rc(rc, "issm_b200_fwd");
+  std::vector<issm_add_item> sums;
+  add_item(sums, out[0], out[1], scale);
+  add_item(sums, fin[0], fin[1], scale);
+  check_rc(issm_b200_add_multi(sums.data(), (int32_t)sums.size(), f.main), "issm_b200_add_multi");
+  return {out[0], fin[0], out_x[0], out_x[1], saved[0], saved[1]};
+}
+
+// Returns (dx, dxb, ddt, dA, dB, dC, dBb, dCb, dD, dz, ddt_bias, dinitial_states); absent ones are 0-element tensors.
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> bi_bwd(
+    const Tensor& dout, const OptTensor& dfinal, const Tensor& x, const Tensor& xb, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C,
+    const Tensor& Bb, const Tensor& Cb, const OptTensor& out_x, const OptTensor& out_xb, int64_t chunk_size, const OptTensor& D, const OptTensor& z,
+    const OptTensor& dt_bias, const OptTensor& initial_states, bool dt_softplus, double dt_min, double dt_max, double scale, int64_t path,
+    const OptTensor& saved_f, const OptTensor& saved_b, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  std::vector<Tensor> keep;
+  const Tensor Ak = par(A, keep);
+  // the scale reaches both directions through their output gradients
+  const Tensor g = act(scale == 1.0 ? dout : at::mul(dout, scale), x.scalar_type(), keep);
+  OptTensor gf;
+  if (dfinal) gf = scale == 1.0 ? *dfinal : at::mul(*dfinal, scale);
+  const OptTensor init = once(initial_states, x.scalar_type()), bias = bias_2d(dt_bias, A);
+  Common c[2];
+  Grads r[2];
+  for (int k = 0; k < 2; ++k) {
+    fill_common(c[k], k ? xb : x, dt, Ak, k ? Bb : B, k ? Cb : C, chunk_size, D, z, bias, init, dt_softplus, dt_min, dt_max, k == 1, path, status);
+    attach_bwd(c[k], g, k ? out_xb : out_x, D, z, bias, init, gf, k ? saved_b : saved_f, r[k]);
+    attach_workspace(c[k], 1);
+  }
+  Fork f(c[0].x);
+  check_rc(issm_b200_bwd(&c[0].p, f.main), "issm_b200_bwd");
+  const int rc = issm_b200_bwd(&c[1].p, f.side.stream);
+  f.join();
+  check_rc(rc, "issm_b200_bwd");
+  std::vector<issm_add_item> sums;
+  add_item(sums, r[0].dt, r[1].dt, 1.0);
+  add_item(sums, r[0].A, r[1].A, 1.0);
+  if (D) add_item(sums, r[0].D, r[1].D, 1.0);
+  if (z) add_item(sums, r[0].z, r[1].z, 1.0);
+  if (dt_bias) add_item(sums, r[0].bias, r[1].bias, 1.0);
+  if (initial_states) add_item(sums, r[0].init, r[1].init, 1.0);
+  check_rc(issm_b200_add_multi(sums.data(), (int32_t)sums.size(), f.main), "issm_b200_add_multi");
+  return {r[0].x, r[1].x, r[0].dt, r[0].A, r[0].B, r[0].C, r[1].B, r[1].C, r[0].D, r[0].z, r[0].bias, r[0].init};
 }
 
 // ---- gated norms ------------------------------------------------------------------------------------
@@ -278,6 +407,13 @@ TORCH_LIBRARY(issm_b200, m) {
   m.def("bwd(Tensor dout, Tensor x, Tensor dt, Tensor A, Tensor B, Tensor C, Tensor? out_x, int chunk_size, Tensor? D, Tensor? z, "
         "Tensor? dt_bias, Tensor? initial_states, Tensor? dfinal_states, bool dt_softplus, float dt_min, float dt_max, bool reverse, "
         "int path, Tensor? saved_states, Tensor status) -> (Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)");
+  m.def("bi_fwd(Tensor x, Tensor xb, Tensor dt, Tensor A, Tensor B, Tensor C, Tensor Bb, Tensor Cb, int chunk_size, Tensor? D, Tensor? z, "
+        "Tensor? dt_bias, Tensor? initial_states, bool dt_softplus, float dt_min, float dt_max, float scale, int path, bool save_states, "
+        "Tensor status) -> (Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)");
+  m.def("bi_bwd(Tensor dout, Tensor? dfinal, Tensor x, Tensor xb, Tensor dt, Tensor A, Tensor B, Tensor C, Tensor Bb, Tensor Cb, "
+        "Tensor? out_x, Tensor? out_xb, int chunk_size, Tensor? D, Tensor? z, Tensor? dt_bias, Tensor? initial_states, bool dt_softplus, "
+        "float dt_min, float dt_max, float scale, int path, Tensor? saved_f, Tensor? saved_b, Tensor status) -> (Tensor, Tensor, Tensor, "
+        "Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor)");
   m.def("norm_fwd(Tensor x, Tensor? z, Tensor weight, Tensor? bias, float eps, int group_size, bool norm_before_gate, bool is_rms) "
         "-> (Tensor, Tensor, Tensor)");
   m.def("norm_bwd(Tensor dy, Tensor x, Tensor? z, Tensor weight, Tensor? bias, Tensor rstd, Tensor? mean, float eps, int group_size, "
@@ -287,6 +423,8 @@ TORCH_LIBRARY(issm_b200, m) {
 TORCH_LIBRARY_IMPL(issm_b200, CUDA, m) {
   m.impl("fwd", &fwd);
   m.impl("bwd", &bwd);
+  m.impl("bi_fwd", &bi_fwd);
+  m.impl("bi_bwd", &bi_bwd);
   m.impl("norm_fwd", &norm_fwd);
   m.impl("norm_bwd", &norm_bwd);
 }

@@ -30,7 +30,9 @@ def _status_word(device):
     """One int32 per device that kernels OR error bits into (bit 0 (value 1): a bounded wait
     expired; bit 2 (value 4), informational: a 64-point block exceeded the decay range of the fast tensor-core
     kernel and its stream was redone by the windowed kernel)."""
-    key = torch.device(device).index if torch.device(device).index is not None else torch.cuda.current_device()
+    key = device.index if isinstance(device, torch.device) else torch.device(device).index
+    if key is None:
+        key = torch.cuda.current_device()
     if key not in _STATUS:
         _STATUS[key] = torch.zeros(1, dtype=torch.int32, device=torch.device("cuda", key))
     return _STATUS[key]
@@ -149,11 +151,17 @@ class _StatusMirror:
                                    f"(status {v}); the results of that call are invalid")
 
     def refresh(self):
-        if torch.cuda.is_current_stream_capturing():
-            return
         self.host.copy_(_status_word(self.device), non_blocking=True)
         self.event.record()
         self.pending = True
+
+
+    def check(self, what):
+        if torch.cuda.is_current_stream_capturing():     # inside a CUDA-graph capture: neither query nor copy
+            return
+        self.poll(what)
+        if not self.pending:                             # one copy in flight at a time: a step of several calls enqueues one
+            self.refresh()
 
 
 _MIRROR = {}
@@ -167,17 +175,18 @@ def _check_status(device, what):
     if os.environ.get("ISSM_B200_CHECK_STATUS") == "1":
         raise_on_device_error(device, what)
         return
-    dev = torch.device(device)
-    key = dev.index if dev.index is not None else torch.cuda.current_device()
+    key = device.index if isinstance(device, torch.device) else torch.device(device).index
+    cur = torch.cuda.current_device()
+    if key is None:
+        key = cur
     m = _MIRROR.get(key)
     if m is None:
         m = _MIRROR[key] = _StatusMirror(torch.device("cuda", key))
-    with torch.cuda.device(key):
-        if torch.cuda.is_current_stream_capturing():     # inside a CUDA-graph capture: neither query nor copy
-            return
-        m.poll(what)
-        if not m.pending:                                # one copy in flight at a time: a step of several calls enqueues one
-            m.refresh()
+    if key == cur:
+        m.check(what)
+    else:
+        with torch.cuda.device(key):
+            m.check(what)
 
 
 def raise_on_device_error(device=None, what="ISSM"):
@@ -393,6 +402,43 @@ def _scan_packed(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, seq_
     return (out, torch.cat(finals, dim=0)) if return_final_states else out
 
 
+class BidirectionalScanFn(torch.autograd.Function):
+    """Both directions in one call of the extension: the second runs on a side stream next to the first (one direction has
+    one block per (sample, head) and leaves SMs idle), what they share is converted once, and one launch joins the
+    results - in the backward the gradients of dt, A, D, z, dt_bias and the entering states."""
+
+    @staticmethod
+    def forward(ctx, x, x_back, dt, A, B, C, B_back, C_back, chunk_size, D, z, dt_bias, initial_states, dt_softplus, dt_limit, out_scale, path):
+        ctx.set_materialize_grads(False)
+        need_grad = any(ctx.needs_input_grad)
+        out, final, ox, oxb, sf, sb = _ext.ops().bi_fwd(
+            x, x_back, dt, A, B, C, B_back, C_back, int(chunk_size), D, z, dt_bias, initial_states, bool(dt_softplus), float(dt_limit[0]),
+            float(dt_limit[1]), float(out_scale), _PATHS[path], need_grad, _status_word(x.device))
+        _check_status(x.device, "issm_b200_fwd")
+        if need_grad:
+            ctx.save_for_backward(x, x_back, dt, A, B, C, B_back, C_back, D, z, dt_bias, initial_states, _ext.opt(ox), _ext.opt(oxb), _ext.opt(sf), _ext.opt(sb))
+            ctx.opts = (int(chunk_size), bool(dt_softplus), float(dt_limit[0]), float(dt_limit[1]), float(out_scale), _PATHS[path])
+        return out, final
+
+    @staticmethod
+    def backward(ctx, dout, dfinal):
+        x, xb, dt, A, B, C, Bb, Cb, D, z, dt_bias, init, ox, oxb, sf, sb = ctx.saved_tensors
+        chunk_size, softplus, lo, hi, scale, path = ctx.opts
+        if dout is None:
+            if dfinal is None:
+                return (None,) * 17
+            dout = torch.zeros_like(x)
+        g = _ext.ops().bi_bwd(dout, dfinal, x, xb, dt, A, B, C, Bb, Cb, ox, oxb, chunk_size, D, z, dt_bias, init, softplus, lo, hi, scale, path,
+                              sf, sb, _status_word(x.device))
+        _check_status(x.device, "issm_b200_bwd")
+        dx, dxb, ddt, dA, dB, dC, dBb, dCb, dD, dz, dbias, dinit = g
+        if dt_bias is not None and dt_bias.dim() != 2:
+            dbias = dbias.sum(dim=1)
+        like = lambda t, ref: None if ref is None else (t if t.dtype == ref.dtype else t.to(ref.dtype))
+        return (dx, like(dxb, xb), like(ddt, dt), like(dA, A), like(dB, B), like(dC, C), like(dBb, Bb), like(dCb, Cb), None, like(dD, D),
+                like(dz, z), like(dbias, dt_bias), like(dinit, init), None, None, None, None)
+
+
 def issm_bidirectional_scan(x, x_back, dt, A, B, C, B_back, C_back, chunk_size, D=None, z=None, dt_bias=None,
                             initial_states=None, dt_softplus=False, dt_limit=(0.0, float("inf")),
                             out_scale=0.5, path="auto"):
@@ -400,6 +446,9 @@ def issm_bidirectional_scan(x, x_back, dt, A, B, C, B_back, C_back, chunk_size, 
     initial states, combined as out_scale * (fwd + bwd): the bidirectional block of
     models/dest_module.py:565-575 (which averages, out_scale = 0.5) without the flipped copies.
     All `_back` tensors are in natural point order.  Returns (out, final_states)."""
+    if BINDING == "torch":
+        return BidirectionalScanFn.apply(x, x_back, dt, A, B, C, B_back, C_back, chunk_size, D, z, dt_bias, initial_states, dt_softplus,
+                                         dt_limit, out_scale, path)
     yf, sf = ISSM_chunk_scan_combined(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, None,
                                       dt_softplus, dt_limit, True, reverse=False, path=path)
     yb, sb = ISSM_chunk_scan_combined(x_back, dt, A, B_back, C_back, chunk_size, D, z, dt_bias, initial_states,

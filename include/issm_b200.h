@@ -258,6 +258,20 @@ int issm_b200_dt_sum(const void* dt, int32_t dt_dtype, int32_t batch, int32_t se
                      int64_t dt_sb, int64_t dt_sl, int64_t dt_sh, const float* dt_bias, int32_t dt_softplus, float dt_min,
                      float dt_max, int32_t rows_per_part, float* part, void* cuda_stream);
 
+/* ---- joining the two scan directions ------------------------------------------------------------------------ */
+
+/* out = (a + b) * scale for up to ISSM_ADD_MAX contiguous arrays in one launch (models/dest_module.py:574 and the
+ * gradients of what the two directions share).  dtype ISSM_F32 or ISSM_BF16 (summed in float, rounded once); 16-byte
+ * aligned pointers; out may be a or b. */
+#define ISSM_ADD_MAX 8
+typedef struct issm_add_item {
+  const void* a; const void* b; void* out;
+  int64_t n;
+  int32_t dtype;
+  float scale;
+} issm_add_item;
+int issm_b200_add_multi(const issm_add_item* items, int32_t count, void* cuda_stream);
+
 /* Number of kernel launches the library has enqueued since load (monotonic, process-wide);
  * used by the benchmark to report how many of its own kernels ran inside a timed region. */
 uint64_t issm_b200_launch_count(void);

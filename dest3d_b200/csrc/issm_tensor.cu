@@ -159,15 +159,11 @@ __device__ __noinline__ void fwd_windowed_passes(const TArgs& a, WinCtx<TDT>& c)
 // every bulk prefetch.  The I/O warps load the x / z rows of the block, build the x operand tile and
 // store the previous block's output rows (D skip and gate applied) with coalesced accesses.
 //
-// Two instantiations walk the streams.  kWin = false is the fast one: it only notices a block outside the range
-// of the single-reference factorisation and marks its (batch, head) stream in a.redo.  kWin = true is launched
-// right behind it, returns at once for unmarked streams and redoes the marked ones from the start with the
-// windowed passes described at fwd_windowed_passes (keeping that code out of the fast kernel is worth 15 %).
-// kMode fixes the row order of the staged tiles at compile time, so that their addresses need no multiply:
-// 1 = dt / B / C tiles staged in scan order (forward scan of regular arrays), 2 = staged in memory order for a
-// reversed scan (walked backwards), 0 = decided at run time (row-by-row copies, mixed layouts).
-template <int NT, typename TDT, bool kWin, int kMode>
-__global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_constant__ TArgs a, const __grid_constant__ FwdMaps maps) {
+// This is the windowed walk: it returns at once unless the pipelined kernel (issm_tensor_fwd.cu) has marked the stream as
+// holding a block outside the range of the single-reference factorisation, and then redoes the stream from the start with
+// the windowed passes described at fwd_windowed_passes (keeping that code out of the fast kernel is worth 15 %).
+template <int NT, typename TDT>
+__global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_windowed(const __grid_constant__ TArgs a, const __grid_constant__ FwdMaps maps) {
   using SM = FwdSmem<NT>;
   constexpr bool kStageDt = sizeof(TDT) == 2;
   constexpr int NTH = 2 * NT;                           // column threads
@@ -193,7 +189,7 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
   const int h = blockIdx.y, b = blockIdx.z, g = h / a.hpg;
   const int n_off = blockIdx.x * NT;                     // first state of this CTA's slice
   const int stream = (blockIdx.x * a.b + b) * a.H + h;
-  if (kWin && !a.redo[stream]) return;                   // the fast kernel finished this stream
+  if (!a.redo[stream]) return;                           // the fast kernel finished this stream
   const int n = tid % NT, half = (tid / NT) & 1;
   const TDT* __restrict__ dtp = (const TDT*)a.dt + b * a.dt_sb + h * a.dt_sh + n_off;
   const bf16* __restrict__ Bp = a.B + b * a.B_sb + g * a.B_sg + n_off;
@@ -202,11 +198,6 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
   const bf16* __restrict__ zp = a.has_z ? a.z + b * a.z_sb + h * a.z_sh : nullptr;
   const float A2 = __ldg(a.A + h * a.N + n_off + n) * LOG2E;
   const float bias = a.has_bias ? __ldg(a.bias + h * a.N + n_off + n) : 0.f;
-  // the same constants for the two adjacent states (2 pr, 2 pr + 1) of the fast instantiation's operand pass
-  const int pr0 = n_off + 2 * (tid % (NT / 2));
-  const float2 A2p = f2(__ldg(a.A + h * a.N + pr0) * LOG2E, __ldg(a.A + h * a.N + pr0 + 1) * LOG2E);
-  const float bsc = a.softplus ? LOG2E : 1.f;
-  const float2 biasL2 = a.has_bias ? f2(__ldg(a.bias + h * a.N + pr0) * bsc, __ldg(a.bias + h * a.N + pr0 + 1) * bsc) : f2(0.f);
   const int nblk = (a.L + QB - 1) / QB;
 
   // one-time setup: zero the padded operand tiles, barriers, TMEM
@@ -384,7 +375,7 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
   };
 
   bool failed = false;
-  uint32_t windowed = 0, unsafe = 0;
+  uint32_t windowed = 0;
 
   // The three roles run their own loop over the blocks (so that the registers of one role's state are not held
   // through the code of the others); they meet at the two block-wide barriers of every iteration.
@@ -433,12 +424,12 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
       // dropped): per window the column threads rebuild Cd / Bd relative to the window start with every row outside
       // the window zero, the MMAs accumulate [M | Y] over the windows (M becomes block diagonal, rows of later
       // windows see earlier ones through the state) and the state is rescaled by the window's decay.
-      const uint32_t flag = kWin ? *sFlag : 0u;
-      const int kw = (kWin && (flag >> 3) == (uint32_t)(blk + 1)) ? (int)(flag & 7) : 0;
+      const uint32_t flag = *sFlag;
+      const int kw = (flag >> 3) == (uint32_t)(blk + 1) ? (int)(flag & 7) : 0;
       const int ws = QB >> kw;
       const int npass = kw ? (rows + ws - 1) / ws : 1;
       // ---- MMAs of the block (of every window of a flagged block) ---------------------------------------------
-      if (!kWin || kw == 0) {
+      if (kw == 0) {
         if (lane == 0) {
           fence_after_sync();
           issue_mmas(false);
@@ -482,15 +473,14 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
 
       // Staged tiles are addressed as base + l * step in units of rows: a tile that was copied in memory
       // order for a reversed scan is walked backwards.  Full blocks run a guard-free instantiation.
-      const bool flipT = kMode ? kMode == 2 : (a.dt_tma && a.rev), flipB = kMode ? kMode == 2 : ((a.bc_contig || a.bc_tma) && a.rev);
+      const bool flipT = a.dt_tma && a.rev, flipB = (a.bc_contig || a.bc_tma) && a.rev;
       const bf16* sdt = (const bf16*)(smem + SM::kSdt) + n + (flipT ? (rows - 1) * NT : 0);
       const int dstep = flipT ? -NT : NT;
       const bf16* sB = (const bf16*)(smem + SM::kSB) + n + (flipB ? (rows - 1) * NT : 0);
       const bf16* sC = (const bf16*)(smem + SM::kSC) + n + (flipB ? (rows - 1) * NT : 0);
       const int bstep = flipB ? -NT : NT;
 
-      if constexpr (kWin) {
-        // the windowed instantiation keeps the one-state-per-thread pass (its window code addresses rows per half)
+      {
         // ---- phase A: dt of this thread's 32 rows and their summed log2-decay -----------------------
         float dtv[32];
         float asum = 0.f;
@@ -519,8 +509,7 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
         // (or over its first half) exceeds 2^120 asks for the block to be redone in 2^k row windows, each with
         // its own reference: the smallest k for which this thread's windows stay within 2^100.
         if (!(fabsf(a0) <= 120.f && fabsf(alast) <= 120.f)) {
-          if (kWin) atomicMax(sFlag, (uint32_t)(blk + 1) * 8 + window_need<TDT>(a, sdt, dstep, dtp, row0, rows, half, n, A2, bias));
-          else unsafe = 1;
+          atomicMax(sFlag, (uint32_t)(blk + 1) * 8 + window_need<TDT>(a, sdt, dstep, dtp, row0, rows, half, n, A2, bias));
         }
 
         // ---- phase B: this thread's rows of column n of Cd = C 2^a and Bd = B dt 2^-a ------------------
@@ -544,80 +533,20 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
           }
         };
         if (rows == QB) phaseB(std::true_type{}); else phaseB(std::false_type{});
-      } else {
-        // ---- operand pass, two adjacent states (2 pr, 2 pr + 1) and the 16 rows of quarter qr per thread: every
-        //      shared-memory access moves a bf16 pair (4 bytes) and the fp32 arithmetic runs as packed pairs --------
-        constexpr int NPR = NT / 2;
-        const int pr = tid % NPR, qr = tid / NPR;
-        const bool flipB2 = kMode ? kMode == 2 : ((a.bc_contig || a.bc_tma) && a.rev);
-        const uint32_t* sdt2 = (const uint32_t*)(smem + SM::kSdt) + pr + (flipT ? (rows - 1) * NPR : 0);
-        const int dstep2 = flipT ? -NPR : NPR;
-        const uint32_t* sB2 = (const uint32_t*)(smem + SM::kSB) + pr + (flipB2 ? (rows - 1) * NPR : 0);
-        const uint32_t* sC2 = (const uint32_t*)(smem + SM::kSC) + pr + (flipB2 ? (rows - 1) * NPR : 0);
-        const int bstep2 = flipB2 ? -NPR : NPR;
-        float2 dtv[16];
-        float2 asum2 = f2(0.f);
-        auto phaseA2 = [&](auto full) {
-          constexpr bool kFull = decltype(full)::value;
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int l = qr * 16 + j;
-            const int sl = kFull ? l : min(l, rows - 1);
-            float2 raw;
-            if constexpr (kStageDt) raw = unpack_bf16(sdt2[sl * dstep2]);
-            else raw = *(const float2*)((const float*)dtp + (int64_t)trow(a, row0 + sl) * a.dt_sl + 2 * pr);
-            float2 v = dt_transform2(a, raw, biasL2);
-            if (!kFull && l >= rows) v = f2(0.f);
-            dtv[j] = v;
-            asum2 = __ffma2_rn(v, A2p, asum2);
-          }
-        };
-        if (rows == QB) phaseA2(std::true_type{}); else phaseA2(std::false_type{});
-        *(float2*)(sAsum + qr * NT + 2 * pr) = asum2;
-        named_barrier(1 + (warp % (NPR / 32)), 128);       // the four warps that share these 64 columns
-        const float2 q0 = *(const float2*)(sAsum + 2 * pr), q1 = *(const float2*)(sAsum + NT + 2 * pr),
-                     q2 = *(const float2*)(sAsum + 2 * NT + 2 * pr), q3 = *(const float2*)(sAsum + 3 * NT + 2 * pr);
-        const float2 c1 = q0, c2 = __fadd2_rn(c1, q1), c3 = __fadd2_rn(c2, q2), c4 = __fadd2_rn(c3, q3);
-        // range of the factorisation (see the windowed instantiation above): every running sum must stay within 2^120
-        const float worst = fmaxf(fmaxf(fmaxf(fabsf(c1.x), fabsf(c1.y)), fmaxf(fabsf(c2.x), fabsf(c2.y))),
-                                  fmaxf(fmaxf(fabsf(c3.x), fabsf(c3.y)), fmaxf(fabsf(c4.x), fabsf(c4.y))));
-        if (!(worst <= 120.f)) unsafe = 1;
-        auto phaseB2 = [&](auto full) {
-          constexpr bool kFull = decltype(full)::value;
-          const int at = pr >> 5, kc = (pr & 31) >> 2;     // 64-state atom, 16-byte chunk inside its 128-byte rows
-          uint8_t* cd_col = smem + SM::kCd + at * (QB * 128) + qr * (16 * 128) + ((pr & 3) << 2);
-          uint8_t* bd_col = smem + SM::kBd + at * SM::kAtomB + qr * (16 * 128) + ((pr & 3) << 2);
-          float2 acc = qr == 0 ? f2(0.f) : (qr == 1 ? c1 : (qr == 2 ? c2 : c3));
-#pragma unroll
-          for (int j = 0; j < 16; ++j) {
-            const int l = qr * 16 + j;
-            const int sl = kFull ? l : min(l, rows - 1);
-            const float2 dtj = dtv[j];
-            acc = __ffma2_rn(dtj, A2p, acc);
-            float2 cd = __fmul2_rn(unpack_bf16(sC2[sl * bstep2]), ex2f2(acc));
-            float2 bd = __fmul2_rn(__fmul2_rn(unpack_bf16(sB2[sl * bstep2]), dtj), ex2f2_neg(acc));
-            if (!kFull && l >= rows) { cd = f2(0.f); bd = f2(0.f); }
-            const uint32_t off = (uint32_t)(j * 128 + ((kc ^ (j & 7)) << 4));
-            *(uint32_t*)(cd_col + off) = pack_bf16(cd);
-            *(uint32_t*)(bd_col + off) = pack_bf16(bd);
-          }
-        };
-        if (rows == QB) phaseB2(std::true_type{}); else phaseB2(std::false_type{});
       }
       fence_async_smem();
       fence_before_sync();
       if (__syncthreads_or(failed)) { failed = true; break; }
-      const uint32_t flag = kWin ? *sFlag : 0u;
-      const int kw = (kWin && (flag >> 3) == (uint32_t)(blk + 1)) ? (int)(flag & 7) : 0;
+      const uint32_t flag = *sFlag;
+      const int kw = (flag >> 3) == (uint32_t)(blk + 1) ? (int)(flag & 7) : 0;
       const int ws = QB >> kw;
       const int npass = kw ? (rows + ws - 1) / ws : 1;
-      if constexpr (!kWin) alast = ((sAsum[n] + sAsum[NT + n]) + sAsum[2 * NT + n]) + sAsum[3 * NT + n];   // summed decay of column n
       // output rows of the previous block, while the MMAs of this one run and the column threads would wait anyway
       if (blk > 0 && !a.no_output) {
 #pragma unroll
         for (int r = 0; r < kColR; ++r) group_store(group_load(row0 - QB, QB, tid + r * NTH), row0 - QB, QB);
       }
-      if (!kWin || kw == 0) {
+      if (kw == 0) {
         if (!mbar_wait_warp(barA, phA)) failed = true;
         phA ^= 1;
         fence_after_sync();
@@ -705,11 +634,8 @@ __global__ void __launch_bounds__(2 * NT + 128, 1) k_fwd_tensor(const __grid_con
 
   // a wait of the last iteration can expire after that iteration's last block-wide vote: make the verdict
   // uniform over the block before anything below depends on it
-  const int votes = __syncthreads_or((int)unsafe | (failed ? 2 : 0));
-  const int any_unsafe = votes & 1;
-  failed = (votes & 2) != 0;
+  failed = __syncthreads_or(failed);
   if (!failed && !a.no_output && nblk > 0) store_tile(prev_row0, prev_rows);   // last block's tile
-  if (!kWin && tid == 0) a.redo[stream] = any_unsafe;
   if (a.status) {
     if (failed && tid == 0) atomicOr(a.status, 1);
     if (windowed && tid == 0) atomicOr(a.status, 4);       // informational: some block ran windowed
@@ -807,6 +733,7 @@ TArgs make_targs(const issm_params& p) {
   a.hpg = p.nheads / p.ngroups; a.rev = p.reverse;
   a.has_D = p.has_D; a.D_has_hdim = p.D_has_hdim; a.has_z = p.has_z; a.has_bias = p.has_dt_bias;
   a.softplus = p.dt_softplus; a.has_init = p.has_init; a.want_final = p.want_final;
+  a.dt_f32 = p.dt_dtype == ISSM_F32;
   a.dtmin = p.dt_min; a.dtmax = p.dt_max;
   a.x = (const bf16*)p.x; a.x_sb = p.x_sb; a.x_sl = p.x_sl; a.x_sh = p.x_sh;
   a.dt = p.dt; a.dt_sb = p.dt_sb; a.dt_sl = p.dt_sl; a.dt_sh = p.dt_sh;
@@ -855,30 +782,23 @@ bool make_rows_tensor_map(const void* base, int64_t sb, int64_t sl, int64_t widt
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+bool make_tile_map(const void* base, int64_t sb, int64_t sl, int64_t width, int batch, int seqlen, CUtensorMap* out) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn || !base || ((uintptr_t)base & 15) || (sl & 7) || (sb & 7) || sl < 64 || sb < sl || width < 64) return false;
+  const cuuint64_t gdim[3] = {(cuuint64_t)width, (cuuint64_t)seqlen, (cuuint64_t)batch};
+  const cuuint64_t gstride[2] = {(cuuint64_t)sl * 2, (cuuint64_t)sb * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)QB, 1};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstride, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool make_dt_tensor_map(const issm_params& p, CUtensorMap* out) {
   memset(out, 0, sizeof(*out));
   if (p.dt_dtype != ISSM_BF16 || (p.dt_sh & 7)) return false;
   // one tile = one 256-state slice (or all 128 / 256 states) of one head, 64 rows
   return make_rows_tensor_map(p.dt, p.dt_sb, p.dt_sl, (int64_t)(p.nheads - 1) * p.dt_sh + p.dstate, p.batch, p.seqlen,
                               p.dstate > 256 ? 256 : p.dstate, out);
-}
-
-template <int NT, typename TDT, int kMode>
-static int launch_fwd_mode(const TArgs& a, const FwdMaps& maps, cudaStream_t s) {
-  const size_t smem = FwdSmem<NT>::kTotal + 1024;
-  struct FastTag {};
-  struct WinTag {};
-  if (SmemAttrOnce<FastTag>::set(k_fwd_tensor<NT, TDT, false, kMode>, smem) != ISSM_OK ||
-      SmemAttrOnce<WinTag>::set(k_fwd_tensor<NT, TDT, true, 0>, smem) != ISSM_OK)
-    return ISSM_ERR_CUDA;
-  const int slices = a.N / NT;
-  ISSM_LAUNCH((k_fwd_tensor<NT, TDT, false, kMode>), dim3(slices, a.H, a.b), 2 * NT + 128, smem, s, a, maps);
-  ISSM_LAUNCH((k_fwd_tensor<NT, TDT, true, 0>), dim3(slices, a.H, a.b), 2 * NT + 128, smem, s, a, maps);   // marked streams only
-  if (slices > 1 && !a.no_output) {
-    const size_t groups = (size_t)a.b * a.L * a.H * (a.P / 4);
-    ISSM_LAUNCH(k_combine_slices, (unsigned)cdiv64(groups, 256), 256, 0, s, a, slices, groups);
-  }
-  return ISSM_OK;
 }
 
 template <int NT, typename TDT>
@@ -892,10 +812,18 @@ static int launch_fwd(TArgs a, const issm_params& p, cudaStream_t s) {
               make_rows_tensor_map(p.B, p.B_sb, p.B_sl, (int64_t)(p.ngroups - 1) * p.B_sg + p.dstate, p.batch, p.seqlen, box, &maps.B) &&
               make_rows_tensor_map(p.C, p.C_sb, p.C_sl, (int64_t)(p.ngroups - 1) * p.C_sg + p.dstate, p.batch, p.seqlen, box, &maps.C)) ? 1 : 0;
   if (!a.bc_tma) { memset(&maps.B, 0, sizeof(maps.B)); memset(&maps.C, 0, sizeof(maps.C)); }
-  // whole-tile copies of dt (when it is staged at all) and of B / C: the row order of the staged tiles is known
-  const bool tiles = (a.bc_contig || a.bc_tma) && (sizeof(TDT) != 2 || a.dt_tma);
-  if (!tiles) return launch_fwd_mode<NT, TDT, 0>(a, maps, s);
-  return a.rev ? launch_fwd_mode<NT, TDT, 2>(a, maps, s) : launch_fwd_mode<NT, TDT, 1>(a, maps, s);
+  const size_t smem = FwdSmem<NT>::kTotal + 1024;
+  struct WinTag {};
+  if (SmemAttrOnce<WinTag>::set(k_fwd_windowed<NT, TDT>, smem) != ISSM_OK) return ISSM_ERR_CUDA;
+  const int slices = a.N / NT;
+  const int rc = launch_fwd_pipe(a, p, NT, s);
+  if (rc) return rc;
+  ISSM_LAUNCH((k_fwd_windowed<NT, TDT>), dim3(slices, a.H, a.b), 2 * NT + 128, smem, s, a, maps);   // marked streams only
+  if (slices > 1 && !a.no_output) {
+    const size_t groups = (size_t)a.b * a.L * a.H * (a.P / 4);
+    ISSM_LAUNCH(k_combine_slices, (unsigned)cdiv64(groups, 256), 256, 0, s, a, slices, groups);
+  }
+  return ISSM_OK;
 }
 
 int tensor_fwd(const issm_params& p, cudaStream_t s) {

@@ -24,6 +24,7 @@ struct TArgs {
   int* redo;        // (batch, nheads) marks: stream holds a block outside the fast kernel's range, redo it windowed
   bf16* dxpart;     // backward with state slices: (slice, b, L, H, P) bf16 partial dx rows (before the D skip)
   float* ypart;     // forward with the states cut into slices of 256 (dstate 512 ...): (slice, b, L, H, P) float partial outputs
+  int dt_f32;       // dt and ddt are float (else bf16)
   int dt_tma;       // dt is a regular 2-D array of rows: a 64-row tile is ONE tiled TMA load through a tensor map
   int bc_contig;    // B and C rows of one (batch, group) are adjacent in memory: a 64-row tile is one bulk copy
   int bc_tma;       // forward: B and C are regular 2-D arrays of rows (any row pitch): a 64-row tile is one tiled TMA load each
@@ -74,14 +75,18 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t w) { return make_float2(_
 
 // dt of one row, two adjacent states: bias, softplus (reference threshold 20, evaluated in the log2 domain: the
 // pre-activation scaled by log2 e is `t`, softplus = ln 2 * lg2(1 + 2^t), and above the threshold t * ln 2), clamp.
-// biasL = bias * log2 e when softplus is on, else the plain bias.
+// biasL = bias * log2 e when softplus is on, else the plain bias.  kThr = false leaves the threshold out: right where the
+// clamp lies below it (an overflowing 2^t then ends at dtmax all the same).
+template <bool kThr = true>
 __device__ __forceinline__ float2 dt_transform2(const TArgs& a, float2 raw, float2 biasL) {
   float2 v;
   if (a.softplus) {
     const float2 t = __ffma2_rn(raw, f2(LOG2E), biasL);
     float2 s = lg2f2(__fadd2_rn(ex2f2(t), f2(1.f)));
-    s.x = t.x <= 20.f * LOG2E ? s.x : t.x;
-    s.y = t.y <= 20.f * LOG2E ? s.y : t.y;
+    if (kThr) {
+      s.x = t.x <= 20.f * LOG2E ? s.x : t.x;
+      s.y = t.y <= 20.f * LOG2E ? s.y : t.y;
+    }
     v = __fmul2_rn(s, f2(LN2));
   } else {
     v = __fadd2_rn(raw, biasL);
@@ -138,6 +143,11 @@ bool make_rows_tensor_map(const void* base, int64_t sb, int64_t sl, int64_t widt
 // the forward kernel's tensor maps (one kernel parameter)
 struct FwdMaps { CUtensorMap dt, B, C; };
 int state_slices(int dstate);
+// the fast forward walk over slices of nt states; streams with a block outside its range are marked in a.redo
+int launch_fwd_pipe(const TArgs& a, const issm_params& p, int nt, cudaStream_t s);
+// Tensor map over the rows of a (batch, seqlen, width) bf16 array, any batch and row pitch, with a 64 x 64 box in the 128-byte
+// swizzle of the operand tiles; rows past seqlen read as zero.  false if TMA does not take the strides
+bool make_tile_map(const void* base, int64_t sb, int64_t sl, int64_t width, int batch, int seqlen, CUtensorMap* out);
 int tensor_fwd_states_only(const issm_params& p, bf16* saved, int* redo, cudaStream_t s);
 size_t tensor_bwd_workspace_bytes(const issm_params& p);
 

@@ -1,0 +1,515 @@
+// Forward of the tcgen05 scan path, pipelined over the 64-point blocks of a stream.
+//
+// One CTA walks one (batch, head) stream (or one 256-state slice of it) as a warp-specialised pipeline, so that the
+// operand pass of block k + 1 runs beside the tensor-core and epilogue chain of block k:
+//   P   2 NT / 32 warps: dt transform, in-block decays, Cd = C 2^a and Bd = B dt 2^-a.  TMA has put the raw C and B rows into
+//       one of two operand sets and P scales them in place; dt comes straight from L2, a block ahead in registers
+//   svc one warp: TMA; M = Cd Bd^T, Y = Cd S, S += Bd^T x, then Y += tril(M) x
+//   E2  NT / 32 warps: S <- 2^a_last S in TMEM, bf16 copy as operand of the next block, saved and final states; then the output
+//       rows (D skip, gate) of the block before, coalesced
+//   E1  4 warps: masked M -> bf16 operand; Y rows -> shared memory
+//   X   3 warps: x operand tiles; announce dt, x, z rows to L2 two blocks ahead
+// The roles meet only at mbarriers (every wait bounded; a role whose wait expired keeps walking without waiting, so that
+// nobody is left behind).  What bounds it: the special-function unit in P - four results per (row, state), 4.1 k cycles of a
+// 64 x 256 block; the serial version of this kernel spent 10.9 k cycles per block with that unit idle 60 % of the time.
+#include "issm_tensor.cuh"
+
+#include <cstring>
+
+namespace issm {
+namespace {
+
+template <int NT>
+struct PipeSmem {
+  static constexpr int kHalf = NT * 128;                 // [NT/64 atoms][64 l][128 B]
+  static constexpr int kSet = 2 * kHalf;                 // Cd, then Bd: TMA puts the raw C and B rows here, P scales them in place
+  static constexpr int kS = 2 * kSet;                    // [NT n][128 B]: state rows, head dim contiguous
+  static constexpr int kX = kS + NT * 128;               // 2 x [64 l][128 B]
+  static constexpr int kMm = kX + 2 * QB * 128;          // [64 l][128 B]
+  static constexpr int kY = kMm + QB * 128;              // [64][PP] float
+  static constexpr int kXch = kY + QB * PP * 4;          // 2 x [4][NT] float: sums of dt*A over the quarters of a block
+  static constexpr int kLast = kXch + 2 * 4 * NT * 4;    // 4 x [NT] float: summed decay of a block
+  static constexpr int kBars = kLast + 4 * NT * 4;
+  static constexpr int kTotal = kBars + 192;
+};
+
+// mbarriers; where there are two of a kind (operand set or x tile, parity of the block) each completes once per two blocks: a
+// waiter that is late then still finds the phase it waits for, since the next one needs its own arrival
+enum { kRaw = 0, kFullP = 2, kFullX = 4, kDoneMY = 6, kDoneS = 8, kDoneB = 10, kReadyS = 12, kReadyM = 13, kYFull = 14, kYEmpty = 15, kNumBars = 17 };
+
+__device__ __forceinline__ void arrive(uint64_t* bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// one arrival per warp, after every lane's writes
+__device__ __forceinline__ void warp_arrive(uint64_t* bar, int lane) {
+  __syncwarp();
+  if (lane == 0) arrive(bar);
+}
+// bounded wait; once a role has failed it stops waiting and only keeps its barriers moving
+__device__ __forceinline__ void wait_or_fail(uint64_t* bar, uint32_t parity, bool& failed) {
+  if (!failed && !__all_sync(0xffffffffu, mbar_wait_suspended(bar, parity) ? 1 : 0)) failed = true;
+}
+
+// Rows keep their memory order inside a block also for a reversed scan (kRev): only the direction of the in-block sums and the
+// side of the mask change, so the tiles can be filled by TMA and scaled in place.
+template <int NT, typename TDT, bool kRev>
+__global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pipe(const __grid_constant__ TArgs a, const __grid_constant__ FwdMaps maps) {
+  using SM = PipeSmem<NT>;
+  constexpr int NP = NT / 16;                            // P warps
+  constexpr int NX = 3;                                  // X warps
+  constexpr int NE2 = NT / 32;                           // E2 warps: one per slab of 128 states and 32 lanes
+  constexpr int kRegP = NT == 256 ? 72 : 104, kRegE = NT == 256 ? 56 : 80;      // registers: 1024 x 64 = 512 x (72 + 56); 640 x 96 >= 256 x 104 + 384 x 80
+  constexpr int NPR = NT / 2;                            // state pairs
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* bars = (uint64_t*)(smem + SM::kBars);
+  uint32_t* tmem_holder = (uint32_t*)(bars + kNumBars);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int h = blockIdx.y, b = blockIdx.z, g = h / a.hpg;
+  const int n_off = blockIdx.x * NT;
+  const int stream = (blockIdx.x * a.b + b) * a.H + h;
+  const int nblk = (a.L + QB - 1) / QB;
+  const bf16* __restrict__ xp = a.x + b * a.x_sb + h * a.x_sh;
+
+  // memory row of a block's tile row 0 (negative in the short last block of a reversed scan, whose rows sit at the tile's end)
+  auto mrow0 = [&](int blk) { return kRev ? a.L - blk * QB - QB : blk * QB; };
+  auto inside = [](int r, int rows) { return kRev ? r >= QB - rows : r < rows; };
+  auto clampr = [](int r, int rows) { return kRev ? max(r, QB - rows) : min(r, rows - 1); };
+
+  for (int i = tid + SM::kS / 16; i < SM::kXch / 16; i += blockDim.x) ((uint4*)smem)[i] = make_uint4(0, 0, 0, 0);
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bars + kRaw + i, 1); mbar_init(bars + kFullP + i, NP); mbar_init(bars + kFullX + i, NX);
+      mbar_init(bars + kDoneMY + i, 1); mbar_init(bars + kDoneS + i, 1); mbar_init(bars + kDoneB + i, 1);
+      mbar_init(bars + kYEmpty + i, NE2);
+    }
+    mbar_init(bars + kReadyS, NE2); mbar_init(bars + kReadyM, 4); mbar_init(bars + kYFull, 4);
+    mbar_fence_init();
+  }
+  if (warp == 0) { tmem_alloc(tmem_holder, 512); tmem_relinquish(); }
+  fence_async_smem();
+  fence_before_sync();
+  __syncthreads();
+  fence_after_sync();
+  const uint32_t tmem = *tmem_holder;
+  const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
+  const uint32_t t_S = tmem + 256;                       // 2 slabs x PP columns; [M | Y] of block k at columns (k & 1) * 128
+  bool failed = false;
+  uint32_t unsafe = 0;
+
+  if (warp < NP) {
+    // ==================================================== P =====================================================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kRegP));
+    const int pr = tid % NPR, qr = tid / NPR;
+    const int hn = h * a.N + n_off + 2 * pr;
+    const float2 A2 = f2(__ldg(a.A + hn) * LOG2E, __ldg(a.A + hn + 1) * LOG2E);
+    const float bsc = a.softplus ? LOG2E : 1.f;
+    const float2 biasL = a.has_bias ? f2(__ldg(a.bias + hn) * bsc, __ldg(a.bias + hn + 1) * bsc) : f2(0.f);
+    const TDT* dtp = (const TDT*)a.dt + b * a.dt_sb + h * a.dt_sh + n_off + 2 * pr;
+    typedef typename std::conditional<sizeof(TDT) == 2, uint32_t, float2>::type Raw;
+    Raw raw[16];
+    const int r0 = qr * 16;                              // this thread's tile rows, visited in scan order: r0 + j or r0 + 15 - j
+    const int64_t dstep = kRev ? -a.dt_sl : a.dt_sl;
+    auto load_dt = [&](int blk, int j0, int j1) {
+      const int rows = min(QB, a.L - blk * QB);
+      if (rows == QB) {
+        const TDT* p = dtp + (int64_t)(mrow0(blk) + r0 + (kRev ? 15 : 0)) * a.dt_sl;
+#pragma unroll
+        for (int j = j0; j < j1; ++j) raw[j] = *(const Raw*)(p + j * dstep);
+      } else {                                           // rows outside the sequence repeat the nearest one inside
+        const TDT* p = dtp + (int64_t)mrow0(blk) * a.dt_sl;
+#pragma unroll
+        for (int j = j0; j < j1; ++j) raw[j] = *(const Raw*)(p + clampr(r0 + (kRev ? 15 - j : j), rows) * a.dt_sl);
+      }
+    };
+    const int at = pr >> 5, kc = (pr & 31) >> 2;         // 64-state atom, 16-byte chunk inside its 128-byte rows
+    const int iq = kRev ? 3 - qr : qr;                   // place of this quarter in scan order
+    const bool thr = !a.softplus || a.dtmax > 20.f;
+    load_dt(0, 0, 16);
+    for (int blk = 0; blk < nblk; ++blk) {
+      const int rows = min(QB, a.L - blk * QB), set = blk & 1;
+      float2 dtv[16], asum = f2(0.f);
+      auto unraw = [&](int j) {
+        if constexpr (sizeof(TDT) == 2) return unpack_bf16(raw[j]);
+        else return raw[j];
+      };
+      if (thr) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) dtv[j] = dt_transform2<true>(a, unraw(j), biasL);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) dtv[j] = dt_transform2<false>(a, unraw(j), biasL);
+      }
+      if (rows < QB) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j)
+          if (!inside(r0 + (kRev ? 15 - j : j), rows)) dtv[j] = f2(0.f);
+      }
+#pragma unroll
+      for (int j = 0; j < 16; ++j) asum = __ffma2_rn(dtv[j], A2, asum);
+      float* xch = (float*)(smem + SM::kXch) + set * (4 * NT);
+      *(float2*)(xch + qr * NT + 2 * pr) = asum;
+      named_barrier(1 + (warp % (NPR / 32)), 128);       // the four warps that share these 64 states
+      const float2 q0 = *(const float2*)(xch + 2 * pr), q1 = *(const float2*)(xch + NT + 2 * pr), q2 = *(const float2*)(xch + 2 * NT + 2 * pr),
+                   q3 = *(const float2*)(xch + 3 * NT + 2 * pr);
+      // running sums after each quarter in scan order: quarters 0, 1, .. or 3, 2, ..
+      const float2 c1 = kRev ? q3 : q0, c2 = __fadd2_rn(c1, kRev ? q2 : q1), c3 = __fadd2_rn(c2, kRev ? q1 : q2), c4 = __fadd2_rn(c3, kRev ? q0 : q3);
+      // range of the factorisation: 2^(+-a) must stay finite in bf16, every running sum within 2^120
+      const float worst = fmaxf(fmaxf(fmaxf(fabsf(c1.x), fabsf(c1.y)), fmaxf(fabsf(c2.x), fabsf(c2.y))),
+                                fmaxf(fmaxf(fabsf(c3.x), fabsf(c3.y)), fmaxf(fabsf(c4.x), fabsf(c4.y))));
+      if (!(worst <= 120.f)) unsafe = 1;
+      float2 acc = iq == 0 ? f2(0.f) : (iq == 1 ? c1 : (iq == 2 ? c2 : c3));
+      if (qr == 0) *(float2*)((float*)(smem + SM::kLast) + (blk & 3) * NT + 2 * pr) = c4;
+      wait_or_fail(bars + kRaw + set, (blk >> 1) & 1, failed);         // the raw C and B rows have landed
+      uint8_t* col = smem + set * SM::kSet + at * (QB * 128) + r0 * 128 + ((pr & 3) << 2);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const int r = kRev ? 15 - i : i;
+        uint32_t* cp = (uint32_t*)(col + (uint32_t)(r * 128 + ((kc ^ (r & 7)) << 4)));
+        uint32_t* bp = cp + SM::kHalf / 4;
+        acc = __ffma2_rn(dtv[i], A2, acc);
+        const float2 cd = __fmul2_rn(unpack_bf16(*cp), ex2f2(acc));
+        const float2 bd = __fmul2_rn(__fmul2_rn(unpack_bf16(*bp), dtv[i]), ex2f2_neg(acc));
+        *cp = pack_bf16(cd);
+        *bp = pack_bf16(bd);
+        if ((i & 3) == 3 && blk + 1 < nblk) load_dt(blk + 1, i - 3, i + 1);   // dt of the next block takes the place of this one's
+      }
+      if (rows < QB) {                                   // rows outside the sequence: zero
+#pragma unroll 1
+        for (int r = 0; r < 16; ++r)
+          if (!inside(r0 + r, rows)) {
+            uint32_t* cp = (uint32_t*)(col + (uint32_t)(r * 128 + ((kc ^ (r & 7)) << 4)));
+            cp[0] = 0;
+            cp[SM::kHalf / 4] = 0;
+          }
+      }
+      fence_async_smem();
+      warp_arrive(bars + kFullP + set, lane);
+    }
+  } else if (warp < NP + NE2) {
+    // ==================================================== E2 ====================================================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegE));
+    const int sl = (warp - NP) >> 2, n = sl * 128 + (warp & 3) * 32 + lane;      // this thread's state
+    bf16* savep = a.saved ? a.saved + (((size_t)b * a.H + h) * (nblk + 1)) * a.N * PP + (size_t)(n_off + n) * 8 : nullptr;
+    // 16 TMEM columns from c0: scaled by el and written back, bf16 copies to the operand tile and to the saved states of
+    // block blk, fp32 to the final states
+    auto pass = [&](int c0, float el, int blk, bool first) {
+      constexpr int CW = 16;
+      const uint32_t t = t_S + lane_base + sl * PP + c0;
+      float sc[CW];
+      if (first) {
+        const bf16* ip = a.init + (((size_t)b * a.H + h) * a.P) * a.N + n_off + n;
+#pragma unroll
+        for (int j = 0; j < CW; ++j) sc[j] = (a.has_init && c0 + j < a.P) ? __bfloat162float(ip[(size_t)(c0 + j) * a.N]) : 0.f;
+      } else {
+        tmem_ld16(t, sc);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < CW; ++j) sc[j] *= el;
+      }
+      tmem_st16(t, sc);
+#pragma unroll
+      for (int c = 0; c < CW / 8; ++c) {
+        const uint4 v = make_uint4(pack_bf16(sc[c * 8], sc[c * 8 + 1]), pack_bf16(sc[c * 8 + 2], sc[c * 8 + 3]),
+                                   pack_bf16(sc[c * 8 + 4], sc[c * 8 + 5]), pack_bf16(sc[c * 8 + 6], sc[c * 8 + 7]));
+        *(uint4*)(smem + SM::kS + sw128_chunk(n, c0 / 8 + c)) = v;
+        if (savep) *(uint4*)(savep + ((size_t)blk * PP + c0 + c * 8) * a.N) = v;
+      }
+      if (blk == nblk && a.want_final) {
+        float* fp = a.final_states + (((size_t)b * a.H + h) * a.P) * a.N + n_off + n;
+#pragma unroll
+        for (int j = 0; j < CW; ++j)
+          if (c0 + j < a.P) fp[(size_t)(c0 + j) * a.N] = sc[j];
+      }
+    };
+    // out = (y + D x) * silu(z) for the rows of a finished block, in groups of 4 consecutive head-dim elements (8-byte
+    // accesses; headdim % 4 == 0): group i of the [64][P / 4] grid
+    constexpr int NIO = NE2 * 32, KG = 3;                // threads, groups in flight
+    const int io_t = tid - NP * 32, ngrp = a.P / 4;
+    const int l0 = io_t / ngrp, g0 = io_t % ngrp, dl = NIO / ngrp, dg = NIO % ngrp;
+    const bf16* zp = a.has_z ? a.z + b * a.z_sb + h * a.z_sh : nullptr;
+    const float dscalar = (a.has_D && !a.D_has_hdim) ? __ldg(a.D + h) : 0.f;
+    auto bf_lo = [](uint32_t w) { return __uint_as_float(w << 16); };
+    auto bf_hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+    auto output = [&](int blk) {
+      const int rows = min(QB, a.L - blk * QB), m0 = mrow0(blk);
+      const uint8_t* xt = smem + SM::kX + (blk & 1) * (QB * 128);
+      int l = l0, gq = g0, lz = l0, gz = g0;
+      bool ready = false;
+#pragma unroll 1
+      for (int i = 0; i < QB * ngrp; i += KG * NIO) {
+        uint2 zv[KG];
+        if (zp) {
+#pragma unroll
+          for (int k = 0; k < KG; ++k) {
+            zv[k] = *(const uint2*)(zp + (int64_t)(m0 + clampr(min(lz, QB - 1), rows)) * a.z_sl + gz * 4);
+            lz += dl; gz += dg;
+            if (gz >= ngrp) { gz -= ngrp; ++lz; }
+          }
+        }
+        if (!ready) { wait_or_fail(bars + kYFull, blk & 1, failed); ready = true; }
+#pragma unroll
+        for (int k = 0; k < KG; ++k) {
+          if (l < QB && inside(l, rows)) {
+            const int q4 = gq * 4;
+            const float4 yv = *(const float4*)(smem + SM::kY + (l * PP + q4) * 4);
+            if (a.ypart) {                               // one slice of the states: the skip and the gate come after the sum
+              *(float4*)(a.ypart + ((((size_t)blockIdx.x * a.b + b) * a.L + m0 + l) * a.H + h) * a.P + q4) = yv;
+            } else {
+              const uint2 xv = *(const uint2*)(xt + sw128_off(l, q4));
+              float y[4] = {yv.x, yv.y, yv.z, yv.w};
+              const float xf[4] = {bf_lo(xv.x), bf_hi(xv.x), bf_lo(xv.y), bf_hi(xv.y)};
+#pragma unroll
+              for (int q = 0; q < 4; ++q) y[q] = fmaf(a.D_has_hdim ? __ldg(a.D + h * a.P + q4 + q) : dscalar, xf[q], y[q]);
+              const int64_t o = b * a.o_sb + (int64_t)(m0 + l) * a.o_sl + h * a.o_sh + q4;
+              if (zp) {
+                *(uint2*)(a.out_x + o) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
+                const float zf[4] = {bf_lo(zv[k].x), bf_hi(zv[k].x), bf_lo(zv[k].y), bf_hi(zv[k].y)};
+#pragma unroll
+                for (int q = 0; q < 4; ++q) y[q] *= __fdividef(zf[q], 1.f + ex2f(-zf[q] * LOG2E));
+              }
+              *(uint2*)(a.out + o) = make_uint2(pack_bf16(y[0], y[1]), pack_bf16(y[2], y[3]));
+            }
+          }
+          l += dl; gq += dg;
+          if (gq >= ngrp) { gq -= ngrp; ++l; }
+        }
+      }
+      warp_arrive(bars + kYEmpty + (blk & 1), lane);
+    };
+    auto publish = [&]() {
+      tmem_st_wait();
+      fence_async_smem();
+      fence_before_sync();
+      warp_arrive(bars + kReadyS, lane);
+    };
+#pragma unroll 1
+    for (int c0 = 0; c0 < PP; c0 += 16) pass(c0, 1.f, 0, true);
+    publish();
+    for (int blk = 0; blk < nblk; ++blk) {
+      wait_or_fail(bars + kDoneS + (blk & 1), (blk >> 1) & 1, failed);
+      fence_after_sync();
+      const float el = ex2f(((const float*)(smem + SM::kLast))[(blk & 3) * NT + n]);
+#pragma unroll 1
+      for (int c0 = 0; c0 < PP; c0 += 16) pass(c0, el, blk + 1, false);
+      publish();
+      if (blk > 0 && !a.no_output) output(blk - 1);      // while the MMAs of the next block run
+    }
+    if (!a.no_output) output(nblk - 1);
+  } else if (warp < NP + NE2 + 4) {
+    // ==================================================== E1 ====================================================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegE));
+    const int l = (warp & 3) * 16 + lane;                // row of this lane (lanes 0..15: a 64-row accumulator)
+    if (!a.no_output)
+      for (int blk = 0; blk < nblk; ++blk) {
+        const uint32_t t = tmem + (blk & 1) * 128 + lane_base, par = (blk >> 1) & 1;
+        wait_or_fail(bars + kDoneMY + (blk & 1), par, failed);
+        fence_after_sync();
+#pragma unroll 1
+        for (int c16 = 0; c16 < 4; ++c16) {
+          float mv[16];
+          tmem_ld16(t + c16 * 16, mv);
+          tmem_ld_wait();
+          if (lane < 16) {
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+              uint32_t pk[4];
+#pragma unroll
+              for (int j = 0; j < 8; j += 2) {
+                const int s = c16 * 16 + c * 8 + j;
+                pk[j >> 1] = pack_bf16((kRev ? s >= l : s <= l) ? mv[c * 8 + j] : 0.f, (kRev ? s + 1 >= l : s + 1 <= l) ? mv[c * 8 + j + 1] : 0.f);
+              }
+              *(uint4*)(smem + SM::kMm + sw128_chunk(l, c16 * 2 + c)) = make_uint4(pk[0], pk[1], pk[2], pk[3]);
+            }
+          }
+        }
+        fence_async_smem();
+        fence_before_sync();
+        warp_arrive(bars + kReadyM, lane);
+        if (blk > 0) wait_or_fail(bars + kYEmpty + ((blk - 1) & 1), ((blk - 1) >> 1) & 1, failed);
+        wait_or_fail(bars + kDoneB + (blk & 1), par, failed);
+        fence_after_sync();
+#pragma unroll 1
+        for (int c16 = 0; c16 < PP / 16; ++c16) {
+          float yv[16];
+          tmem_ld16(t + 64 + c16 * 16, yv);
+          tmem_ld_wait();
+          if (lane < 16) {
+            float4* dst = (float4*)(smem + SM::kY + (l * PP + c16 * 16) * 4);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) dst[c] = make_float4(yv[c * 4], yv[c * 4 + 1], yv[c * 4 + 2], yv[c * 4 + 3]);
+          }
+        }
+        fence_before_sync();
+        warp_arrive(bars + kYFull, lane);
+      }
+  } else if (warp < NP + NE2 + 4 + NX) {
+    // ==================================================== X =====================================================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegE));
+    // x rows -> operand tile, in groups of 4 consecutive head-dim elements (8-byte accesses; headdim % 4 == 0)
+    constexpr int KG = 7, NXT = NX * 32;                 // groups in flight, threads
+    // dt (128-byte lines), x and z rows of a block to L2
+    auto announce = [&](int blk) {
+      if (blk >= nblk) return;
+      const int rows = min(QB, a.L - blk * QB), m0 = mrow0(blk);
+      constexpr int kLines = NT * (int)sizeof(TDT) / 128;
+      for (int i = tid - (NP + NE2 + 4) * 32; i < QB * kLines; i += NXT) {
+        const int l = i / kLines;
+        if (inside(l, rows))
+          asm volatile("prefetch.global.L2 [%0];" ::"l"((const char*)((const TDT*)a.dt + b * a.dt_sb + h * a.dt_sh + n_off + (int64_t)(m0 + l) * a.dt_sl) + (i % kLines) * 128));
+      }
+      for (int l = tid - (NP + NE2 + 4) * 32; l < QB; l += NXT) {
+        if (!inside(l, rows)) continue;
+        const char* q = (const char*)(xp + (int64_t)(m0 + l) * a.x_sl);
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(q + a.P * 2 - 1));
+        if (a.has_z && !a.no_output) {
+          const char* z = (const char*)(a.z + b * a.z_sb + h * a.z_sh + (int64_t)(m0 + l) * a.z_sl);
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(z));
+          asm volatile("prefetch.global.L2 [%0];" ::"l"(z + a.P * 2 - 1));
+        }
+      }
+    };
+    announce(1);
+    const int x_t = tid - (NP + NE2 + 4) * 32, ngrp = a.P / 4, l0 = x_t / ngrp, g0 = x_t % ngrp, dl = NXT / ngrp, dg = NXT % ngrp;
+    for (int blk = 0; blk < nblk; ++blk) {
+      const int rows = min(QB, a.L - blk * QB);
+      announce(blk + 2);
+      const bf16* p = xp + (int64_t)mrow0(blk) * a.x_sl;
+      uint8_t* tile = smem + SM::kX + (blk & 1) * (QB * 128);
+      int l = l0, gq = g0, ls = l0, gs = g0;
+      bool ready = blk < 2;
+#pragma unroll 1
+      for (int i = 0; i < QB * ngrp; i += KG * NXT) {
+        uint2 v[KG];
+#pragma unroll
+        for (int k = 0; k < KG; ++k) {
+          v[k] = *(const uint2*)(p + (int64_t)clampr(min(l, QB - 1), rows) * a.x_sl + gq * 4);
+          l += dl; gq += dg;
+          if (gq >= ngrp) { gq -= ngrp; ++l; }
+        }
+        if (!ready) {                                    // block blk - 2: its MMAs and its output rows have read this tile
+          ready = true;
+          wait_or_fail(bars + kDoneB + (blk & 1), ((blk >> 1) - 1) & 1, failed);
+          if (!a.no_output) wait_or_fail(bars + kYEmpty + (blk & 1), ((blk >> 1) - 1) & 1, failed);
+        }
+#pragma unroll
+        for (int k = 0; k < KG; ++k) {
+          if (ls < QB) *(uint2*)(tile + sw128_off(ls, gs * 4)) = inside(ls, rows) ? v[k] : make_uint2(0, 0);
+          ls += dl; gs += dg;
+          if (gs >= ngrp) { gs -= ngrp; ++ls; }
+        }
+      }
+      fence_async_smem();
+      warp_arrive(bars + kFullX + (blk & 1), lane);
+    }
+  } else {
+    // =================================================== service =================================================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegE));
+    const uint32_t sb = smem_u32(smem);
+    const uint64_t dK = desc_sw128(sb), dMN = desc_sw128_mn(sb, QB * 128);
+    // raw C and B rows of a block into its operand set, one TMA tile per 64 states
+    auto fill = [&](int blk) {
+      if (blk >= nblk || lane != 0) return;
+      uint64_t* bar = bars + kRaw + (blk & 1);
+      uint8_t* dst = smem + (blk & 1) * SM::kSet;
+      mbar_expect_tx(bar, SM::kSet);
+#pragma unroll
+      for (int at = 0; at < NT / 64; ++at) {
+        tma_load_3d(dst + at * (QB * 128), &maps.C, g * (int)a.C_sg + n_off + at * 64, mrow0(blk), b, bar);
+        tma_load_3d(dst + SM::kHalf + at * (QB * 128), &maps.B, g * (int)a.B_sg + n_off + at * 64, mrow0(blk), b, bar);
+      }
+    };
+    fill(0);
+    fill(1);
+    for (int blk = 0; blk < nblk; ++blk) {
+      const int set = blk & 1;
+      const uint32_t par = (blk >> 1) & 1, oC = set * SM::kSet, oB = oC + SM::kHalf, oX = SM::kX + set * (QB * 128);
+      wait_or_fail(bars + kFullP + set, par, failed);
+      wait_or_fail(bars + kReadyS, blk & 1, failed);
+      fence_after_sync();
+      if (lane == 0 && !a.no_output) {
+#pragma unroll
+        for (int at = 0; at < NT / 64; ++at)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)                 // M = Cd Bd^T
+            mma_bf16_off(tmem + set * 128, dK, oC + at * (QB * 128) + kk * 32, dK, oB + at * (QB * 128) + kk * 32, idesc_bf16(64, 64), (at | kk) != 0);
+        mma_commit(bars + kDoneMY + set);
+#pragma unroll
+        for (int at = 0; at < NT / 64; ++at)
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)                 // Y = Cd S
+            mma_bf16_off(tmem + set * 128 + 64, dK, oC + at * (QB * 128) + kk * 32, dMN, SM::kS + (at * 4 + kk) * 2048, idesc_bf16(64, PP, 0, 1), (at | kk) != 0);
+      }
+      wait_or_fail(bars + kFullX + set, par, failed);
+      if (lane == 0) {
+#pragma unroll
+        for (int sl = 0; sl < NT / 128; ++sl)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {                  // S += Bd^T x, rows in scan order (a reversed scan equals the flipped one)
+            const int kk = kRev ? 3 - k : k;
+            mma_bf16_off(t_S + sl * PP, dMN, oB + sl * (2 * QB * 128) + kk * 2048, dMN, oX + kk * 2048, idesc_bf16(128, PP, 1, 1), 1);
+          }
+        mma_commit(bars + kDoneS + set);
+      }
+      __syncwarp();
+      if (!a.no_output) wait_or_fail(bars + kReadyM, blk & 1, failed);
+      fence_after_sync();
+      if (lane == 0) {
+        if (!a.no_output) {
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {                  // Y += tril(M) x
+            const int kk = kRev ? 3 - k : k;
+            mma_bf16_off(tmem + set * 128 + 64, dK, SM::kMm + kk * 32, dMN, oX + kk * 2048, idesc_bf16(64, PP, 0, 1), 1);
+          }
+        }
+        mma_commit(bars + kDoneB + set);
+      }
+      __syncwarp();
+      if (blk + 2 < nblk) {
+        wait_or_fail(bars + kDoneS + set, par, failed);  // the set has been read
+        fill(blk + 2);
+      }
+      __syncwarp();
+    }
+    wait_or_fail(bars + kDoneB + ((nblk - 1) & 1), ((nblk - 1) >> 1) & 1, failed);       // no MMA in flight when TMEM is freed
+  }
+  const int votes = __syncthreads_or((int)unsafe | (failed ? 2 : 0));
+  if (tid == 0) {
+    a.redo[stream] = votes & 1;
+    if (a.status && (votes & 2)) atomicOr(a.status, 1);
+  }
+  fence_before_sync();
+  __syncthreads();
+  if (warp == 0) tmem_dealloc(tmem, 512);
+}
+
+template <int NT, typename TDT, bool kRev>
+int launch(const TArgs& a, const FwdMaps& maps, cudaStream_t s) {
+  const size_t smem = PipeSmem<NT>::kTotal + 1024;
+  struct Tag {};
+  if (SmemAttrOnce<Tag>::set(k_fwd_pipe<NT, TDT, kRev>, smem) != ISSM_OK) return ISSM_ERR_CUDA;
+  ISSM_LAUNCH((k_fwd_pipe<NT, TDT, kRev>), dim3(a.N / NT, a.H, a.b), 2 * NT + (NT == 256 ? 512 : 384), smem, s, a, maps);
+  return ISSM_OK;
+}
+template <int NT>
+int launch_nt(const TArgs& a, const FwdMaps& maps, cudaStream_t s) {
+  if (a.dt_f32) return a.rev ? launch<NT, float, true>(a, maps, s) : launch<NT, float, false>(a, maps, s);
+  return a.rev ? launch<NT, bf16, true>(a, maps, s) : launch<NT, bf16, false>(a, maps, s);
+}
+}  // namespace
+
+// the fast forward walk; streams with a block outside its range are marked in a.redo.  Where B or C has no tensor map (strides
+// that TMA does not take) every stream is marked, which leaves it to the windowed kernel
+int launch_fwd_pipe(const TArgs& a, const issm_params& p, int nt, cudaStream_t s) {
+  FwdMaps maps;
+  memset(&maps, 0, sizeof(maps));
+  if (!make_tile_map(p.B, p.B_sb, p.B_sl, (int64_t)(p.ngroups - 1) * p.B_sg + p.dstate, p.batch, p.seqlen, &maps.B) ||
+      !make_tile_map(p.C, p.C_sb, p.C_sl, (int64_t)(p.ngroups - 1) * p.C_sg + p.dstate, p.batch, p.seqlen, &maps.C)) {
+    const size_t n = (size_t)(a.N / nt) * a.b * a.H * sizeof(int);
+    return cudaMemsetAsync(a.redo, 1, n, s) == cudaSuccess ? ISSM_OK : ISSM_ERR_CUDA;
+  }
+  return nt == 256 ? launch_nt<256>(a, maps, s) : launch_nt<128>(a, maps, s);
+}
+
+}  // namespace issm

@@ -156,6 +156,18 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, uint32
   }
   return false;
 }
+// Waits of warps that idle beside working ones: the hardware suspends the warp (up to 20 us per poll) instead of letting it spin
+// through issue slots; about a second in all.
+__device__ __forceinline__ bool mbar_wait_suspended(uint64_t* bar, uint32_t parity, uint32_t limit = 1u << 16) {
+  for (uint32_t i = 0; i < limit; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok) : "r"(smem_u32(bar)), "r"(parity), "r"(20000u) : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
 // Same wait with a warp-uniform verdict (every lane of a full warp must call it): the warp-collective
 // tcgen05.ld / tcgen05.st that follow a wait may only run under a condition all 32 lanes agree on.
 __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t limit = 1u << 22) {
@@ -174,6 +186,12 @@ __device__ __forceinline__ void bulk_g2s(void* dst_smem, const void* src_gmem, u
 __device__ __forceinline__ void tma_load_2d(void* dst_smem, const void* tmap, int c0, int c1, uint64_t* bar) {
   asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
                ::"r"(smem_u32(dst_smem)), "l"(tmap), "r"(c0), "r"(c1), "r"(smem_u32(bar)) : "memory");
+}
+
+// 3-D form: c0 innermost in elements (16-byte granules), c1, c2
+__device__ __forceinline__ void tma_load_3d(void* dst_smem, const void* tmap, int c0, int c1, int c2, uint64_t* bar) {
+  asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+               ::"r"(smem_u32(dst_smem)), "l"(tmap), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar)) : "memory");
 }
 
 // bring the 32-byte sectors of [p, p + bytes) into L2 (no register result, nothing to wait for)

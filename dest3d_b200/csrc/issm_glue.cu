@@ -11,9 +11,12 @@
 // fixed order.
 #include "issm_common.cuh"
 
+#include <type_traits>
+
 namespace issm {
 
 constexpr int GLUE_MAX_ROWS = 16;
+constexpr int GLUE_FWD_BLOCKS = 148 * 16;
 
 struct GlueArgs {
   int L, K, H, G, back, RW, RO;                            // RW = H + 2G weight rows; RO = H + 2G (+ 2G) output rows
@@ -92,297 +95,310 @@ __device__ __forceinline__ float glue_softplus(float v) {
 // reading four weights per shared-memory access
 // TD: element type of dist (and ddist), T: of dt / bc and their gradients (float dist with bfloat16 outputs is what
 // autocast hands the block: the features stay float32, the activations are bfloat16)
+// Weights wait in shared memory as pairs (w, w): a 128-bit access gives two packed operands, where the scalar form cost a move
+// per multiply-add.  Blocks walk the points with a grid stride, so the weights are laid out once per block and not per point.
+// 16 x 4096 points x 256 states x 16 features bf16: 312 us before.
+template <int M>
+__device__ __forceinline__ void weights_to_smem(const GlueArgs& a, float2* sw) {
+  for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) { const float w = a.w[i]; sw[i] = make_float2(w, w); }
+}
+template <int M>
+__device__ __forceinline__ float2 row_dot(const float2* w, const float2 (&dp)[M], float2 pre) {
+#pragma unroll
+  for (int c = 0; c < M; c += 2) {
+    const float4 q = *(const float4*)(w + c);
+    pre = __ffma2_rn(dp[c], make_float2(q.x, q.y), pre);
+    pre = __ffma2_rn(dp[c + 1], make_float2(q.z, q.w), pre);
+  }
+  return pre;
+}
 template <typename TD, typename T, int M>
-__global__ void __launch_bounds__(128) k_glue_fwd(GlueArgs a) {
-  __shared__ __align__(16) float sw[GLUE_MAX_ROWS * M];
-  __shared__ float stok[GLUE_MAX_ROWS + 8];
-  const int l = blockIdx.x, b = blockIdx.y;
-  for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) sw[i] = a.w[i];
-  for (int i = threadIdx.x; i < a.RO; i += blockDim.x) stok[i] = a.tok[((int64_t)b * a.L + l) * a.RO + i];
+__global__ void __launch_bounds__(128) k_glue_fwd(GlueArgs a, int npoints) {
+  __shared__ __align__(16) float2 sw[GLUE_MAX_ROWS * M];
+  weights_to_smem<M>(a, sw);
   __syncthreads();
-  const TD* drow = (const TD*)a.dist + b * a.d_sb + l * a.d_sl;
-  const int64_t row = (int64_t)b * a.L + l;
-  T* dt = (T*)a.dt + row * a.H * a.K;
-  T* bc = (T*)a.bc + row * (a.RO - a.H) * a.K;
   const bool pair_store = !(a.K & 1);                      // rows of an even number of states keep pairs aligned
-  for (int k = 2 * threadIdx.x; k < a.K; k += 2 * blockDim.x) {
+  auto put = [&](T* p, float2 v, bool two) {
+    if (pair_store) {
+      if constexpr (sizeof(T) == 2) *(__nv_bfloat162*)p = __float22bfloat162_rn(v);
+      else *(float2*)p = v;
+    } else {
+      stf(p, v.x);
+      if (two) stf(p + 1, v.y);
+    }
+  };
+  const int half = (a.K + 1) / 2, items = npoints * half;
+  // item = (point, pair of states); consecutive threads take consecutive pairs
+  for (int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; item < items; item += (int64_t)gridDim.x * blockDim.x) {
+    const int row = (int)(item / half), k = 2 * (int)(item - (int64_t)row * half), b = row / a.L, l = row - b * a.L;
+    const TD* drow = (const TD*)a.dist + b * a.d_sb + l * a.d_sl;
+    const float* tok = a.tok + (int64_t)row * a.RO;
+    T* dt = (T*)a.dt + (int64_t)row * a.H * a.K + k;
+    T* bc = (T*)a.bc + (int64_t)row * (a.RO - a.H) * a.K + k;
     const bool two = k + 1 < a.K;
     float d0[M], d1[M];
     load_feats<TD, M>(drow + (int64_t)k * a.d_sk, d0);
     load_feats<TD, M>(drow + (int64_t)(two ? k + 1 : k) * a.d_sk, d1);
+    float2 mk = make_float2(1.f, 1.f);
+    if (a.mask) mk = make_float2(a.mask[(int64_t)row * a.K + k], a.mask[(int64_t)row * a.K + (two ? k + 1 : k)]);
     float2 dp[M];
 #pragma unroll
     for (int j = 0; j < M; ++j) dp[j] = make_float2(d0[j], d1[j]);
-    float2 mk = make_float2(1.f, 1.f);
-    if (a.mask) mk = make_float2(a.mask[row * a.K + k], a.mask[row * a.K + (two ? k + 1 : k)]);
-    auto put = [&](T* p, float2 v) {
-      if (pair_store) {
-        if constexpr (sizeof(T) == 2) *(__nv_bfloat162*)p = __float22bfloat162_rn(v);
-        else *(float2*)p = v;
-      } else {
-        stf(p, v.x);
-        if (two) stf(p + 1, v.y);
-      }
-    };
-    for (int r = 0; r < a.RW; ++r) {
-      float2 pre = make_float2(stok[r], stok[r]);
-#pragma unroll
-      for (int c = 0; c < M / 4; ++c) {
-        const float4 w4 = *(const float4*)&sw[r * M + c * 4];
-        pre = __ffma2_rn(dp[c * 4], make_float2(w4.x, w4.x), pre);
-        pre = __ffma2_rn(dp[c * 4 + 1], make_float2(w4.y, w4.y), pre);
-        pre = __ffma2_rn(dp[c * 4 + 2], make_float2(w4.z, w4.z), pre);
-        pre = __ffma2_rn(dp[c * 4 + 3], make_float2(w4.w, w4.w), pre);
-      }
-      if (r < a.H) {
-        put(dt + (int64_t)r * a.K + k, __fmul2_rn(make_float2(glue_softplus(pre.x), glue_softplus(pre.y)), mk));
-      } else {
-        put(bc + (int64_t)(r - a.H) * a.K + k, pre);
-        if (a.back) {
-          const float dlt = stok[r + 2 * a.G] - stok[r];
-          put(bc + (int64_t)(r - a.H + 2 * a.G) * a.K + k, __fadd2_rn(pre, make_float2(dlt, dlt)));
-        }
+#pragma unroll 2
+    for (int r = 0; r < a.H; ++r) {
+      const float t = __ldg(tok + r);
+      const float2 pre = row_dot<M>(sw + r * M, dp, make_float2(t, t));
+      put(dt + (int64_t)r * a.K, __fmul2_rn(make_float2(glue_softplus(pre.x), glue_softplus(pre.y)), mk), two);
+    }
+#pragma unroll 2
+    for (int r = a.H; r < a.RW; ++r) {
+      const float2 pre = row_dot<M>(sw + r * M, dp, make_float2(0.f, 0.f));
+      const float t = __ldg(tok + r);
+      put(bc + (int64_t)(r - a.H) * a.K, __fadd2_rn(pre, make_float2(t, t)), two);
+      if (a.back) {
+        const float u = __ldg(tok + r + 2 * a.G);
+        put(bc + (int64_t)(r - a.H + 2 * a.G) * a.K, __fadd2_rn(pre, make_float2(u, u)), two);
       }
     }
   }
 }
 
-constexpr int GLUE_KT = 256;                               // states per shared-memory tile of the weight-gradient product
-constexpr int GLUE_BWD_BLOCKS = 148 * 8;
+constexpr int GLUE_BWD_WARPS = 4;
+constexpr int GLUE_BWD_BLOCKS = 148 * 3;                   // two (16 features) or three blocks of four warps per SM: registers
 
-__device__ __forceinline__ void cp_async(void* smem_dst, const void* gsrc, int bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(smem_dst);
-  if (bytes == 16) asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(d), "l"(gsrc) : "memory");
-  else if (bytes == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(gsrc) : "memory");
-  else asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(gsrc) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
-
-// One stage of the backward's input pipeline: everything a (point, tile of 256 states) needs, as raw bytes.  The
-// number of gradient rows is the call's (RO), so the layout is computed at run time.
-template <typename TD, typename T, int M>
-struct GlueStage {
-  unsigned char* base;
-  int ro;
-  __host__ __device__ static size_t bytes(int ro) {
-    return ((size_t)GLUE_KT * M * sizeof(TD) + (size_t)ro * GLUE_KT * sizeof(T) + GLUE_KT * 4 + (GLUE_MAX_ROWS + 8) * 4 + 15) / 16 * 16;
-  }
-  __device__ TD* dist(int kk) const { return (TD*)base + (size_t)kk * M; }                       // [GLUE_KT][M]
-  __device__ T* grad(int r) const { return (T*)(base + (size_t)GLUE_KT * M * sizeof(TD)) + (size_t)r * GLUE_KT; }   // ddt rows, then the B / C rows
-  __device__ float* mask() const { return (float*)(base + (size_t)GLUE_KT * (M * sizeof(TD) + ro * sizeof(T))); }
-  __device__ float* tok() const { return mask() + GLUE_KT; }
-};
-
-// A block walks (point, tile of 256 states) items with a grid stride over the points, two items in flight: the
-// inputs of the next item are copied into shared memory (cp.async) while the current one is computed.  Per item:
-// (1) a thread takes two adjacent states: g, ddist, token sums; g and the features are parked in shared memory;
-// (2) thread (row r, four features, a range of the tile's states) adds sum_k g[r, k] dist[k, j] to its accumulators of
-// the weight gradient.  The accumulators go out once per block and are summed in a fixed order.
-template <typename TD, typename T, int M>
-__global__ void __launch_bounds__(128) k_glue_bwd(GlueArgs a, int npoints, int vec_ok) {
-  extern __shared__ __align__(16) unsigned char glue_dyn[];
-  const size_t stage_bytes = GlueStage<TD, T, M>::bytes(a.RO);
-  auto stage_of = [&](int it) { return GlueStage<TD, T, M>{glue_dyn + (it & 1) * stage_bytes, a.RO}; };
-  __shared__ __align__(16) float sw[GLUE_MAX_ROWS * M];
-  __shared__ float sred[4][GLUE_MAX_ROWS + 8];
-  __shared__ __align__(16) float sg[GLUE_MAX_ROWS][GLUE_KT + 4];   // g of the tile, read four states at a time
-  // float copy of the tile's features for the weight gradient (rows 16 bytes apart from a power of two: 128-bit accesses
-  // without conflicts); float features are read from the stage itself
-  constexpr bool kCopy = sizeof(TD) != 4;
-  __shared__ __align__(16) float sd[kCopy ? GLUE_KT : 1][M + 4];
+// Backward: a warp takes whole points and walks their states 64 at a time, two adjacent states per lane; it shares nothing with
+// the other warps of the block but the weights, so there is no block barrier in the walk.  Per 64 states:
+//  (1) g = d out / d pre per row and ddist = sum_r g[r] W[r, :] with packed pairs; the inputs of the next 64 states are loaded
+//      (packed, in registers) before the current ones are worked on;
+//  (2) g and the features go through the warp's part of shared memory for the weight gradient sum_k g[r, k] dist[k, j]: a lane
+//      owns NR / 2 rows x M / 2 features of it and every eighth state - 48 multiply-adds for four shared-memory reads at
+//      10 rows x 16 features - in registers over the whole walk.
+// Bound: the fp32 pipe (450 multiply-adds per (point, state)); the block-wide version with staged inputs held 12 warps per SM
+// that met at three barriers per point and used a fifth of the issue slots: 16 x 4096 x 256 x 16 bf16 1730 us.
+// NR: weight rows padded to 12 or 16.
+template <typename TD, typename T, int M, int NR>
+__global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_bwd(GlueArgs a, int npoints, int pairs_ok) {
+  constexpr int RH = NR / 2, MH = M / 2, GS = NR, DS = M + 4;      // rows / features of a lane's tile; row strides in shared memory
+  __shared__ __align__(16) float2 sw[NR * M];
+  __shared__ __align__(16) float sg_all[GLUE_BWD_WARPS][64 * GS];
+  __shared__ __align__(16) float sd_all[GLUE_BWD_WARPS][64 * DS];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) sw[i] = a.w[i];
-  // weight gradient: thread = (row r, four features 4 jq .. 4 jq + 3, one of NKG ranges of the tile's states)
-  constexpr int JQ = M / 4;
-  const int tiles = a.RW * JQ, NKG = 128 / tiles > 0 ? 128 / tiles : 1;
-  const int tile = threadIdx.x % tiles, kg = threadIdx.x / tiles;
-  const int wr = tile / JQ, wj = (tile % JQ) * 4;
-  const int kspan = ((GLUE_KT + NKG - 1) / NKG + 3) & ~3;  // a multiple of four states
-  float wacc[4] = {0.f, 0.f, 0.f, 0.f};
-  const int ntile = (a.K + GLUE_KT - 1) / GLUE_KT;
-  const int my_points = blockIdx.x < npoints ? (npoints - blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-  const int nitems = my_points * ntile;
-
-  // copies of item `it` into stage `st`.  vec_ok: every row of states starts on a 16-byte boundary, so the gradient rows
-  // and the mask go in 16-byte pieces; otherwise element by element through registers.
-  auto issue = [&](int it, const GlueStage<TD, T, M>& st) {
-    const int pt = blockIdx.x + (it / ntile) * gridDim.x, k0 = (it % ntile) * GLUE_KT;
-    const int b = pt / a.L, l = pt - b * a.L;
-    const int nk = min(GLUE_KT, a.K - k0);
-    const TD* drow = (const TD*)a.dist + b * a.d_sb + l * a.d_sl + (int64_t)k0 * a.d_sk;
-    constexpr int RB = M * (int)sizeof(TD), CS = RB >= 16 ? 16 : RB, CH = RB / CS;     // bytes per state, per piece, pieces per state
-    for (int c = threadIdx.x; c < nk * CH; c += blockDim.x) {
-      const int kk = c / CH, part = c % CH;
-      cp_async((char*)st.dist(kk) + part * CS, (const char*)(drow + (int64_t)kk * a.d_sk) + part * CS, CS);
-    }
-    const int nrow = a.RO;
-    const T* ddt = a.ddt ? (const T*)a.ddt + (int64_t)pt * a.H * a.K + k0 : nullptr;
-    const T* dbc = a.dbc ? (const T*)a.dbc + (int64_t)pt * (a.RO - a.H) * a.K + k0 : nullptr;
-    constexpr int EPC = 16 / (int)sizeof(T);               // elements per 16-byte piece
-    if (vec_ok) {
-      const int pieces = nk / EPC;                         // K is a multiple of EPC here
-      for (int c = threadIdx.x; c < nrow * pieces; c += blockDim.x) {
-        const int ro = c / pieces, q = c % pieces;
-        const T* src = ro < a.H ? (ddt ? ddt + (int64_t)ro * a.K : nullptr) : (dbc ? dbc + (int64_t)(ro - a.H) * a.K : nullptr);
-        if (src) cp_async(st.grad(ro) + q * EPC, src + q * EPC, 16);
-      }
-      if (a.mask)
-        for (int c = threadIdx.x; c < nk / 4; c += blockDim.x) cp_async(st.mask() + c * 4, a.mask + (int64_t)pt * a.K + k0 + c * 4, 16);
-    } else {
-      for (int c = threadIdx.x; c < nrow * nk; c += blockDim.x) {
-        const int ro = c / nk, kk = c % nk;
-        const T* src = ro < a.H ? (ddt ? ddt + (int64_t)ro * a.K : nullptr) : (dbc ? dbc + (int64_t)(ro - a.H) * a.K : nullptr);
-        if (src) st.grad(ro)[kk] = src[kk];
-      }
-      if (a.mask)
-        for (int c = threadIdx.x; c < nk; c += blockDim.x) st.mask()[c] = a.mask[(int64_t)pt * a.K + k0 + c];
-    }
-    for (int i = threadIdx.x; i < a.RO; i += blockDim.x) cp_async(st.tok() + i, a.tok + (int64_t)pt * a.RO + i, 4);
-    cp_async_commit();
+  float* sg = sg_all[warp];
+  float* sd = sd_all[warp];
+  for (int i = threadIdx.x; i < NR * M; i += blockDim.x) { const float w = i < a.RW * M ? a.w[i] : 0.f; sw[i] = make_float2(w, w); }
+  for (int i = lane; i < 64 * GS; i += 32) sg[i] = 0.f;
+  __syncthreads();
+  const int rh = lane & 1, jh = (lane >> 1) & 1, kq = lane >> 2;   // the lane's tile and its share of the states
+  float2 acc[RH][MH / 2];
+#pragma unroll
+  for (int r = 0; r < RH; ++r)
+#pragma unroll
+    for (int j = 0; j < MH / 2; ++j) acc[r][j] = make_float2(0.f, 0.f);
+  constexpr int FW = M * (int)sizeof(TD) / 8;              // 8-byte words of one state's features
+  typedef typename std::conditional<sizeof(T) == 2, uint32_t, float2>::type GP;      // a pair of gradients as loaded
+  auto up = [](GP v) {
+    if constexpr (sizeof(T) == 2) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
+    else return v;
   };
-
-  float tsum[GLUE_MAX_ROWS + 8];                            // per output row: sum over this thread's states of the point
+  const int per = gridDim.x * GLUE_BWD_WARPS, first = blockIdx.x * GLUE_BWD_WARPS + warp;
+  const int nstep = (a.K + 63) / 64, nb = a.RO - a.H;      // steps per point; B / C gradient rows
+  uint2 fx[2][FW];
+  GP gh[8];                                  // dt gradient rows, loaded eight at a time
+  float2 mk;
+  auto pair_at = [&](const T* p, bool in0, bool in1) {
+    GP v;
+    if constexpr (sizeof(T) == 2) {
+      if (pairs_ok) v = in0 ? *(const uint32_t*)p : 0u;
+      else v = (in0 ? (uint32_t)*(const uint16_t*)p : 0u) | (in1 ? (uint32_t)*((const uint16_t*)p + 1) << 16 : 0u);
+    } else {
+      if (pairs_ok) v = in0 ? *(const float2*)p : make_float2(0.f, 0.f);
+      else v = make_float2(in0 ? p[0] : 0.f, in1 ? p[1] : 0.f);
+    }
+    return v;
+  };
+  auto load = [&](int pt, int step) {                      // features, mask and the first eight dt gradient rows of 64 states
+    const int k = step * 64 + 2 * lane;
+    const bool in0 = k < a.K, in1 = k + 1 < a.K;
+    const int b = pt / a.L, l = pt - b * a.L;
+    const TD* d = (const TD*)a.dist + b * a.d_sb + l * a.d_sl;
 #pragma unroll
-  for (int r = 0; r < GLUE_MAX_ROWS + 8; ++r) tsum[r] = 0.f;
-  if (nitems > 0) issue(0, stage_of(0));
-  for (int it = 0; it < nitems; ++it) {
-    const GlueStage<TD, T, M> st = stage_of(it);
-    if (it + 1 < nitems) { issue(it + 1, stage_of(it + 1)); cp_async_wait<1>(); }
-    else cp_async_wait<0>();
-    __syncthreads();                                       // this item's inputs are in shared memory
-    const int pt = blockIdx.x + (it / ntile) * gridDim.x, k0 = (it % ntile) * GLUE_KT;
-    const int64_t row = pt;
-    TD* ddist = (TD*)a.ddist + row * a.K * M;
-    {                                                      // two adjacent states per thread: 128 threads cover the tile
-      const int kk = 2 * threadIdx.x, k = k0 + kk;
-      const bool in0 = k < a.K, in1 = k + 1 < a.K;
-      float d0[M], d1[M];
+    for (int s2 = 0; s2 < 2; ++s2) {
+      const bool in = s2 ? in1 : in0;
+      const uint2* p = (const uint2*)(d + (int64_t)(k + s2) * a.d_sk);
+      if constexpr (FW % 2 == 0) {
 #pragma unroll
-      for (int j = 0; j < M; ++j) { d0[j] = 0.f; d1[j] = 0.f; }
-      if (in0) load_feats<TD, M>(st.dist(kk), d0);
-      if (in1) load_feats<TD, M>(st.dist(kk + 1), d1);
-      float2 dp[M], dd[M];
-#pragma unroll
-      for (int j = 0; j < M; ++j) { dp[j] = make_float2(d0[j], d1[j]); dd[j] = make_float2(0.f, 0.f); }
-      if constexpr (kCopy) {
-#pragma unroll
-        for (int c = 0; c < M / 4; ++c) {
-          *(float4*)&sd[kk][c * 4] = make_float4(d0[c * 4], d0[c * 4 + 1], d0[c * 4 + 2], d0[c * 4 + 3]);
-          *(float4*)&sd[kk + 1][c * 4] = make_float4(d1[c * 4], d1[c * 4 + 1], d1[c * 4 + 2], d1[c * 4 + 3]);
+        for (int c = 0; c < FW / 2; ++c) {
+          const uint4 v = in ? ((const uint4*)p)[c] : make_uint4(0, 0, 0, 0);
+          fx[s2][2 * c] = make_uint2(v.x, v.y);
+          fx[s2][2 * c + 1] = make_uint2(v.z, v.w);
         }
-      } else {                                             // rows of the stage beyond the last state: zero, not stale
+      } else {
 #pragma unroll
-        for (int c = 0; c < M / 4; ++c) {
-          if (!in0) *(float4*)((float*)st.dist(kk) + c * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (!in1) *(float4*)((float*)st.dist(kk + 1) + c * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-        }
+        for (int c = 0; c < FW; ++c) fx[s2][c] = in ? p[c] : make_uint2(0, 0);
       }
-      const float2 inm = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f);
-      float2 mk = inm;
-      if (a.mask) mk = make_float2(in0 ? st.mask()[kk] : 0.f, in1 ? st.mask()[kk + 1] : 0.f);
-      auto get = [&](int ro) {                             // the pair (k, k + 1) of one gradient row; zero outside the row
-        float2 v;
-        if constexpr (sizeof(T) == 2) v = __bfloat1622float2(*(const __nv_bfloat162*)(st.grad(ro) + kk));
-        else v = *(const float2*)(st.grad(ro) + kk);
-        return make_float2(in0 ? v.x : 0.f, in1 ? v.y : 0.f);
-      };
+    }
+    mk = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f);
+    if (a.mask) {
+      if (in0) mk.x = a.mask[(int64_t)pt * a.K + k];
+      if (in1) mk.y = a.mask[(int64_t)pt * a.K + k + 1];
+    }
+    if (a.ddt) {
+      const T* g = (const T*)a.ddt + (int64_t)pt * a.H * a.K + k;
 #pragma unroll
-      for (int r = 0; r < GLUE_MAX_ROWS; ++r) {
+      for (int r = 0; r < 8; ++r)
+        if (r < a.H) gh[r] = pair_at(g + (int64_t)r * a.K, in0, in1);
+    }
+  };
+  float tsum[NR + 8];
+#pragma unroll
+  for (int r = 0; r < NR + 8; ++r) tsum[r] = 0.f;
+  if (first < npoints) load(first, 0);
+  for (int pt = first; pt < npoints; pt += per) {
+    const float* tok = a.tok + (int64_t)pt * a.RO;
+    for (int step = 0; step < nstep; ++step) {
+      const int k = step * 64 + 2 * lane;
+      const bool in0 = k < a.K, in1 = k + 1 < a.K;
+      float2 dp[M], dd[M], m2 = mk;
+      GP g8[8];
+#pragma unroll
+      for (int s2 = 0; s2 < 2; ++s2) {                     // features: float pairs over the two states; rows of sd
+        float f[M];
+#pragma unroll
+        for (int c = 0; c < FW; ++c) {
+          if constexpr (sizeof(TD) == 2) {
+            f[4 * c] = __uint_as_float(fx[s2][c].x << 16); f[4 * c + 1] = __uint_as_float(fx[s2][c].x & 0xffff0000u);
+            f[4 * c + 2] = __uint_as_float(fx[s2][c].y << 16); f[4 * c + 3] = __uint_as_float(fx[s2][c].y & 0xffff0000u);
+          } else {
+            f[2 * c] = __uint_as_float(fx[s2][c].x); f[2 * c + 1] = __uint_as_float(fx[s2][c].y);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < M; ++j) { if (s2) dp[j].y = f[j]; else dp[j].x = f[j]; }
+#pragma unroll
+        for (int c = 0; c < M / 4; ++c) *(float4*)(sd + (2 * lane + s2) * DS + c * 4) = make_float4(f[c * 4], f[c * 4 + 1], f[c * 4 + 2], f[c * 4 + 3]);
+      }
+#pragma unroll
+      for (int r = 0; r < 8; ++r) g8[r] = gh[r];
+      // gradients of the B / C rows of this step and the inputs of the next one
+      GP gb[8];
+      const T* pb = a.dbc ? (const T*)a.dbc + (int64_t)pt * nb * a.K + k : nullptr;
+      if (pb) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (r < nb) gb[r] = pair_at(pb + (int64_t)r * a.K, in0, in1);
+      }
+      if (step + 1 < nstep) load(pt, step + 1);
+      else if (pt + per < npoints) load(pt + per, 0);
+#pragma unroll
+      for (int j = 0; j < M; ++j) dd[j] = make_float2(0.f, 0.f);
+      float2 gq[4];                                        // g of four rows on their way to sg
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        float2 g = make_float2(0.f, 0.f);
         if (r < a.RW) {
-          float2 g = make_float2(0.f, 0.f);
-          float4 wrow[M / 4];                              // the row's weights: read once, used for pre and for ddist
-#pragma unroll
-          for (int c = 0; c < M / 4; ++c) wrow[c] = *(const float4*)&sw[r * M + c * 4];
+          const float2* w = sw + r * M;
           if (r < a.H) {
             if (a.ddt) {
-              float2 pre = make_float2(st.tok()[r], st.tok()[r]);
-#pragma unroll
-              for (int c = 0; c < M / 4; ++c) {
-                pre = __ffma2_rn(dp[c * 4], make_float2(wrow[c].x, wrow[c].x), pre);
-                pre = __ffma2_rn(dp[c * 4 + 1], make_float2(wrow[c].y, wrow[c].y), pre);
-                pre = __ffma2_rn(dp[c * 4 + 2], make_float2(wrow[c].z, wrow[c].z), pre);
-                pre = __ffma2_rn(dp[c * 4 + 3], make_float2(wrow[c].w, wrow[c].w), pre);
-              }
-              const float2 sg2 = make_float2(pre.x <= 20.f ? glue_sigmoid(pre.x) : 1.f, pre.y <= 20.f ? glue_sigmoid(pre.y) : 1.f);
-              g = __fmul2_rn(__fmul2_rn(get(r), mk), sg2);
+              const float t = __ldg(tok + r);
+              const float2 pre = row_dot<M>(w, dp, make_float2(t, t));
+              const float2 s2 = make_float2(pre.x <= 20.f ? glue_sigmoid(pre.x) : 1.f, pre.y <= 20.f ? glue_sigmoid(pre.y) : 1.f);
+              const float2 go = r < 8 ? up(g8[r & 7]) : up(pair_at((const T*)a.ddt + ((int64_t)pt * a.H + r) * a.K + k, in0, in1));
+              g = __fmul2_rn(__fmul2_rn(go, m2), s2);
             }
             tsum[r] += g.x + g.y;
-          } else if (a.dbc) {
-            g = get(r);
-            if (a.back) g = __fadd2_rn(g, get(r + 2 * a.G));   // both directions share the weight row
+          } else if (pb) {
+            const int q = r - a.H;                         // both directions share the weight row
+            g = q == 0 ? up(gb[0]) : q == 1 ? up(gb[1]) : up(pair_at(pb + (int64_t)q * a.K, in0, in1));
+            if (a.back) {
+              const int q2 = q + 2 * a.G;
+              g = __fadd2_rn(g, q2 == 2 ? up(gb[2]) : q2 == 3 ? up(gb[3]) : up(pair_at(pb + (int64_t)q2 * a.K, in0, in1)));
+            }
           }
-          *(float2*)&sg[r][kk] = g;
 #pragma unroll
-          for (int c = 0; c < M / 4; ++c) {
-            dd[c * 4] = __ffma2_rn(g, make_float2(wrow[c].x, wrow[c].x), dd[c * 4]);
-            dd[c * 4 + 1] = __ffma2_rn(g, make_float2(wrow[c].y, wrow[c].y), dd[c * 4 + 1]);
-            dd[c * 4 + 2] = __ffma2_rn(g, make_float2(wrow[c].z, wrow[c].z), dd[c * 4 + 2]);
-            dd[c * 4 + 3] = __ffma2_rn(g, make_float2(wrow[c].w, wrow[c].w), dd[c * 4 + 3]);
+          for (int c = 0; c < M; c += 2) {
+            const float4 q = *(const float4*)(w + c);
+            dd[c] = __ffma2_rn(g, make_float2(q.x, q.y), dd[c]);
+            dd[c + 1] = __ffma2_rn(g, make_float2(q.z, q.w), dd[c + 1]);
           }
         }
+        gq[r & 3] = g;
+        if ((r & 3) == 3) {
+          *(float4*)(sg + (2 * lane) * GS + r - 3) = make_float4(gq[0].x, gq[1].x, gq[2].x, gq[3].x);
+          *(float4*)(sg + (2 * lane + 1) * GS + r - 3) = make_float4(gq[0].y, gq[1].y, gq[2].y, gq[3].y);
+        }
       }
+      if (pb) {                                            // token terms of the B / C rows (each output row has its own)
 #pragma unroll
-      for (int j = 0; j < M; ++j) { d0[j] = dd[j].x; d1[j] = dd[j].y; }
-      if (in0) store_feats<TD, M>(ddist + (int64_t)k * M, d0);
-      if (in1) store_feats<TD, M>(ddist + (int64_t)(k + 1) * M, d1);
-      if (a.dbc) {                                         // token terms of the B / C rows (each output row has its own)
-#pragma unroll
-        for (int ro = 0; ro < GLUE_MAX_ROWS + 8; ++ro)
-          if (ro >= a.H && ro < a.RO) {
-            const float2 v = get(ro);
-            tsum[ro] += v.x + v.y;
+        for (int q = 0; q < 8; ++q)
+          if (q < nb) {
+            const float2 v = q < 4 ? up(gb[q & 3]) : up(pair_at(pb + (int64_t)q * a.K, in0, in1));
+            tsum[NR + q] += v.x + v.y;
           }
+        for (int q = 8; q < nb; ++q) {                     // more than two groups: straight to the token gradient
+          const float2 v = up(pair_at(pb + (int64_t)q * a.K, in0, in1));
+          const float t = warp_sum(v.x + v.y);
+          if (lane == 0) { float* o = a.dtok + (int64_t)pt * a.RO + a.H + q; *o = step ? *o + t : t; }
+        }
       }
-    }
-    __syncthreads();
-    if (kg < NKG) {
-      const int k1 = min(GLUE_KT, (kg + 1) * kspan);       // rows beyond the last state hold g = 0 and zero features
+      TD* ddist = (TD*)a.ddist + ((int64_t)pt * a.K + k) * M;
+      {
+        float f[M];
+#pragma unroll
+        for (int j = 0; j < M; ++j) f[j] = dd[j].x;
+        if (in0) store_feats<TD, M>(ddist, f);
+#pragma unroll
+        for (int j = 0; j < M; ++j) f[j] = dd[j].y;
+        if (in1) store_feats<TD, M>(ddist + M, f);
+      }
+      __syncwarp();
 #pragma unroll 2
-      for (int kk = kg * kspan; kk < k1; kk += 4) {
-        const float4 g4 = *(const float4*)&sg[wr][kk];
-        const float gs[4] = {g4.x, g4.y, g4.z, g4.w};
+      for (int i = 0; i < 8; ++i) {
+        const float* gp = sg + (kq + 8 * i) * GS + rh * RH;
+        const float* dq = sd + (kq + 8 * i) * DS + jh * MH;
+        float gv[RH];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          float4 f;
-          if constexpr (kCopy) f = *(const float4*)&sd[kk + i][wj];
-          else f = *(const float4*)((const float*)st.dist(kk + i) + wj);
-          wacc[0] = fmaf(gs[i], f.x, wacc[0]); wacc[1] = fmaf(gs[i], f.y, wacc[1]);
-          wacc[2] = fmaf(gs[i], f.z, wacc[2]); wacc[3] = fmaf(gs[i], f.w, wacc[3]);
+        for (int r = 0; r < RH; r += 2) { const float2 v = *(const float2*)(gp + r); gv[r] = v.x; gv[r + 1] = v.y; }
+#pragma unroll
+        for (int j = 0; j < MH / 2; ++j) {
+          const float2 dv = *(const float2*)(dq + 2 * j);
+#pragma unroll
+          for (int r = 0; r < RH; ++r) acc[r][j] = __ffma2_rn(make_float2(gv[r], gv[r]), dv, acc[r][j]);
         }
       }
+      __syncwarp();
     }
-    if (k0 + GLUE_KT >= a.K) {
-      // last tile of the point: token terms, summed over the states by warp shuffles, then the four warps in a fixed order
+    // token gradients of the point: sums over its states
 #pragma unroll
-      for (int r = 0; r < GLUE_MAX_ROWS + 8; ++r) {
-        if (r < a.RO) {
-          float v = tsum[r];
-#pragma unroll
-          for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) sred[warp][r] = v;
-        }
-        tsum[r] = 0.f;
+    for (int r = 0; r < NR + 8; ++r) {
+      const bool head = r < NR;
+      const int o = head ? r : a.H + r - NR;
+      if (head ? r < a.H : r - NR < nb) {
+        const float t = warp_sum(tsum[r]);
+        if (lane == 0) a.dtok[(int64_t)pt * a.RO + o] = t;
       }
-      __syncthreads();
-      for (int r = threadIdx.x; r < a.RO; r += blockDim.x)
-        a.dtok[row * a.RO + r] = ((sred[0][r] + sred[1][r]) + sred[2][r]) + sred[3][r];
+      tsum[r] = 0.f;
     }
-    __syncthreads();                                       // sg / sd / sred and this stage may be overwritten
   }
-  // the NKG ranges of a tile are summed in a fixed order through shared memory, then one partial per block goes out
+  // the eight shares of the states, then the four warps, in a fixed order
   __syncthreads();
-  float* sacc = &sg[0][0];                                 // 128 x 4 floats fit
 #pragma unroll
-  for (int c = 0; c < 4; ++c) sacc[threadIdx.x * 4 + c] = wacc[c];
-  __syncthreads();
-  if (threadIdx.x < tiles) {
+  for (int r = 0; r < RH; ++r)
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      float acc = 0.f;
-      for (int q = 0; q < NKG; ++q) acc += sacc[(q * tiles + threadIdx.x) * 4 + c];
-      a.dwpart[(size_t)blockIdx.x * GLUE_MAX_ROWS * M + wr * M + wj + c] = acc;
+    for (int j = 0; j < MH / 2; ++j) {
+      float2 v = acc[r][j];
+#pragma unroll
+      for (int o = 4; o < 32; o <<= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+      }
+      if (kq == 0) *(float2*)(sg + (rh * RH + r) * M + jh * MH + 2 * j) = v;
     }
+  __syncthreads();
+  for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < GLUE_BWD_WARPS; ++w) t += sg_all[w][i];
+    a.dwpart[(size_t)blockIdx.x * GLUE_MAX_ROWS * M + i] = t;
   }
 }
 
@@ -436,34 +452,34 @@ static GlueArgs glue_args(const issm_glue_params& p) {
 
 using namespace issm;
 
-#define GLUE_DISPATCH_M(KERNEL, TD, T)                                                                \
-  do {                                                                                                \
-    if (p->nfeat == 16) ISSM_LAUNCH((KERNEL<TD, T, 16>), grid, 128, 0, s, a);                         \
-    else if (p->nfeat == 8) ISSM_LAUNCH((KERNEL<TD, T, 8>), grid, 128, 0, s, a);                      \
-    else ISSM_LAUNCH((KERNEL<TD, T, 4>), grid, 128, 0, s, a);                                         \
-  } while (0)
-#define GLUE_DISPATCH(KERNEL)                                                                         \
-  do {                                                                                                \
-    const dim3 grid(p->seqlen, p->batch);                                                             \
-    cudaStream_t s = (cudaStream_t)stream;                                                            \
-    if (p->io_dtype == ISSM_F32) GLUE_DISPATCH_M(KERNEL, float, float);                               \
-    else if (p->dist_dtype == ISSM_F32) GLUE_DISPATCH_M(KERNEL, float, bf16);                         \
-    else GLUE_DISPATCH_M(KERNEL, bf16, bf16);                                                         \
-  } while (0)
-
 extern "C" size_t issm_b200_sizeof_glue_params(void) { return sizeof(issm_glue_params); }
 
 extern "C" int issm_b200_glue_fwd(const issm_glue_params* p, void* stream) {
   int rc = glue_validate(p, false);
   if (rc) return rc;
   const GlueArgs a = glue_args(*p);
-  GLUE_DISPATCH(k_glue_fwd);
+  if ((int64_t)p->batch * p->seqlen * ((p->nstates + 1) / 2) > 0x7fffffff) return ISSM_ERR_SHAPE;
+  const int npoints = p->batch * p->seqlen;
+  const int64_t want = cdiv64((int64_t)npoints * ((p->nstates + 1) / 2), 128);
+  const unsigned grid = (unsigned)(want < GLUE_FWD_BLOCKS ? want : GLUE_FWD_BLOCKS);
+  cudaStream_t s = (cudaStream_t)stream;
+#define GLUE_FWD_M(TD, T)                                                                             \
+  do {                                                                                                \
+    if (p->nfeat == 16) ISSM_LAUNCH((k_glue_fwd<TD, T, 16>), grid, 128, 0, s, a, npoints);            \
+    else if (p->nfeat == 8) ISSM_LAUNCH((k_glue_fwd<TD, T, 8>), grid, 128, 0, s, a, npoints);         \
+    else ISSM_LAUNCH((k_glue_fwd<TD, T, 4>), grid, 128, 0, s, a, npoints);                            \
+  } while (0)
+  if (p->io_dtype == ISSM_F32) GLUE_FWD_M(float, float);
+  else if (p->dist_dtype == ISSM_F32) GLUE_FWD_M(float, bf16);
+  else GLUE_FWD_M(bf16, bf16);
+#undef GLUE_FWD_M
   return ISSM_OK;
 }
 
 static int glue_bwd_blocks(const issm_glue_params* p) {
-  const int64_t pts = (int64_t)p->batch * p->seqlen;
-  return (int)(pts < GLUE_BWD_BLOCKS ? pts : GLUE_BWD_BLOCKS);
+  const int64_t need = cdiv64((int64_t)p->batch * p->seqlen, GLUE_BWD_WARPS);
+  const int64_t most = p->nfeat == 16 ? 148 * 2 : GLUE_BWD_BLOCKS;
+  return (int)(need < most ? need : most);
 }
 
 extern "C" size_t issm_b200_glue_workspace_bytes(const issm_glue_params* p) {
@@ -480,15 +496,12 @@ extern "C" int issm_b200_glue_bwd(const issm_glue_params* p, void* stream) {
   const int blocks = glue_bwd_blocks(p), npoints = p->batch * p->seqlen;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t es = p->io_dtype == ISSM_F32 ? 4 : 2;
-  // 16-byte copies of the gradient rows and the mask need every row of states to start on a 16-byte boundary
-  const int vec_ok = !((p->nstates * es) % 16) && !(p->nstates % 4) && !((uintptr_t)p->ddt % 16) && !((uintptr_t)p->dbc % 16) &&
-                     !((uintptr_t)p->mask % 16);
+  // pairs of gradients are one access where every row of states starts on the pair's alignment
+  const int pairs_ok = !(p->nstates & 1) && !((uintptr_t)p->ddt % (2 * es)) && !((uintptr_t)p->dbc % (2 * es));
 #define GLUE_BWD(TD, TT, MM)                                                                          \
   do {                                                                                                \
-    const size_t dyn = 2 * GlueStage<TD, TT, MM>::bytes(a.RO);                                        \
-    struct Tag {};                                                                                    \
-    if (int rc2 = SmemAttrOnce<Tag>::set(k_glue_bwd<TD, TT, MM>, 2 * GlueStage<TD, TT, MM>::bytes(GLUE_MAX_ROWS + 8))) return rc2; \
-    ISSM_LAUNCH((k_glue_bwd<TD, TT, MM>), blocks, 128, dyn, s, a, npoints, vec_ok);                   \
+    if (a.RW <= 12) ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 12>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok); \
+    else ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 16>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok);            \
   } while (0)
 #define GLUE_BWD_M(TD, TT)                                                                            \
   do {                                                                                                \

@@ -394,6 +394,207 @@ __global__ void __launch_bounds__(NORM_BWD_WARPS * 32, (CH == 1 && !HB) ? 5 : 0)
   }
 }
 
+// ---- RMS norm of x * silu(z) without bias: the detector's key_norm ------------------------------------------
+// The general vector kernels spend 39 (forward) and 73 (backward) instructions per element and are bound by instruction
+// issue in bf16.  Here two features go through each packed instruction, the sigmoid is evaluated once, and what the call
+// never asks for (mean, bias, the other gate) is left out: about 8 and 15 per element, so the memory system is the bound.
+// 2^18 rows x 288 features bf16, forward + backward call: see the table of the kernels' numbers at launch_norm_bwd_main.
+template <typename T> struct Pairs {                       // 16 bytes of a row as float pairs
+  static constexpr int NP = Vec16<T>::N / 2;
+  static __device__ __forceinline__ void unpack(uint4 w, float2* v) {
+    float f[2 * NP];
+    Vec16<T>::unpack(w, f);
+#pragma unroll
+    for (int i = 0; i < NP; ++i) v[i] = make_float2(f[2 * i], f[2 * i + 1]);
+  }
+  static __device__ __forceinline__ void store(T* p, const float2* v) {
+    float f[2 * NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) { f[2 * i] = v[i].x; f[2 * i + 1] = v[i].y; }
+    Vec16<T>::store(p, f);
+  }
+};
+__device__ __forceinline__ float2 bc2(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 sigmoid2(float2 z) {
+  const float2 t = __fmul2_rn(z, bc2(-1.4426950408889634f));
+  float2 e;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(t.x));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(t.y));
+  e = __fadd2_rn(e, bc2(1.f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(e.x) : "f"(e.x));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(e.y) : "f"(e.y));
+  return e;
+}
+
+template <typename T, int CH, int TL>
+__global__ void __launch_bounds__(256, CH == 1 ? 4 : 2) k_rmsgate_fwd(issm_norm_params np) {
+  constexpr int V = Vec16<T>::N, NP = V / 2, FT = CH * 32 * V;
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5, H = np.hidden;
+  const bool z16 = !(((uintptr_t)np.z | (uintptr_t)(np.z_sr * (int64_t)sizeof(T))) & 15);
+  auto in = [&](int c) { return TL || (c * 32 + lane) * V < H; };
+  uint4 nx[CH], nz[CH];
+  float nxt = 0.f, nzt = 0.f;
+  auto issue = [&](int row) {
+    const T* x = (const T*)np.x + (int64_t)row * np.x_sr;
+    const T* z = (const T*)np.z + (int64_t)row * np.z_sr;
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (in(c)) {
+        nx[c] = *(const uint4*)(x + (c * 32 + lane) * V);
+        nz[c] = ld16(z + (c * 32 + lane) * V, z16);
+      } else {
+        nx[c] = nz[c] = make_uint4(0, 0, 0, 0);
+      }
+    if constexpr (TL) { nxt = ldf(x + FT + lane); nzt = ldf(z + FT + lane); }
+  };
+  const float wt = TL ? np.weight[FT + lane] : 0.f, inv = 1.f / H;
+  int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (row < np.rows) issue(row);
+  for (; row < np.rows; row += warps) {
+    float2 v[CH][NP], s2 = bc2(0.f);
+    float vt = 0.f;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      float2 z[NP];
+      Pairs<T>::unpack(nx[c], v[c]);
+      Pairs<T>::unpack(nz[c], z);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        v[c][i] = __fmul2_rn(v[c][i], __fmul2_rn(z[i], sigmoid2(z[i])));
+        s2 = __ffma2_rn(v[c][i], v[c][i], s2);
+      }
+    }
+    float s = s2.x + s2.y;
+    if constexpr (TL) {
+      vt = nxt * siluf_(nzt);
+      s = fmaf(vt, vt, s);
+    }
+    if (row + warps < np.rows) issue(row + warps);
+    const float rstd = rsqrtf(warp_sum(s) * inv + np.eps);
+    if (lane == 0) np.rstd[row] = rstd;
+    T* y = (T*)np.y + (int64_t)row * np.y_sr;
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (in(c)) {
+        const float4* w = (const float4*)(np.weight + (c * 32 + lane) * V);
+        float2 wv[NP];
+#pragma unroll
+        for (int i = 0; i < NP; i += 2) { const float4 q = __ldg(w + i / 2); wv[i] = make_float2(q.x, q.y); wv[i + 1] = make_float2(q.z, q.w); }
+#pragma unroll
+        for (int i = 0; i < NP; ++i) v[c][i] = __fmul2_rn(__fmul2_rn(v[c][i], bc2(rstd)), wv[i]);
+        Pairs<T>::store(y + (c * 32 + lane) * V, v[c]);
+      }
+    if constexpr (TL) stf(y + FT + lane, vt * rstd * wt);
+  }
+}
+
+// dx, dz and the weight gradient partials (dw only: layout of k_norm_bwd_vec)
+template <typename T, int CH, int TL>
+__global__ void __launch_bounds__(128, CH == 1 ? 5 : 2) k_rmsgate_bwd(issm_norm_params np, int rpb, float* __restrict__ dwpart) {
+  constexpr int V = Vec16<T>::N, NP = V / 2, FT = CH * 32 * V, WARPS = 4;
+  extern __shared__ float sm[];                            // [WARPS][hidden]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, H = np.hidden;
+  const bool z16 = !(((uintptr_t)np.z | (uintptr_t)(np.z_sr * (int64_t)sizeof(T))) & 15);
+  auto in = [&](int c) { return TL || (c * 32 + lane) * V < H; };
+  float2 dw[CH][NP], w[CH][NP];
+#pragma unroll
+  for (int c = 0; c < CH; ++c)
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      dw[c][i] = bc2(0.f);
+      w[c][i] = in(c) ? *(const float2*)(np.weight + (c * 32 + lane) * V + 2 * i) : bc2(0.f);
+    }
+  float dwt = 0.f;
+  const float wt = TL ? np.weight[FT + lane] : 0.f, inv = 1.f / H;
+  const int r_end = min(np.rows, (int)(blockIdx.x + 1) * rpb);
+  uint4 nx[CH], ng[CH], nz[CH];
+  float nxt = 0.f, ngt = 0.f, nzt = 0.f, nrstd = 0.f;
+  auto issue = [&](int row) {
+    const T* x = (const T*)np.x + (int64_t)row * np.x_sr;
+    const T* z = (const T*)np.z + (int64_t)row * np.z_sr;
+    const T* dy = (const T*)np.dy + (int64_t)row * np.dy_sr;
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      const int f0 = (c * 32 + lane) * V;
+      if (in(c)) {
+        nx[c] = *(const uint4*)(x + f0);
+        ng[c] = *(const uint4*)(dy + f0);
+        nz[c] = ld16(z + f0, z16);
+      } else {
+        nx[c] = ng[c] = nz[c] = make_uint4(0, 0, 0, 0);
+      }
+    }
+    if constexpr (TL) { nxt = ldf(x + FT + lane); ngt = ldf(dy + FT + lane); nzt = ldf(z + FT + lane); }
+    nrstd = np.rstd[row];
+  };
+  int row = blockIdx.x * rpb + warp;
+  if (row < r_end) issue(row);
+  for (; row < r_end; row += WARPS) {
+    const float rstd = nrstd;
+    // kept over the statistics: x, silu(z), d silu / dz, dy
+    float2 x[CH][NP], sz[CH][NP], ds[CH][NP], go[CH][NP], c2 = bc2(0.f);
+#pragma unroll
+    for (int c = 0; c < CH; ++c) {
+      Pairs<T>::unpack(nx[c], x[c]);
+      Pairs<T>::unpack(ng[c], go[c]);
+      Pairs<T>::unpack(nz[c], sz[c]);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const float2 sg = sigmoid2(sz[c][i]);
+        sz[c][i] = __fmul2_rn(sz[c][i], sg);
+        ds[c][i] = __ffma2_rn(sz[c][i], __ffma2_rn(sg, bc2(-1.f), bc2(1.f)), sg);     // sg (1 + z (1 - sg))
+        c2 = __ffma2_rn(__fmul2_rn(x[c][i], sz[c][i]), __fmul2_rn(go[c][i], w[c][i]), c2);
+      }
+    }
+    float s = c2.x + c2.y;
+    const float xt = nxt, got = ngt;
+    float szt = 0.f, dst = 0.f;
+    if constexpr (TL) {
+      const float sg = fast_sigmoid(nzt);
+      szt = nzt * sg;
+      dst = fmaf(szt, 1.f - sg, sg);
+      s = fmaf(xt * szt, got * wt, s);
+    }
+    if (row + WARPS < r_end) issue(row + WARPS);
+    // c1 = mean(xhat * wdy), xhat = v rstd; dv = (wdy - xhat c1) rstd = wdy rstd - v (c1 rstd^2)
+    const float c1 = warp_sum(s) * inv * rstd, k = -c1 * rstd * rstd;
+    T* dx = (T*)np.dx + (int64_t)row * H;
+    T* dz = (T*)np.dz + (int64_t)row * H;
+#pragma unroll
+    for (int c = 0; c < CH; ++c)
+      if (in(c)) {
+        float2 ox[NP], oz[NP];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          const float2 v = __fmul2_rn(x[c][i], sz[c][i]), gr = __fmul2_rn(go[c][i], bc2(rstd));
+          dw[c][i] = __ffma2_rn(gr, v, dw[c][i]);
+          const float2 dv = __ffma2_rn(gr, w[c][i], __fmul2_rn(v, bc2(k)));
+          ox[i] = __fmul2_rn(dv, sz[c][i]);
+          oz[i] = __fmul2_rn(__fmul2_rn(dv, x[c][i]), ds[c][i]);
+        }
+        Pairs<T>::store(dx + (c * 32 + lane) * V, ox);
+        Pairs<T>::store(dz + (c * 32 + lane) * V, oz);
+      }
+    if constexpr (TL) {
+      const float v = xt * szt, gr = got * rstd, dv = fmaf(gr, wt, v * k);
+      dwt = fmaf(gr, v, dwt);
+      stf(dx + FT + lane, dv * szt);
+      stf(dz + FT + lane, dv * xt * dst);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CH; ++c)
+    if (in(c)) {
+#pragma unroll
+      for (int i = 0; i < NP; ++i) *(float2*)(sm + (size_t)warp * H + (c * 32 + lane) * V + 2 * i) = dw[c][i];
+    }
+  if constexpr (TL) sm[(size_t)warp * H + FT + lane] = dwt;
+  __syncthreads();
+  for (int f = threadIdx.x; f < H; f += blockDim.x)
+    dwpart[(size_t)blockIdx.x * H + f] = ((sm[f] + sm[H + f]) + sm[2 * H + f]) + sm[3 * H + f];
+}
+static bool norm_rmsgate(const issm_norm_params& p) { return p.is_rms && p.has_z && !p.norm_before_gate && !p.has_bias; }
+
 // chunks per lane the vector kernels need for this call, or 0 when it has to take the general kernels
 static int norm_vec_chunks(const issm_norm_params& p, bool bwd) {
   const int V = p.io_dtype == ISSM_BF16 ? 8 : 4, esz = p.io_dtype == ISSM_BF16 ? 2 : 4;
@@ -483,26 +684,29 @@ __global__ void k_norm_bwd(issm_norm_params np, int rpb, float* __restrict__ dwp
   }
 }
 
-// out[j] = sum over the `count` partial rows of part[i][j], in a fixed order: 32 features x 8 row groups per block;
-// group g adds rows g, g + 8, ... in order, then the eight group sums are added in order
-__global__ void __launch_bounds__(256) k_norm_reduce(const float* __restrict__ part, int count, int stride, float* __restrict__ out) {
-  __shared__ float sacc[8][33];
+// out[j] = sum over the `count` partial rows of part[i][j], in a fixed order: 32 features x 32 row groups per block;
+// group g adds rows g, g + 32, ..., then the group sums are added in order (eight groups left each thread a chain of 93
+// dependent loads at 740 rows: 13 us)
+__global__ void __launch_bounds__(1024) k_norm_reduce(const float* __restrict__ part, int count, int stride, float* __restrict__ out) {
+  __shared__ float sacc[32][33];
   const int fx = threadIdx.x & 31, gy = threadIdx.x >> 5;
   const int j = blockIdx.x * 32 + fx;
   float acc = 0.f;
-  if (j < stride)
-    for (int i = gy; i < count; i += 8) acc += part[(size_t)i * stride + j];
+  if (j < stride) {
+#pragma unroll 4
+    for (int i = gy; i < count; i += 32) acc += part[(size_t)i * stride + j];
+  }
   sacc[gy][fx] = acc;
   __syncthreads();
   if (gy == 0 && j < stride) {
     float t = 0.f;
 #pragma unroll
-    for (int g = 0; g < 8; ++g) t += sacc[g][fx];
+    for (int g = 0; g < 32; ++g) t += sacc[g][fx];
     out[j] = t;
   }
 }
 
-// blocks of the backward: one resident wave (five blocks of four warps per SM fit the bias-free vector kernel; the
+// blocks of the backward: one resident wave (five blocks of four warps per SM fit the one-chunk kernels without bias; the
 // workspace-free entry point keeps to its built-in scratch of 148 * 4 partial rows)
 static int norm_blocks(const issm_norm_params& p, int want = 148 * 5) {
   return p.rows < want ? (p.rows > 0 ? p.rows : 1) : want;
@@ -522,6 +726,18 @@ static int norm_validate(const issm_norm_params* p, bool bwd) {
 // the backward main kernel of one call (vector kernels when the call qualifies, see norm_vec_chunks)
 static int launch_norm_bwd_main(const issm_norm_params& p, int nblk, int rpb, float* dwpart, float* dbpart, size_t smem, cudaStream_t s) {
   const int ch = norm_vec_chunks(p, true);
+#define ISSM_NORM_RMSGATE_BWD(T)                                                                          \
+  do {                                                                                                    \
+    if (ch == 17) ISSM_LAUNCH((k_rmsgate_bwd<T, 1, 1>), nblk, 128, smem, s, p, rpb, dwpart);              \
+    else if (ch == 18) ISSM_LAUNCH((k_rmsgate_bwd<T, 2, 1>), nblk, 128, smem, s, p, rpb, dwpart);         \
+    else if (ch == 1) ISSM_LAUNCH((k_rmsgate_bwd<T, 1, 0>), nblk, 128, smem, s, p, rpb, dwpart);          \
+    else if (ch == 2) ISSM_LAUNCH((k_rmsgate_bwd<T, 2, 0>), nblk, 128, smem, s, p, rpb, dwpart);          \
+    else ISSM_LAUNCH((k_rmsgate_bwd<T, 4, 0>), nblk, 128, smem, s, p, rpb, dwpart);                       \
+  } while (0)
+  if (ch && norm_rmsgate(p)) {
+    if (p.io_dtype == ISSM_F32) ISSM_NORM_RMSGATE_BWD(float); else ISSM_NORM_RMSGATE_BWD(bf16);
+    return ISSM_OK;
+  }
 #define ISSM_NORM_BWD_VEC2(T, HBV)                                                                                            \
   do {                                                                                                                      \
     if (ch == 17) ISSM_LAUNCH((k_norm_bwd_vec<T, 1, 1, HBV>), nblk, NORM_BWD_WARPS * 32, smem, s, p, rpb, dwpart, dbpart);      \
@@ -562,6 +778,18 @@ extern "C" int issm_b200_norm_fwd(const issm_norm_params* p, void* stream) {
   const unsigned grid = (p->rows + wpb - 1) / wpb;
   const int ch = norm_vec_chunks(*p, false);
   const unsigned vgrid = grid < 148u * 4u ? grid : 148u * 4u;   // the vector kernel walks the rows with a grid stride (one resident wave)
+#define ISSM_NORM_RMSGATE_FWD(T)                                                                                \
+  do {                                                                                                         \
+    if (ch == 17) ISSM_LAUNCH((k_rmsgate_fwd<T, 1, 1>), vgrid, wpb * 32, 0, s, *p);                               \
+    else if (ch == 18) ISSM_LAUNCH((k_rmsgate_fwd<T, 2, 1>), vgrid, wpb * 32, 0, s, *p);                       \
+    else if (ch == 1) ISSM_LAUNCH((k_rmsgate_fwd<T, 1, 0>), vgrid, wpb * 32, 0, s, *p);                           \
+    else if (ch == 2) ISSM_LAUNCH((k_rmsgate_fwd<T, 2, 0>), vgrid, wpb * 32, 0, s, *p);                        \
+    else ISSM_LAUNCH((k_rmsgate_fwd<T, 4, 0>), vgrid, wpb * 32, 0, s, *p);                                     \
+  } while (0)
+  if (ch && norm_rmsgate(*p)) {
+    if (p->io_dtype == ISSM_F32) ISSM_NORM_RMSGATE_FWD(float); else ISSM_NORM_RMSGATE_FWD(bf16);
+    return ISSM_OK;
+  }
 #define ISSM_NORM_FWD_VEC(T)                                                                                   \
   do {                                                                                                         \
     if (ch == 17) ISSM_LAUNCH((k_norm_fwd_vec<T, 1, 1>), vgrid, wpb * 32, 0, s, *p);                           \
@@ -602,8 +830,8 @@ extern "C" int issm_b200_norm_bwd(const issm_norm_params* p, void* stream) {
   }
   rc = launch_norm_bwd_main(*p, nblk, rpb, dwpart, dbpart, smem, s);
   if (rc) return rc;
-  ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 256, 0, s, dwpart, nblk, p->hidden, p->dweight);
-  if (p->has_bias) ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 256, 0, s, dbpart, nblk, p->hidden, p->dbias);
+  ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 1024, 0, s, dwpart, nblk, p->hidden, p->dweight);
+  if (p->has_bias) ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 1024, 0, s, dbpart, nblk, p->hidden, p->dbias);
   return ISSM_OK;
 }
 
@@ -660,7 +888,7 @@ extern "C" int issm_b200_norm_bwd_noalloc(const issm_norm_params* p, void* strea
   // every block writes its whole row of partials, so nothing in the scratch has to start at zero
   rc = launch_norm_bwd_main(*p, nblk, rpb, dwpart, dbpart, smem, s);
   if (rc) return rc;
-  ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 256, 0, s, dwpart, nblk, p->hidden, p->dweight);
-  if (p->has_bias) ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 256, 0, s, dbpart, nblk, p->hidden, p->dbias);
+  ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 1024, 0, s, dwpart, nblk, p->hidden, p->dweight);
+  if (p->has_bias) ISSM_LAUNCH(k_norm_reduce, (p->hidden + 31) / 32, 1024, 0, s, dbpart, nblk, p->hidden, p->dbias);
   return ISSM_OK;
 }

@@ -7,30 +7,58 @@
 // every access is coalesced.  Gradients of weight and bias are accumulated per block and reduced in a fixed order.
 #include "issm_common.cuh"
 
+#include <type_traits>
+
 namespace issm {
 
 constexpr int CONV_K = 7, CONV_PAD = 3;
 
 
 // ---- gather ----------------------------------------------------------------------------------------------
-// one warp per destination row; VEC = bytes per lane access (16, 4 or 2)
+// A warp copies kGatherRows destination rows; VEC = bytes per lane access (16, 4 or 2).  The bound is latency: with one row per
+// warp (an index, then five 4-byte loads per lane at 290 bf16 channels) too few bytes were in flight: 64 x 16384 x 290 bf16
+// 289 us = 4.2 TB/s.  All rows' loads of a step go out before the first store.
+constexpr int kGatherRows = 4;
+template <int VEC> struct GatherWord { using t = uint16_t; };
+template <> struct GatherWord<4> { using t = uint32_t; };
+template <> struct GatherWord<16> { using t = uint4; };
 template <int VEC>
-__global__ void k_gather_rows(const char* __restrict__ src, const int64_t* __restrict__ index, char* __restrict__ dst,
+__global__ void __launch_bounds__(256) k_gather_rows(const char* __restrict__ src, const int64_t* __restrict__ index, char* __restrict__ dst,
                               int n_out, int n_src, int64_t row_bytes, int64_t src_batch_bytes, int64_t src_row_bytes, int* status) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  using W = typename GatherWord<VEC>::t;
+  constexpr int STEP = VEC == 16 ? 1 : 3;                // accesses per row and step: 12 in flight per lane (4 of 16 bytes)
+  const int row0 = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * kGatherRows, lane = threadIdx.x & 31;
   const int b = blockIdx.y;
-  if (warp >= n_out) return;
-  int64_t j = index[(int64_t)b * n_out + warp];
-  if (j < 0 || j >= n_src) {                               // an index outside the source: flag it, copy nothing
-    if (lane == 0 && status) atomicOr(status, 2);
-    return;
+  if (row0 >= n_out) return;
+  int64_t j = -1;
+  if (lane < kGatherRows && row0 + lane < n_out) {
+    j = index[(int64_t)b * n_out + row0 + lane];
+    if (j < 0 || j >= n_src) {                           // an index outside the source: flag it, copy nothing
+      j = -1;
+      if (status) atomicOr(status, 2);
+    }
   }
-  const char* s = src + b * src_batch_bytes + j * src_row_bytes;
-  char* d = dst + ((int64_t)b * n_out + warp) * row_bytes;
-  for (int64_t o = (int64_t)lane * VEC; o < row_bytes; o += 32 * VEC) {
-    if (VEC == 16) *(uint4*)(d + o) = *(const uint4*)(s + o);
-    else if (VEC == 4) *(uint32_t*)(d + o) = *(const uint32_t*)(s + o);
-    else *(uint16_t*)(d + o) = *(const uint16_t*)(s + o);
+  const char* s[kGatherRows];
+  bool ok[kGatherRows];
+#pragma unroll
+  for (int r = 0; r < kGatherRows; ++r) {
+    const int64_t jr = __shfl_sync(0xffffffffu, j, r);
+    ok[r] = jr >= 0;
+    s[r] = src + b * src_batch_bytes + jr * src_row_bytes;
+  }
+  char* d = dst + ((int64_t)b * n_out + row0) * row_bytes;
+  for (int64_t o0 = (int64_t)lane * VEC; o0 < row_bytes; o0 += 32 * VEC * STEP) {
+    W v[kGatherRows][STEP];
+#pragma unroll
+    for (int k = 0; k < STEP; ++k)
+#pragma unroll
+      for (int r = 0; r < kGatherRows; ++r)
+        if (ok[r] && o0 + k * 32 * VEC < row_bytes) v[r][k] = *(const W*)(s[r] + o0 + k * 32 * VEC);
+#pragma unroll
+    for (int r = 0; r < kGatherRows; ++r)
+#pragma unroll
+      for (int k = 0; k < STEP; ++k)
+        if (ok[r] && o0 + k * 32 * VEC < row_bytes) *(W*)(d + r * row_bytes + o0 + k * 32 * VEC) = v[r][k];
   }
 }
 
@@ -85,6 +113,23 @@ __device__ __forceinline__ void ldv(const float* p, float& v) { v = *p; }
 __device__ __forceinline__ void ldv(const float* p, float2& v) { v = *(const float2*)p; }
 __device__ __forceinline__ void ldv(const bf16* p, float& v) { v = __bfloat162float(*p); }
 __device__ __forceinline__ void ldv(const bf16* p, float2& v) { v = __bfloat1622float2(*(const __nv_bfloat162*)p); }
+// a row value as loaded (packed for a pair of bf16 channels), so that the loads of the next rows can be in flight at one
+// register each while the current ones are worked on
+template <typename T, int V> struct RawVal { using t = typename Val<V>::t; };
+template <> struct RawVal<bf16, 2> { using t = uint32_t; };
+template <> struct RawVal<bf16, 1> { using t = bf16; };
+__device__ __forceinline__ void ldraw(const float* p, float& v) { v = *p; }
+__device__ __forceinline__ void ldraw(const float* p, float2& v) { v = *(const float2*)p; }
+__device__ __forceinline__ void ldraw(const bf16* p, bf16& v) { v = *p; }
+__device__ __forceinline__ void ldraw(const bf16* p, uint32_t& v) { v = *(const uint32_t*)p; }
+__device__ __forceinline__ void rawzero(float& v) { v = 0.f; }
+__device__ __forceinline__ void rawzero(float2& v) { v = make_float2(0.f, 0.f); }
+__device__ __forceinline__ void rawzero(bf16& v) { v = __float2bfloat16(0.f); }
+__device__ __forceinline__ void rawzero(uint32_t& v) { v = 0; }
+__device__ __forceinline__ void unraw(float r, float& v) { v = r; }
+__device__ __forceinline__ void unraw(float2 r, float2& v) { v = r; }
+__device__ __forceinline__ void unraw(bf16 r, float& v) { v = __bfloat162float(r); }
+__device__ __forceinline__ void unraw(uint32_t r, float2& v) { v = make_float2(__uint_as_float(r << 16), __uint_as_float(r & 0xffff0000u)); }
 __device__ __forceinline__ void stv(float* p, float v) { *p = v; }
 __device__ __forceinline__ void stv(float* p, float2 v) { *(float2*)p = v; }
 __device__ __forceinline__ void stv(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
@@ -109,23 +154,35 @@ __global__ void __launch_bounds__(256) k_dwconv7_silu_fwd(ConvArgs a) {
   if (a.bias) ldw(a.bias, a.C, c, 1, 0, bias);
 #pragma unroll
   for (int k = 0; k < CONV_K; ++k) ldw(a.w, a.C, c, CONV_K, k, w[k]);
-  auto fetch = [&](int n, F& d) {
-    if (n >= 0 && n < a.N) ldv(x + (int64_t)n * a.x_sl, d);
-    else vzero(d);
+  using Raw = typename RawVal<T, V>::t;
+  auto fetch = [&](int n, Raw& d) {
+    if (n >= 0 && n < a.N) ldraw(x + (int64_t)n * a.x_sl, d);
+    else rawzero(d);
   };
-  // rows n - 3 .. n + R + 2 of a batch of R output rows; the R loads of a batch are issued before any is used
+  // rows n - 3 .. n + R + 2 of a batch of R output rows; the R loads of the NEXT batch are in flight while one is worked on
   F buf[CONV_K - 1 + R];
-#pragma unroll
-  for (int k = 0; k < CONV_K - 1; ++k) fetch(n0 - CONV_PAD + k, buf[k]);
-  for (int n = n0; n < n1; n += R) {
+  Raw nx[R];
+  auto issue = [&](int n) {
     if (n + CONV_PAD + R <= a.N) {                         // the whole batch lies inside the sequence: no per-row test
       const T* px = x + (int64_t)(n + CONV_PAD) * a.x_sl;
 #pragma unroll
-      for (int r = 0; r < R; ++r) ldv(px + (int64_t)r * a.x_sl, buf[CONV_K - 1 + r]);
+      for (int r = 0; r < R; ++r) ldraw(px + (int64_t)r * a.x_sl, nx[r]);
     } else {
 #pragma unroll
-      for (int r = 0; r < R; ++r) fetch(n + CONV_PAD + r, buf[CONV_K - 1 + r]);
+      for (int r = 0; r < R; ++r) fetch(n + CONV_PAD + r, nx[r]);
     }
+  };
+#pragma unroll
+  for (int k = 0; k < CONV_K - 1; ++k) {
+    Raw t;
+    fetch(n0 - CONV_PAD + k, t);
+    unraw(t, buf[k]);
+  }
+  issue(n0);
+  for (int n = n0; n < n1; n += R) {
+#pragma unroll
+    for (int r = 0; r < R; ++r) unraw(nx[r], buf[CONV_K - 1 + r]);
+    if (n + R < n1) issue(n + R);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (n + r < n1) {
@@ -144,9 +201,10 @@ __global__ void __launch_bounds__(256) k_dwconv7_silu_fwd(ConvArgs a) {
 // Backward in one pass: g[m] = dy[m] * dsilu(pre[m]) is recomputed for the 3 halo rows on either side of the segment
 // and kept in a 7-row register window, so dx[n] = sum_k w[k] g[n - k + 3] needs no intermediate in global memory.
 template <typename T, int V>
-__global__ void __launch_bounds__(256) k_dwconv7_silu_bwd(ConvArgs a) {
+__global__ void __launch_bounds__(256, 2) k_dwconv7_silu_bwd(ConvArgs a) {
   using F = typename Val<V>::t;
-  constexpr int R = CONV_R;
+  using Raw = typename RawVal<T, V>::t;
+  constexpr int R = 4;                                     // half the forward's: x, dy and g windows, and the next rows in flight
   __shared__ float red[CONV_SEGS][8][32 * V];
   const int c = (blockIdx.x * 32 + threadIdx.x) * V;
   const int b = blockIdx.z;
@@ -165,56 +223,71 @@ __global__ void __launch_bounds__(256) k_dwconv7_silu_bwd(ConvArgs a) {
     if (a.bias) ldw(a.bias, a.C, c, 1, 0, bias);
 #pragma unroll
     for (int k = 0; k < CONV_K; ++k) ldw(a.w, a.C, c, CONV_K, k, w[k]);
-    auto fetch = [&](const T* base, int64_t stride, int n, F& d) {
-      if (n >= 0 && n < a.N) ldv(base + (int64_t)n * stride, d);
-      else vzero(d);
+    auto fetch = [&](const T* base, int64_t stride, int n, Raw& d) {
+      if (n >= 0 && n < a.N) ldraw(base + (int64_t)n * stride, d);
+      else rawzero(d);
     };
-    F xb[CONV_K - 1 + R], gyb[R], gb[CONV_K - 1 + R];      // x[m - 3 .. m + R + 2]; dy[m .. m + R); g[m - 6 .. m + R)
+    F xb[CONV_K - 1 + R], gb[CONV_K - 1 + R];              // x[m - 3 .. m + R + 2]; g[m - 6 .. m + R)
+    Raw nx[R], ng[R], gyb[R];                              // the next rows of x and dy; dy[m .. m + R)
     const int m0 = n0 - CONV_PAD, m1 = n1 + CONV_PAD;
-#pragma unroll
-    for (int k = 0; k < CONV_K - 1; ++k) fetch(x, a.x_sl, m0 - CONV_PAD + k, xb[k]);
-#pragma unroll
-    for (int k = 0; k < CONV_K - 1; ++k) vzero(gb[k]);
-    for (int mb = m0; mb < m1; mb += R) {
+    auto issue = [&](int mb) {
       if (mb >= 0 && mb + CONV_PAD + R <= a.N) {           // whole batch inside the sequence
         const T* px = x + (int64_t)(mb + CONV_PAD) * a.x_sl;
         const T* pg = dy + (int64_t)mb * a.dy_sl;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          ldv(px + (int64_t)r * a.x_sl, xb[CONV_K - 1 + r]);
-          ldv(pg + (int64_t)r * a.dy_sl, gyb[r]);
+          ldraw(px + (int64_t)r * a.x_sl, nx[r]);
+          ldraw(pg + (int64_t)r * a.dy_sl, ng[r]);
         }
       } else {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          fetch(x, a.x_sl, mb + CONV_PAD + r, xb[CONV_K - 1 + r]);
-          fetch(dy, a.dy_sl, mb + r, gyb[r]);              // zero outside the sequence, so g is zero there too
+          fetch(x, a.x_sl, mb + CONV_PAD + r, nx[r]);
+          fetch(dy, a.dy_sl, mb + r, ng[r]);               // zero outside the sequence, so g is zero there too
         }
       }
+    };
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const int m = mb + r;
-        if (m < m1) {
-          F pre = bias;
+    for (int k = 0; k < CONV_K - 1; ++k) {
+      Raw t;
+      fetch(x, a.x_sl, m0 - CONV_PAD + k, t);
+      unraw(t, xb[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < CONV_K - 1; ++k) vzero(gb[k]);
+    issue(m0);
+    for (int mb = m0; mb < m1; mb += R) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) { unraw(nx[r], xb[CONV_K - 1 + r]); gyb[r] = ng[r]; }
+      if (mb + R < m1) issue(mb + R);
+      auto rows = [&](auto inner) {                        // inner: every row of the batch and of its dx lies in the segment
+        constexpr bool kInner = decltype(inner)::value;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int m = mb + r;
+          if (!kInner && m >= m1) continue;
+          F pre = bias, gy;
 #pragma unroll
           for (int k = 0; k < CONV_K; ++k) pre = vfma(w[k], xb[r + k], pre);
-          const F g = vmul(gyb[r], vdsilu(pre, vsigmoid(pre)));
+          unraw(gyb[r], gy);
+          const F g = vmul(gy, vdsilu(pre, vsigmoid(pre)));
           gb[CONV_K - 1 + r] = g;
-          if (m >= n0 && m < n1) {                         // rows of this segment; halo rows belong to a neighbour
+          if (kInner || (m >= n0 && m < n1)) {             // rows of this segment; halo rows belong to a neighbour
             db = vadd(db, g);
 #pragma unroll
             for (int k = 0; k < CONV_K; ++k) dw[k] = vfma(g, xb[r + k], dw[k]);
           }
           const int n = m - CONV_PAD;                      // gb[r .. r + 6] = g[n - 3 .. n + 3]
-          if (n >= n0) {
-            F acc;
-            vzero(acc);
+          if (kInner || n >= n0) {
+            F acc = vmul(w[0], gb[r + CONV_K - 1]);
 #pragma unroll
-            for (int k = 0; k < CONV_K; ++k) acc = vfma(w[k], gb[r + CONV_K - 1 - k], acc);
+            for (int k = 1; k < CONV_K; ++k) acc = vfma(w[k], gb[r + CONV_K - 1 - k], acc);
             stv(dx + (int64_t)n * a.C, acc);
           }
         }
-      }
+      };
+      if (mb - CONV_PAD >= n0 && mb + R <= n1) rows(std::true_type{});
+      else rows(std::false_type{});
 #pragma unroll
       for (int k = 0; k < CONV_K - 1; ++k) { xb[k] = xb[R + k]; gb[k] = gb[R + k]; }
     }
@@ -309,7 +382,7 @@ extern "C" int issm_b200_gather_rows(const void* src, const int64_t* index, void
   if (!src || !index || !dst) return ISSM_ERR_NULL;
   if (batch <= 0 || batch > 65535 || n_out <= 0 || n_src <= 0 || row_bytes <= 0 || (row_bytes & 1)) return ISSM_ERR_SHAPE;
   cudaStream_t s = (cudaStream_t)stream;
-  const dim3 grid((n_out + 7) / 8, batch);
+  const dim3 grid((n_out + 8 * kGatherRows - 1) / (8 * kGatherRows), batch);
   const bool a16 = !(((uintptr_t)src | (uintptr_t)dst | (uintptr_t)row_bytes | (uintptr_t)src_batch_bytes | (uintptr_t)src_row_bytes) & 15);
   const bool a4 = !(((uintptr_t)src | (uintptr_t)dst | (uintptr_t)row_bytes | (uintptr_t)src_batch_bytes | (uintptr_t)src_row_bytes) & 3);
   if (a16) ISSM_LAUNCH(k_gather_rows<16>, grid, 256, 0, s, (const char*)src, index, (char*)dst, n_out, n_src, row_bytes, src_batch_bytes, src_row_bytes, status);

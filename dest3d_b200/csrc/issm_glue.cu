@@ -98,24 +98,35 @@ __device__ __forceinline__ float glue_softplus(float v) {
 // Weights wait in shared memory as pairs (w, w): a 128-bit access gives two packed operands, where the scalar form cost a move
 // per multiply-add.  Blocks walk the points with a grid stride, so the weights are laid out once per block and not per point.
 // 16 x 4096 points x 256 states x 16 features bf16: 312 us before.
+// The dt rows are padded to a multiple of four (zero weights) and the B / C rows follow: rows are worked on four at a time, four
+// independent chains of multiply-adds (one row at a time left the fp32 pipe waiting for its own results).
+constexpr int GLUE_PAD_ROWS = 20;
+__host__ __device__ __forceinline__ int glue_hp(int H) { return (H + 3) & ~3; }
 template <int M>
-__device__ __forceinline__ void weights_to_smem(const GlueArgs& a, float2* sw) {
-  for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) { const float w = a.w[i]; sw[i] = make_float2(w, w); }
-}
-template <int M>
-__device__ __forceinline__ float2 row_dot(const float2* w, const float2 (&dp)[M], float2 pre) {
-#pragma unroll
-  for (int c = 0; c < M; c += 2) {
-    const float4 q = *(const float4*)(w + c);
-    pre = __ffma2_rn(dp[c], make_float2(q.x, q.y), pre);
-    pre = __ffma2_rn(dp[c + 1], make_float2(q.z, q.w), pre);
+__device__ __forceinline__ void weights_to_smem(const GlueArgs& a, float2* sw, int rows) {
+  const int hp = glue_hp(a.H);
+  for (int i = threadIdx.x; i < rows * M; i += blockDim.x) {
+    const int r = i / M, src = r < hp ? (r < a.H ? r : -1) : (r - hp < 2 * a.G ? a.H + r - hp : -1);
+    const float w = src >= 0 ? a.w[src * M + i % M] : 0.f;
+    sw[i] = make_float2(w, w);
   }
-  return pre;
+}
+// pre[q] += sum_j dp[j] w[q][j] for four consecutive rows
+template <int M>
+__device__ __forceinline__ void quad_dot(const float2* w, const float2 (&dp)[M], float2 (&pre)[4]) {
+#pragma unroll
+  for (int c = 0; c < M; c += 2)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float4 v = *(const float4*)(w + q * M + c);
+      pre[q] = __ffma2_rn(dp[c], make_float2(v.x, v.y), pre[q]);
+      pre[q] = __ffma2_rn(dp[c + 1], make_float2(v.z, v.w), pre[q]);
+    }
 }
 template <typename TD, typename T, int M>
 __global__ void __launch_bounds__(128) k_glue_fwd(GlueArgs a, int npoints) {
-  __shared__ __align__(16) float2 sw[GLUE_MAX_ROWS * M];
-  weights_to_smem<M>(a, sw);
+  __shared__ __align__(16) float2 sw[GLUE_PAD_ROWS * M];
+  weights_to_smem<M>(a, sw, GLUE_PAD_ROWS);
   __syncthreads();
   const bool pair_store = !(a.K & 1);                      // rows of an even number of states keep pairs aligned
   auto put = [&](T* p, float2 v, bool two) {
@@ -127,38 +138,54 @@ __global__ void __launch_bounds__(128) k_glue_fwd(GlueArgs a, int npoints) {
       if (two) stf(p + 1, v.y);
     }
   };
-  const int half = (a.K + 1) / 2, items = npoints * half;
+  const unsigned half = (a.K + 1) / 2, items = (unsigned)npoints * half;
+  const int hp = glue_hp(a.H), nbc = 2 * a.G;
   // item = (point, pair of states); consecutive threads take consecutive pairs
-  for (int64_t item = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; item < items; item += (int64_t)gridDim.x * blockDim.x) {
-    const int row = (int)(item / half), k = 2 * (int)(item - (int64_t)row * half), b = row / a.L, l = row - b * a.L;
-    const TD* drow = (const TD*)a.dist + b * a.d_sb + l * a.d_sl;
-    const float* tok = a.tok + (int64_t)row * a.RO;
-    T* dt = (T*)a.dt + (int64_t)row * a.H * a.K + k;
-    T* bc = (T*)a.bc + (int64_t)row * (a.RO - a.H) * a.K + k;
+  for (unsigned item = blockIdx.x * blockDim.x + threadIdx.x; item < items; item += gridDim.x * blockDim.x) {
+    const unsigned row = item / half, b = row / a.L, l = row - b * a.L;
+    const int k = 2 * (int)(item - row * half);
+    const TD* drow = (const TD*)a.dist + b * a.d_sb + l * a.d_sl + (int64_t)k * a.d_sk;
+    const float* tok = a.tok + (size_t)row * a.RO;
     const bool two = k + 1 < a.K;
     float d0[M], d1[M];
-    load_feats<TD, M>(drow + (int64_t)k * a.d_sk, d0);
-    load_feats<TD, M>(drow + (int64_t)(two ? k + 1 : k) * a.d_sk, d1);
+    load_feats<TD, M>(drow, d0);
+    load_feats<TD, M>(drow + (two ? a.d_sk : 0), d1);
     float2 mk = make_float2(1.f, 1.f);
-    if (a.mask) mk = make_float2(a.mask[(int64_t)row * a.K + k], a.mask[(int64_t)row * a.K + (two ? k + 1 : k)]);
+    if (a.mask) mk = make_float2(a.mask[(size_t)row * a.K + k], a.mask[(size_t)row * a.K + (two ? k + 1 : k)]);
     float2 dp[M];
 #pragma unroll
     for (int j = 0; j < M; ++j) dp[j] = make_float2(d0[j], d1[j]);
-#pragma unroll 2
-    for (int r = 0; r < a.H; ++r) {
-      const float t = __ldg(tok + r);
-      const float2 pre = row_dot<M>(sw + r * M, dp, make_float2(t, t));
-      put(dt + (int64_t)r * a.K, __fmul2_rn(make_float2(glue_softplus(pre.x), glue_softplus(pre.y)), mk), two);
-    }
-#pragma unroll 2
-    for (int r = a.H; r < a.RW; ++r) {
-      const float2 pre = row_dot<M>(sw + r * M, dp, make_float2(0.f, 0.f));
-      const float t = __ldg(tok + r);
-      put(bc + (int64_t)(r - a.H) * a.K, __fadd2_rn(pre, make_float2(t, t)), two);
-      if (a.back) {
-        const float u = __ldg(tok + r + 2 * a.G);
-        put(bc + (int64_t)(r - a.H + 2 * a.G) * a.K, __fadd2_rn(pre, make_float2(u, u)), two);
+    T* out = (T*)a.dt + (size_t)row * a.H * a.K + k;
+#pragma unroll 1
+    for (int r = 0; r < hp; r += 4) {
+      float2 pre[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) { const float t = r + q < a.H ? __ldg(tok + r + q) : 0.f; pre[q] = make_float2(t, t); }
+      quad_dot<M>(sw + r * M, dp, pre);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (r + q < a.H) put(out, __fmul2_rn(make_float2(glue_softplus(pre[q].x), glue_softplus(pre[q].y)), mk), two);
+        out += a.K;
       }
+    }
+    out = (T*)a.bc + (size_t)row * (a.RO - a.H) * a.K + k;
+    const float* tk = tok + a.H;
+#pragma unroll 1
+    for (int r = 0; r < nbc; r += 4) {
+      float2 pre[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) pre[q] = make_float2(0.f, 0.f);
+      quad_dot<M>(sw + (hp + r) * M, dp, pre);              // rows past the last one have zero weights
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (r + q < nbc) {
+          const float t = __ldg(tk + r + q);
+          put(out + (r + q) * a.K, __fadd2_rn(pre[q], make_float2(t, t)), two);
+          if (a.back) {
+            const float u = __ldg(tk + nbc + r + q);
+            put(out + (nbc + r + q) * a.K, __fadd2_rn(pre[q], make_float2(u, u)), two);
+          }
+        }
     }
   }
 }
@@ -175,7 +202,7 @@ constexpr int GLUE_BWD_BLOCKS = 148 * 3;                   // two (16 features) 
 //      10 rows x 16 features - in registers over the whole walk.
 // Bound: the fp32 pipe (450 multiply-adds per (point, state)); the block-wide version with staged inputs held 12 warps per SM
 // that met at three barriers per point and used a fifth of the issue slots: 16 x 4096 x 256 x 16 bf16 1730 us.
-// NR: weight rows padded to 12 or 16.
+// NR: weight rows padded to 12 or 20 (dt rows to a multiple of four, then the B / C rows).
 template <typename TD, typename T, int M, int NR>
 __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_bwd(GlueArgs a, int npoints, int pairs_ok) {
   constexpr int RH = NR / 2, MH = M / 2, GS = NR, DS = M + 4;      // rows / features of a lane's tile; row strides in shared memory
@@ -185,7 +212,7 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   float* sg = sg_all[warp];
   float* sd = sd_all[warp];
-  for (int i = threadIdx.x; i < NR * M; i += blockDim.x) { const float w = i < a.RW * M ? a.w[i] : 0.f; sw[i] = make_float2(w, w); }
+  weights_to_smem<M>(a, sw, NR);
   for (int i = lane; i < 64 * GS; i += 32) sg[i] = 0.f;
   __syncthreads();
   const int rh = lane & 1, jh = (lane >> 1) & 1, kq = lane >> 2;   // the lane's tile and its share of the states
@@ -201,7 +228,7 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
     else return v;
   };
   const int per = gridDim.x * GLUE_BWD_WARPS, first = blockIdx.x * GLUE_BWD_WARPS + warp;
-  const int nstep = (a.K + 63) / 64, nb = a.RO - a.H;      // steps per point; B / C gradient rows
+  const int nstep = (a.K + 63) / 64, nb = a.RO - a.H, hp = glue_hp(a.H);      // steps per point; B / C gradient rows; padded dt rows
   uint2 fx[2][FW];
   GP gh[8];                                  // dt gradient rows, loaded eight at a time
   float2 mk;
@@ -291,41 +318,46 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
       else if (pt + per < npoints) load(pt + per, 0);
 #pragma unroll
       for (int j = 0; j < M; ++j) dd[j] = make_float2(0.f, 0.f);
-      float2 gq[4];                                        // g of four rows on their way to sg
 #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        float2 g = make_float2(0.f, 0.f);
-        if (r < a.RW) {
-          const float2* w = sw + r * M;
-          if (r < a.H) {
-            if (a.ddt) {
-              const float t = __ldg(tok + r);
-              const float2 pre = row_dot<M>(w, dp, make_float2(t, t));
-              const float2 s2 = make_float2(pre.x <= 20.f ? glue_sigmoid(pre.x) : 1.f, pre.y <= 20.f ? glue_sigmoid(pre.y) : 1.f);
-              const float2 go = r < 8 ? up(g8[r & 7]) : up(pair_at((const T*)a.ddt + ((int64_t)pt * a.H + r) * a.K + k, in0, in1));
-              g = __fmul2_rn(__fmul2_rn(go, m2), s2);
-            }
-            tsum[r] += g.x + g.y;
-          } else if (pb) {
-            const int q = r - a.H;                         // both directions share the weight row
-            g = q == 0 ? up(gb[0]) : q == 1 ? up(gb[1]) : up(pair_at(pb + (int64_t)q * a.K, in0, in1));
-            if (a.back) {
-              const int q2 = q + 2 * a.G;
-              g = __fadd2_rn(g, q2 == 2 ? up(gb[2]) : q2 == 3 ? up(gb[3]) : up(pair_at(pb + (int64_t)q2 * a.K, in0, in1)));
+      for (int rq = 0; rq < NR; rq += 4) {
+        float2 g[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) g[q] = make_float2(0.f, 0.f);
+        if (rq < hp) {
+          if (a.ddt) {
+            float2 pre[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) { const float t = rq + q < a.H ? __ldg(tok + rq + q) : 0.f; pre[q] = make_float2(t, t); }
+            quad_dot<M>(sw + rq * M, dp, pre);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const int r = rq + q;
+              const float2 s2 = make_float2(pre[q].x <= 20.f ? glue_sigmoid(pre[q].x) : 1.f, pre[q].y <= 20.f ? glue_sigmoid(pre[q].y) : 1.f);
+              float2 go = make_float2(0.f, 0.f);
+              if (r < a.H) go = r < 8 ? up(g8[r & 7]) : up(pair_at((const T*)a.ddt + ((int64_t)pt * a.H + r) * a.K + k, in0, in1));
+              g[q] = __fmul2_rn(__fmul2_rn(go, m2), s2);
+              tsum[r] += g[q].x + g[q].y;
             }
           }
+        } else if (pb) {
 #pragma unroll
-          for (int c = 0; c < M; c += 2) {
-            const float4 q = *(const float4*)(w + c);
-            dd[c] = __ffma2_rn(g, make_float2(q.x, q.y), dd[c]);
-            dd[c + 1] = __ffma2_rn(g, make_float2(q.z, q.w), dd[c + 1]);
+          for (int q = 0; q < 4; ++q) {
+            const int c = rq - hp + q, c2 = c + 2 * a.G;   // both directions share the weight row
+            if (c >= 2 * a.G) continue;
+            g[q] = c == 0 ? up(gb[0]) : c == 1 ? up(gb[1]) : up(pair_at(pb + (int64_t)c * a.K, in0, in1));
+            if (a.back) g[q] = __fadd2_rn(g[q], c2 == 2 ? up(gb[2]) : c2 == 3 ? up(gb[3]) : up(pair_at(pb + (int64_t)c2 * a.K, in0, in1)));
           }
         }
-        gq[r & 3] = g;
-        if ((r & 3) == 3) {
-          *(float4*)(sg + (2 * lane) * GS + r - 3) = make_float4(gq[0].x, gq[1].x, gq[2].x, gq[3].x);
-          *(float4*)(sg + (2 * lane + 1) * GS + r - 3) = make_float4(gq[0].y, gq[1].y, gq[2].y, gq[3].y);
-        }
+#pragma unroll
+        for (int c = 0; c < M; c += 2)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const float4 v = *(const float4*)(sw + (rq + q) * M + c);
+            dd[c] = __ffma2_rn(g[q], make_float2(v.x, v.y), dd[c]);
+            dd[c + 1] = __ffma2_rn(g[q], make_float2(v.z, v.w), dd[c + 1]);
+          }
+        *(float4*)(sg + (2 * lane) * GS + rq) = make_float4(g[0].x, g[1].x, g[2].x, g[3].x);
+        *(float4*)(sg + (2 * lane + 1) * GS + rq) = make_float4(g[0].y, g[1].y, g[2].y, g[3].y);
       }
       if (pb) {                                            // token terms of the B / C rows (each output row has its own)
 #pragma unroll
@@ -395,9 +427,10 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
     }
   __syncthreads();
   for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) {
+    const int r = i / M, at = (r < a.H ? r : hp + r - a.H) * M + i % M;
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < GLUE_BWD_WARPS; ++w) t += sg_all[w][i];
+    for (int w = 0; w < GLUE_BWD_WARPS; ++w) t += sg_all[w][at];
     a.dwpart[(size_t)blockIdx.x * GLUE_MAX_ROWS * M + i] = t;
   }
 }
@@ -458,7 +491,7 @@ extern "C" int issm_b200_glue_fwd(const issm_glue_params* p, void* stream) {
   int rc = glue_validate(p, false);
   if (rc) return rc;
   const GlueArgs a = glue_args(*p);
-  if ((int64_t)p->batch * p->seqlen * ((p->nstates + 1) / 2) > 0x7fffffff) return ISSM_ERR_SHAPE;
+  if ((int64_t)p->batch * p->seqlen * ((p->nstates + 1) / 2) > 0x7fffffff - 148 * 16 * 128) return ISSM_ERR_SHAPE;
   const int npoints = p->batch * p->seqlen;
   const int64_t want = cdiv64((int64_t)npoints * ((p->nstates + 1) / 2), 128);
   const unsigned grid = (unsigned)(want < GLUE_FWD_BLOCKS ? want : GLUE_FWD_BLOCKS);
@@ -500,8 +533,8 @@ extern "C" int issm_b200_glue_bwd(const issm_glue_params* p, void* stream) {
   const int pairs_ok = !(p->nstates & 1) && !((uintptr_t)p->ddt % (2 * es)) && !((uintptr_t)p->dbc % (2 * es));
 #define GLUE_BWD(TD, TT, MM)                                                                          \
   do {                                                                                                \
-    if (a.RW <= 12) ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 12>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok); \
-    else ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 16>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok);            \
+    if (glue_hp(a.H) + 2 * a.G <= 12) ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 12>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok); \
+    else ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 20>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok);            \
   } while (0)
 #define GLUE_BWD_M(TD, TT)                                                                            \
   do {                                                                                                \

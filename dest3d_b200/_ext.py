@@ -1,5 +1,6 @@
 """Loader of the torch C++ extension (`libissm_b200_torch.so`, TORCH_LIBRARY namespace `issm_b200`): ops
-`fwd`, `bwd`, `norm_fwd`, `norm_bwd` over the C ABI.  Like the C-ABI library itself it has to be built first;
+`fwd`, `bwd`, `norm_fwd`, `norm_bwd` over the C ABI and the differentiable `scan`, `bi_scan`, `norm`, `conv_silu`, `reorder`,
+`dt_bc` and `block`.  Like the C-ABI library itself it has to be built first;
 there is no fallback."""
 import os
 
@@ -22,6 +23,17 @@ def ops():
         torch.ops.load_library(_EXT_PATH)
         _loaded = True
     return torch.ops.issm_b200
+
+
+_calls = {}
+
+
+def call(name):
+    """One operation of the extension, resolved once (the packet lookup costs as much as a small call)."""
+    f = _calls.get(name)
+    if f is None:
+        f = _calls[name] = getattr(ops(), name).default
+    return f
 
 
 def opt(t):

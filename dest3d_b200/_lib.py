@@ -66,7 +66,7 @@ class IssmGlueParams(C.Structure):
         [(n, i32) for n in ("batch", "seqlen", "nstates", "nfeat", "nheads", "ngroups", "has_back", "io_dtype", "dist_dtype")]
         + [("dist", vp), ("dist_sb", i64), ("dist_sl", i64), ("dist_sk", i64), ("weight", vp), ("tok", vp), ("mask", vp),
            ("dt", vp), ("bc", vp), ("ddt", vp), ("dbc", vp), ("ddist", vp), ("dweight", vp), ("dtok", vp),
-           ("workspace", vp), ("workspace_bytes", C.c_size_t)]
+           ("workspace", vp), ("workspace_bytes", C.c_size_t), ("weight_bc", vp), ("dbc_part", vp * 4)]
     )
 
 

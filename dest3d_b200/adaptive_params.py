@@ -11,12 +11,15 @@ import ctypes as ct
 
 import torch
 
-from . import _lib
+from . import _ext, _lib, issm_combined
 
 
 def _empty(shape, dtype, device):
     """Every output and workspace of this module is allocated here (the guard-band tests substitute it)."""
     return torch.empty(tuple(shape), dtype=dtype, device=device)
+
+
+_default_empty = _empty
 
 
 def _params(dist, w, tok, mask, H, G, back, out_dtype):
@@ -97,6 +100,9 @@ def adaptive_dt_bc(dist, dt_proj_weight, bc_proj_weight, dt_bias_tok, dt_bias, b
     bfloat16 next to a float32 dist is what autocast calls for, without a cast pass over dist).  Returns (dt, B, C) or (dt, B, C, B_back, C_back)."""
     H, G = dt_proj_weight.shape[0], bc_proj_weight.shape[0] // 2
     back = b_bias_back is not None
+    if issm_combined.BINDING == "torch" and _empty is _default_empty:      # the C++ operation; a substituted allocator keeps to the code below
+        src = [dt_bias_tok, b_bias, c_bias] + ([b_bias_back, c_bias_back] if back else [])
+        return tuple(_ext.call("dt_bc")(dist, dt_proj_weight, bc_proj_weight, dt_bias, mask, out_dtype or dist.dtype, src))
     terms = [dt_bias_tok.float() + dt_bias.float(), b_bias.float(), c_bias.float()]
     if back:
         terms += [b_bias_back.float(), c_bias_back.float()]

@@ -13,7 +13,8 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 LIB = os.path.join(PKG, "libissm_b200.so")
 TORCH_LIB = os.path.join(PKG, "libissm_b200_torch.so")
-TORCH_SRC = os.path.join(CSRC, "issm_torch.cpp")
+TORCH_SRCS = [os.path.join(CSRC, f) for f in ("issm_torch.cpp", "issm_autograd.cpp")]
+TORCH_DEPS = TORCH_SRCS + [os.path.join(CSRC, "issm_torch.h")]
 SOURCES = ["issm_abi.cu", "issm_simt.cu", "issm_blocked.cu", "issm_norm.cu", "issm_tensor.cu", "issm_tensor_fwd.cu", "issm_tensor_bwd.cu", "issm_pointops.cu", "issm_seqpar.cu", "issm_glue.cu", "issm_combine.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-shared", "-Xptxas", "-v"]
@@ -33,15 +34,15 @@ def _stale():
     if not os.path.exists(LIB):
         return True
     t = os.path.getmtime(LIB)
-    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith(".cpp")] + [HEADER]
+    deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if not f.endswith((".cpp", "issm_torch.h"))] + [HEADER]
     return any(os.path.getmtime(d) > t for d in deps)
 
 
 def build_torch_extension(force=False, verbose=False):
-    """Compile csrc/issm_torch.cpp against the installed torch and link it to libissm_b200.so (found next to
+    """Compile csrc/issm_torch.cpp and issm_autograd.cpp against the installed torch and link it to libissm_b200.so (found next to
     it at run time through an $ORIGIN rpath).  Returns the extension's path."""
     if (not force and os.path.exists(TORCH_LIB)
-            and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_LIB) for d in (TORCH_SRC, HEADER, LIB))):
+            and all(os.path.getmtime(d) <= os.path.getmtime(TORCH_LIB) for d in TORCH_DEPS + [HEADER, LIB])):
         return TORCH_LIB
     import torch
     from torch.utils import cpp_extension as ce
@@ -49,7 +50,7 @@ def build_torch_extension(force=False, verbose=False):
     # the host compiler nvcc itself uses (g++ on PATH), so that the extension shares the process-wide libstdc++ with
     # torch: a compiler that links its own C++ runtime statically breaks exceptions thrown across the libraries
     cmd = ([os.environ.get("ISSM_B200_CXX") or shutil.which("g++") or "g++", "-O2", "-std=c++17", "-fPIC", "-shared",
-            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", TORCH_SRC]
+            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"] + TORCH_SRCS
            + [f"-I{d}" for d in ce.include_paths()] + [f"-I{os.path.join(cuda_home, 'include')}"]
            + [f"-L{d}" for d in ce.library_paths()] + ["-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch",
               f"-L{PKG}", "-lissm_b200", "-Wl,-rpath,$ORIGIN", "-o", TORCH_LIB])

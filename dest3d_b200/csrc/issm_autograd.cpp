@@ -1,0 +1,451 @@
+// The library's differentiable operations as C++ autograd functions (`torch.ops.issm_b200.*`): the calls of a training or
+// inference step at the detector's sizes are bound by host time, and a Python autograd function costs two interpreter round
+// trips and its argument parsing per direction.  Same checks, results and dtypes as the Python classes they stand in for
+// (issm_combined.py, layernorm_gated.py, pointops.py, adaptive_params.py), which remain for the foreign-language binding.
+// Host code only; every kernel is behind the C ABI.
+#include "issm_torch.h"
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAException.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/library.h>
+
+#include <cstdlib>
+#include <cstring>
+#include <mutex>
+
+namespace issm_host {
+using torch::autograd::AutogradContext;
+using torch::autograd::Function;
+using torch::autograd::variable_list;
+
+// ---- device status word ------------------------------------------------------------------------------------------------
+// One pinned copy per device, enqueued behind a call's kernels, looked at by a later call once it has landed; one copy in
+// flight at a time.  Surfaces bit 0 (a bounded wait expired) without blocking; nothing happens inside a graph capture.
+void check_status(const Tensor& status, const char* what) {
+  struct Mirror {
+    std::mutex mu;
+    int* host = nullptr;
+    cudaEvent_t ev = nullptr;
+    bool pending = false;
+  };
+  static Mirror mirrors[64];
+  const int dev = status.device().index();
+  if (dev < 0 || dev >= 64) return;
+  const cudaStream_t s = c10::cuda::getCurrentCUDAStream(dev).stream();
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) { (void)cudaGetLastError(); return; }
+  int value = 0;
+  {
+    Mirror& m = mirrors[dev];
+    std::lock_guard<std::mutex> lock(m.mu);
+    if (!m.host) {
+      C10_CUDA_CHECK(cudaHostAlloc((void**)&m.host, sizeof(int), cudaHostAllocDefault));
+      *m.host = 0;
+      C10_CUDA_CHECK(cudaEventCreateWithFlags(&m.ev, cudaEventDisableTiming));
+    }
+    const char* now = std::getenv("ISSM_B200_CHECK_STATUS");
+    const bool sync = now && !std::strcmp(now, "1");       // debug aid: every call synchronises and raises at once
+    if (m.pending) {
+      const cudaError_t q = sync ? cudaEventSynchronize(m.ev) : cudaEventQuery(m.ev);
+      if (q == cudaSuccess) { m.pending = false; value |= *m.host; }
+      else (void)cudaGetLastError();
+    }
+    if (!m.pending) {
+      C10_CUDA_CHECK(cudaMemcpyAsync(m.host, status.data_ptr<int>(), sizeof(int), cudaMemcpyDeviceToHost, s));
+      C10_CUDA_CHECK(cudaEventRecord(m.ev, s));
+      m.pending = true;
+      if (sync) {
+        C10_CUDA_CHECK(cudaEventSynchronize(m.ev));
+        m.pending = false;
+        value |= *m.host;
+      }
+    }
+    if (value & 1) {
+      if (m.pending) { C10_CUDA_CHECK(cudaEventSynchronize(m.ev)); m.pending = false; }
+      *m.host = 0;
+      C10_CUDA_CHECK(cudaMemsetAsync(status.data_ptr<int>(), 0, sizeof(int), s));
+    }
+  }
+  TORCH_CHECK(!(value & 1), what, ": a bounded device-side wait expired in an earlier ISSM call on ", status.device(), " (status ", value,
+              "); the results of that call are invalid");
+}
+
+static Tensor like(const Tensor& g, const Tensor& ref) { return g.scalar_type() == ref.scalar_type() ? g : g.to(ref.scalar_type()); }
+static OptTensor some(const Tensor& t) { return t.defined() ? OptTensor(t) : OptTensor(); }
+static Tensor none(const OptTensor& t) { return t ? *t : Tensor(); }
+static Tensor filled(const Tensor& t) { return t.defined() && t.numel() ? t : Tensor(); }
+
+// ---- scans -------------------------------------------------------------------------------------------------------------
+struct ScanFn : public Function<ScanFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C,
+                               int64_t chunk, const OptTensor& D, const OptTensor& z, const OptTensor& bias, const OptTensor& init, bool softplus,
+                               double lo, double hi, bool want_final, bool reverse, int64_t path, const Tensor& status, bool need) {
+    ctx->set_materialize_grads(false);
+    auto [out, out_x, fin, saved] = fwd(x, dt, A, B, C, chunk, D, z, bias, init, softplus, lo, hi, reverse, path, want_final, need, status);
+    check_status(status, "issm_b200_fwd");
+    if (need) {
+      ctx->save_for_backward({x, dt, A, B, C, none(D), none(z), none(bias), none(init), filled(out_x), filled(saved), status});
+      ctx->saved_data["i"] = c10::IValue(std::vector<int64_t>{chunk, softplus, reverse, path});
+      ctx->saved_data["f"] = c10::IValue(std::vector<double>{lo, hi});
+    }
+    if (want_final) return {out, fin};
+    return {out};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const auto i = ctx->saved_data["i"].toIntVector();
+    const auto f = ctx->saved_data["f"].toDoubleVector();
+    variable_list r(18);
+    const Tensor dfin = g.size() > 1 ? g[1] : Tensor();
+    if (!g[0].defined() && !dfin.defined()) return r;
+    const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(s[0]);
+    auto [dx, ddt, dA, dB, dC, dD, dz, db, di] = bwd(dout, s[0], s[1], s[2], s[3], s[4], some(s[9]), i[0], some(s[5]), some(s[6]), some(s[7]), some(s[8]),
+                                                     some(dfin), i[1] != 0, f[0], f[1], i[2] != 0, i[3], some(s[10]), s[11]);
+    check_status(s[11], "issm_b200_bwd");
+    r[0] = dx; r[1] = like(ddt, s[1]); r[2] = like(dA, s[2]); r[3] = like(dB, s[3]); r[4] = like(dC, s[4]);
+    if (s[5].defined()) r[6] = like(dD, s[5]);
+    if (s[6].defined()) r[7] = like(dz, s[6]);
+    if (s[7].defined()) r[8] = like(s[7].dim() == 2 ? db : db.sum(1), s[7]);
+    if (s[8].defined()) r[9] = like(di, s[8]);
+    return r;
+  }
+};
+
+struct BiScanFn : public Function<BiScanFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& xb, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C,
+                               const Tensor& Bb, const Tensor& Cb, int64_t chunk, const OptTensor& D, const OptTensor& z, const OptTensor& bias,
+                               const OptTensor& init, bool softplus, double lo, double hi, double scale, int64_t path, const Tensor& status, bool need) {
+    ctx->set_materialize_grads(false);
+    auto [out, fin, ox, oxb, sf, sb] = bi_fwd(x, xb, dt, A, B, C, Bb, Cb, chunk, D, z, bias, init, softplus, lo, hi, scale, path, need, status);
+    check_status(status, "issm_b200_fwd");
+    if (need) {
+      ctx->save_for_backward({x, xb, dt, A, B, C, Bb, Cb, none(D), none(z), none(bias), none(init), filled(ox), filled(oxb), filled(sf), filled(sb), status});
+      ctx->saved_data["i"] = c10::IValue(std::vector<int64_t>{chunk, softplus, path});
+      ctx->saved_data["f"] = c10::IValue(std::vector<double>{lo, hi, scale});
+    }
+    return {out, fin};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const auto i = ctx->saved_data["i"].toIntVector();
+    const auto f = ctx->saved_data["f"].toDoubleVector();
+    variable_list r(20);
+    if (!g[0].defined() && !g[1].defined()) return r;
+    const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(s[0]);
+    auto [dx, dxb, ddt, dA, dB, dC, dBb, dCb, dD, dz, db, di] =
+        bi_bwd(dout, some(g[1]), s[0], s[1], s[2], s[3], s[4], s[5], s[6], s[7], some(s[12]), some(s[13]), i[0], some(s[8]), some(s[9]), some(s[10]),
+               some(s[11]), i[1] != 0, f[0], f[1], f[2], i[2], some(s[14]), some(s[15]), s[16]);
+    check_status(s[16], "issm_b200_bwd");
+    r[0] = dx; r[1] = like(dxb, s[1]); r[2] = like(ddt, s[2]); r[3] = like(dA, s[3]);
+    r[4] = like(dB, s[4]); r[5] = like(dC, s[5]); r[6] = like(dBb, s[6]); r[7] = like(dCb, s[7]);
+    if (s[8].defined()) r[9] = like(dD, s[8]);
+    if (s[9].defined()) r[10] = like(dz, s[9]);
+    if (s[10].defined()) r[11] = like(s[10].dim() == 2 ? db : db.sum(1), s[10]);
+    if (s[11].defined()) r[12] = like(di, s[11]);
+    return r;
+  }
+};
+
+// ---- gated norms -------------------------------------------------------------------------------------------------------
+static Tensor rows_of(const Tensor& t) {
+  Tensor r = t.reshape({-1, t.size(-1)});
+  return r.stride(-1) == 1 ? r : r.contiguous();
+}
+static Tensor f32(const Tensor& t) { return t.detach().to(at::kFloat).contiguous(); }
+
+struct NormFn : public Function<NormFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const OptTensor& b, const OptTensor& z, double eps, int64_t group,
+                        bool before, bool rms) {
+    TORCH_CHECK(x.is_cuda(), "the gated norm runs on CUDA tensors only; there is no CPU path");
+    const Tensor x2 = rows_of(x);
+    OptTensor z2;
+    if (z) {
+      TORCH_CHECK(z->sizes() == x.sizes(), "issm_b200: z must have the shape of x");
+      z2 = rows_of(z->scalar_type() == x.scalar_type() ? *z : z->to(x.scalar_type()));
+    }
+    const OptTensor bf = b ? OptTensor(f32(*b)) : OptTensor();
+    auto [y, rstd, mean] = norm_fwd(x2, z2, f32(w), bf, eps, group, before, rms);
+    ctx->save_for_backward({x2, w, none(b), filled(mean), rstd, none(z2)});
+    ctx->saved_data["s"] = c10::IValue(x.sizes().vec());
+    ctx->saved_data["i"] = c10::IValue(std::vector<int64_t>{group, before, rms, z ? (int64_t)z->scalar_type() : 0});
+    ctx->saved_data["e"] = c10::IValue(eps);
+    return y.reshape(x.sizes());
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const auto i = ctx->saved_data["i"].toIntVector();
+    const auto shape = ctx->saved_data["s"].toIntVector();
+    const Tensor dy = rows_of(g[0].scalar_type() == s[0].scalar_type() ? g[0] : g[0].to(s[0].scalar_type()));
+    auto [dx, dz, dw, db] = norm_bwd(dy, s[0], some(s[5]), f32(s[1]), s[2].defined() ? OptTensor(f32(s[2])) : OptTensor(), s[4], some(s[3]),
+                                     ctx->saved_data["e"].toDouble(), i[0], i[1] != 0, i[2] != 0);
+    variable_list r(8);
+    r[0] = dx.reshape(shape);
+    r[1] = like(dw, s[1]);
+    if (s[2].defined()) r[2] = like(db, s[2]);
+    if (s[5].defined()) {
+      const Tensor t = dz.reshape(shape);
+      const auto zt = (at::ScalarType)i[3];
+      r[3] = t.scalar_type() == zt ? t : t.to(zt);
+    }
+    return r;
+  }
+};
+
+// ---- PointLiteConv, row gather -------------------------------------------------------------------------------------------
+static issm_conv_params conv_params(const Tensor& x, const Tensor& w, const OptTensor& b) {
+  issm_conv_params p{};
+  p.batch = (int32_t)x.size(0); p.seqlen = (int32_t)x.size(1); p.channels = (int32_t)x.size(2);
+  p.io_dtype = dtype_code(x.scalar_type());
+  p.x = x.data_ptr(); p.x_sb = x.stride(0); p.x_sl = x.stride(1);
+  p.weight = w.data_ptr<float>();
+  p.bias = b ? b->data_ptr<float>() : nullptr;
+  return p;
+}
+struct ConvFn : public Function<ConvFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& xi, const Tensor& w, const OptTensor& b) {
+    TORCH_CHECK(xi.is_cuda(), "dest3d_b200.pointops runs on CUDA tensors only");
+    TORCH_CHECK_VALUE(xi.dim() == 3 && w.dim() == 3 && w.size(0) == xi.size(2) && w.size(1) == 1 && w.size(2) == 7, "x must be (B, N, C) and weight (C, 1, 7)");
+    const c10::cuda::CUDAGuard guard(xi.device());
+    const Tensor x = xi.stride(2) == 1 ? xi : xi.contiguous();
+    Tensor y = at::empty(x.sizes(), x.options());
+    if (y.numel()) {
+      const Tensor wf = f32(w);
+      const OptTensor bf = b ? OptTensor(f32(*b)) : OptTensor();
+      issm_conv_params p = conv_params(x, wf, bf);
+      p.y = y.data_ptr();
+      check_rc(issm_b200_dwconv7_silu_fwd(&p, stream_of(x)), "issm_b200_dwconv7_silu_fwd");
+    }
+    ctx->save_for_backward({x, w, none(b)});
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const Tensor& x = s[0];
+    const c10::cuda::CUDAGuard guard(x.device());
+    Tensor dy = g[0].stride(2) == 1 ? g[0] : g[0].contiguous();
+    if (dy.scalar_type() != x.scalar_type()) dy = dy.to(x.scalar_type());
+    const auto fo = x.options().dtype(at::kFloat);
+    Tensor dx = at::empty(x.sizes(), x.options()), dw = at::empty({x.size(2), 7}, fo), db = s[2].defined() ? at::empty({x.size(2)}, fo) : Tensor();
+    if (!x.numel()) {
+      dw.zero_();
+      if (db.defined()) db.zero_();
+    } else {
+      const Tensor wf = f32(s[1]);
+      const OptTensor bf = s[2].defined() ? OptTensor(f32(s[2])) : OptTensor();
+      issm_conv_params p = conv_params(x, wf, bf);
+      p.dy = dy.data_ptr(); p.dy_sb = dy.stride(0); p.dy_sl = dy.stride(1);
+      p.dx = dx.data_ptr(); p.dweight = dw.data_ptr<float>(); p.dbias = db.defined() ? db.data_ptr<float>() : nullptr;
+      const size_t need = issm_b200_dwconv_workspace_bytes(&p);
+      Tensor ws = at::empty({(int64_t)need}, x.options().dtype(at::kByte));
+      p.workspace = ws.data_ptr(); p.workspace_bytes = need;
+      check_rc(issm_b200_dwconv7_silu_bwd(&p, stream_of(x)), "issm_b200_dwconv7_silu_bwd");
+    }
+    return {dx, like(dw.reshape(s[1].sizes()), s[1]), db.defined() ? like(db, s[2]) : Tensor()};
+  }
+};
+
+static Tensor gather_rows(const Tensor& src_, const Tensor& index_) {
+  TORCH_CHECK(src_.is_cuda(), "dest3d_b200.pointops runs on CUDA tensors only");
+  TORCH_CHECK_VALUE(src_.dim() == 3 && index_.dim() == 2 && index_.size(0) == src_.size(0), "points must be (B, N, C) and index (B, M)");
+  const c10::cuda::CUDAGuard guard(src_.device());
+  const Tensor src = src_.stride(2) == 1 ? src_ : src_.contiguous(), index = index_.to(at::kLong).contiguous();
+  Tensor dst = at::empty({src.size(0), index.size(1), src.size(2)}, src.options());
+  if (!dst.numel()) return dst;
+  TORCH_CHECK_INDEX(src.size(1) > 0, "reorder_points: gather from an empty point set");
+  const int64_t es = src.element_size();
+  TORCH_CHECK_VALUE((src.size(2) * es) % 2 == 0, "rows must be an even number of bytes");
+  check_rc(issm_b200_gather_rows(src.data_ptr(), index.data_ptr<int64_t>(), dst.data_ptr(), (int32_t)src.size(0), (int32_t)index.size(1), (int32_t)src.size(1),
+                                 src.size(2) * es, src.stride(0) * es, src.stride(1) * es, nullptr, stream_of(src)), "issm_b200_gather_rows");
+  return dst;
+}
+struct ReorderFn : public Function<ReorderFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& points, const Tensor& index, const OptTensor& inverse) {
+    ctx->save_for_backward({index, none(inverse)});
+    ctx->saved_data["n"] = c10::IValue(points.size(1));
+    return gather_rows(points, index);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    if (s[1].defined()) return {gather_rows(g[0], s[1]), Tensor(), Tensor()};          // a permutation: the adjoint is the inverse gather
+    Tensor d = at::zeros({g[0].size(0), ctx->saved_data["n"].toInt(), g[0].size(2)}, g[0].options());
+    d.scatter_add_(1, s[0].unsqueeze(-1).expand({-1, -1, g[0].size(2)}), g[0]);
+    return {d, Tensor(), Tensor()};
+  }
+};
+
+// ---- dt / B / C generation -----------------------------------------------------------------------------------------------
+static issm_glue_params glue_params(const Tensor& dist, const Tensor& w, const Tensor& wbc, const Tensor& tok, const Tensor& mask, int64_t H, int64_t G, bool back,
+                                    at::ScalarType out) {
+  issm_glue_params p{};
+  p.batch = (int32_t)dist.size(0); p.seqlen = (int32_t)dist.size(1); p.nstates = (int32_t)dist.size(2); p.nfeat = (int32_t)dist.size(3);
+  p.nheads = (int32_t)H; p.ngroups = (int32_t)G; p.has_back = back;
+  p.io_dtype = dtype_code(out); p.dist_dtype = dtype_code(dist.scalar_type());
+  p.dist = dist.data_ptr(); p.dist_sb = dist.stride(0); p.dist_sl = dist.stride(1); p.dist_sk = dist.stride(2);
+  p.weight = w.data_ptr<float>(); p.weight_bc = wbc.data_ptr<float>(); p.tok = tok.data_ptr<float>();
+  p.mask = mask.defined() ? mask.data_ptr<float>() : nullptr;
+  return p;
+}
+struct GlueFn : public Function<GlueFn> {
+  // terms: dt_tok (b, L, H), then b_bias, c_bias (, b_bias_back, c_bias_back) (b, L, G)
+  static variable_list forward(AutogradContext* ctx, const Tensor& dist_, const Tensor& w_dt, const Tensor& w_bc, const Tensor& dt_bias, const OptTensor& mask_,
+                               at::ScalarType out, at::TensorList terms_) {
+    TORCH_CHECK(dist_.is_cuda(), "dest3d_b200.adaptive_params runs on CUDA tensors only");
+    TORCH_CHECK_TYPE(out == dist_.scalar_type() || (dist_.scalar_type() == at::kFloat && out == at::kBFloat16),
+                     "adaptive_dt_bc: outputs take the dtype of dist, or bfloat16 next to a float32 dist");
+    const c10::cuda::CUDAGuard guard(dist_.device());
+    const Tensor dist = dist_.stride(3) == 1 ? dist_ : dist_.contiguous();
+    const int64_t b = dist.size(0), L = dist.size(1), K = dist.size(2), H = w_dt.size(0), G = w_bc.size(0) / 2;
+    const bool back = terms_.size() == 5;
+    const Tensor w = f32(w_dt), wbc = f32(w_bc), bias = f32(dt_bias), mask = mask_ ? f32(*mask_) : Tensor();
+    issm_glue_tok t{};
+    t.batch = (int32_t)b; t.seqlen = (int32_t)L; t.nheads = (int32_t)H; t.ngroups = (int32_t)G; t.nsrc = (int32_t)terms_.size();
+    std::vector<Tensor> keep;
+    std::vector<int64_t> types;
+    for (size_t i = 0; i < terms_.size(); ++i) {
+      Tensor x = terms_[i];
+      TORCH_CHECK(x.dim() == 3 && x.size(0) == b && x.size(1) == L && x.size(2) == (i ? G : H), "adaptive_dt_bc: token terms must be (b, L, H) and (b, L, G)");
+      types.push_back((int64_t)x.scalar_type());
+      if (x.scalar_type() != at::kFloat && x.scalar_type() != at::kBFloat16) x = x.to(at::kFloat);
+      if (x.stride(2) != 1 && x.size(2) > 1) x = x.contiguous();
+      keep.push_back(x);
+      t.dtype[i] = dtype_code(x.scalar_type()); t.src[i] = x.data_ptr(); t.sb[i] = x.stride(0); t.sl[i] = x.stride(1);
+    }
+    const int64_t RO = H + 2 * G * (back ? 2 : 1);
+    Tensor tok = at::empty({b, L, RO}, dist.options().dtype(at::kFloat));
+    t.dt_bias = bias.data_ptr<float>(); t.tok = tok.data_ptr<float>();
+    check_rc(issm_b200_glue_tok_pack(&t, stream_of(dist)), "issm_b200_glue_tok_pack");
+    const auto o = dist.options().dtype(out);
+    Tensor dt = at::empty({b, L, H, K}, o), bc = at::empty({b, L, RO - H, K}, o);
+    issm_glue_params p = glue_params(dist, w, wbc, tok, mask, H, G, back, out);
+    p.dt = dt.data_ptr(); p.bc = bc.data_ptr();
+    check_rc(issm_b200_glue_fwd(&p, stream_of(dist)), "issm_b200_glue_fwd");
+    ctx->save_for_backward({dist, w, wbc, tok, mask, w_dt, w_bc, dt_bias});
+    types.push_back((int64_t)out);
+    ctx->saved_data["t"] = c10::IValue(types);
+    ctx->set_materialize_grads(false);
+    variable_list r{dt};
+    for (int64_t i = 0; i < (RO - H) / G; ++i) r.push_back(bc.slice(2, i * G, (i + 1) * G));
+    return r;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const auto types = ctx->saved_data["t"].toIntVector();
+    const Tensor &dist = s[0], &w = s[1], &wbc = s[2], &tok = s[3], &mask = s[4];
+    const c10::cuda::CUDAGuard guard(dist.device());
+    const int64_t b = dist.size(0), L = dist.size(1), H = w.size(0), G = wbc.size(0) / 2, M = dist.size(3);
+    const size_t nt = types.size() - 1;
+    const auto out = (at::ScalarType)types.back();
+    const auto fo = dist.options().dtype(at::kFloat);
+    Tensor ddist = at::empty(dist.sizes(), dist.options().memory_format(at::MemoryFormat::Contiguous)), dw = at::empty({H + 2 * G, M}, fo), dtok = at::empty(tok.sizes(), fo);
+    issm_glue_params p = glue_params(dist, w, wbc, tok, mask, H, G, nt == 5, out);
+    std::vector<Tensor> keep;
+    for (size_t i = 0; i < g.size(); ++i) {
+      if (!g[i].defined()) continue;
+      keep.push_back((g[i].scalar_type() == out ? g[i] : g[i].to(out)).contiguous());
+      if (i == 0) p.ddt = keep.back().data_ptr();
+      else p.dbc_part[i - 1] = keep.back().data_ptr();
+    }
+    p.ddist = ddist.data_ptr(); p.dweight = dw.data_ptr<float>(); p.dtok = dtok.data_ptr<float>();
+    const size_t need = issm_b200_glue_workspace_bytes(&p);
+    Tensor ws = at::empty({(int64_t)need}, dist.options().dtype(at::kByte));
+    p.workspace = ws.data_ptr(); p.workspace_bytes = need;
+    check_rc(issm_b200_glue_bwd(&p, stream_of(dist)), "issm_b200_glue_bwd");
+    issm_glue_tok t{};
+    t.batch = (int32_t)b; t.seqlen = (int32_t)L; t.nheads = (int32_t)H; t.ngroups = (int32_t)G; t.nsrc = (int32_t)nt;
+    t.dtok = dtok.data_ptr<float>();
+    variable_list r(6 + nt);
+    for (size_t i = 0; i < nt; ++i) {
+      const auto st = (at::ScalarType)types[i];
+      const auto kt = st == at::kFloat || st == at::kBFloat16 ? st : at::kFloat;
+      r[6 + i] = at::empty({b, L, i ? G : H}, dist.options().dtype(kt));
+      t.dtype[i] = dtype_code(kt);
+      t.dsrc[i] = r[6 + i].data_ptr();
+    }
+    check_rc(issm_b200_glue_tok_unpack(&t, stream_of(dist)), "issm_b200_glue_tok_unpack");
+    for (size_t i = 0; i < nt; ++i)
+      if (r[6 + i].scalar_type() != (at::ScalarType)types[i]) r[6 + i] = r[6 + i].to((at::ScalarType)types[i]);
+    r[0] = ddist;
+    r[1] = like(dw.slice(0, 0, H), s[5]);
+    r[2] = like(dw.slice(0, H), s[6]);
+    r[3] = like(dtok.slice(2, 0, H).sum(at::IntArrayRef{0, 1}), s[7]);
+    return r;
+  }
+};
+
+// ---- what Python calls -----------------------------------------------------------------------------------------------------
+static bool wants_grad(std::initializer_list<const Tensor*> req, std::initializer_list<const OptTensor*> opt) {
+  if (!at::GradMode::is_enabled()) return false;
+  for (const Tensor* t : req)
+    if (t->requires_grad()) return true;
+  for (const OptTensor* t : opt)
+    if (*t && (*t)->requires_grad()) return true;
+  return false;
+}
+std::vector<Tensor> scan(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, const OptTensor& D,
+                         const OptTensor& z, const OptTensor& bias, const OptTensor& init, bool softplus, double lo, double hi, bool want_final,
+                         bool reverse, int64_t path, const Tensor& status) {
+  return ScanFn::apply(x, dt, A, B, C, chunk, D, z, bias, init, softplus, lo, hi, want_final, reverse, path, status,
+                       wants_grad({&x, &dt, &A, &B, &C}, {&D, &z, &bias, &init}));
+}
+std::tuple<Tensor, Tensor> bi_scan(const Tensor& x, const Tensor& xb, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& Bb,
+                                   const Tensor& Cb, int64_t chunk, const OptTensor& D, const OptTensor& z, const OptTensor& bias, const OptTensor& init,
+                                   bool softplus, double lo, double hi, double scale, int64_t path, const Tensor& status) {
+  const auto r = BiScanFn::apply(x, xb, dt, A, B, C, Bb, Cb, chunk, D, z, bias, init, softplus, lo, hi, scale, path, status,
+                                 wants_grad({&x, &xb, &dt, &A, &B, &C, &Bb, &Cb}, {&D, &z, &bias, &init}));
+  return {r[0], r[1]};
+}
+Tensor norm(const Tensor& x, const Tensor& w, const OptTensor& b, const OptTensor& z, double eps, int64_t group, bool before, bool rms) {
+  return NormFn::apply(x, w, b, z, eps, group, before, rms);
+}
+Tensor conv_silu(const Tensor& x, const Tensor& w, const OptTensor& b) { return ConvFn::apply(x, w, b); }
+Tensor reorder(const Tensor& points, const Tensor& index, const OptTensor& inverse) { return ReorderFn::apply(points, index, inverse); }
+std::vector<Tensor> dt_bc(const Tensor& dist, const Tensor& w_dt, const Tensor& w_bc, const Tensor& dt_bias, const OptTensor& mask, at::ScalarType out,
+                          at::TensorList terms) {
+  // bool mask: dt is zeroed where it is true (models/dest_module.py:554-558)
+  const OptTensor m = mask && mask->scalar_type() == at::kBool ? OptTensor(mask->logical_not().to(at::kFloat)) : mask;
+  return GlueFn::apply(dist, w_dt, w_bc, dt_bias, m, out, terms);
+}
+
+// The bidirectional ISSM block (issm_block.py MultiHeadISSMScan.forward; models/dest_module.py:519-612) in one call.  Ordinary
+// differentiable operations in order; autocast applies to the projections and the layer norm as it does from Python.
+std::tuple<Tensor, Tensor> block(const Tensor& in_key, const Tensor& in_query, const Tensor& dist, const OptTensor& mask, const Tensor& key_w,
+                                 const Tensor& conv_w, const OptTensor& conv_b, const Tensor& convb_w, const OptTensor& convb_b, const Tensor& query_w,
+                                 const Tensor& bc_w, const Tensor& dt_w, const Tensor& dt_bias, const Tensor& A_log, const Tensor& D, const Tensor& kn_w,
+                                 double kn_eps, const Tensor& okey_w, const Tensor& qn_w, const OptTensor& qn_b, double qn_eps, const Tensor& oquery_w,
+                                 int64_t H, int64_t G, int64_t d_state, int64_t chunk, double lo, double hi, const Tensor& status) {
+  const int64_t di = query_w.size(0), P = di / H;
+  const Tensor zx = at::linear(in_key, key_w);
+  const Tensor z = zx.narrow(-1, 0, di), dt_tok = zx.narrow(-1, 2 * di + 2 * G, H);
+  const Tensor xbc = conv_silu(zx.narrow(-1, di, di + 2 * G), conv_w, conv_b);
+  const Tensor back = conv_silu(xbc, convb_w, convb_b);    // the second convolution takes the OUTPUT of the first (dest_module.py:534)
+  const auto b = in_key.size(0), L = in_key.size(1), K = in_query.size(1);
+  auto heads = [&](const Tensor& t) { return t.narrow(-1, 0, di).contiguous().view({b, L, H, P}); };
+  const Tensor init = at::linear(in_query, query_w).view({b, K, H, P}).permute({0, 2, 3, 1});
+  const Tensor A = at::exp(A_log.to(at::kFloat)).neg().unsqueeze(1).expand({H, d_state});
+  const auto act = xbc.scalar_type();
+  const Tensor feats = dist.scalar_type() == act || (dist.scalar_type() == at::kFloat && act == at::kBFloat16) ? dist : dist.to(act);
+  const std::vector<Tensor> terms{dt_tok, xbc.narrow(-1, di, G), xbc.narrow(-1, di + G, G), back.narrow(-1, di, G), back.narrow(-1, di + G, G)};
+  const auto g = dt_bc(feats, dt_w, bc_w, dt_bias, mask, act, terms);
+  const auto [key, last] = bi_scan(heads(xbc), heads(back), g[0], A, g[1], g[2], g[3], g[4], chunk, D, {}, {}, init, false, lo, hi, 0.5, 0, status);
+  const Tensor out_key = at::linear(norm(key.view({b, L, di}), kn_w, {}, z, kn_eps, 0, false, true), okey_w);
+  const Tensor q = last.permute({0, 3, 1, 2}).reshape({b, K, di}).to(out_key.scalar_type());
+  return {out_key, at::linear(at::layer_norm(q, {di}, qn_w, qn_b, qn_eps), oquery_w)};
+}
+}  // namespace issm_host
+
+using namespace issm_host;
+TORCH_LIBRARY_FRAGMENT(issm_b200, m) {
+  m.def("scan(Tensor x, Tensor dt, Tensor A, Tensor B, Tensor C, int chunk, Tensor? D, Tensor? z, Tensor? dt_bias, Tensor? init, bool softplus, float lo, "
+        "float hi, bool want_final, bool reverse, int path, Tensor status) -> Tensor[]", &scan);
+  m.def("bi_scan(Tensor x, Tensor xb, Tensor dt, Tensor A, Tensor B, Tensor C, Tensor Bb, Tensor Cb, int chunk, Tensor? D, Tensor? z, Tensor? dt_bias, "
+        "Tensor? init, bool softplus, float lo, float hi, float scale, int path, Tensor status) -> (Tensor, Tensor)", &bi_scan);
+  m.def("norm(Tensor x, Tensor w, Tensor? b, Tensor? z, float eps, int group, bool before, bool rms) -> Tensor", &norm);
+  m.def("conv_silu(Tensor x, Tensor w, Tensor? b) -> Tensor", &conv_silu);
+  m.def("reorder(Tensor points, Tensor index, Tensor? inverse) -> Tensor", &reorder);
+  m.def("dt_bc(Tensor dist, Tensor w_dt, Tensor w_bc, Tensor dt_bias, Tensor? mask, ScalarType out, Tensor[] terms) -> Tensor[]", &dt_bc);
+  m.def("block(Tensor in_key, Tensor in_query, Tensor dist, Tensor? mask, Tensor key_w, Tensor conv_w, Tensor? conv_b, Tensor convb_w, Tensor? convb_b, "
+        "Tensor query_w, Tensor bc_w, Tensor dt_w, Tensor dt_bias, Tensor A_log, Tensor D, Tensor kn_w, float kn_eps, Tensor okey_w, Tensor qn_w, "
+        "Tensor? qn_b, float qn_eps, Tensor oquery_w, int H, int G, int d_state, int chunk, float lo, float hi, Tensor status) -> (Tensor, Tensor)", &block);
+}

@@ -21,11 +21,12 @@ constexpr int GLUE_FWD_BLOCKS = 148 * 16;
 struct GlueArgs {
   int L, K, H, G, back, RW, RO;                            // RW = H + 2G weight rows; RO = H + 2G (+ 2G) output rows
   const void* dist; int64_t d_sb, d_sl, d_sk;
-  const float* w;                                          // (RW, M)
+  const float* w; const float* wbc;                        // dt rows (H, M); B / C rows (2G, M)
   const float* tok;                                        // (b, L, RO)
   const float* mask;                                       // (b, L, K) or null
   void* dt; void* bc;                                      // (b, L, H, K), (b, L, RO - H, K)
-  const void* ddt; const void* dbc;                        // same shapes, either may be null
+  const void* ddt;                                         // (b, L, H, K) or null
+  const void* gb[4]; int64_t gb_rs;                        // gradients of B, C (, second B, second C): rows of G x K, gb_rs elements per point; null: zero
   void* ddist;                                             // (b, L, K, M)
   float* dwpart;                                           // (blocks, GLUE_MAX_ROWS * M) partial weight gradients
   float* dtok;                                             // (b, L, RO)
@@ -106,8 +107,8 @@ template <int M>
 __device__ __forceinline__ void weights_to_smem(const GlueArgs& a, float2* sw, int rows) {
   const int hp = glue_hp(a.H);
   for (int i = threadIdx.x; i < rows * M; i += blockDim.x) {
-    const int r = i / M, src = r < hp ? (r < a.H ? r : -1) : (r - hp < 2 * a.G ? a.H + r - hp : -1);
-    const float w = src >= 0 ? a.w[src * M + i % M] : 0.f;
+    const int r = i / M, j = i % M;
+    const float w = r < hp ? (r < a.H ? a.w[r * M + j] : 0.f) : (r - hp < 2 * a.G ? a.wbc[(r - hp) * M + j] : 0.f);
     sw[i] = make_float2(w, w);
   }
 }
@@ -229,6 +230,7 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
   };
   const int per = gridDim.x * GLUE_BWD_WARPS, first = blockIdx.x * GLUE_BWD_WARPS + warp;
   const int nstep = (a.K + 63) / 64, nb = a.RO - a.H, hp = glue_hp(a.H);      // steps per point; B / C gradient rows; padded dt rows
+  const bool has_bc = a.gb[0] || a.gb[1] || a.gb[2] || a.gb[3];
   uint2 fx[2][FW];
   GP gh[8];                                  // dt gradient rows, loaded eight at a time
   float2 mk;
@@ -308,11 +310,15 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
       for (int r = 0; r < 8; ++r) g8[r] = gh[r];
       // gradients of the B / C rows of this step and the inputs of the next one
       GP gb[8];
-      const T* pb = a.dbc ? (const T*)a.dbc + (int64_t)pt * nb * a.K + k : nullptr;
-      if (pb) {
+      auto row_grad = [&](int q) {                         // B / C gradient row q of this step
+        const int which = q / a.G;
+        const T* p = (const T*)a.gb[which];
+        return p ? pair_at(p + (int64_t)pt * a.gb_rs + (int64_t)(q - which * a.G) * a.K + k, in0, in1) : GP{};
+      };
+      if (has_bc) {
 #pragma unroll
         for (int r = 0; r < 4; ++r)
-          if (r < nb) gb[r] = pair_at(pb + (int64_t)r * a.K, in0, in1);
+          if (r < nb) gb[r] = row_grad(r);
       }
       if (step + 1 < nstep) load(pt, step + 1);
       else if (pt + per < npoints) load(pt + per, 0);
@@ -339,13 +345,13 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
               tsum[r] += g[q].x + g[q].y;
             }
           }
-        } else if (pb) {
+        } else if (has_bc) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int c = rq - hp + q, c2 = c + 2 * a.G;   // both directions share the weight row
             if (c >= 2 * a.G) continue;
-            g[q] = c == 0 ? up(gb[0]) : c == 1 ? up(gb[1]) : up(pair_at(pb + (int64_t)c * a.K, in0, in1));
-            if (a.back) g[q] = __fadd2_rn(g[q], c2 == 2 ? up(gb[2]) : c2 == 3 ? up(gb[3]) : up(pair_at(pb + (int64_t)c2 * a.K, in0, in1)));
+            g[q] = c == 0 ? up(gb[0]) : c == 1 ? up(gb[1]) : up(row_grad(c));
+            if (a.back) g[q] = __fadd2_rn(g[q], c2 == 2 ? up(gb[2]) : c2 == 3 ? up(gb[3]) : up(row_grad(c2)));
           }
         }
 #pragma unroll
@@ -359,15 +365,15 @@ __global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_b
         *(float4*)(sg + (2 * lane) * GS + rq) = make_float4(g[0].x, g[1].x, g[2].x, g[3].x);
         *(float4*)(sg + (2 * lane + 1) * GS + rq) = make_float4(g[0].y, g[1].y, g[2].y, g[3].y);
       }
-      if (pb) {                                            // token terms of the B / C rows (each output row has its own)
+      if (has_bc) {                                        // token terms of the B / C rows (each output row has its own)
 #pragma unroll
         for (int q = 0; q < 8; ++q)
           if (q < nb) {
-            const float2 v = q < 4 ? up(gb[q & 3]) : up(pair_at(pb + (int64_t)q * a.K, in0, in1));
+            const float2 v = q < 4 ? up(gb[q & 3]) : up(row_grad(q));
             tsum[NR + q] += v.x + v.y;
           }
         for (int q = 8; q < nb; ++q) {                     // more than two groups: straight to the token gradient
-          const float2 v = up(pair_at(pb + (int64_t)q * a.K, in0, in1));
+          const float2 v = up(row_grad(q));
           const float t = warp_sum(v.x + v.y);
           if (lane == 0) { float* o = a.dtok + (int64_t)pt * a.RO + a.H + q; *o = step ? *o + t : t; }
         }
@@ -477,13 +483,61 @@ static GlueArgs glue_args(const issm_glue_params& p) {
   a.L = p.seqlen; a.K = p.nstates; a.H = p.nheads; a.G = p.ngroups; a.back = p.has_back;
   a.RW = p.nheads + 2 * p.ngroups; a.RO = a.RW + (p.has_back ? 2 * p.ngroups : 0);
   a.dist = p.dist; a.d_sb = p.dist_sb; a.d_sl = p.dist_sl; a.d_sk = p.dist_sk;
-  a.w = p.weight; a.tok = p.tok; a.mask = p.mask; a.dt = p.dt; a.bc = p.bc;
-  a.ddt = p.ddt; a.dbc = p.dbc; a.ddist = p.ddist; a.dwpart = (float*)p.workspace; a.dtok = p.dtok;
+  a.w = p.weight; a.wbc = p.weight_bc ? p.weight_bc : p.weight + (size_t)p.nheads * p.nfeat; a.tok = p.tok; a.mask = p.mask; a.dt = p.dt; a.bc = p.bc;
+  a.ddt = p.ddt; a.ddist = p.ddist; a.dwpart = (float*)p.workspace; a.dtok = p.dtok;
+  const int64_t part = (int64_t)p.ngroups * p.nstates;
+  a.gb_rs = p.dbc ? (a.RO - p.nheads) * (int64_t)p.nstates : part;
+  for (int i = 0; i < (p.has_back ? 4 : 2); ++i)
+    a.gb[i] = p.dbc ? (const void*)((const char*)p.dbc + i * part * (p.io_dtype == ISSM_F32 ? 4 : 2)) : p.dbc_part[i];
   return a;
+}
+
+// ---- token terms ---------------------------------------------------------------------------------------------------
+// one thread per (point, output row): float copies of up to five narrow tensors into one array, and the way back
+struct TokSrc { const void* src[5]; void* dst[5]; int64_t sb[5], sl[5]; int f32[5]; };
+__global__ void k_glue_tok(TokSrc t, int L, int H, int G, int RO, unsigned n, const float* __restrict__ bias, float* __restrict__ tok,
+                           const float* __restrict__ dtok) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const unsigned row = i / RO;
+  int r = (int)(i - row * RO), s = 0, w = H;
+  if (r >= H) { s = 1 + (r - H) / G; r = (r - H) % G; w = G; }
+  if (tok) {
+    const unsigned b = row / L, l = row - b * L;
+    const int64_t at = b * t.sb[s] + l * t.sl[s] + r;
+    float v = t.f32[s] ? ((const float*)t.src[s])[at] : ldf((const bf16*)t.src[s] + at);
+    if (s == 0 && bias) v += bias[r];
+    tok[i] = v;
+  } else if (t.dst[s]) {
+    const float v = dtok[i];
+    if (t.f32[s]) ((float*)t.dst[s])[(size_t)row * w + r] = v;
+    else stf((bf16*)t.dst[s] + (size_t)row * w + r, v);
+  }
 }
 }  // namespace issm
 
 using namespace issm;
+
+extern "C" size_t issm_b200_sizeof_glue_tok(void) { return sizeof(issm_glue_tok); }
+static int glue_tok_run(const issm_glue_tok* p, void* stream, bool pack) {
+  if (!p) return ISSM_ERR_NULL;
+  if (p->batch <= 0 || p->seqlen <= 0 || p->nheads <= 0 || p->ngroups <= 0 || (p->nsrc != 3 && p->nsrc != 5)) return ISSM_ERR_SHAPE;
+  const int RO = p->nheads + (p->nsrc - 1) * p->ngroups;
+  const int64_t n = (int64_t)p->batch * p->seqlen * RO;
+  if (n > 0x7fffffff) return ISSM_ERR_SHAPE;
+  if (pack ? !p->tok : !p->dtok) return ISSM_ERR_NULL;
+  TokSrc t{};
+  for (int i = 0; i < p->nsrc; ++i) {
+    if (p->dtype[i] != ISSM_F32 && p->dtype[i] != ISSM_BF16) return ISSM_ERR_DTYPE;
+    if (pack && !p->src[i]) return ISSM_ERR_NULL;
+    t.src[i] = p->src[i]; t.dst[i] = p->dsrc[i]; t.sb[i] = p->sb[i]; t.sl[i] = p->sl[i]; t.f32[i] = p->dtype[i] == ISSM_F32;
+  }
+  ISSM_LAUNCH(k_glue_tok, (unsigned)cdiv64(n, 256), 256, 0, (cudaStream_t)stream, t, p->seqlen, p->nheads, p->ngroups, RO, (unsigned)n, p->dt_bias,
+              pack ? p->tok : nullptr, p->dtok);
+  return ISSM_OK;
+}
+extern "C" int issm_b200_glue_tok_pack(const issm_glue_tok* p, void* stream) { return glue_tok_run(p, stream, true); }
+extern "C" int issm_b200_glue_tok_unpack(const issm_glue_tok* p, void* stream) { return glue_tok_run(p, stream, false); }
 
 extern "C" size_t issm_b200_sizeof_glue_params(void) { return sizeof(issm_glue_params); }
 
@@ -530,7 +584,8 @@ extern "C" int issm_b200_glue_bwd(const issm_glue_params* p, void* stream) {
   cudaStream_t s = (cudaStream_t)stream;
   const size_t es = p->io_dtype == ISSM_F32 ? 4 : 2;
   // pairs of gradients are one access where every row of states starts on the pair's alignment
-  const int pairs_ok = !(p->nstates & 1) && !((uintptr_t)p->ddt % (2 * es)) && !((uintptr_t)p->dbc % (2 * es));
+  const int pairs_ok = !(p->nstates & 1) && !((uintptr_t)p->ddt % (2 * es)) && !((uintptr_t)p->dbc % (2 * es)) &&
+                       !(((uintptr_t)p->dbc_part[0] | (uintptr_t)p->dbc_part[1] | (uintptr_t)p->dbc_part[2] | (uintptr_t)p->dbc_part[3]) % (2 * es));
 #define GLUE_BWD(TD, TT, MM)                                                                          \
   do {                                                                                                \
     if (glue_hp(a.H) + 2 * a.G <= 12) ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 12>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok); \

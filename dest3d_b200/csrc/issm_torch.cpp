@@ -4,7 +4,8 @@
 // (unit stride in the last dimension), allocates outputs and workspace with torch's caching allocator, fills
 // the parameter struct and calls the library on the current stream of the tensors' device.  No kernel lives
 // here: this file is host-side C++ only and links against libissm_b200.so.
-#include <ATen/ATen.h>
+#include "issm_torch.h"
+
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAException.h>
@@ -15,12 +16,7 @@
 #include <tuple>
 #include <vector>
 
-#include "../../include/issm_b200.h"
-
-namespace {
-
-using at::Tensor;
-using OptTensor = c10::optional<Tensor>;
+namespace issm_host {
 
 int dtype_code(at::ScalarType t) {
   if (t == at::kFloat) return ISSM_F32;
@@ -409,8 +405,9 @@ std::tuple<Tensor, Tensor, Tensor, Tensor> norm_bwd(const Tensor& dy2, const Ten
   return {dx, dz, dw, db};
 }
 
-}  // namespace
+}  // namespace issm_host
 
+using namespace issm_host;
 TORCH_LIBRARY(issm_b200, m) {
   m.def("fwd(Tensor x, Tensor dt, Tensor A, Tensor B, Tensor C, int chunk_size, Tensor? D, Tensor? z, Tensor? dt_bias, "
         "Tensor? initial_states, bool dt_softplus, float dt_min, float dt_max, bool reverse, int path, bool want_final, "

@@ -12,6 +12,7 @@ import math
 import torch
 from torch import nn
 
+from . import _ext, issm_combined
 from .adaptive_params import adaptive_dt_bc
 from .issm_combined import issm_bidirectional_scan, ISSM_chunk_scan_combined
 from .layernorm_gated import RMSNorm as RMSNormGated
@@ -54,6 +55,14 @@ class MultiHeadISSMScan(nn.Module):
     def forward(self, in_key, in_query, dist, key_xyz, mask=None):
         """in_key (B, L, D), in_query (B, K, D), dist (B, L, K, M), mask (B, L, K) -> out_key (B, L, D), out_query (B, K, D)."""
         G, H, P = self.ngroups, self.nheads, self.headdim
+        if self.use_biscan and issm_combined.BINDING == "torch" and in_key.is_cuda and not any(m._forward_hooks or m._forward_pre_hooks for m in self.children()):
+            # the same operations in the same order from C++: at the detector's size the block is bound by host time
+            return _ext.call("block")(
+                in_key, in_query, dist, mask, self.key_proj.weight, self.key_conv.dwconv.weight, self.key_conv.dwconv.bias,
+                self.key_conv_back.dwconv.weight, self.key_conv_back.dwconv.bias, self.query_proj.weight, self.bc_proj.weight, self.dt_proj.weight,
+                self.dt_bias, self.A_log, self.D, self.key_norm.weight, self.key_norm.eps, self.out_key_proj.weight, self.query_norm.weight,
+                self.query_norm.bias, self.query_norm.eps, self.out_query_proj.weight, H, G, self.d_state, self.chunk_size,
+                float(self.dt_limit[0]), float(self.dt_limit[1]), issm_combined._status_word(in_key.device))
         zxbcdt = self.key_proj(in_key)
         z, xbc, dt_tok = torch.split(zxbcdt, [self.d_inner, self.d_inner + 2 * G, H], dim=-1)
         xbc = self.key_conv(key_xyz, xbc)

@@ -361,6 +361,10 @@ def ISSM_chunk_scan_combined(x, dt, A, B, C, chunk_size, D=None, z=None, dt_bias
     if seq_idx is not None:
         return _scan_packed(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, seq_idx, dt_softplus, dt_limit,
                             return_final_states, reverse, path)
+    if BINDING == "torch":
+        res = _ext.call("scan")(x, dt, A, B, C, int(chunk_size), D, z, dt_bias, initial_states, bool(dt_softplus), float(dt_limit[0]), float(dt_limit[1]),
+                                bool(return_final_states), bool(reverse), _PATHS[path], _status_word(x.device))
+        return tuple(res) if return_final_states else res[0]
     return ISSMChunkScanCombinedFn.apply(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, None,
                                          dt_softplus, dt_limit, return_final_states, reverse, path)
 
@@ -402,43 +406,6 @@ def _scan_packed(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, seq_
     return (out, torch.cat(finals, dim=0)) if return_final_states else out
 
 
-class BidirectionalScanFn(torch.autograd.Function):
-    """Both directions in one call of the extension: the second runs on a side stream next to the first (one direction has
-    one block per (sample, head) and leaves SMs idle), what they share is converted once, and one launch joins the
-    results - in the backward the gradients of dt, A, D, z, dt_bias and the entering states."""
-
-    @staticmethod
-    def forward(ctx, x, x_back, dt, A, B, C, B_back, C_back, chunk_size, D, z, dt_bias, initial_states, dt_softplus, dt_limit, out_scale, path):
-        ctx.set_materialize_grads(False)
-        need_grad = any(ctx.needs_input_grad)
-        out, final, ox, oxb, sf, sb = _ext.ops().bi_fwd(
-            x, x_back, dt, A, B, C, B_back, C_back, int(chunk_size), D, z, dt_bias, initial_states, bool(dt_softplus), float(dt_limit[0]),
-            float(dt_limit[1]), float(out_scale), _PATHS[path], need_grad, _status_word(x.device))
-        _check_status(x.device, "issm_b200_fwd")
-        if need_grad:
-            ctx.save_for_backward(x, x_back, dt, A, B, C, B_back, C_back, D, z, dt_bias, initial_states, _ext.opt(ox), _ext.opt(oxb), _ext.opt(sf), _ext.opt(sb))
-            ctx.opts = (int(chunk_size), bool(dt_softplus), float(dt_limit[0]), float(dt_limit[1]), float(out_scale), _PATHS[path])
-        return out, final
-
-    @staticmethod
-    def backward(ctx, dout, dfinal):
-        x, xb, dt, A, B, C, Bb, Cb, D, z, dt_bias, init, ox, oxb, sf, sb = ctx.saved_tensors
-        chunk_size, softplus, lo, hi, scale, path = ctx.opts
-        if dout is None:
-            if dfinal is None:
-                return (None,) * 17
-            dout = torch.zeros_like(x)
-        g = _ext.ops().bi_bwd(dout, dfinal, x, xb, dt, A, B, C, Bb, Cb, ox, oxb, chunk_size, D, z, dt_bias, init, softplus, lo, hi, scale, path,
-                              sf, sb, _status_word(x.device))
-        _check_status(x.device, "issm_b200_bwd")
-        dx, dxb, ddt, dA, dB, dC, dBb, dCb, dD, dz, dbias, dinit = g
-        if dt_bias is not None and dt_bias.dim() != 2:
-            dbias = dbias.sum(dim=1)
-        like = lambda t, ref: None if ref is None else (t if t.dtype == ref.dtype else t.to(ref.dtype))
-        return (dx, like(dxb, xb), like(ddt, dt), like(dA, A), like(dB, B), like(dC, C), like(dBb, Bb), like(dCb, Cb), None, like(dD, D),
-                like(dz, z), like(dbias, dt_bias), like(dinit, init), None, None, None, None)
-
-
 def issm_bidirectional_scan(x, x_back, dt, A, B, C, B_back, C_back, chunk_size, D=None, z=None, dt_bias=None,
                             initial_states=None, dt_softplus=False, dt_limit=(0.0, float("inf")),
                             out_scale=0.5, path="auto"):
@@ -447,8 +414,10 @@ def issm_bidirectional_scan(x, x_back, dt, A, B, C, B_back, C_back, chunk_size, 
     models/dest_module.py:565-575 (which averages, out_scale = 0.5) without the flipped copies.
     All `_back` tensors are in natural point order.  Returns (out, final_states)."""
     if BINDING == "torch":
-        return BidirectionalScanFn.apply(x, x_back, dt, A, B, C, B_back, C_back, chunk_size, D, z, dt_bias, initial_states, dt_softplus,
-                                         dt_limit, out_scale, path)
+        # one operation: the second direction next to the first, what they share converted once, one launch joins the results
+        # (in the backward the gradients of dt, A, D, z, dt_bias and the entering states)
+        return _ext.call("bi_scan")(x, x_back, dt, A, B, C, B_back, C_back, int(chunk_size), D, z, dt_bias, initial_states, bool(dt_softplus),
+                                    float(dt_limit[0]), float(dt_limit[1]), float(out_scale), _PATHS[path], _status_word(x.device))
     yf, sf = ISSM_chunk_scan_combined(x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, None,
                                       dt_softplus, dt_limit, True, reverse=False, path=path)
     yb, sb = ISSM_chunk_scan_combined(x_back, dt, A, B_back, C_back, chunk_size, D, z, dt_bias, initial_states,

@@ -124,11 +124,13 @@ class LayerNormFn(torch.autograd.Function):
 
 
 def layernorm_fn(x, weight, bias, z=None, eps=1e-6, group_size=None, norm_before_gate=True, is_rms_norm=False):
+    if issm_combined.BINDING == "torch":
+        return _ext.call("norm")(x, weight, bias, z, float(eps), int(group_size or 0), bool(norm_before_gate), bool(is_rms_norm))
     return LayerNormFn.apply(x, weight, bias, z, eps, group_size, norm_before_gate, is_rms_norm)
 
 
 def rmsnorm_fn(x, weight, bias, z=None, eps=1e-6, group_size=None, norm_before_gate=True):
-    return LayerNormFn.apply(x, weight, bias, z, eps, group_size, norm_before_gate, True)
+    return layernorm_fn(x, weight, bias, z, eps, group_size, norm_before_gate, True)
 
 
 class LayerNorm(torch.nn.Module):

@@ -13,12 +13,21 @@ import ctypes as ct
 import torch
 from torch import nn
 
-from . import _lib
+from . import _ext, _lib, issm_combined
 
 
 def _empty(shape, dtype, device):
     """Every output and workspace of this module is allocated here (the guard-band tests substitute it)."""
     return torch.empty(tuple(shape), dtype=dtype, device=device)
+
+
+_default_empty = _empty
+
+
+def _native():
+    """The C++ operations of the torch extension serve the calls unless the ctypes binding is selected or a test has put an
+    allocator of its own in `_empty`'s place."""
+    return issm_combined.BINDING == "torch" and _empty is _default_empty
 
 
 def _gather_rows(src, index):
@@ -74,6 +83,8 @@ def reorder_points(points, index, inverse_index=None, check=False):
     permutation and `inverse_index` its inverse (the reference keeps both, models/dest_module.py:340-344), the
     backward is one more gather; otherwise it is a scatter-add.  `check=True` synchronises and raises on an index
     outside [0, N) (such rows are left unwritten)."""
+    if not check and _native():
+        return _ext.call("reorder")(points, index, inverse_index)
     return _ReorderFn.apply(points, index, inverse_index, check)
 
 
@@ -149,4 +160,6 @@ class PointLiteConv(nn.Module):
 
     def forward(self, xyz, feature):
         """xyz (B, N, 3) is unused, as in the reference; feature (B, N, C) -> (B, N, C)."""
+        if _native():
+            return _ext.call("conv_silu")(feature, self.dwconv.weight, self.dwconv.bias)
         return DwConv7SiluFn.apply(feature, self.dwconv.weight, self.dwconv.bias)

@@ -239,7 +239,26 @@ typedef struct issm_glue_params {
   const void* ddt; const void* dbc;
   void* ddist; float* dweight; float* dtok;
   void* workspace; size_t workspace_bytes;
+  /* optional: the B / C weight rows as an array of their own, (2 ngroups, nfeat); null: they follow the dt rows in `weight` */
+  const float* weight_bc;
+  /* optional, backward with dbc null: the gradients of B, C [, second B, second C] as separate contiguous
+   * (batch, seqlen, ngroups, nstates) arrays; null entries count as zero */
+  const void* dbc_part[4];
 } issm_glue_params;
+/* The token terms of a call from the tensors they come from: tok[b, l, :] = [dt_tok[b, l, h] + dt_bias[h], b, c (, b_back,
+ * c_back)], float; the backward splits dtok into gradients of the same element types (contiguous; any may be null).
+ * Sources have element strides sb (batch) and sl (point) and a unit last stride; dtype per source, ISSM_F32 or ISSM_BF16. */
+typedef struct issm_glue_tok {
+  int32_t batch, seqlen, nheads, ngroups, nsrc;   /* nsrc = 3, or 5 with the second direction */
+  int32_t dtype[5];
+  const void* src[5]; int64_t sb[5], sl[5];       /* dt_tok (nheads wide), then ngroups wide each */
+  const float* dt_bias;                           /* (nheads) or null */
+  float* tok;
+  const float* dtok; void* dsrc[5];
+} issm_glue_tok;
+size_t issm_b200_sizeof_glue_tok(void);
+int issm_b200_glue_tok_pack(const issm_glue_tok* p, void* cuda_stream);
+int issm_b200_glue_tok_unpack(const issm_glue_tok* p, void* cuda_stream);
 
 size_t issm_b200_sizeof_glue_params(void);
 size_t issm_b200_glue_workspace_bytes(const issm_glue_params* p);

@@ -374,6 +374,19 @@ struct GlueFn : public Function<GlueFn> {
   }
 };
 
+// A[h, n] = -exp(A_log[h]) for every state
+struct DecayFn : public Function<DecayFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& A_log, int64_t states) {
+    const Tensor a = at::exp(A_log.detach().to(at::kFloat)).neg_();
+    ctx->save_for_backward({a, A_log});
+    return a.unsqueeze(1).expand({a.size(0), states}).contiguous();
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    return {like(g[0].sum(1).mul_(s[0]), s[1]), Tensor()};
+  }
+};
+
 // ---- what Python calls -----------------------------------------------------------------------------------------------------
 static bool wants_grad(std::initializer_list<const Tensor*> req, std::initializer_list<const OptTensor*> opt) {
   if (!at::GradMode::is_enabled()) return false;
@@ -416,20 +429,21 @@ std::tuple<Tensor, Tensor> block(const Tensor& in_key, const Tensor& in_query, c
                                  double kn_eps, const Tensor& okey_w, const Tensor& qn_w, const OptTensor& qn_b, double qn_eps, const Tensor& oquery_w,
                                  int64_t H, int64_t G, int64_t d_state, int64_t chunk, double lo, double hi, const Tensor& status) {
   const int64_t di = query_w.size(0), P = di / H;
-  const Tensor zx = at::linear(in_key, key_w);
-  const Tensor z = zx.narrow(-1, 0, di), dt_tok = zx.narrow(-1, 2 * di + 2 * G, H);
-  const Tensor xbc = conv_silu(zx.narrow(-1, di, di + 2 * G), conv_w, conv_b);
+  // split, not narrow: its gradient is one concatenation
+  const auto zx = at::linear(in_key, key_w).split_with_sizes({di, di + 2 * G, H}, -1);
+  const Tensor xbc = conv_silu(zx[1], conv_w, conv_b);
   const Tensor back = conv_silu(xbc, convb_w, convb_b);    // the second convolution takes the OUTPUT of the first (dest_module.py:534)
+  const auto f = xbc.split_with_sizes({di, G, G}, -1), r = back.split_with_sizes({di, G, G}, -1);
   const auto b = in_key.size(0), L = in_key.size(1), K = in_query.size(1);
-  auto heads = [&](const Tensor& t) { return t.narrow(-1, 0, di).contiguous().view({b, L, H, P}); };
+  auto heads = [&](const Tensor& t) { return t.contiguous().view({b, L, H, P}); };
   const Tensor init = at::linear(in_query, query_w).view({b, K, H, P}).permute({0, 2, 3, 1});
-  const Tensor A = at::exp(A_log.to(at::kFloat)).neg().unsqueeze(1).expand({H, d_state});
+  const Tensor A = DecayFn::apply(A_log, d_state);
   const auto act = xbc.scalar_type();
   const Tensor feats = dist.scalar_type() == act || (dist.scalar_type() == at::kFloat && act == at::kBFloat16) ? dist : dist.to(act);
-  const std::vector<Tensor> terms{dt_tok, xbc.narrow(-1, di, G), xbc.narrow(-1, di + G, G), back.narrow(-1, di, G), back.narrow(-1, di + G, G)};
+  const std::vector<Tensor> terms{zx[2], f[1], f[2], r[1], r[2]};
   const auto g = dt_bc(feats, dt_w, bc_w, dt_bias, mask, act, terms);
-  const auto [key, last] = bi_scan(heads(xbc), heads(back), g[0], A, g[1], g[2], g[3], g[4], chunk, D, {}, {}, init, false, lo, hi, 0.5, 0, status);
-  const Tensor out_key = at::linear(norm(key.view({b, L, di}), kn_w, {}, z, kn_eps, 0, false, true), okey_w);
+  const auto [key, last] = bi_scan(heads(f[0]), heads(r[0]), g[0], A, g[1], g[2], g[3], g[4], chunk, D, {}, {}, init, false, lo, hi, 0.5, 0, status);
+  const Tensor out_key = at::linear(norm(key.view({b, L, di}), kn_w, {}, zx[0], kn_eps, 0, false, true), okey_w);
   const Tensor q = last.permute({0, 3, 1, 2}).reshape({b, K, di}).to(out_key.scalar_type());
   return {out_key, at::linear(at::layer_norm(q, {di}, qn_w, qn_b, qn_eps), oquery_w)};
 }

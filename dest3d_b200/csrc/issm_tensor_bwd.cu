@@ -1220,13 +1220,15 @@ __global__ void k_reduce_heads_bf16(int hpg, int N, int H, size_t total, const u
                                                  pack_bf16(accC[4], accC[5]), pack_bf16(accC[6], accC[7]));
 }
 
-// out[h, j] = sum_b part[b, h, j]   (fixed order)
-__global__ void k_reduce_batch(const float* __restrict__ part, int batch, int stride, float* __restrict__ out) {
-  const int j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= stride) return;
+// out[j] = sum_b part[b, j] (fixed order) for up to three arrays in one launch: dA, ddt_bias and the per-head dD
+struct BatchSums { const float* part[3]; float* out[3]; int stride[3]; };
+__global__ void k_reduce_batch(BatchSums q, int batch) {
+  int j = blockIdx.x * blockDim.x + threadIdx.x, k = 0;
+  while (k < 3 && j >= q.stride[k]) j -= q.stride[k++];
+  if (k == 3) return;
   float acc = 0.f;
-  for (int i = 0; i < batch; ++i) acc += part[(size_t)i * stride + j];
-  out[j] = acc;
+  for (int i = 0; i < batch; ++i) acc += q.part[k][(size_t)i * q.stride[k] + j];
+  q.out[k][j] = acc;
 }
 // dD from (b, H, PP) partials: (H, P) or (H)
 __global__ void k_reduce_dD(const float* __restrict__ part, int batch, int H, int P, int has_hdim, float* __restrict__ out) {
@@ -1334,15 +1336,14 @@ int tensor_bwd(const issm_params& p, cudaStream_t s) {
   const size_t tot = (size_t)p.batch * p.seqlen * p.ngroups * (p.dstate / 8);
   ISSM_LAUNCH(k_reduce_heads_bf16, (unsigned)cdiv64(tot, 256), 256, 0, s, hpg, p.dstate, p.nheads, tot, w.dBCh, (bf16*)p.dB, (bf16*)p.dC);
   const int HN = p.nheads * p.dstate;
-  ISSM_LAUNCH(k_reduce_batch, (HN + 127) / 128, 128, 0, s, w.dApart, p.batch, HN, p.dA);
-  if (p.has_dt_bias) ISSM_LAUNCH(k_reduce_batch, (HN + 127) / 128, 128, 0, s, w.dbpart, p.batch, HN, p.ddt_bias);
-  if (p.has_D) {
-    if (p.D_has_hdim) {
-      ISSM_LAUNCH(k_dD_hdim, dim3(p.nheads, p.batch), 256, 0, s, a);
-      ISSM_LAUNCH(k_reduce_dD, (p.nheads * p.headdim + 63) / 64, 64, 0, s, w.dDpart, p.batch, p.nheads, p.headdim, 1, p.dD);
-    } else {
-      ISSM_LAUNCH(k_reduce_batch, (p.nheads + 63) / 64, 64, 0, s, w.dDpart, p.batch, p.nheads, p.dD);
-    }
+  BatchSums q{};
+  q.part[0] = w.dApart; q.out[0] = p.dA; q.stride[0] = HN;
+  if (p.has_dt_bias) { q.part[1] = w.dbpart; q.out[1] = p.ddt_bias; q.stride[1] = HN; }
+  if (p.has_D && !p.D_has_hdim) { q.part[2] = w.dDpart; q.out[2] = p.dD; q.stride[2] = p.nheads; }
+  ISSM_LAUNCH(k_reduce_batch, (q.stride[0] + q.stride[1] + q.stride[2] + 127) / 128, 128, 0, s, q, p.batch);
+  if (p.has_D && p.D_has_hdim) {
+    ISSM_LAUNCH(k_dD_hdim, dim3(p.nheads, p.batch), 256, 0, s, a);
+    ISSM_LAUNCH(k_reduce_dD, (p.nheads * p.headdim + 63) / 64, 64, 0, s, w.dDpart, p.batch, p.nheads, p.headdim, 1, p.dD);
   }
   return ISSM_OK;
 }

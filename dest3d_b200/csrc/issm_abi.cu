@@ -15,11 +15,16 @@ static int validate(const issm_params* p, int pass) {
   if ((p->io_dtype != ISSM_F32 && p->io_dtype != ISSM_BF16) || (p->dt_dtype != ISSM_F32 && p->dt_dtype != ISSM_BF16))
     return ISSM_ERR_DTYPE;
   if (p->path < ISSM_PATH_AUTO || p->path > ISSM_PATH_TENSOR) return ISSM_ERR_UNSUPPORTED;
-  if (!(p->dt_min <= p->dt_max)) return ISSM_ERR_SHAPE;
+  if (!(p->dt_min <= p->dt_max) || p->states_only < 0 || p->states_only > 2) return ISSM_ERR_SHAPE;
   return ISSM_OK;
 }
 
 static int validate_ptrs(const issm_params* p, int pass) {
+  if (pass == 0 && p->states_only) {
+    if (!p->dt || !p->A || !p->final_states || (p->has_dt_bias && !p->dt_bias)) return ISSM_ERR_NULL;
+    if (p->states_only == 1) return (!p->x || !p->B || (p->has_init && !p->initial_states)) ? ISSM_ERR_NULL : ISSM_OK;
+    return (!p->dout || !p->C || (p->has_z && !p->z)) ? ISSM_ERR_NULL : ISSM_OK;
+  }
   if (!p->x || !p->dt || !p->A || !p->B || !p->C) return ISSM_ERR_NULL;
   if (p->has_D && !p->D) return ISSM_ERR_NULL;
   if (p->has_z && (!p->z || !p->out_x)) return ISSM_ERR_NULL;
@@ -113,7 +118,7 @@ static int run(const issm_params* in, void* stream, int pass) {
   const issm_params q = canonical(*in);
   const issm_params* p = &q;
   const int path = resolve(*p, pass);
-  if (path < 0) return ISSM_ERR_UNSUPPORTED;
+  if (path < 0 || (pass == 0 && p->states_only && path != ISSM_PATH_TENSOR)) return ISSM_ERR_UNSUPPORTED;
   const size_t need = path == ISSM_PATH_TENSOR ? tensor_workspace_bytes(*p, pass) : simt_workspace_bytes(*p, pass);
   if (need && (!p->workspace || p->workspace_bytes < need)) return ISSM_ERR_WORKSPACE;
   if ((uintptr_t)p->workspace % 256) return ISSM_ERR_ALIGN;

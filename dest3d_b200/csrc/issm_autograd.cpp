@@ -148,6 +148,42 @@ struct BiScanFn : public Function<BiScanFn> {
   }
 };
 
+struct SlicedFn : public Function<SlicedFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk,
+                               const OptTensor& D, const OptTensor& z, const OptTensor& bias, const OptTensor& init, bool softplus, double lo, double hi,
+                               bool reverse, int64_t path, int64_t slices, const Tensor& status, bool need) {
+    ctx->set_materialize_grads(false);
+    const auto r = sliced_fwd(x, dt, A, B, C, chunk, D, z, bias, init, softplus, lo, hi, reverse, path, slices, need, status);
+    check_status(status, "issm_b200_fwd");
+    if (need) {
+      variable_list keep{x, dt, A, B, C, none(D), none(z), none(bias), none(init), status};
+      for (size_t i = 2; i < r.size(); ++i) keep.push_back(filled(r[i]));
+      ctx->save_for_backward(keep);
+      ctx->saved_data["i"] = c10::IValue(std::vector<int64_t>{chunk, softplus, reverse, path, slices});
+      ctx->saved_data["f"] = c10::IValue(std::vector<double>{lo, hi});
+    }
+    return {r[0], r[1]};
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const auto s = ctx->get_saved_variables();
+    const auto i = ctx->saved_data["i"].toIntVector();
+    const auto f = ctx->saved_data["f"].toDoubleVector();
+    variable_list r(18);
+    if (!g[0].defined() && !g[1].defined()) return r;
+    const Tensor dout = g[0].defined() ? g[0] : at::zeros_like(s[0]);
+    const std::vector<Tensor> kept(s.begin() + 10, s.end());
+    auto [dx, ddt, dA, dB, dC, dD, dz, db, di] = sliced_bwd(dout, some(g[1]), s[0], s[1], s[2], s[3], s[4], i[0], some(s[5]), some(s[6]), some(s[7]), some(s[8]),
+                                                            i[1] != 0, f[0], f[1], i[2] != 0, i[3], i[4], kept, s[9]);
+    check_status(s[9], "issm_b200_bwd");
+    r[0] = dx; r[1] = like(ddt, s[1]); r[2] = like(dA, s[2]); r[3] = like(dB, s[3]); r[4] = like(dC, s[4]);
+    if (s[5].defined()) r[6] = like(dD, s[5]);
+    if (s[6].defined()) r[7] = like(dz, s[6]);
+    if (s[7].defined()) r[8] = like(s[7].dim() == 2 ? db : db.sum(1), s[7]);
+    if (s[8].defined()) r[9] = like(di, s[8]);
+    return r;
+  }
+};
+
 // ---- gated norms -------------------------------------------------------------------------------------------------------
 static Tensor rows_of(const Tensor& t) {
   Tensor r = t.reshape({-1, t.size(-1)});
@@ -402,6 +438,15 @@ std::vector<Tensor> scan(const Tensor& x, const Tensor& dt, const Tensor& A, con
   return ScanFn::apply(x, dt, A, B, C, chunk, D, z, bias, init, softplus, lo, hi, want_final, reverse, path, status,
                        wants_grad({&x, &dt, &A, &B, &C}, {&D, &z, &bias, &init}));
 }
+// scan over `slices` slices per sequence; always with the final state
+std::vector<Tensor> sliced_scan(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, const OptTensor& D,
+                                const OptTensor& z, const OptTensor& bias, const OptTensor& init, bool softplus, double lo, double hi, bool reverse,
+                                int64_t path, int64_t slices, const Tensor& status) {
+  const int64_t R = usable_slices(x, dt, A, B, C, chunk, path, status, slices);
+  if (R <= 1) return scan(x, dt, A, B, C, chunk, D, z, bias, init, softplus, lo, hi, true, reverse, path, status);
+  return SlicedFn::apply(x, dt, A, B, C, chunk, D, z, bias, init, softplus, lo, hi, reverse, path, R, status,
+                         wants_grad({&x, &dt, &A, &B, &C}, {&D, &z, &bias, &init}));
+}
 std::tuple<Tensor, Tensor> bi_scan(const Tensor& x, const Tensor& xb, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, const Tensor& Bb,
                                    const Tensor& Cb, int64_t chunk, const OptTensor& D, const OptTensor& z, const OptTensor& bias, const OptTensor& init,
                                    bool softplus, double lo, double hi, double scale, int64_t path, const Tensor& status) {
@@ -453,6 +498,8 @@ using namespace issm_host;
 TORCH_LIBRARY_FRAGMENT(issm_b200, m) {
   m.def("scan(Tensor x, Tensor dt, Tensor A, Tensor B, Tensor C, int chunk, Tensor? D, Tensor? z, Tensor? dt_bias, Tensor? init, bool softplus, float lo, "
         "float hi, bool want_final, bool reverse, int path, Tensor status) -> Tensor[]", &scan);
+  m.def("sliced_scan(Tensor x, Tensor dt, Tensor A, Tensor B, Tensor C, int chunk, Tensor? D, Tensor? z, Tensor? dt_bias, Tensor? init, bool softplus, "
+        "float lo, float hi, bool reverse, int path, int slices, Tensor status) -> Tensor[]", &sliced_scan);
   m.def("bi_scan(Tensor x, Tensor xb, Tensor dt, Tensor A, Tensor B, Tensor C, Tensor Bb, Tensor Cb, int chunk, Tensor? D, Tensor? z, Tensor? dt_bias, "
         "Tensor? init, bool softplus, float lo, float hi, float scale, int path, Tensor status) -> (Tensor, Tensor)", &bi_scan);
   m.def("norm(Tensor x, Tensor w, Tensor? b, Tensor? z, float eps, int group, bool before, bool rms) -> Tensor", &norm);

@@ -44,3 +44,39 @@ extern "C" int issm_b200_dt_sum(const void* dt, int32_t dt_dtype, int32_t batch,
     ISSM_LAUNCH(k_dt_sum<bf16>, grid, threads, 0, s, (const bf16*)dt, dt_sb, dt_sl, dt_sh, dt_bias, dt_softplus, dt_min, dt_max, seqlen, rows_per_part, dstate, part);
   return ISSM_OK;
 }
+
+// One thread per (sequence, head, channel, state) walks the slices: run = F + 2^sums run, coalesced over the states.
+namespace issm {
+__global__ void k_slice_chain(const __grid_constant__ issm_slice_chain q) {
+  const int64_t hpn = (int64_t)q.nheads * q.headdim * q.dstate, i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= q.batch * hpn) return;
+  const int64_t b = i / hpn, e = i - b * hpn;
+  const int n = (int)(e % q.dstate), h = (int)(e / ((int64_t)q.headdim * q.dstate));
+  const int64_t hn = (int64_t)q.nheads * q.dstate, sn = (int64_t)h * q.dstate + n;
+  const int total = q.nmain + (q.f_tail ? 1 : 0);
+  float run = !q.start ? 0.f : q.start_f32 ? ((const float*)q.start)[i] : ldf((const bf16*)q.start + i);
+#pragma unroll 4
+  for (int k = 0; k < total; ++k) {
+    const int s = q.descending ? total - 1 - k : k;
+    const bool tail = s == q.nmain;
+    const int64_t row = tail ? b : b * q.nmain + s, at = row * hpn + e;
+    void* en = tail ? q.enter_tail : q.enter_main;
+    if (q.enter_f32) ((float*)en)[at] = run;
+    else stf((bf16*)en + at, run);
+    run = fmaf(exp2f((tail ? q.s_tail : q.s_main)[row * hn + sn]), run, (tail ? q.f_tail : q.f_main)[at]);
+  }
+  if (q.last) {
+    if (q.last_f32) ((float*)q.last)[i] = run;
+    else stf((bf16*)q.last + i, run);
+  }
+}
+}  // namespace issm
+
+extern "C" size_t issm_b200_sizeof_slice_chain(void) { return sizeof(issm_slice_chain); }
+extern "C" int issm_b200_slice_chain(const issm_slice_chain* p, void* stream) {
+  if (!p || !p->f_main || !p->s_main || !p->enter_main || (p->f_tail && (!p->s_tail || !p->enter_tail))) return ISSM_ERR_NULL;
+  if (p->batch <= 0 || p->nmain <= 0 || p->nheads <= 0 || p->headdim <= 0 || p->dstate <= 0) return ISSM_ERR_SHAPE;
+  const int64_t n = (int64_t)p->batch * p->nheads * p->headdim * p->dstate;
+  ISSM_LAUNCH(k_slice_chain, (unsigned)cdiv64(n, 128), 128, 0, (cudaStream_t)stream, *p);
+  return ISSM_OK;
+}

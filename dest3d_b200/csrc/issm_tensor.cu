@@ -744,6 +744,7 @@ TArgs make_targs(const issm_params& p) {
   a.out = (bf16*)p.out; a.o_sb = p.out_sb; a.o_sl = p.out_sl; a.o_sh = p.out_sh;
   a.out_x = p.has_z ? (bf16*)p.out_x : nullptr;
   a.final_states = p.final_states;
+  a.sums = p.state_sums;
   a.status = p.status;
   a.saved = (bf16*)p.saved_states;
   // a whole 64-row tile of B / C is one contiguous copy only when a row IS the tile's row (not a 256-state slice of it)
@@ -816,7 +817,7 @@ static int launch_fwd(TArgs a, const issm_params& p, cudaStream_t s) {
   struct WinTag {};
   if (SmemAttrOnce<WinTag>::set(k_fwd_windowed<NT, TDT>, smem) != ISSM_OK) return ISSM_ERR_CUDA;
   const int slices = a.N / NT;
-  const int rc = launch_fwd_pipe(a, p, NT, s);
+  const int rc = launch_fwd_pipe(a, NT, a.no_output ? 1 : 0, s);
   if (rc) return rc;
   ISSM_LAUNCH((k_fwd_windowed<NT, TDT>), dim3(slices, a.H, a.b), 2 * NT + 128, smem, s, a, maps);   // marked streams only
   if (slices > 1 && !a.no_output) {
@@ -830,6 +831,21 @@ int tensor_fwd(const issm_params& p, cudaStream_t s) {
   TArgs a = make_targs(p);
   a.redo = (int*)p.workspace;
   const int slices = state_slices(p.dstate);
+  if (p.states_only == 2) {                               // the adjoint walks against the scan; dy in x's place, C in B's
+    a.rev = !p.reverse;
+    a.no_output = a.want_final = 1;
+    a.x = (const bf16*)p.dout; a.x_sb = p.dout_sb; a.x_sl = p.dout_sl; a.x_sh = p.dout_sh;
+    a.B = a.C; a.B_sb = a.C_sb; a.B_sl = a.C_sl; a.B_sg = a.C_sg;
+    a.saved = nullptr;
+    a.out_x = nullptr;
+    const int nt = p.dstate == 128 ? 128 : 256;
+    const int rc = launch_fwd_pipe(a, nt, 2, s);
+    return rc ? rc : launch_grad_states_rows(a, nt, s);
+  }
+  if (p.states_only == 1) {
+    a.no_output = a.want_final = 1;
+    a.saved = nullptr;
+  }
   if (slices > 1) {
     a.ypart = (float*)((char*)p.workspace + align_up((size_t)slices * p.batch * p.nheads * sizeof(int), 256));
   }

@@ -39,6 +39,7 @@ struct TArgs {
   bf16* out; int64_t o_sb, o_sl, o_sh;
   bf16* out_x;
   float* final_states;
+  float* sums;      // states-only walks: (b, H, N) summed log2 decay of the sequence
   bf16* saved;      // optional (b, H, nblk + 1, PP / 8, N, 8) bf16: state entering every 64-point block, and the final one
   int* status;
   // backward
@@ -144,7 +145,9 @@ bool make_rows_tensor_map(const void* base, int64_t sb, int64_t sl, int64_t widt
 struct FwdMaps { CUtensorMap dt, B, C; };
 int state_slices(int dstate);
 // the fast forward walk over slices of nt states; streams with a block outside its range are marked in a.redo
-int launch_fwd_pipe(const TArgs& a, const issm_params& p, int nt, cudaStream_t s);
+// (mode 0: the scan, 1: states only, 2: gradient states - see k_fwd_pipe)
+int launch_fwd_pipe(const TArgs& a, int nt, int mode, cudaStream_t s);
+int launch_grad_states_rows(const TArgs& a, int nt, cudaStream_t s);   // redo of marked streams in mode 2
 // Tensor map over the rows of a (batch, seqlen, width) bf16 array, any batch and row pitch, with a 64 x 64 box in the 128-byte
 // swizzle of the operand tiles; rows past seqlen read as zero.  false if TMA does not take the strides
 bool make_tile_map(const void* base, int64_t sb, int64_t sl, int64_t width, int batch, int seqlen, CUtensorMap* out);

@@ -52,7 +52,10 @@ __device__ __forceinline__ void wait_or_fail(uint64_t* bar, uint32_t parity, boo
 
 // Rows keep their memory order inside a block also for a reversed scan (kRev): only the direction of the in-block sums and the
 // side of the mask change, so the tiles can be filled by TMA and scaled in place.
-template <int NT, typename TDT, bool kRev>
+// kMode: 0 the scan; 1 states only (no output rows: Cd, M and Y are left out); 2 gradient states: the adjoint recurrence
+// G <- 2^a_last G + sum_l C 2^a_l dy_l, which is the states-only walk against the scan order with dy for x and C 2^(a_l - a_last)
+// for B dt 2^-a - the in-block sum from the other end without the row itself.
+template <int NT, typename TDT, bool kRev, int kMode>
 __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pipe(const __grid_constant__ TArgs a, const __grid_constant__ FwdMaps maps) {
   using SM = PipeSmem<NT>;
   constexpr int NP = NT / 16;                            // P warps
@@ -167,11 +170,11 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
         const int r = kRev ? 15 - i : i;
         uint32_t* cp = (uint32_t*)(col + (uint32_t)(r * 128 + ((kc ^ (r & 7)) << 4)));
         uint32_t* bp = cp + SM::kHalf / 4;
+        const float2 before = acc;
         acc = __ffma2_rn(dtv[i], A2, acc);
-        const float2 cd = __fmul2_rn(unpack_bf16(*cp), ex2f2(acc));
-        const float2 bd = __fmul2_rn(__fmul2_rn(unpack_bf16(*bp), dtv[i]), ex2f2_neg(acc));
-        *cp = pack_bf16(cd);
-        *bp = pack_bf16(bd);
+        if constexpr (kMode == 0) *cp = pack_bf16(__fmul2_rn(unpack_bf16(*cp), ex2f2(acc)));
+        if constexpr (kMode == 2) *bp = pack_bf16(__fmul2_rn(unpack_bf16(*bp), ex2f2_neg(before)));
+        else *bp = pack_bf16(__fmul2_rn(__fmul2_rn(unpack_bf16(*bp), dtv[i]), ex2f2_neg(acc)));
         if ((i & 3) == 3 && blk + 1 < nblk) load_dt(blk + 1, i - 3, i + 1);   // dt of the next block takes the place of this one's
       }
       if (rows < QB) {                                   // rows outside the sequence: zero
@@ -179,7 +182,7 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
         for (int r = 0; r < 16; ++r)
           if (!inside(r0 + r, rows)) {
             uint32_t* cp = (uint32_t*)(col + (uint32_t)(r * 128 + ((kc ^ (r & 7)) << 4)));
-            cp[0] = 0;
+            if (kMode == 0) cp[0] = 0;
             cp[SM::kHalf / 4] = 0;
           }
       }
@@ -200,7 +203,7 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
       if (first) {
         const bf16* ip = a.init + (((size_t)b * a.H + h) * a.P) * a.N + n_off + n;
 #pragma unroll
-        for (int j = 0; j < CW; ++j) sc[j] = (a.has_init && c0 + j < a.P) ? __bfloat162float(ip[(size_t)(c0 + j) * a.N]) : 0.f;
+        for (int j = 0; j < CW; ++j) sc[j] = (kMode != 2 && a.has_init && c0 + j < a.P) ? __bfloat162float(ip[(size_t)(c0 + j) * a.N]) : 0.f;
       } else {
         tmem_ld16(t, sc);
         tmem_ld_wait();
@@ -212,7 +215,7 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
       for (int c = 0; c < CW / 8; ++c) {
         const uint4 v = make_uint4(pack_bf16(sc[c * 8], sc[c * 8 + 1]), pack_bf16(sc[c * 8 + 2], sc[c * 8 + 3]),
                                    pack_bf16(sc[c * 8 + 4], sc[c * 8 + 5]), pack_bf16(sc[c * 8 + 6], sc[c * 8 + 7]));
-        *(uint4*)(smem + SM::kS + sw128_chunk(n, c0 / 8 + c)) = v;
+        if (kMode == 0) *(uint4*)(smem + SM::kS + sw128_chunk(n, c0 / 8 + c)) = v;
         if (savep) *(uint4*)(savep + ((size_t)blk * PP + c0 + c * 8) * a.N) = v;
       }
       if (blk == nblk && a.want_final) {
@@ -286,21 +289,24 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
 #pragma unroll 1
     for (int c0 = 0; c0 < PP; c0 += 16) pass(c0, 1.f, 0, true);
     publish();
+    float asum = 0.f;
     for (int blk = 0; blk < nblk; ++blk) {
       wait_or_fail(bars + kDoneS + (blk & 1), (blk >> 1) & 1, failed);
       fence_after_sync();
-      const float el = ex2f(((const float*)(smem + SM::kLast))[(blk & 3) * NT + n]);
+      const float last = ((const float*)(smem + SM::kLast))[(blk & 3) * NT + n], el = ex2f(last);
+      asum += last;
 #pragma unroll 1
       for (int c0 = 0; c0 < PP; c0 += 16) pass(c0, el, blk + 1, false);
       publish();
-      if (blk > 0 && !a.no_output) output(blk - 1);      // while the MMAs of the next block run
+      if (blk > 0 && kMode == 0) output(blk - 1);      // while the MMAs of the next block run
     }
-    if (!a.no_output) output(nblk - 1);
+    if (kMode == 0) output(nblk - 1);
+    if (kMode != 0 && a.sums) a.sums[((size_t)b * a.H + h) * a.N + n_off + n] = asum;
   } else if (warp < NP + NE2 + 4) {
     // ==================================================== E1 ====================================================
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kRegE));
     const int l = (warp & 3) * 16 + lane;                // row of this lane (lanes 0..15: a 64-row accumulator)
-    if (!a.no_output)
+    if (kMode == 0)
       for (int blk = 0; blk < nblk; ++blk) {
         const uint32_t t = tmem + (blk & 1) * 128 + lane_base, par = (blk >> 1) & 1;
         wait_or_fail(bars + kDoneMY + (blk & 1), par, failed);
@@ -363,7 +369,7 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
         const char* q = (const char*)(xp + (int64_t)(m0 + l) * a.x_sl);
         asm volatile("prefetch.global.L2 [%0];" ::"l"(q));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(q + a.P * 2 - 1));
-        if (a.has_z && !a.no_output) {
+        if (a.has_z && kMode == 0) {
           const char* z = (const char*)(a.z + b * a.z_sb + h * a.z_sh + (int64_t)(m0 + l) * a.z_sl);
           asm volatile("prefetch.global.L2 [%0];" ::"l"(z));
           asm volatile("prefetch.global.L2 [%0];" ::"l"(z + a.P * 2 - 1));
@@ -391,10 +397,16 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
         if (!ready) {                                    // block blk - 2: its MMAs and its output rows have read this tile
           ready = true;
           wait_or_fail(bars + kDoneB + (blk & 1), ((blk >> 1) - 1) & 1, failed);
-          if (!a.no_output) wait_or_fail(bars + kYEmpty + (blk & 1), ((blk >> 1) - 1) & 1, failed);
+          if (kMode == 0) wait_or_fail(bars + kYEmpty + (blk & 1), ((blk >> 1) - 1) & 1, failed);
         }
 #pragma unroll
         for (int k = 0; k < KG; ++k) {
+          if (kMode == 2 && a.has_z && ls < QB) {            // dy = dout silu(z), rounded as the backward rounds it
+            const uint2 zw = *(const uint2*)(a.z + b * a.z_sb + h * a.z_sh + (int64_t)(mrow0(blk) + clampr(ls, rows)) * a.z_sl + gs * 4);
+            const float2 z0 = unpack_bf16(zw.x), z1 = unpack_bf16(zw.y), g0 = unpack_bf16(v[k].x), g1 = unpack_bf16(v[k].y);
+            auto silu = [](float z) { return __fdividef(z, 1.f + ex2f(-z * LOG2E)); };
+            v[k] = make_uint2(pack_bf16(g0.x * silu(z0.x), g0.y * silu(z0.y)), pack_bf16(g1.x * silu(z1.x), g1.y * silu(z1.y)));
+          }
           if (ls < QB) *(uint2*)(tile + sw128_off(ls, gs * 4)) = inside(ls, rows) ? v[k] : make_uint2(0, 0);
           ls += dl; gs += dg;
           if (gs >= ngrp) { gs -= ngrp; ++ls; }
@@ -413,10 +425,10 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
       if (blk >= nblk || lane != 0) return;
       uint64_t* bar = bars + kRaw + (blk & 1);
       uint8_t* dst = smem + (blk & 1) * SM::kSet;
-      mbar_expect_tx(bar, SM::kSet);
+      mbar_expect_tx(bar, kMode == 0 ? SM::kSet : SM::kHalf);
 #pragma unroll
       for (int at = 0; at < NT / 64; ++at) {
-        tma_load_3d(dst + at * (QB * 128), &maps.C, g * (int)a.C_sg + n_off + at * 64, mrow0(blk), b, bar);
+        if (kMode == 0) tma_load_3d(dst + at * (QB * 128), &maps.C, g * (int)a.C_sg + n_off + at * 64, mrow0(blk), b, bar);
         tma_load_3d(dst + SM::kHalf + at * (QB * 128), &maps.B, g * (int)a.B_sg + n_off + at * 64, mrow0(blk), b, bar);
       }
     };
@@ -428,7 +440,7 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
       wait_or_fail(bars + kFullP + set, par, failed);
       wait_or_fail(bars + kReadyS, blk & 1, failed);
       fence_after_sync();
-      if (lane == 0 && !a.no_output) {
+      if (lane == 0 && kMode == 0) {
 #pragma unroll
         for (int at = 0; at < NT / 64; ++at)
 #pragma unroll
@@ -453,10 +465,10 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
         mma_commit(bars + kDoneS + set);
       }
       __syncwarp();
-      if (!a.no_output) wait_or_fail(bars + kReadyM, blk & 1, failed);
+      if (kMode == 0) wait_or_fail(bars + kReadyM, blk & 1, failed);
       fence_after_sync();
       if (lane == 0) {
-        if (!a.no_output) {
+        if (kMode == 0) {
 #pragma unroll
           for (int k = 0; k < 4; ++k) {                  // Y += tril(M) x
             const int kk = kRev ? 3 - k : k;
@@ -484,32 +496,71 @@ __global__ void __launch_bounds__(2 * NT + (NT == 256 ? 512 : 384), 1) k_fwd_pip
   if (warp == 0) tmem_dealloc(tmem, 512);
 }
 
-template <int NT, typename TDT, bool kRev>
+template <int NT, typename TDT, bool kRev, int kMode>
 int launch(const TArgs& a, const FwdMaps& maps, cudaStream_t s) {
   const size_t smem = PipeSmem<NT>::kTotal + 1024;
   struct Tag {};
-  if (SmemAttrOnce<Tag>::set(k_fwd_pipe<NT, TDT, kRev>, smem) != ISSM_OK) return ISSM_ERR_CUDA;
-  ISSM_LAUNCH((k_fwd_pipe<NT, TDT, kRev>), dim3(a.N / NT, a.H, a.b), 2 * NT + (NT == 256 ? 512 : 384), smem, s, a, maps);
+  if (SmemAttrOnce<Tag>::set(k_fwd_pipe<NT, TDT, kRev, kMode>, smem) != ISSM_OK) return ISSM_ERR_CUDA;
+  ISSM_LAUNCH((k_fwd_pipe<NT, TDT, kRev, kMode>), dim3(a.N / NT, a.H, a.b), 2 * NT + (NT == 256 ? 512 : 384), smem, s, a, maps);
   return ISSM_OK;
 }
-template <int NT>
+template <int NT, int kMode>
 int launch_nt(const TArgs& a, const FwdMaps& maps, cudaStream_t s) {
-  if (a.dt_f32) return a.rev ? launch<NT, float, true>(a, maps, s) : launch<NT, float, false>(a, maps, s);
-  return a.rev ? launch<NT, bf16, true>(a, maps, s) : launch<NT, bf16, false>(a, maps, s);
+  if (a.dt_f32) return a.rev ? launch<NT, float, true, kMode>(a, maps, s) : launch<NT, float, false, kMode>(a, maps, s);
+  return a.rev ? launch<NT, bf16, true, kMode>(a, maps, s) : launch<NT, bf16, false, kMode>(a, maps, s);
+}
+template <int NT>
+int launch_mode(const TArgs& a, const FwdMaps& maps, int mode, cudaStream_t s) {
+  return mode == 0 ? launch_nt<NT, 0>(a, maps, s) : mode == 1 ? launch_nt<NT, 1>(a, maps, s) : launch_nt<NT, 2>(a, maps, s);
+}
+
+// Gradient states of the streams that the pipelined walk has marked (a block outside its range): the recurrence row by row,
+// thread = state.  Rare; a.rev is the direction of the WALK, i.e. against the scan.
+template <typename TDT>
+__global__ void k_grad_states_rows(const __grid_constant__ TArgs a, int nt) {
+  const int h = blockIdx.y, b = blockIdx.z, g = h / a.hpg, n = blockIdx.x * nt + threadIdx.x;
+  if (!a.redo[(blockIdx.x * a.b + b) * a.H + h]) return;
+  const float A2 = a.A[h * a.N + n] * LOG2E, bias = a.has_bias ? a.bias[h * a.N + n] : 0.f;
+  float G[40], sum = 0.f;
+  for (int p = 0; p < 40; ++p) G[p] = 0.f;
+  for (int t = 0; t < a.L; ++t) {
+    const int64_t mr = trow(a, t);
+    bool clamped;
+    const float d = dt_transform(a, ldf((const TDT*)a.dt + b * a.dt_sb + mr * a.dt_sl + h * a.dt_sh + n), bias, clamped);
+    const float c = ldf(a.B + b * a.B_sb + mr * a.B_sl + g * a.B_sg + n), e = ex2f(d * A2);
+    sum += d * A2;
+    for (int p = 0; p < a.P; ++p) {
+      float dy = ldf(a.x + b * a.x_sb + mr * a.x_sl + h * a.x_sh + p);
+      if (a.has_z) {
+        const float z = ldf(a.z + b * a.z_sb + mr * a.z_sl + h * a.z_sh + p);
+        dy = __bfloat162float(__float2bfloat16_rn(dy * __fdividef(z, 1.f + ex2f(-z * LOG2E))));
+      }
+      G[p] = e * fmaf(c, dy, G[p]);
+    }
+  }
+  for (int p = 0; p < a.P; ++p) a.final_states[(((size_t)b * a.H + h) * a.P + p) * a.N + n] = G[p];
+  if (a.sums) a.sums[((size_t)b * a.H + h) * a.N + n] = sum;
 }
 }  // namespace
 
+int launch_grad_states_rows(const TArgs& a, int nt, cudaStream_t s) {
+  const dim3 grid(a.N / nt, a.H, a.b);
+  if (a.dt_f32) ISSM_LAUNCH(k_grad_states_rows<float>, grid, nt, 0, s, a, nt);
+  else ISSM_LAUNCH(k_grad_states_rows<bf16>, grid, nt, 0, s, a, nt);
+  return ISSM_OK;
+}
+
 // the fast forward walk; streams with a block outside its range are marked in a.redo.  Where B or C has no tensor map (strides
 // that TMA does not take) every stream is marked, which leaves it to the windowed kernel
-int launch_fwd_pipe(const TArgs& a, const issm_params& p, int nt, cudaStream_t s) {
+int launch_fwd_pipe(const TArgs& a, int nt, int mode, cudaStream_t s) {
   FwdMaps maps;
   memset(&maps, 0, sizeof(maps));
-  if (!make_tile_map(p.B, p.B_sb, p.B_sl, (int64_t)(p.ngroups - 1) * p.B_sg + p.dstate, p.batch, p.seqlen, &maps.B) ||
-      !make_tile_map(p.C, p.C_sb, p.C_sl, (int64_t)(p.ngroups - 1) * p.C_sg + p.dstate, p.batch, p.seqlen, &maps.C)) {
+  if (!make_tile_map(a.B, a.B_sb, a.B_sl, (int64_t)(a.G - 1) * a.B_sg + a.N, a.b, a.L, &maps.B) ||
+      (mode == 0 && !make_tile_map(a.C, a.C_sb, a.C_sl, (int64_t)(a.G - 1) * a.C_sg + a.N, a.b, a.L, &maps.C))) {
     const size_t n = (size_t)(a.N / nt) * a.b * a.H * sizeof(int);
     return cudaMemsetAsync(a.redo, 1, n, s) == cudaSuccess ? ISSM_OK : ISSM_ERR_CUDA;
   }
-  return nt == 256 ? launch_nt<256>(a, maps, s) : launch_nt<128>(a, maps, s);
+  return nt == 256 ? launch_mode<256>(a, maps, mode, s) : launch_mode<128>(a, maps, mode, s);
 }
 
 }  // namespace issm

@@ -339,6 +339,141 @@ std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tenso
   return {r[0].x, r[1].x, r[0].dt, r[0].A, r[0].B, r[0].C, r[1].B, r[1].C, r[0].D, r[0].z, r[0].bias, r[0].init};
 }
 
+// ---- one sequence cut into slices that run as extra batch entries (seqpar.py describes the algorithm) ---------------------
+// Tensor-core path: pass 1 walks states only (issm_params.states_only), one kernel chains the slices, pass 2 is the scan itself.
+struct Fold {                                              // `n` equal slices of `len` points folded into the batch axis, then a tail
+  int64_t n, len, tail, b, L;
+  Fold(int64_t b_, int64_t L_, int64_t R) : b(b_), L(L_) {
+    for (int64_t r = R; r > std::max<int64_t>(1, R / 2); --r)       // a slice count that divides the length, if there is one near
+      if (L % r == 0) { n = r; len = L / r; tail = 0; return; }
+    len = (L + R - 1) / R; n = L / len; tail = L % len;
+  }
+  int groups() const { return tail ? 2 : 1; }
+  Tensor part(const Tensor& t, int g) const {
+    if (g) return t.narrow(1, n * len, tail);
+    auto shape = t.sizes().vec();
+    shape[0] = b * n;
+    shape[1] = len;
+    return t.narrow(1, 0, n * len).reshape(shape);
+  }
+  OptTensor part(const OptTensor& t, int g) const { return t ? OptTensor(part(*t, g)) : t; }
+  Tensor join(const Tensor& main, const Tensor& rest) const {
+    auto shape = main.sizes().vec();
+    shape[0] = b;
+    shape[1] = n * len;
+    const Tensor m = main.reshape(shape);
+    return tail ? at::cat({m, rest}, 1) : m;
+  }
+};
+void chain(const Fold& f, const Tensor (&F)[2], const Tensor (&sums)[2], const OptTensor& start, bool descending, Tensor (&enter)[2], at::ScalarType enter_type,
+           const Tensor& last) {
+  issm_slice_chain q{};
+  q.batch = (int32_t)f.b; q.nmain = (int32_t)f.n; q.nheads = (int32_t)F[0].size(1); q.headdim = (int32_t)F[0].size(2); q.dstate = (int32_t)F[0].size(3);
+  q.descending = descending; q.enter_f32 = enter_type == at::kFloat;
+  for (int g = 0; g < f.groups(); ++g) enter[g] = at::empty(F[g].sizes(), F[g].options().dtype(enter_type));
+  q.f_main = F[0].data_ptr<float>(); q.s_main = sums[0].data_ptr<float>(); q.enter_main = enter[0].data_ptr();
+  if (f.tail) { q.f_tail = F[1].data_ptr<float>(); q.s_tail = sums[1].data_ptr<float>(); q.enter_tail = enter[1].data_ptr(); }
+  Tensor st;
+  if (start) {
+    st = start->contiguous();
+    q.start = st.data_ptr(); q.start_f32 = dtype_code(st.scalar_type()) == ISSM_F32;
+  }
+  if (last.defined()) { q.last = last.data_ptr(); q.last_f32 = dtype_code(last.scalar_type()) == ISSM_F32; }
+  check_rc(issm_b200_slice_chain(&q, stream_of(F[0])), "issm_b200_slice_chain");
+}
+void states_pass(Common& c, int mode, Tensor& F, Tensor& sums) {
+  issm_params& p = c.p;
+  const auto fo = c.x.options().dtype(at::kFloat);
+  F = at::empty({p.batch, p.nheads, p.headdim, p.dstate}, fo);
+  sums = at::empty({p.batch, p.nheads, p.dstate}, fo);
+  p.states_only = mode; p.want_final = 1;
+  p.final_states = F.data_ptr<float>(); p.state_sums = sums.data_ptr<float>();
+  attach_workspace(c, 0);
+  check_rc(issm_b200_fwd(&p, stream_of(c.x)), "issm_b200_fwd");
+}
+
+// Slices for a call, or 1 where it does not take the tensor-core kernels (the fp32 kernels cut the sequence themselves).
+int64_t usable_slices(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, int64_t path, const Tensor& status,
+                      int64_t slices) {
+  if (slices <= 1 || path == ISSM_PATH_SIMT || !x.is_cuda()) return 1;
+  Common c;
+  fill_common(c, x, dt, A, B, C, chunk, {}, {}, {}, {}, false, 0.0, 3e38, false, path, status);
+  return issm_b200_resolve_path_pass(&c.p, 1) == ISSM_PATH_TENSOR ? slices : 1;
+}
+
+// (out, final, then per group - main slices, tail - the entering states, out_x, saved states and sums)
+std::vector<Tensor> sliced_fwd(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, const OptTensor& D,
+                               const OptTensor& z, const OptTensor& dt_bias, const OptTensor& initial_states, bool dt_softplus, double dt_min, double dt_max,
+                               bool reverse, int64_t path, int64_t slices, bool save, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Fold f(x.size(0), x.size(1), slices);
+  std::vector<Tensor> keep;
+  const Tensor Ak = par(A, keep);
+  const OptTensor bias = bias_2d(dt_bias, A), init = once(initial_states, x.scalar_type());
+  Tensor F[2], sums[2], enter[2], out[2], out_x[2], none_fin, saved[2];
+  for (int g = 0; g < f.groups(); ++g) {
+    Common c;
+    fill_common(c, f.part(x, g), f.part(dt, g), Ak, f.part(B, g), f.part(C, g), chunk, {}, {}, bias, {}, dt_softplus, dt_min, dt_max, reverse, path, status);
+    states_pass(c, 1, F[g], sums[g]);
+  }
+  Tensor fin = at::empty({x.size(0), x.size(2), x.size(3), A.size(1)}, x.options().dtype(at::kFloat));
+  chain(f, F, sums, init, reverse, enter, x.scalar_type(), fin);
+  for (int g = 0; g < f.groups(); ++g) {
+    Common c;
+    fill_common(c, f.part(x, g), f.part(dt, g), Ak, f.part(B, g), f.part(C, g), chunk, D, f.part(z, g), bias, enter[g], dt_softplus, dt_min, dt_max, reverse,
+                path, status);
+    attach_fwd(c, z.has_value(), false, save, out[g], out_x[g], none_fin, saved[g]);
+    attach_workspace(c, 0);
+    check_rc(issm_b200_fwd(&c.p, stream_of(c.x)), "issm_b200_fwd");
+  }
+  std::vector<Tensor> r{f.join(out[0], out[1]), fin};
+  for (int g = 0; g < f.groups(); ++g)
+    for (const Tensor& t : {enter[g], out_x[g], saved[g], sums[g]}) r.push_back(t);
+  return r;
+}
+
+// The tuple of `bwd` for the whole sequence; `kept`: what sliced_fwd returned behind (out, final).
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> sliced_bwd(
+    const Tensor& dout, const OptTensor& dfinal, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk,
+    const OptTensor& D, const OptTensor& z, const OptTensor& dt_bias, const OptTensor& initial_states, bool dt_softplus, double dt_min, double dt_max,
+    bool reverse, int64_t path, int64_t slices, const std::vector<Tensor>& kept, const Tensor& status) {
+  const c10::cuda::CUDAGuard guard(x.device());
+  const Fold f(x.size(0), x.size(1), slices);
+  std::vector<Tensor> keep;
+  const Tensor Ak = par(A, keep), gy = act(dout, x.scalar_type(), keep);
+  const OptTensor bias = bias_2d(dt_bias, A), dfin = dfinal ? OptTensor(dfinal->to(at::kFloat).contiguous()) : OptTensor();
+  Tensor G[2], sums[2], leave[2];
+  for (int g = 0; g < f.groups(); ++g) {
+    Common c;
+    fill_common(c, f.part(x, g), f.part(dt, g), Ak, f.part(B, g), f.part(C, g), chunk, {}, f.part(z, g), bias, {}, dt_softplus, dt_min, dt_max, reverse, path,
+                status);
+    const Tensor d = act(f.part(gy, g), x.scalar_type(), c.keep);
+    c.p.dout = d.data_ptr(); c.p.dout_sb = d.stride(0); c.p.dout_sl = d.stride(1); c.p.dout_sh = d.stride(2);
+    states_pass(c, 2, G[g], sums[g]);
+  }
+  Tensor dinit = initial_states ? at::empty(initial_states->sizes(), x.options()) : Tensor();
+  chain(f, G, sums, dfin, !reverse, leave, at::kFloat, dinit);
+  Grads r[2];
+  for (int g = 0; g < f.groups(); ++g) {
+    Common c;
+    const Tensor &enter = kept[g * 4], &out_x = kept[g * 4 + 1], &saved = kept[g * 4 + 2];
+    fill_common(c, f.part(x, g), f.part(dt, g), Ak, f.part(B, g), f.part(C, g), chunk, D, f.part(z, g), bias, enter, dt_softplus, dt_min, dt_max, reverse, path,
+                status);
+    attach_bwd(c, f.part(gy, g), out_x.defined() && out_x.numel() ? OptTensor(out_x) : OptTensor(), D, f.part(z, g), bias, enter, leave[g], saved, r[g]);
+    attach_workspace(c, 1);
+    check_rc(issm_b200_bwd(&c.p, stream_of(c.x)), "issm_b200_bwd");
+  }
+  if (f.tail) {
+    std::vector<issm_add_item> add;
+    add_item(add, r[0].A, r[1].A, 1.0);
+    if (D) add_item(add, r[0].D, r[1].D, 1.0);
+    if (dt_bias) add_item(add, r[0].bias, r[1].bias, 1.0);
+    check_rc(issm_b200_add_multi(add.data(), (int32_t)add.size(), stream_of(x)), "issm_b200_add_multi");
+  }
+  return {f.join(r[0].x, r[1].x), f.join(r[0].dt, r[1].dt), r[0].A, f.join(r[0].B, r[1].B), f.join(r[0].C, r[1].C), r[0].D,
+          z ? f.join(r[0].z, r[1].z) : r[0].z, r[0].bias, dinit.defined() ? dinit : r[0].z};
+}
+
 // ---- gated norms ------------------------------------------------------------------------------------
 void fill_norm(issm_norm_params& p, const Tensor& x2, const OptTensor& z2, const Tensor& weight, const OptTensor& bias,
                double eps, int64_t group_size, bool norm_before_gate, bool is_rms) {

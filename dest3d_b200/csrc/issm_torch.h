@@ -39,4 +39,13 @@ std::tuple<Tensor, Tensor, Tensor> norm_fwd(const Tensor& x2, const OptTensor& z
 std::tuple<Tensor, Tensor, Tensor, Tensor> norm_bwd(const Tensor& dy2, const Tensor& x2, const OptTensor& z2, const Tensor& weight, const OptTensor& bias,
                                                     const Tensor& rstd, const OptTensor& mean, double eps, int64_t group_size, bool norm_before_gate,
                                                     bool is_rms);
+int64_t usable_slices(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, int64_t path, const Tensor& status,
+                      int64_t slices);
+std::vector<Tensor> sliced_fwd(const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk, const OptTensor& D,
+                               const OptTensor& z, const OptTensor& dt_bias, const OptTensor& initial_states, bool dt_softplus, double dt_min, double dt_max,
+                               bool reverse, int64_t path, int64_t slices, bool save, const Tensor& status);
+std::tuple<Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor, Tensor> sliced_bwd(
+    const Tensor& dout, const OptTensor& dfinal, const Tensor& x, const Tensor& dt, const Tensor& A, const Tensor& B, const Tensor& C, int64_t chunk,
+    const OptTensor& D, const OptTensor& z, const OptTensor& dt_bias, const OptTensor& initial_states, bool dt_softplus, double dt_min, double dt_max,
+    bool reverse, int64_t path, int64_t slices, const std::vector<Tensor>& kept, const Tensor& status);
 }  // namespace issm_host

@@ -25,7 +25,7 @@ input dtype (bf16 inputs: rounded to bf16 there, like the initial_states of any 
 import torch
 import torch.distributed as dist
 
-from . import issm_combined
+from . import _ext, issm_combined
 
 
 def _wide(t):
@@ -304,6 +304,11 @@ def issm_scan_chunk_parallel(x, dt, A, B, C, chunk_size, D=None, z=None, dt_bias
         return issm_combined.ISSM_chunk_scan_combined(x, dt, A, B, C, chunk_size, D=D, z=z, dt_bias=dt_bias, initial_states=initial_states,
                                                       dt_softplus=dt_softplus, dt_limit=dt_limit, return_final_states=return_final_states,
                                                       reverse=reverse, path=path)
+    if backend is KernelBackend and issm_combined.BINDING == "torch":
+        # one operation: states-only first passes, one kernel for the chain
+        out, final = _ext.call("sliced_scan")(x, dt, A, B, C, int(chunk_size), D, z, dt_bias, initial_states, bool(dt_softplus), float(dt_limit[0]),
+                                              float(dt_limit[1]), bool(reverse), issm_combined._PATHS[path], R, issm_combined._status_word(x.device))
+        return (out, final) if return_final_states else out
     out, final = _sliced(Solo(), R, x, dt, A, B, C, chunk_size, D, z, dt_bias, initial_states, dt_softplus, dt_limit, reverse, path, backend)
     return (out, final) if return_final_states else out
 

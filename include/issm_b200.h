@@ -106,6 +106,12 @@ typedef struct issm_params {
    * forward stores the state entering every 64-point block (and the final state) here; a backward given
    * the same buffer skips recomputing them (the reference recomputes: issm_combined.py:136-144). */
   void* saved_states;
+  /* Slices of a sequence (tensor-core path, forward entry point only).  states_only = 1: no output rows, only final_states from
+   * initial_states.  states_only = 2: the adjoint - final_states receives the gradient that the outputs' gradient `dout` (through
+   * the gate z when has_z) sends to the state ENTERING the sequence; x, B, initial_states are not read.  state_sums (optional,
+   * (batch, nheads, dstate) float): log2 of the factor the sequence applies to the state entering it. */
+  int32_t states_only;
+  float* state_sums;
 } issm_params;
 
 /* Gated RMS / Layer norm over the last dimension of a (rows, hidden) matrix
@@ -276,6 +282,20 @@ int issm_b200_glue_bwd(const issm_glue_params* p, void* cuda_stream);
 int issm_b200_dt_sum(const void* dt, int32_t dt_dtype, int32_t batch, int32_t seqlen, int32_t nheads, int32_t dstate,
                      int64_t dt_sb, int64_t dt_sl, int64_t dt_sh, const float* dt_bias, int32_t dt_softplus, float dt_min,
                      float dt_max, int32_t rows_per_part, float* part, void* cuda_stream);
+
+/* The chain of the slices of each sequence, in scan order (or against it for the adjoint): with local end states F and log2
+ * factors sums of every slice, run = start; per slice: enter[slice] = run, run = F + 2^sums * run; last = run.
+ * Slices of one sequence are `nmain` consecutive entries of the `main` arrays (batch * nmain, nheads, headdim, dstate) and, when
+ * the tail pointers are given, one more behind them (batch, ...).  descending: the slices are visited from the last to the first.
+ * Types: F float; start and last float or the activation type (is_f32 flags); enter float or bfloat16. */
+typedef struct issm_slice_chain {
+  int32_t batch, nmain, nheads, headdim, dstate, descending, start_f32, last_f32, enter_f32;
+  const float* f_main; const float* s_main; const float* f_tail; const float* s_tail;
+  const void* start;              /* or null (zero) */
+  void* enter_main; void* enter_tail; void* last;
+} issm_slice_chain;
+size_t issm_b200_sizeof_slice_chain(void);
+int issm_b200_slice_chain(const issm_slice_chain* p, void* cuda_stream);
 
 /* ---- joining the two scan directions ------------------------------------------------------------------------ */
 

@@ -398,7 +398,7 @@ __global__ void __launch_bounds__(NORM_BWD_WARPS * 32, (CH == 1 && !HB) ? 5 : 0)
 // The general vector kernels spend 39 (forward) and 73 (backward) instructions per element and are bound by instruction
 // issue in bf16.  Here two features go through each packed instruction, the sigmoid is evaluated once, and what the call
 // never asks for (mean, bias, the other gate) is left out: about 8 and 15 per element, so the memory system is the bound.
-// 2^18 rows x 288 features bf16, forward + backward call: see the table of the kernels' numbers at launch_norm_bwd_main.
+// 2^18 rows x 288 features bf16, forward + backward call: 373 us with the general kernels, 240 us with these (82 + 145 us on the device).
 template <typename T> struct Pairs {                       // 16 bytes of a row as float pairs
   static constexpr int NP = Vec16<T>::N / 2;
   static __device__ __forceinline__ void unpack(uint4 w, float2* v) {

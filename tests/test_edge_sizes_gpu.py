@@ -1,0 +1,113 @@
+"""The kernels at the sizes where their tiles, remainders and dispatch rules change, against the oracle or the plain formula in
+float64: blocked float32 scan (32-row blocks, 32-state warps), pipelined bf16 forward (64-row blocks), joined scan directions,
+gated RMS norm rows of several widths, row gather in fours, parameter generation in quads of rows, sliced scan with a tail."""
+import ctypes as ct
+
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle import issm_oracle as O
+from tests import parity
+
+pytestmark = pytest.mark.gpu
+BENCH = dict(dt_softplus=True, dt_limit=(1e-3, 1e-1))
+
+
+@pytest.mark.parametrize("dtype,b,L,H,P,N,G,opts", [
+    (torch.float32, 1, 1, 1, 1, 1, 1, {}), (torch.float32, 2, 31, 2, 32, 31, 1, {}), (torch.float32, 1, 32, 2, 33, 33, 2, {}),
+    (torch.float32, 1, 33, 2, 40, 32, 1, dict(reverse=True)), (torch.float32, 1, 65, 2, 41, 100, 1, {}),
+    (torch.float32, 1, 700, 1, 36, 48, 1, dict(reverse=True)), (torch.float32, 1, 96, 2, 80, 64, 2, dict(use_z=False)),
+    (torch.float32, 1, 64, 1, 128, 65, 1, {}), (torch.float32, 1, 40, 1, 130, 40, 1, {}),
+    (torch.float32, 1, 100, 2, 36, 64, 1, dict(offset=3.0, dt_limit=(0.0, float("inf")), loosen=4.0)),       # leaves the blocked range
+    (torch.bfloat16, 1, 96, 2, 64, 64, 1, {}), (torch.bfloat16, 1, 1, 2, 36, 256, 1, dict(reverse=True)),
+    (torch.bfloat16, 1, 63, 2, 4, 128, 1, {}), (torch.bfloat16, 1, 65, 2, 40, 128, 1, dict(reverse=True)),
+    (torch.bfloat16, 1, 129, 2, 36, 512, 1, dict(use_initial_states=False)), (torch.bfloat16, 1, 200, 2, 36, 256, 2, dict(noncontig_bc=True))])
+def test_scan(dtype, b, L, H, P, N, G, opts):
+    opts = dict(BENCH, **opts)
+    inp = O.make_inputs(b, L, H, P, N, G=G, seed=L + N, dtype=dtype)
+    inp["dt"] = inp["dt"] + opts.get("offset", 0.0)
+    ref = parity.oracle_run(inp, 64, opts)
+    parity.compare(parity.cuda_run(inp, 64, opts), ref, dtype, loosen=opts.get("loosen", 1.0))
+
+
+@pytest.mark.parametrize("offset,z,L,reverse", [(0.0, True, 523, False), (0.0, False, 512, True), (2.0, True, 523, True)])
+def test_sliced_scan(offset, z, L, reverse):
+    """Tail, gate, and the row-by-row gradient states of streams outside the range of the tensor-core factorisation."""
+    from dest3d_b200.seqpar import issm_scan_chunk_parallel
+    inp = O.make_inputs(1, L, 2, 36, 256, seed=5, dtype=torch.bfloat16)
+    inp["dt"] = inp["dt"] + offset
+    opts = dict(BENCH, reverse=reverse, use_z=z)
+    if offset:
+        opts["dt_limit"] = (0.0, float("inf"))
+    ref = parity.oracle_run(inp, 64, opts)
+    lv = {k: inp[k].cuda().requires_grad_() for k in parity.GRADS if k != "z" or z}
+    out, fin = issm_scan_chunk_parallel(lv["x"], lv["dt"], lv["A"], lv["B"], lv["C"], 64, D=lv["D"], z=lv.get("z"), dt_bias=lv["dt_bias"],
+                                        initial_states=lv["initial_states"], return_final_states=True, reverse=reverse, path="tensor", slices=3,
+                                        dt_softplus=True, dt_limit=opts["dt_limit"])
+    ((out.float() * inp["dout"].cuda().float()).sum() + (fin * inp["dfinal"].cuda()).sum()).backward()
+    got = dict({"out": out.detach(), "final": fin.detach()}, **{"d" + k: v.grad for k, v in lv.items()})
+    parity.compare(got, ref, torch.bfloat16)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("sizes", [(1,), (7, 8, 9), (4096, 16385, 3, 8193)])
+def test_add_multi(dtype, sizes):
+    from dest3d_b200 import _lib
+    pairs = [(torch.randn(n, device="cuda").to(dtype), torch.randn(n, device="cuda").to(dtype)) for n in sizes]
+    outs = [torch.empty_like(a) for a, _ in pairs]
+    lib = _lib.lib()
+
+    class Item(ct.Structure):
+        _fields_ = [("a", ct.c_void_p), ("b", ct.c_void_p), ("out", ct.c_void_p), ("n", ct.c_int64), ("dtype", ct.c_int32), ("scale", ct.c_float)]
+    items = (Item * len(sizes))(*[Item(a.data_ptr(), b.data_ptr(), o.data_ptr(), a.numel(), 0 if dtype == torch.float32 else 1, 0.5)
+                                  for (a, b), o in zip(pairs, outs)])
+    lib.issm_b200_add_multi.argtypes = [ct.c_void_p, ct.c_int32, ct.c_void_p]
+    assert lib.issm_b200_add_multi(items, len(sizes), torch.cuda.current_stream().cuda_stream) == 0
+    for (a, b), o in zip(pairs, outs):
+        assert torch.equal(o, ((a.float() + b.float()) * 0.5).to(dtype))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("rows,width", [(1, 8), (5, 128), (33, 256), (9, 264), (130, 288), (3, 512), (2, 520)])
+def test_gated_rms_norm(dtype, rows, width):
+    from dest3d_b200 import layernorm_fn
+    g = torch.Generator().manual_seed(rows + width)
+    x, z, dy = (torch.randn(rows, width, generator=g).to(dtype) for _ in range(3))
+    w = 1 + 0.02 * torch.randn(width, generator=g)
+    xr, wr, zr = (t.double().requires_grad_() for t in (x, w, z))
+    v = xr * F.silu(zr)
+    yr = v * torch.rsqrt(v.square().mean(-1, keepdim=True) + 1e-5) * wr
+    (yr * dy.double()).sum().backward()
+    xc, wc, zc = (t.cuda().requires_grad_() for t in (x, w, z))
+    y = layernorm_fn(xc, wc, None, zc, eps=1e-5, group_size=None, norm_before_gate=False, is_rms_norm=True)
+    (y.float() * dy.cuda().float()).sum().backward()
+    for name, got, ref in (("y", y, yr), ("dx", xc.grad, xr.grad), ("dw", wc.grad, wr.grad), ("dz", zc.grad, zr.grad)):
+        parity.close(got, ref, dtype, name)
+
+
+@pytest.mark.parametrize("N,C", [(1, 1), (3, 288), (4, 290), (5, 2), (1021, 36)])
+def test_gather_rows(N, C):
+    from dest3d_b200 import reorder_points
+    pts = torch.randn(2, N, C, device="cuda").bfloat16()
+    order = torch.stack([torch.randperm(N, device="cuda") for _ in range(2)])
+    assert torch.equal(reorder_points(pts, order), pts.gather(1, order.unsqueeze(-1).expand(-1, -1, C)))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("L,K,M,H,G", [(1, 1, 16, 1, 1), (3, 31, 16, 5, 1), (4, 34, 4, 3, 3), (9, 127, 8, 6, 2), (2, 258, 16, 7, 4)])
+def test_parameter_generation(dtype, L, K, M, H, G):
+    from dest3d_b200.adaptive_params import adaptive_dt_bc
+    from tests.test_adaptive_gpu import _reference
+    g = torch.Generator().manual_seed(L + K + H)
+    rn = lambda *s: torch.randn(*s, generator=g)
+    host = [rn(2, L, K, M).to(dtype), rn(H, M) * 0.3, rn(2 * G, M) * 0.3, rn(2, L, H).to(dtype), rn(H) - 2.0] + [rn(2, L, G).to(dtype) for _ in range(4)]
+    dev, ref_in = [v.cuda().requires_grad_() for v in host], [v.double().requires_grad_() for v in host]
+    got, ref = adaptive_dt_bc(*dev, None), _reference(*ref_in, None, G)
+    douts = [rn(*r.shape) for r in ref]
+    sum((o.float() * d.cuda()).sum() for o, d in zip(got, douts)).backward()
+    sum((r * d.double()).sum() for r, d in zip(ref, douts)).backward()
+    lim = 3e-2 if dtype == torch.bfloat16 else 1e-4
+    for u, v in list(zip(got, ref)) + [(d.grad, r.grad) for d, r in zip(dev, ref_in)]:
+        v = v.detach()
+        assert (u.double().cpu() - v).abs().max().item() <= lim * max(1.0, v.abs().max().item())

@@ -4,11 +4,10 @@
 //                                                                             their own token terms, alike)
 // where the reference runs dt_proj / bc_proj as two Linear layers over dist, transposes both results to the
 // (b, l, h, k) layout the scan wants, adds the per-token terms, applies softplus and multiplies by the mask in
-// separate elementwise passes.  Here a thread owns one state k of one point: it holds the M distance features in
-// registers, forms every output row, and stores each row coalesced over k in the scan's layout.
+// separate elementwise passes.  Here a warp takes 64 states of one point, forms every output row from one read of the
+// features, and stores each row in the scan's layout.
 // Backward: g = d(out) / d(pre) per output row; ddist = sum_r g[r] W[r, :]; the weight gradient sum_k g[r, k] dist[k, j]
-// is formed per point from shared-memory tiles and accumulated per block; the token terms are g summed over k in a
-// fixed order.
+// is accumulated per warp and block; the token terms are g summed over k in a fixed order.
 #include "issm_common.cuh"
 
 #include <type_traits>
@@ -32,53 +31,6 @@ struct GlueArgs {
   float* dtok;                                             // (b, L, RO)
 };
 
-template <typename T, int M>
-__device__ __forceinline__ void load_feats(const T* p, float (&d)[M]) {
-  if constexpr (sizeof(T) == 2 && M % 8 == 0) {
-#pragma unroll
-    for (int c = 0; c < M / 8; ++c) {
-      const uint4 u = ((const uint4*)p)[c];
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        d[c * 8 + 2 * i] = __uint_as_float(w[i] << 16);
-        d[c * 8 + 2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
-      }
-    }
-  } else if constexpr (sizeof(T) == 4 && M % 4 == 0) {
-#pragma unroll
-    for (int c = 0; c < M / 4; ++c) {
-      const float4 u = ((const float4*)p)[c];
-      d[c * 4] = u.x; d[c * 4 + 1] = u.y; d[c * 4 + 2] = u.z; d[c * 4 + 3] = u.w;
-    }
-  } else {
-#pragma unroll
-    for (int j = 0; j < M; ++j) d[j] = ldf(p + j);
-  }
-}
-
-template <typename T, int M>
-__device__ __forceinline__ void store_feats(T* p, const float (&d)[M]) {
-  if constexpr (sizeof(T) == 2 && M % 8 == 0) {
-#pragma unroll
-    for (int c = 0; c < M / 8; ++c) {
-      uint32_t w[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const __nv_bfloat162 h = __floats2bfloat162_rn(d[c * 8 + 2 * i], d[c * 8 + 2 * i + 1]);
-        w[i] = *(const uint32_t*)&h;
-      }
-      ((uint4*)p)[c] = make_uint4(w[0], w[1], w[2], w[3]);
-    }
-  } else if constexpr (sizeof(T) == 4 && M % 4 == 0) {
-#pragma unroll
-    for (int c = 0; c < M / 4; ++c) ((float4*)p)[c] = make_float4(d[c * 4], d[c * 4 + 1], d[c * 4 + 2], d[c * 4 + 3]);
-  } else {
-#pragma unroll
-    for (int j = 0; j < M; ++j) stf(p + j, d[j]);
-  }
-}
-
 __device__ __forceinline__ float glue_sigmoid(float v) { return __fdividef(1.f, 1.f + __expf(-v)); }
 
 // softplus with threshold 20 in the log2 domain (hardware ex2 / lg2); below -4 the series of log1p in u = e^v, where
@@ -92,351 +44,398 @@ __device__ __forceinline__ float glue_softplus(float v) {
   return v <= 20.f ? r : v;
 }
 
-// one block per point (b, l); a thread owns two adjacent states and computes them with packed fp32 instructions,
-// reading four weights per shared-memory access
+// ---- the contractions on the matrix pipe -----------------------------------------------------------------------------
+// Both directions contract over at most 16 features and 16 rows: one m16n8k16 tile in either index.  On the fp32 pipe the
+// backward spent 450 multiply-adds per (point, state) and shared-memory traffic for the weight gradient: 16 x 4096 points x 256
+// states x 16 features bf16 1200 us, forward 347 us; here 717 and 237 us (forward 4 TB/s).  float operands go in as three bf16 terms (24 bits: the value itself),
+// products down to 2^-24 of the largest are formed, sums are float, so nothing is lost against float multiply-adds.  The tiles
+// are too small for the tensor memory path: 16 rows x 16 deep, with element-wise work between the products in registers.
+//
+// A warp works on 64 states of a point.  Lane = (c, q) = (lane / 4, lane % 4).  The orders of states and features inside a tile
+// are free, so they are chosen for the memory accesses: column c of tile j (8 columns each) is state 16 (c / 2) + 2 j + (c & 1),
+// so that in the row-major fragments lane q owns the 16 CONSECUTIVE states from 16 q of rows c and c + 8 (32 bytes of bf16);
+// features 4 q .. 4 q + 3 sit with lane q, so a state's 32 bytes of bf16 features are one sector read by four lanes.
+constexpr int GLUE_WARPS = 4;
+__device__ __forceinline__ uint32_t pk(float lo, float hi) {
+  const __nv_bfloat162 h = __floats2bfloat162_rn(lo, hi);
+  return *(const uint32_t*)&h;
+}
+__device__ __forceinline__ float2 upk(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+__device__ __forceinline__ float2 upk(float2 v) { return v; }
+__device__ __forceinline__ void split3(float2 v, uint32_t (&s)[3]) {
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    s[i] = pk(v.x, v.y);
+    const float2 h = upk(s[i]);
+    if (i < 2) v = make_float2(v.x - h.x, v.y - h.y);
+  }
+}
+struct Frag { uint32_t r[4]; };
+__device__ __forceinline__ void mma16(float (&d)[4], const Frag& a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a.r[0]), "r"(a.r[1]), "r"(a.r[2]), "r"(a.r[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t transpose8(uint32_t v) {
+  uint32_t r;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+  return r;
+}
+// d += sum over the terms s of A and t of B with s + t <= 2, smallest first
+template <int NA, int NB, typename FA, typename FB>
+__device__ __forceinline__ void mma_terms(float (&d)[4], FA a, FB b) {
+#pragma unroll
+  for (int tot = 2; tot >= 0; --tot)
+#pragma unroll
+    for (int s = 0; s <= tot; ++s)
+      if (s < NA && tot - s < NB) {
+        uint32_t b0, b1;
+        b(tot - s, b0, b1);
+        mma16(d, a(s), b0, b1);
+      }
+}
+__device__ __forceinline__ float glue_w(const GlueArgs& a, int M, int r, int f) {
+  return f >= M ? 0.f : r < a.H ? a.w[r * M + f] : r < a.RW ? a.wbc[(r - a.H) * M + f] : 0.f;
+}
+// weights as the A operand of pre[row][state] = sum_f W[row][f] dist[state][f]
+__device__ __forceinline__ void weight_rows(const GlueArgs& a, int M, int c, int q, Frag (&w)[3]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = c + 8 * (i & 1), f = 4 * q + (i & 2);
+    uint32_t s[3];
+    split3(make_float2(glue_w(a, M, r, f), glue_w(a, M, r, f + 1)), s);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) w[k].r[i] = s[k];
+  }
+}
+// features 4 q .. of the eight states of column c, as loaded
+template <typename TD> struct Feat { using t = uint2; };
+template <> struct Feat<float> { using t = float4; };
+__device__ __forceinline__ void feat_terms(uint2 v, uint32_t (&s)[1][2]) { s[0][0] = v.x; s[0][1] = v.y; }
+__device__ __forceinline__ void feat_terms(float4 v, uint32_t (&s)[3][2]) {
+  uint32_t lo[3], hi[3];
+  split3(make_float2(v.x, v.y), lo);
+  split3(make_float2(v.z, v.w), hi);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) { s[k][0] = lo[k]; s[k][1] = hi[k]; }
+}
+template <typename TD>
+__device__ __forceinline__ void load_states(const GlueArgs& a, int M, int pt, int k0, int c, int q, typename Feat<TD>::t (&d)[8]) {
+  using F = typename Feat<TD>::t;
+  const int b = pt / a.L, l = pt - b * a.L, kc = k0 + 16 * (c >> 1) + (c & 1);
+  const TD* p = (const TD*)a.dist + b * a.d_sb + l * a.d_sl + (int64_t)kc * a.d_sk + 4 * q;
+  const bool has = 4 * q < M;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    F v{};
+    if (has && kc + 2 * j < a.K) v = *(const F*)(p + (int64_t)(2 * j) * a.d_sk);
+    d[j] = v;
+  }
+}
+// lane (c, q) holds the mask of states 16 q + 2 c, + 1: tile j's pair of lane q is with lane (j, q)
+__device__ __forceinline__ float2 load_mask(const GlueArgs& a, int pt, int k0, int c, int q) {
+  const int k = k0 + 16 * q + 2 * c;
+  if (!a.mask) return make_float2(1.f, 1.f);
+  const float* p = a.mask + (int64_t)pt * a.K + k;
+  return make_float2(k < a.K ? p[0] : 0.f, k + 1 < a.K ? p[1] : 0.f);
+}
+__device__ __forceinline__ float2 mask_of(float2 m, int j, int q) {
+  return make_float2(__shfl_sync(0xffffffffu, m.x, j * 4 + q), __shfl_sync(0xffffffffu, m.y, j * 4 + q));
+}
+// 16 consecutive states of a row as eight pairs; vec: rows start on 16-byte boundaries
+__device__ __forceinline__ void load_row(const bf16* p, int k, int K, bool vec, uint32_t (&v)[8]) {
+  if (vec && k + 16 <= K) {
+    const uint4 x = ((const uint4*)(p + k))[0], y = ((const uint4*)(p + k))[1];
+    v[0] = x.x; v[1] = x.y; v[2] = x.z; v[3] = x.w; v[4] = y.x; v[5] = y.y; v[6] = y.z; v[7] = y.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const uint16_t* u = (const uint16_t*)p + k + 2 * j;
+      v[j] = (k + 2 * j < K ? (uint32_t)u[0] : 0u) | (k + 2 * j + 1 < K ? (uint32_t)u[1] << 16 : 0u);
+    }
+  }
+}
+__device__ __forceinline__ void load_row(const float* p, int k, int K, bool vec, float2 (&v)[8]) {
+  if (vec && k + 16 <= K) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float4 x = ((const float4*)(p + k))[j];
+      v[2 * j] = make_float2(x.x, x.y); v[2 * j + 1] = make_float2(x.z, x.w);
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = make_float2(k + 2 * j < K ? p[k + 2 * j] : 0.f, k + 2 * j + 1 < K ? p[k + 2 * j + 1] : 0.f);
+  }
+}
+__device__ __forceinline__ void store_row(bf16* p, int k, int K, bool vec, const float2 (&v)[8]) {
+  if (vec && k + 16 <= K) {
+    ((uint4*)(p + k))[0] = make_uint4(pk(v[0].x, v[0].y), pk(v[1].x, v[1].y), pk(v[2].x, v[2].y), pk(v[3].x, v[3].y));
+    ((uint4*)(p + k))[1] = make_uint4(pk(v[4].x, v[4].y), pk(v[5].x, v[5].y), pk(v[6].x, v[6].y), pk(v[7].x, v[7].y));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (k + 2 * j < K) stf(p + k + 2 * j, v[j].x);
+      if (k + 2 * j + 1 < K) stf(p + k + 2 * j + 1, v[j].y);
+    }
+  }
+}
+__device__ __forceinline__ void store_row(float* p, int k, int K, bool vec, const float2 (&v)[8]) {
+  if (vec && k + 16 <= K) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) ((float4*)(p + k))[j] = make_float4(v[2 * j].x, v[2 * j].y, v[2 * j + 1].x, v[2 * j + 1].y);
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      if (k + 2 * j < K) p[k + 2 * j] = v[j].x;
+      if (k + 2 * j + 1 < K) p[k + 2 * j + 1] = v[j].y;
+    }
+  }
+}
+
+// Forward: warps walk the (point, 64 states) items; the features of the next item are on their way while one is worked on.
 // TD: element type of dist (and ddist), T: of dt / bc and their gradients (float dist with bfloat16 outputs is what
 // autocast hands the block: the features stay float32, the activations are bfloat16)
-// Weights wait in shared memory as pairs (w, w): a 128-bit access gives two packed operands, where the scalar form cost a move
-// per multiply-add.  Blocks walk the points with a grid stride, so the weights are laid out once per block and not per point.
-// 16 x 4096 points x 256 states x 16 features bf16: 312 us before.
-// The dt rows are padded to a multiple of four (zero weights) and the B / C rows follow: rows are worked on four at a time, four
-// independent chains of multiply-adds (one row at a time left the fp32 pipe waiting for its own results).
-constexpr int GLUE_PAD_ROWS = 20;
-__host__ __device__ __forceinline__ int glue_hp(int H) { return (H + 3) & ~3; }
-template <int M>
-__device__ __forceinline__ void weights_to_smem(const GlueArgs& a, float2* sw, int rows) {
-  const int hp = glue_hp(a.H);
-  for (int i = threadIdx.x; i < rows * M; i += blockDim.x) {
-    const int r = i / M, j = i % M;
-    const float w = r < hp ? (r < a.H ? a.w[r * M + j] : 0.f) : (r - hp < 2 * a.G ? a.wbc[(r - hp) * M + j] : 0.f);
-    sw[i] = make_float2(w, w);
-  }
-}
-// pre[q] += sum_j dp[j] w[q][j] for four consecutive rows
-template <int M>
-__device__ __forceinline__ void quad_dot(const float2* w, const float2 (&dp)[M], float2 (&pre)[4]) {
-#pragma unroll
-  for (int c = 0; c < M; c += 2)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const float4 v = *(const float4*)(w + q * M + c);
-      pre[q] = __ffma2_rn(dp[c], make_float2(v.x, v.y), pre[q]);
-      pre[q] = __ffma2_rn(dp[c + 1], make_float2(v.z, v.w), pre[q]);
-    }
-}
-template <typename TD, typename T, int M>
-__global__ void __launch_bounds__(128) k_glue_fwd(GlueArgs a, int npoints) {
-  __shared__ __align__(16) float2 sw[GLUE_PAD_ROWS * M];
-  weights_to_smem<M>(a, sw, GLUE_PAD_ROWS);
-  __syncthreads();
-  const bool pair_store = !(a.K & 1);                      // rows of an even number of states keep pairs aligned
-  auto put = [&](T* p, float2 v, bool two) {
-    if (pair_store) {
-      if constexpr (sizeof(T) == 2) *(__nv_bfloat162*)p = __float22bfloat162_rn(v);
-      else *(float2*)p = v;
-    } else {
-      stf(p, v.x);
-      if (two) stf(p + 1, v.y);
-    }
-  };
-  const unsigned half = (a.K + 1) / 2, items = (unsigned)npoints * half;
-  const int hp = glue_hp(a.H), nbc = 2 * a.G;
-  // item = (point, pair of states); consecutive threads take consecutive pairs
-  for (unsigned item = blockIdx.x * blockDim.x + threadIdx.x; item < items; item += gridDim.x * blockDim.x) {
-    const unsigned row = item / half, b = row / a.L, l = row - b * a.L;
-    const int k = 2 * (int)(item - row * half);
-    const TD* drow = (const TD*)a.dist + b * a.d_sb + l * a.d_sl + (int64_t)k * a.d_sk;
-    const float* tok = a.tok + (size_t)row * a.RO;
-    const bool two = k + 1 < a.K;
-    float d0[M], d1[M];
-    load_feats<TD, M>(drow, d0);
-    load_feats<TD, M>(drow + (two ? a.d_sk : 0), d1);
-    float2 mk = make_float2(1.f, 1.f);
-    if (a.mask) mk = make_float2(a.mask[(size_t)row * a.K + k], a.mask[(size_t)row * a.K + (two ? k + 1 : k)]);
-    float2 dp[M];
-#pragma unroll
-    for (int j = 0; j < M; ++j) dp[j] = make_float2(d0[j], d1[j]);
-    T* out = (T*)a.dt + (size_t)row * a.H * a.K + k;
-#pragma unroll 1
-    for (int r = 0; r < hp; r += 4) {
-      float2 pre[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) { const float t = r + q < a.H ? __ldg(tok + r + q) : 0.f; pre[q] = make_float2(t, t); }
-      quad_dot<M>(sw + r * M, dp, pre);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (r + q < a.H) put(out, __fmul2_rn(make_float2(glue_softplus(pre[q].x), glue_softplus(pre[q].y)), mk), two);
-        out += a.K;
-      }
-    }
-    out = (T*)a.bc + (size_t)row * (a.RO - a.H) * a.K + k;
-    const float* tk = tok + a.H;
-#pragma unroll 1
-    for (int r = 0; r < nbc; r += 4) {
-      float2 pre[4];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) pre[q] = make_float2(0.f, 0.f);
-      quad_dot<M>(sw + (hp + r) * M, dp, pre);              // rows past the last one have zero weights
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (r + q < nbc) {
-          const float t = __ldg(tk + r + q);
-          put(out + (r + q) * a.K, __fadd2_rn(pre[q], make_float2(t, t)), two);
-          if (a.back) {
-            const float u = __ldg(tk + nbc + r + q);
-            put(out + (nbc + r + q) * a.K, __fadd2_rn(pre[q], make_float2(u, u)), two);
-          }
-        }
-    }
-  }
-}
-
-constexpr int GLUE_BWD_WARPS = 4;
-constexpr int GLUE_BWD_BLOCKS = 148 * 3;                   // two (16 features) or three blocks of four warps per SM: registers
-
-// Backward: a warp takes whole points and walks their states 64 at a time, two adjacent states per lane; it shares nothing with
-// the other warps of the block but the weights, so there is no block barrier in the walk.  Per 64 states:
-//  (1) g = d out / d pre per row and ddist = sum_r g[r] W[r, :] with packed pairs; the inputs of the next 64 states are loaded
-//      (packed, in registers) before the current ones are worked on;
-//  (2) g and the features go through the warp's part of shared memory for the weight gradient sum_k g[r, k] dist[k, j]: a lane
-//      owns NR / 2 rows x M / 2 features of it and every eighth state - 48 multiply-adds for four shared-memory reads at
-//      10 rows x 16 features - in registers over the whole walk.
-// Bound: the fp32 pipe (450 multiply-adds per (point, state)); the block-wide version with staged inputs held 12 warps per SM
-// that met at three barriers per point and used a fifth of the issue slots: 16 x 4096 x 256 x 16 bf16 1730 us.
-// NR: weight rows padded to 12 or 20 (dt rows to a multiple of four, then the B / C rows).
-template <typename TD, typename T, int M, int NR>
-__global__ void __launch_bounds__(GLUE_BWD_WARPS * 32, M == 16 ? 2 : 3) k_glue_bwd(GlueArgs a, int npoints, int pairs_ok) {
-  constexpr int RH = NR / 2, MH = M / 2, GS = NR, DS = M + 4;      // rows / features of a lane's tile; row strides in shared memory
-  __shared__ __align__(16) float2 sw[NR * M];
-  __shared__ __align__(16) float sg_all[GLUE_BWD_WARPS][64 * GS];
-  __shared__ __align__(16) float sd_all[GLUE_BWD_WARPS][64 * DS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  float* sg = sg_all[warp];
-  float* sd = sd_all[warp];
-  weights_to_smem<M>(a, sw, NR);
-  for (int i = lane; i < 64 * GS; i += 32) sg[i] = 0.f;
-  __syncthreads();
-  const int rh = lane & 1, jh = (lane >> 1) & 1, kq = lane >> 2;   // the lane's tile and its share of the states
-  float2 acc[RH][MH / 2];
-#pragma unroll
-  for (int r = 0; r < RH; ++r)
-#pragma unroll
-    for (int j = 0; j < MH / 2; ++j) acc[r][j] = make_float2(0.f, 0.f);
-  constexpr int FW = M * (int)sizeof(TD) / 8;              // 8-byte words of one state's features
-  typedef typename std::conditional<sizeof(T) == 2, uint32_t, float2>::type GP;      // a pair of gradients as loaded
-  auto up = [](GP v) {
-    if constexpr (sizeof(T) == 2) return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u));
-    else return v;
-  };
-  const int per = gridDim.x * GLUE_BWD_WARPS, first = blockIdx.x * GLUE_BWD_WARPS + warp;
-  const int nstep = (a.K + 63) / 64, nb = a.RO - a.H, hp = glue_hp(a.H);      // steps per point; B / C gradient rows; padded dt rows
-  const bool has_bc = a.gb[0] || a.gb[1] || a.gb[2] || a.gb[3];
-  uint2 fx[2][FW];
-  GP gh[8];                                  // dt gradient rows, loaded eight at a time
+template <typename TD, typename T>
+__global__ void __launch_bounds__(GLUE_WARPS * 32, sizeof(TD) == 2 ? 4 : 3) k_glue_fwd(GlueArgs a, int npoints, int M, int vec) {
+  constexpr int ND = sizeof(TD) == 2 ? 1 : 3;
+  const int lane = threadIdx.x & 31, c = lane >> 2, q = lane & 3;
+  Frag w[3];
+  weight_rows(a, M, c, q, w);
+  const int per_point = (a.K + 63) / 64;
+  const unsigned items = (unsigned)npoints * per_point, stride = gridDim.x * GLUE_WARPS;
+  unsigned item = blockIdx.x * GLUE_WARPS + (threadIdx.x >> 5);
+  typename Feat<TD>::t next[8];
+  float tk[2], tk2[2];
   float2 mk;
-  auto pair_at = [&](const T* p, bool in0, bool in1) {
-    GP v;
-    if constexpr (sizeof(T) == 2) {
-      if (pairs_ok) v = in0 ? *(const uint32_t*)p : 0u;
-      else v = (in0 ? (uint32_t)*(const uint16_t*)p : 0u) | (in1 ? (uint32_t)*((const uint16_t*)p + 1) << 16 : 0u);
-    } else {
-      if (pairs_ok) v = in0 ? *(const float2*)p : make_float2(0.f, 0.f);
-      else v = make_float2(in0 ? p[0] : 0.f, in1 ? p[1] : 0.f);
+  auto load = [&](unsigned at) {
+    const int pt = at / per_point, k0 = (int)(at - pt * (unsigned)per_point) * 64;
+    load_states<TD>(a, M, pt, k0, c, q, next);
+    mk = load_mask(a, pt, k0, c, q);
+    const float* tok = a.tok + (int64_t)pt * a.RO;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int r = c + 8 * s;
+      tk[s] = r < a.RW ? tok[r] : 0.f;
+      tk2[s] = a.back && r >= a.H && r < a.RW ? tok[r + 2 * a.G] : 0.f;
     }
-    return v;
   };
-  auto load = [&](int pt, int step) {                      // features, mask and the first eight dt gradient rows of 64 states
-    const int k = step * 64 + 2 * lane;
-    const bool in0 = k < a.K, in1 = k + 1 < a.K;
-    const int b = pt / a.L, l = pt - b * a.L;
-    const TD* d = (const TD*)a.dist + b * a.d_sb + l * a.d_sl;
+  if (item < items) load(item);
+  for (; item < items; item += stride) {
+    const int pt = item / per_point, k = (int)(item - pt * (unsigned)per_point) * 64 + 16 * q;
+    float pre[8][4];
+    const float2 m = mk;
+    const float t0 = tk[0], t1 = tk[1], v0 = tk2[0], v1 = tk2[1];
 #pragma unroll
-    for (int s2 = 0; s2 < 2; ++s2) {
-      const bool in = s2 ? in1 : in0;
-      const uint2* p = (const uint2*)(d + (int64_t)(k + s2) * a.d_sk);
-      if constexpr (FW % 2 == 0) {
+    for (int j = 0; j < 8; ++j) {
+      uint32_t f[ND][2];
+      feat_terms(next[j], f);
+      pre[j][0] = pre[j][1] = pre[j][2] = pre[j][3] = 0.f;
+      mma_terms<3, ND>(pre[j], [&](int s) { return w[s]; }, [&](int t, uint32_t& b0, uint32_t& b1) { b0 = f[t][0]; b1 = f[t][1]; });
+    }
+    if (item + stride < items) load(item + stride);
 #pragma unroll
-        for (int c = 0; c < FW / 2; ++c) {
-          const uint4 v = in ? ((const uint4*)p)[c] : make_uint4(0, 0, 0, 0);
-          fx[s2][2 * c] = make_uint2(v.x, v.y);
-          fx[s2][2 * c + 1] = make_uint2(v.z, v.w);
+    for (int s = 0; s < 2; ++s) {
+      const int r = c + 8 * s;
+      const float t = s ? t1 : t0, u = s ? v1 : v0;
+      float2 o[8];
+      if (8 * s < a.H) {                                    // some row of this half is a dt row (the mask pairs cross lanes)
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float2 mj = mask_of(m, j, q);
+          o[j] = make_float2(glue_softplus(pre[j][2 * s] + t) * mj.x, glue_softplus(pre[j][2 * s + 1] + t) * mj.y);
         }
-      } else {
+        if (r < a.H) store_row((T*)a.dt + ((int64_t)pt * a.H + r) * a.K, k, a.K, vec, o);
+      }
+      if (r >= a.H && r < a.RW) {
+        T* out = (T*)a.bc + ((int64_t)pt * (a.RO - a.H) + r - a.H) * a.K;
 #pragma unroll
-        for (int c = 0; c < FW; ++c) fx[s2][c] = in ? p[c] : make_uint2(0, 0);
+        for (int j = 0; j < 8; ++j) o[j] = make_float2(pre[j][2 * s] + t, pre[j][2 * s + 1] + t);
+        store_row(out, k, a.K, vec, o);
+        if (a.back) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = make_float2(pre[j][2 * s] + u, pre[j][2 * s + 1] + u);
+          store_row(out + (int64_t)(2 * a.G) * a.K, k, a.K, vec, o);
+        }
       }
     }
-    mk = make_float2(in0 ? 1.f : 0.f, in1 ? 1.f : 0.f);
-    if (a.mask) {
-      if (in0) mk.x = a.mask[(int64_t)pt * a.K + k];
-      if (in1) mk.y = a.mask[(int64_t)pt * a.K + k + 1];
-    }
-    if (a.ddt) {
-      const T* g = (const T*)a.ddt + (int64_t)pt * a.H * a.K + k;
+  }
+}
+
+constexpr int GLUE_BWD_BLOCKS = 148 * 3;                   // resident blocks (two per SM where features or gradients are float: registers)
+
+// Backward: a warp takes whole points, 64 states at a time; the warps of a block share nothing until the end.  Per 16 states:
+// pre again (for the softplus derivative), g = d out / d pre; ddist = sum_r g[r] W[r, :] with the 8x8 blocks of g transposed in
+// registers (movmatrix) as the A operand; dW = sum over states g[r] dist with g as it lies and the features transposed.  The weight
+// gradient of 64 states is formed on the matrix pipe and added to the lane's float sums, so long sums are rounded as float sums.
+// kSplit: the dt rows are exactly the first eight (every detector configuration here), so each half of the rows is of one kind.
+template <typename TD, typename T, bool kSplit>
+__global__ void __launch_bounds__(GLUE_WARPS * 32, sizeof(TD) == 2 ? 3 : 2) k_glue_bwd(GlueArgs a, int npoints, int M, int vec, int ddvec) {
+  constexpr int ND = sizeof(TD) == 2 ? 1 : 3;
+  using GP = typename std::conditional<sizeof(T) == 2, uint32_t, float2>::type;      // a pair of gradients as loaded
+  __shared__ float part[GLUE_WARPS][16 * 16];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, c = lane >> 2, q = lane & 3;
+  Frag w[3];
+  weight_rows(a, M, c, q, w);
+  uint32_t wb[2][3][2];                                     // weights as the B operand of ddist: [feature half][term][row half]
 #pragma unroll
-      for (int r = 0; r < 8; ++r)
-        if (r < a.H) gh[r] = pair_at(g + (int64_t)r * a.K, in0, in1);
+  for (int t = 0; t < 2; ++t)
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int r = 2 * q + 8 * i, f = 4 * (c >> 1) + 2 * t + (c & 1);
+      uint32_t s[3];
+      split3(make_float2(glue_w(a, M, r, f), glue_w(a, M, r + 1, f)), s);
+#pragma unroll
+      for (int k = 0; k < 3; ++k) wb[t][k][i] = s[k];
+    }
+  const T *rp[2], *rp2[2];                                  // this lane's gradient rows (dt, or B / C and the second direction's)
+  int64_t rst[2];
+  bool is_dt[2];
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const int r = c + 8 * s, n = r - a.H;
+    is_dt[s] = r < a.H;
+    rp[s] = rp2[s] = nullptr;
+    rst[s] = is_dt[s] ? (int64_t)a.H * a.K : a.gb_rs;
+    if (is_dt[s]) {
+      if (a.ddt) rp[s] = (const T*)a.ddt + (int64_t)r * a.K;
+    } else if (r < a.RW) {
+      const int which = n / a.G;
+      const int64_t at = (int64_t)(n - which * a.G) * a.K;
+      if (a.gb[which]) rp[s] = (const T*)a.gb[which] + at;
+      if (a.back && a.gb[which + 2]) rp2[s] = (const T*)a.gb[which + 2] + at;
+    }
+  }
+  typename Feat<TD>::t fn[8];
+  GP gn[2][8], hn[2][8];
+  float2 mn;
+  auto load = [&](int pt, int k0) {
+    load_states<TD>(a, M, pt, k0, c, q, fn);
+    mn = load_mask(a, pt, k0, c, q);
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) { gn[s][j] = GP{}; hn[s][j] = GP{}; }
+      if (rp[s]) load_row(rp[s] + pt * rst[s], k0 + 16 * q, a.K, vec, gn[s]);
+      if (!(kSplit && s == 0) && rp2[s]) load_row(rp2[s] + pt * rst[s], k0 + 16 * q, a.K, vec, hn[s]);
     }
   };
-  float tsum[NR + 8];
-#pragma unroll
-  for (int r = 0; r < NR + 8; ++r) tsum[r] = 0.f;
-  if (first < npoints) load(first, 0);
-  for (int pt = first; pt < npoints; pt += per) {
+  float acc[2][4] = {};
+  const int per = gridDim.x * GLUE_WARPS;
+  int pt = blockIdx.x * GLUE_WARPS + warp;
+  if (pt < npoints) load(pt, 0);
+  for (; pt < npoints; pt += per) {
     const float* tok = a.tok + (int64_t)pt * a.RO;
-    for (int step = 0; step < nstep; ++step) {
-      const int k = step * 64 + 2 * lane;
-      const bool in0 = k < a.K, in1 = k + 1 < a.K;
-      float2 dp[M], dd[M], m2 = mk;
-      GP g8[8];
+    const float tk[2] = {is_dt[0] ? tok[c] : 0.f, is_dt[1] ? tok[c + 8] : 0.f};
+    float ts[2] = {}, ts2[2] = {};
+    for (int k0 = 0; k0 < a.K; k0 += 64) {
+      typename Feat<TD>::t f[8];
+      GP g[2][8], h[2][8];
+      const float2 m = mn;
 #pragma unroll
-      for (int s2 = 0; s2 < 2; ++s2) {                     // features: float pairs over the two states; rows of sd
-        float f[M];
+      for (int j = 0; j < 8; ++j) {
+        f[j] = fn[j];
 #pragma unroll
-        for (int c = 0; c < FW; ++c) {
-          if constexpr (sizeof(TD) == 2) {
-            f[4 * c] = __uint_as_float(fx[s2][c].x << 16); f[4 * c + 1] = __uint_as_float(fx[s2][c].x & 0xffff0000u);
-            f[4 * c + 2] = __uint_as_float(fx[s2][c].y << 16); f[4 * c + 3] = __uint_as_float(fx[s2][c].y & 0xffff0000u);
-          } else {
-            f[2 * c] = __uint_as_float(fx[s2][c].x); f[2 * c + 1] = __uint_as_float(fx[s2][c].y);
+        for (int s = 0; s < 2; ++s) { g[s][j] = gn[s][j]; h[s][j] = hn[s][j]; }
+      }
+      if (k0 + 64 < a.K) load(pt, k0 + 64);
+      else if (pt + per < npoints) load(pt + per, 0);
+      float dw[2][4] = {};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        uint32_t fd[2][ND][2], gs[2][2][3];                 // features [tile][term][half]; g [tile][row half][term]
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int j = 2 * i + e;
+          feat_terms(f[j], fd[e]);
+          float pre[4] = {tk[0], tk[0], tk[1], tk[1]};
+          mma_terms<3, ND>(pre, [&](int s) { return w[s]; }, [&](int t, uint32_t& b0, uint32_t& b1) { b0 = fd[e][t][0]; b1 = fd[e][t][1]; });
+          const float2 mj = mask_of(m, j, q);
+#pragma unroll
+          for (int s = 0; s < 2; ++s) {
+            const float2 go = upk(g[s][j]);
+            float2 v;
+            auto through = [&] {
+              const float p0 = pre[2 * s], p1 = pre[2 * s + 1];
+              return make_float2(go.x * mj.x * (p0 <= 20.f ? glue_sigmoid(p0) : 1.f), go.y * mj.y * (p1 <= 20.f ? glue_sigmoid(p1) : 1.f));
+            };
+            if (kSplit && s == 0) {
+              v = through();
+              ts[s] += v.x + v.y;
+            } else {
+              const float2 ho = upk(h[s][j]);
+              v = make_float2(go.x + ho.x, go.y + ho.y);
+              if (!kSplit && 8 * s < a.H) {
+                const float2 d = through();
+                if (is_dt[s]) v = d;
+              }
+              ts[s] += !kSplit && is_dt[s] ? v.x + v.y : go.x + go.y;
+              ts2[s] += ho.x + ho.y;
+            }
+            split3(v, gs[e][s]);
           }
         }
+        float dd[2][4] = {};
+        Frag at[3];
 #pragma unroll
-        for (int j = 0; j < M; ++j) { if (s2) dp[j].y = f[j]; else dp[j].x = f[j]; }
+        for (int s = 0; s < 3; ++s) at[s] = Frag{{transpose8(gs[0][0][s]), transpose8(gs[1][0][s]), transpose8(gs[0][1][s]), transpose8(gs[1][1][s])}};
 #pragma unroll
-        for (int c = 0; c < M / 4; ++c) *(float4*)(sd + (2 * lane + s2) * DS + c * 4) = make_float4(f[c * 4], f[c * 4 + 1], f[c * 4 + 2], f[c * 4 + 3]);
-      }
+        for (int t = 0; t < 2; ++t)
+          mma_terms<3, 3>(dd[t], [&](int s) { return at[s]; }, [&](int u, uint32_t& b0, uint32_t& b1) { b0 = wb[t][u][0]; b1 = wb[t][u][1]; });
 #pragma unroll
-      for (int r = 0; r < 8; ++r) g8[r] = gh[r];
-      // gradients of the B / C rows of this step and the inputs of the next one
-      GP gb[8];
-      auto row_grad = [&](int q) {                         // B / C gradient row q of this step
-        const int which = q / a.G;
-        const T* p = (const T*)a.gb[which];
-        return p ? pair_at(p + (int64_t)pt * a.gb_rs + (int64_t)(q - which * a.G) * a.K + k, in0, in1) : GP{};
-      };
-      if (has_bc) {
+        for (int t = 0; t < 2; ++t) {
+          uint32_t ft[ND][2];
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-          if (r < nb) gb[r] = row_grad(r);
-      }
-      if (step + 1 < nstep) load(pt, step + 1);
-      else if (pt + per < npoints) load(pt + per, 0);
+          for (int u = 0; u < ND; ++u) { ft[u][0] = transpose8(fd[0][u][t]); ft[u][1] = transpose8(fd[1][u][t]); }
+          mma_terms<3, ND>(dw[t], [&](int s) { return Frag{{gs[0][0][s], gs[0][1][s], gs[1][0][s], gs[1][1][s]}}; },
+                           [&](int u, uint32_t& b0, uint32_t& b1) { b0 = ft[u][0]; b1 = ft[u][1]; });
+        }
 #pragma unroll
-      for (int j = 0; j < M; ++j) dd[j] = make_float2(0.f, 0.f);
+        for (int e = 0; e < 2; ++e) {
+          const int k = k0 + 16 * (c >> 1) + (c & 1) + 2 * (2 * i + e);
+          if (k < a.K && 4 * q < M) {
+            TD* o = (TD*)a.ddist + ((int64_t)pt * a.K + k) * M + 4 * q;
+            const float v[4] = {dd[0][2 * e], dd[0][2 * e + 1], dd[1][2 * e], dd[1][2 * e + 1]};
+            if (ddvec) {
+              if constexpr (sizeof(TD) == 2) *(uint2*)o = make_uint2(pk(v[0], v[1]), pk(v[2], v[3]));
+              else *(float4*)o = make_float4(v[0], v[1], v[2], v[3]);
+            } else {
 #pragma unroll
-      for (int rq = 0; rq < NR; rq += 4) {
-        float2 g[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) g[q] = make_float2(0.f, 0.f);
-        if (rq < hp) {
-          if (a.ddt) {
-            float2 pre[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) { const float t = rq + q < a.H ? __ldg(tok + rq + q) : 0.f; pre[q] = make_float2(t, t); }
-            quad_dot<M>(sw + rq * M, dp, pre);
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const int r = rq + q;
-              const float2 s2 = make_float2(pre[q].x <= 20.f ? glue_sigmoid(pre[q].x) : 1.f, pre[q].y <= 20.f ? glue_sigmoid(pre[q].y) : 1.f);
-              float2 go = make_float2(0.f, 0.f);
-              if (r < a.H) go = r < 8 ? up(g8[r & 7]) : up(pair_at((const T*)a.ddt + ((int64_t)pt * a.H + r) * a.K + k, in0, in1));
-              g[q] = __fmul2_rn(__fmul2_rn(go, m2), s2);
-              tsum[r] += g[q].x + g[q].y;
+              for (int x = 0; x < 4; ++x) stf(o + x, v[x]);
             }
           }
-        } else if (has_bc) {
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int c = rq - hp + q, c2 = c + 2 * a.G;   // both directions share the weight row
-            if (c >= 2 * a.G) continue;
-            g[q] = c == 0 ? up(gb[0]) : c == 1 ? up(gb[1]) : up(row_grad(c));
-            if (a.back) g[q] = __fadd2_rn(g[q], c2 == 2 ? up(gb[2]) : c2 == 3 ? up(gb[3]) : up(row_grad(c2)));
-          }
-        }
-#pragma unroll
-        for (int c = 0; c < M; c += 2)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const float4 v = *(const float4*)(sw + (rq + q) * M + c);
-            dd[c] = __ffma2_rn(g[q], make_float2(v.x, v.y), dd[c]);
-            dd[c + 1] = __ffma2_rn(g[q], make_float2(v.z, v.w), dd[c + 1]);
-          }
-        *(float4*)(sg + (2 * lane) * GS + rq) = make_float4(g[0].x, g[1].x, g[2].x, g[3].x);
-        *(float4*)(sg + (2 * lane + 1) * GS + rq) = make_float4(g[0].y, g[1].y, g[2].y, g[3].y);
-      }
-      if (has_bc) {                                        // token terms of the B / C rows (each output row has its own)
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          if (q < nb) {
-            const float2 v = q < 4 ? up(gb[q & 3]) : up(row_grad(q));
-            tsum[NR + q] += v.x + v.y;
-          }
-        for (int q = 8; q < nb; ++q) {                     // more than two groups: straight to the token gradient
-          const float2 v = up(row_grad(q));
-          const float t = warp_sum(v.x + v.y);
-          if (lane == 0) { float* o = a.dtok + (int64_t)pt * a.RO + a.H + q; *o = step ? *o + t : t; }
         }
       }
-      TD* ddist = (TD*)a.ddist + ((int64_t)pt * a.K + k) * M;
-      {
-        float f[M];
 #pragma unroll
-        for (int j = 0; j < M; ++j) f[j] = dd[j].x;
-        if (in0) store_feats<TD, M>(ddist, f);
+      for (int t = 0; t < 2; ++t)
 #pragma unroll
-        for (int j = 0; j < M; ++j) f[j] = dd[j].y;
-        if (in1) store_feats<TD, M>(ddist + M, f);
-      }
-      __syncwarp();
-#pragma unroll 2
-      for (int i = 0; i < 8; ++i) {
-        const float* gp = sg + (kq + 8 * i) * GS + rh * RH;
-        const float* dq = sd + (kq + 8 * i) * DS + jh * MH;
-        float gv[RH];
-#pragma unroll
-        for (int r = 0; r < RH; r += 2) { const float2 v = *(const float2*)(gp + r); gv[r] = v.x; gv[r + 1] = v.y; }
-#pragma unroll
-        for (int j = 0; j < MH / 2; ++j) {
-          const float2 dv = *(const float2*)(dq + 2 * j);
-#pragma unroll
-          for (int r = 0; r < RH; ++r) acc[r][j] = __ffma2_rn(make_float2(gv[r], gv[r]), dv, acc[r][j]);
-        }
-      }
-      __syncwarp();
+        for (int i = 0; i < 4; ++i) acc[t][i] += dw[t][i];
     }
     // token gradients of the point: sums over its states
 #pragma unroll
-    for (int r = 0; r < NR + 8; ++r) {
-      const bool head = r < NR;
-      const int o = head ? r : a.H + r - NR;
-      if (head ? r < a.H : r - NR < nb) {
-        const float t = warp_sum(tsum[r]);
-        if (lane == 0) a.dtok[(int64_t)pt * a.RO + o] = t;
+    for (int s = 0; s < 2; ++s) {
+      float u = ts[s], v = ts2[s];
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        u += __shfl_xor_sync(0xffffffffu, u, o);
+        v += __shfl_xor_sync(0xffffffffu, v, o);
       }
-      tsum[r] = 0.f;
+      const int r = c + 8 * s;
+      if (q == 0 && r < a.RW) {
+        float* d = a.dtok + (int64_t)pt * a.RO + r;
+        d[0] = u;
+        if (a.back && !is_dt[s]) d[2 * a.G] = v;
+      }
     }
   }
-  // the eight shares of the states, then the four warps, in a fixed order
-  __syncthreads();
+  // the warps of the block in a fixed order
 #pragma unroll
-  for (int r = 0; r < RH; ++r)
+  for (int t = 0; t < 2; ++t)
 #pragma unroll
-    for (int j = 0; j < MH / 2; ++j) {
-      float2 v = acc[r][j];
-#pragma unroll
-      for (int o = 4; o < 32; o <<= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-      }
-      if (kq == 0) *(float2*)(sg + (rh * RH + r) * M + jh * MH + 2 * j) = v;
-    }
+    for (int i = 0; i < 4; ++i) part[warp][(c + 8 * (i >> 1)) * 16 + 4 * q + 2 * t + (i & 1)] = acc[t][i];
   __syncthreads();
   for (int i = threadIdx.x; i < a.RW * M; i += blockDim.x) {
-    const int r = i / M, at = (r < a.H ? r : hp + r - a.H) * M + i % M;
     float t = 0.f;
 #pragma unroll
-    for (int w = 0; w < GLUE_BWD_WARPS; ++w) t += sg_all[w][at];
+    for (int x = 0; x < GLUE_WARPS; ++x) t += part[x][(i / M) * 16 + i % M];
     a.dwpart[(size_t)blockIdx.x * GLUE_MAX_ROWS * M + i] = t;
   }
 }
@@ -545,27 +544,23 @@ extern "C" int issm_b200_glue_fwd(const issm_glue_params* p, void* stream) {
   int rc = glue_validate(p, false);
   if (rc) return rc;
   const GlueArgs a = glue_args(*p);
-  if ((int64_t)p->batch * p->seqlen * ((p->nstates + 1) / 2) > 0x7fffffff - 148 * 16 * 128) return ISSM_ERR_SHAPE;
+  const int64_t items = (int64_t)p->batch * p->seqlen * ((p->nstates + 63) / 64);
+  if (items > 0x7fffffff - GLUE_FWD_BLOCKS * GLUE_WARPS) return ISSM_ERR_SHAPE;
   const int npoints = p->batch * p->seqlen;
-  const int64_t want = cdiv64((int64_t)npoints * ((p->nstates + 1) / 2), 128);
+  const int64_t want = cdiv64(items, GLUE_WARPS);
   const unsigned grid = (unsigned)(want < GLUE_FWD_BLOCKS ? want : GLUE_FWD_BLOCKS);
   cudaStream_t s = (cudaStream_t)stream;
-#define GLUE_FWD_M(TD, T)                                                                             \
-  do {                                                                                                \
-    if (p->nfeat == 16) ISSM_LAUNCH((k_glue_fwd<TD, T, 16>), grid, 128, 0, s, a, npoints);            \
-    else if (p->nfeat == 8) ISSM_LAUNCH((k_glue_fwd<TD, T, 8>), grid, 128, 0, s, a, npoints);         \
-    else ISSM_LAUNCH((k_glue_fwd<TD, T, 4>), grid, 128, 0, s, a, npoints);                            \
-  } while (0)
-  if (p->io_dtype == ISSM_F32) GLUE_FWD_M(float, float);
-  else if (p->dist_dtype == ISSM_F32) GLUE_FWD_M(float, bf16);
-  else GLUE_FWD_M(bf16, bf16);
-#undef GLUE_FWD_M
+  const size_t es = p->io_dtype == ISSM_F32 ? 4 : 2;
+  const int vec = (p->nstates * es) % 16 == 0 && !(((uintptr_t)p->dt | (uintptr_t)p->bc) % 16);      // rows of states start on 16 bytes
+  if (p->io_dtype == ISSM_F32) ISSM_LAUNCH((k_glue_fwd<float, float>), grid, GLUE_WARPS * 32, 0, s, a, npoints, p->nfeat, vec);
+  else if (p->dist_dtype == ISSM_F32) ISSM_LAUNCH((k_glue_fwd<float, bf16>), grid, GLUE_WARPS * 32, 0, s, a, npoints, p->nfeat, vec);
+  else ISSM_LAUNCH((k_glue_fwd<bf16, bf16>), grid, GLUE_WARPS * 32, 0, s, a, npoints, p->nfeat, vec);
   return ISSM_OK;
 }
 
 static int glue_bwd_blocks(const issm_glue_params* p) {
-  const int64_t need = cdiv64((int64_t)p->batch * p->seqlen, GLUE_BWD_WARPS);
-  const int64_t most = p->nfeat == 16 ? 148 * 2 : GLUE_BWD_BLOCKS;
+  const int64_t need = cdiv64((int64_t)p->batch * p->seqlen, GLUE_WARPS);
+  const int64_t most = p->dist_dtype == ISSM_F32 ? 148 * 2 : GLUE_BWD_BLOCKS;
   return (int)(need < most ? need : most);
 }
 
@@ -583,22 +578,18 @@ extern "C" int issm_b200_glue_bwd(const issm_glue_params* p, void* stream) {
   const int blocks = glue_bwd_blocks(p), npoints = p->batch * p->seqlen;
   cudaStream_t s = (cudaStream_t)stream;
   const size_t es = p->io_dtype == ISSM_F32 ? 4 : 2;
-  // pairs of gradients are one access where every row of states starts on the pair's alignment
-  const int pairs_ok = !(p->nstates & 1) && !((uintptr_t)p->ddt % (2 * es)) && !((uintptr_t)p->dbc % (2 * es)) &&
-                       !(((uintptr_t)p->dbc_part[0] | (uintptr_t)p->dbc_part[1] | (uintptr_t)p->dbc_part[2] | (uintptr_t)p->dbc_part[3]) % (2 * es));
-#define GLUE_BWD(TD, TT, MM)                                                                          \
-  do {                                                                                                \
-    if (glue_hp(a.H) + 2 * a.G <= 12) ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 12>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok); \
-    else ISSM_LAUNCH((k_glue_bwd<TD, TT, MM, 20>), blocks, GLUE_BWD_WARPS * 32, 0, s, a, npoints, pairs_ok);            \
+  // rows of states start on 16 bytes; four features of ddist are one access
+  const int vec = (p->nstates * es) % 16 == 0 && !(((uintptr_t)p->ddt | (uintptr_t)p->dbc) % 16) &&
+                  !(((uintptr_t)p->dbc_part[0] | (uintptr_t)p->dbc_part[1] | (uintptr_t)p->dbc_part[2] | (uintptr_t)p->dbc_part[3]) % 16);
+  const int ddvec = (uintptr_t)p->ddist % (p->dist_dtype == ISSM_F32 ? 16 : 8) == 0;
+#define GLUE_BWD(TD, TT)                                                                                                                  \
+  do {                                                                                                                                    \
+    if (a.H == 8) ISSM_LAUNCH((k_glue_bwd<TD, TT, true>), blocks, GLUE_WARPS * 32, 0, s, a, npoints, p->nfeat, vec, ddvec);                \
+    else ISSM_LAUNCH((k_glue_bwd<TD, TT, false>), blocks, GLUE_WARPS * 32, 0, s, a, npoints, p->nfeat, vec, ddvec);                        \
   } while (0)
-#define GLUE_BWD_M(TD, TT)                                                                            \
-  do {                                                                                                \
-    if (p->nfeat == 16) GLUE_BWD(TD, TT, 16); else if (p->nfeat == 8) GLUE_BWD(TD, TT, 8); else GLUE_BWD(TD, TT, 4); \
-  } while (0)
-  if (p->io_dtype == ISSM_F32) GLUE_BWD_M(float, float);
-  else if (p->dist_dtype == ISSM_F32) GLUE_BWD_M(float, bf16);
-  else GLUE_BWD_M(bf16, bf16);
-#undef GLUE_BWD_M
+  if (p->io_dtype == ISSM_F32) GLUE_BWD(float, float);
+  else if (p->dist_dtype == ISSM_F32) GLUE_BWD(float, bf16);
+  else GLUE_BWD(bf16, bf16);
 #undef GLUE_BWD
   const int n = a.RW * p->nfeat;
   ISSM_LAUNCH(k_glue_reduce, (n + 31) / 32, dim3(32, 8), 0, s, a.dwpart, blocks, GLUE_MAX_ROWS * p->nfeat, n, p->dweight);

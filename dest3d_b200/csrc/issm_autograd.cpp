@@ -5,6 +5,7 @@
 // Host code only; every kernel is behind the C ABI.
 #include "issm_torch.h"
 
+#include <ATen/autocast_mode.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAException.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -466,6 +467,59 @@ std::vector<Tensor> dt_bc(const Tensor& dist, const Tensor& w_dt, const Tensor& 
   return GlueFn::apply(dist, w_dt, w_bc, dt_bias, m, out, terms);
 }
 
+// Float operands of the projections under bfloat16 autocast, converted in one launch each way; the values are those of the
+// conversions that autocast itself would make, one by one.  Tensors it does not suit stay as they are, for autocast.
+struct CastFn : public Function<CastFn> {
+  static variable_list run(const variable_list& from, at::ScalarType to) {
+    variable_list out(from.size());
+    std::vector<issm_cast_item> items;
+    variable_list keep;
+    for (size_t i = 0; i < from.size(); ++i) {
+      if (!from[i].defined()) continue;
+      keep.push_back(from[i].contiguous());
+      out[i] = at::empty(from[i].sizes(), from[i].options().dtype(to));
+      issm_cast_item it{};
+      it.src = keep.back().data_ptr(); it.dst = out[i].data_ptr(); it.n = out[i].numel(); it.to_bf16 = to == at::kBFloat16;
+      if ((uintptr_t)it.src % 16) { out[i] = from[i].to(to); continue; }
+      items.push_back(it);
+    }
+    if (!items.empty())
+      check_rc(issm_b200_cast_multi(items.data(), (int32_t)items.size(), stream_of(keep[0])), "issm_b200_cast_multi");
+    return out;
+  }
+  static variable_list forward(AutogradContext* ctx, at::TensorList from) {
+    ctx->set_materialize_grads(false);
+    const c10::cuda::CUDAGuard guard(from[0].device());
+    return run(from.vec(), at::kBFloat16);
+  }
+  static variable_list backward(AutogradContext*, variable_list g) {
+    for (const Tensor& t : g)
+      if (t.defined()) {
+        const c10::cuda::CUDAGuard guard(t.device());
+        return run(g, at::kFloat);
+      }
+    return g;
+  }
+};
+static variable_list projection_operands(variable_list t) {
+  if (!t[0].is_cuda() || !at::autocast::is_autocast_enabled(at::kCUDA) || at::autocast::get_autocast_dtype(at::kCUDA) != at::kBFloat16) return t;
+  const c10::cuda::CUDAGuard guard(t[0].device());
+  for (const bool grad : {false, true}) {                   // apart: an output of a function with any such input asks for gradients
+    std::vector<size_t> which;
+    variable_list from;
+    for (size_t i = 0; i < t.size() && from.size() < ISSM_ADD_MAX; ++i)
+      if (t[i].is_cuda() && t[i].scalar_type() == at::kFloat && t[i].device() == t[0].device() &&
+          (at::GradMode::is_enabled() && t[i].requires_grad()) == grad) {
+        from.push_back(t[i]);
+        which.push_back(i);
+      }
+    if (from.size() < 2) continue;
+    const auto c = grad ? CastFn::apply(at::TensorList(from)) : CastFn::run(from, at::kBFloat16);
+    for (size_t i = 0; i < which.size(); ++i) t[which[i]] = c[i];
+  }
+  return t;
+}
+
 // The bidirectional ISSM block (issm_block.py MultiHeadISSMScan.forward; models/dest_module.py:519-612) in one call.  Ordinary
 // differentiable operations in order; autocast applies to the projections and the layer norm as it does from Python.
 std::tuple<Tensor, Tensor> block(const Tensor& in_key, const Tensor& in_query, const Tensor& dist, const OptTensor& mask, const Tensor& key_w,
@@ -475,22 +529,23 @@ std::tuple<Tensor, Tensor> block(const Tensor& in_key, const Tensor& in_query, c
                                  int64_t H, int64_t G, int64_t d_state, int64_t chunk, double lo, double hi, const Tensor& status) {
   const int64_t di = query_w.size(0), P = di / H;
   // split, not narrow: its gradient is one concatenation
-  const auto zx = at::linear(in_key, key_w).split_with_sizes({di, di + 2 * G, H}, -1);
+  const auto po = projection_operands({in_key, key_w, in_query, query_w, okey_w, oquery_w});
+  const auto zx = at::linear(po[0], po[1]).split_with_sizes({di, di + 2 * G, H}, -1);
   const Tensor xbc = conv_silu(zx[1], conv_w, conv_b);
   const Tensor back = conv_silu(xbc, convb_w, convb_b);    // the second convolution takes the OUTPUT of the first (dest_module.py:534)
   const auto f = xbc.split_with_sizes({di, G, G}, -1), r = back.split_with_sizes({di, G, G}, -1);
   const auto b = in_key.size(0), L = in_key.size(1), K = in_query.size(1);
   auto heads = [&](const Tensor& t) { return t.contiguous().view({b, L, H, P}); };
-  const Tensor init = at::linear(in_query, query_w).view({b, K, H, P}).permute({0, 2, 3, 1});
+  const Tensor init = at::linear(po[2], po[3]).view({b, K, H, P}).permute({0, 2, 3, 1});
   const Tensor A = DecayFn::apply(A_log, d_state);
   const auto act = xbc.scalar_type();
   const Tensor feats = dist.scalar_type() == act || (dist.scalar_type() == at::kFloat && act == at::kBFloat16) ? dist : dist.to(act);
   const std::vector<Tensor> terms{zx[2], f[1], f[2], r[1], r[2]};
   const auto g = dt_bc(feats, dt_w, bc_w, dt_bias, mask, act, terms);
   const auto [key, last] = bi_scan(heads(f[0]), heads(r[0]), g[0], A, g[1], g[2], g[3], g[4], chunk, D, {}, {}, init, false, lo, hi, 0.5, 0, status);
-  const Tensor out_key = at::linear(norm(key.view({b, L, di}), kn_w, {}, zx[0], kn_eps, 0, false, true), okey_w);
+  const Tensor out_key = at::linear(norm(key.view({b, L, di}), kn_w, {}, zx[0], kn_eps, 0, false, true), po[4]);
   const Tensor q = last.permute({0, 3, 1, 2}).reshape({b, K, di}).to(out_key.scalar_type());
-  return {out_key, at::linear(at::layer_norm(q, {di}, qn_w, qn_b, qn_eps), oquery_w)};
+  return {out_key, at::linear(at::layer_norm(q, {di}, qn_w, qn_b, qn_eps), po[5])};
 }
 }  // namespace issm_host
 

@@ -50,6 +50,42 @@ __global__ void __launch_bounds__(kThreads) k_add_multi(const __grid_constant__ 
     }
   }
 }
+
+// A projection's operands are 0.1 to 10 MB each at the detector's sizes, so a conversion is its launch: six of them in one.
+struct CastArgs { issm_cast_item item[ISSM_ADD_MAX]; unsigned first_block[ISSM_ADD_MAX + 1]; int n; };
+constexpr int kCast = kThreads * 2 * 8;                    // elements per block
+__global__ void __launch_bounds__(kThreads) k_cast_multi(const __grid_constant__ CastArgs p) {
+  int k = 0;
+  while (k + 1 < p.n && blockIdx.x >= p.first_block[k + 1]) ++k;
+  const issm_cast_item& it = p.item[k];
+  const int64_t e0 = (int64_t)(blockIdx.x - p.first_block[k]) * kCast + threadIdx.x * 8;
+  const float* sf = (const float*)it.src;
+  const bf16* sh = (const bf16*)it.src;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int64_t e = e0 + i * (kThreads * 8);
+    if (e + 8 <= it.n) {
+      if (it.to_bf16) {
+        const float4 u = *(const float4*)(sf + e), v = *(const float4*)(sf + e + 4);
+        const __nv_bfloat162 o[4] = {__floats2bfloat162_rn(u.x, u.y), __floats2bfloat162_rn(u.z, u.w), __floats2bfloat162_rn(v.x, v.y),
+                                     __floats2bfloat162_rn(v.z, v.w)};
+        const uint32_t* w = (const uint32_t*)o;
+        *(uint4*)((bf16*)it.dst + e) = make_uint4(w[0], w[1], w[2], w[3]);
+      } else {
+        const uint4 w = *(const uint4*)(sh + e);
+        auto lo = [](uint32_t x) { return __uint_as_float(x << 16); };
+        auto hi = [](uint32_t x) { return __uint_as_float(x & 0xffff0000u); };
+        *(float4*)((float*)it.dst + e) = make_float4(lo(w.x), hi(w.x), lo(w.y), hi(w.y));
+        *(float4*)((float*)it.dst + e + 4) = make_float4(lo(w.z), hi(w.z), lo(w.w), hi(w.w));
+      }
+    } else {
+      for (int64_t j = e; j < it.n && j < e + 8; ++j) {
+        if (it.to_bf16) stf((bf16*)it.dst + j, sf[j]);
+        else ((float*)it.dst)[j] = ldf(sh + j);
+      }
+    }
+  }
+}
 }  // namespace
 }  // namespace issm
 
@@ -76,5 +112,27 @@ extern "C" int issm_b200_add_multi(const issm_add_item* items, int32_t count, vo
   if (blocks > 0x7fffffffull) return ISSM_ERR_SHAPE;
   p.first_block[p.n] = (unsigned)blocks;
   ISSM_LAUNCH(k_add_multi, (unsigned)blocks, kThreads, 0, (cudaStream_t)stream, p);
+  return ISSM_OK;
+}
+
+extern "C" int issm_b200_cast_multi(const issm_cast_item* items, int32_t count, void* stream) {
+  if (!items) return ISSM_ERR_NULL;
+  if (count < 0 || count > ISSM_ADD_MAX) return ISSM_ERR_SHAPE;
+  CastArgs p{};
+  uint64_t blocks = 0;
+  for (int i = 0; i < count; ++i) {
+    const issm_cast_item& it = items[i];
+    if (it.n == 0) continue;
+    if (it.n < 0) return ISSM_ERR_SHAPE;
+    if (!it.src || !it.dst) return ISSM_ERR_NULL;
+    if (((uintptr_t)it.src | (uintptr_t)it.dst) & 15) return ISSM_ERR_ALIGN;
+    p.item[p.n] = it;
+    p.first_block[p.n++] = (unsigned)blocks;
+    blocks += (uint64_t)cdiv64(it.n, kCast);
+  }
+  if (!p.n) return ISSM_OK;
+  if (blocks > 0x7fffffffull) return ISSM_ERR_SHAPE;
+  p.first_block[p.n] = (unsigned)blocks;
+  ISSM_LAUNCH(k_cast_multi, (unsigned)blocks, kThreads, 0, (cudaStream_t)stream, p);
   return ISSM_OK;
 }

@@ -311,6 +311,15 @@ typedef struct issm_add_item {
 } issm_add_item;
 int issm_b200_add_multi(const issm_add_item* items, int32_t count, void* cuda_stream);
 
+/* dst = src converted between float and bfloat16 (to nearest even) for up to ISSM_ADD_MAX contiguous arrays in one launch: the
+ * operands of the block's projections under autocast, and their gradients on the way back.  16-byte aligned pointers. */
+typedef struct issm_cast_item {
+  const void* src; void* dst;
+  int64_t n;
+  int32_t to_bf16;                /* 1: float to bfloat16, 0: bfloat16 to float */
+} issm_cast_item;
+int issm_b200_cast_multi(const issm_cast_item* items, int32_t count, void* cuda_stream);
+
 /* Number of kernel launches the library has enqueued since load (monotonic, process-wide);
  * used by the benchmark to report how many of its own kernels ran inside a timed region. */
 uint64_t issm_b200_launch_count(void);

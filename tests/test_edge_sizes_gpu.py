@@ -111,3 +111,20 @@ def test_parameter_generation(dtype, L, K, M, H, G):
     for u, v in list(zip(got, ref)) + [(d.grad, r.grad) for d, r in zip(dev, ref_in)]:
         v = v.detach()
         assert (u.double().cpu() - v).abs().max().item() <= lim * max(1.0, v.abs().max().item())
+
+
+@pytest.mark.parametrize("sizes", [(1,), (7, 8, 9), (4095, 4096, 4097, 16388)])
+def test_cast_multi(sizes):
+    from dest3d_b200 import _lib
+    lib = _lib.lib()
+
+    class Item(ct.Structure):
+        _fields_ = [("src", ct.c_void_p), ("dst", ct.c_void_p), ("n", ct.c_int64), ("to_bf16", ct.c_int32)]
+    lib.issm_b200_cast_multi.argtypes = [ct.c_void_p, ct.c_int32, ct.c_void_p]
+    src = [torch.randn(n, device="cuda") for n in sizes]
+    half, back = [torch.empty_like(t, dtype=torch.bfloat16) for t in src], [torch.empty_like(t) for t in src]
+    for a, b, to in ((src, half, 1), (half, back, 0)):
+        items = (Item * len(sizes))(*[Item(u.data_ptr(), v.data_ptr(), u.numel(), to) for u, v in zip(a, b)])
+        assert lib.issm_b200_cast_multi(items, len(sizes), torch.cuda.current_stream().cuda_stream) == 0
+    for t, h, k in zip(src, half, back):
+        assert torch.equal(h, t.bfloat16()) and torch.equal(k, t.bfloat16().float())

@@ -425,12 +425,22 @@ __global__ void k_blk_chain(const __grid_constant__ BArgs a, int PW, int reverse
     if (reverse) run = a.dfinal ? a.dfinal[e] : 0.f;
     else run = a.init ? ldf((const TIO*)a.init + e) : 0.f;
   }
-  for (int k = 0; k < a.nseg; ++k) {
-    const int s = reverse ? a.nseg - 1 - k : k;
-    const size_t at = (stream * a.nseg + s) * a.N + n;
-    const float local = a.seg_out[at * PW + p];
-    a.seg_out[at * PW + p] = run;
-    run = fmaf(exp2f(a.seg_sum[at]), run, local);
+  for (int k0 = 0; k0 < a.nseg; k0 += 8) {                 // eight segments' loads at once: one latency, not eight
+    float local[8], sum[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int c = min(k0 + k, a.nseg - 1), s = reverse ? a.nseg - 1 - c : c;
+      const size_t at = (stream * a.nseg + s) * a.N + n;
+      local[k] = a.seg_out[at * PW + p];
+      sum[k] = a.seg_sum[at];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= a.nseg) break;
+      const int s = reverse ? a.nseg - 1 - k0 - k : k0 + k;
+      a.seg_out[((stream * a.nseg + s) * a.N + n) * PW + p] = run;
+      run = fmaf(exp2f(sum[k]), run, local[k]);
+    }
   }
   if (p < a.P && fin) fin[e] = run;
   if (p < a.P && fin_io) stf(fin_io + e, run);

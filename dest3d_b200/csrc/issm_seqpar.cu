@@ -55,15 +55,27 @@ __global__ void k_slice_chain(const __grid_constant__ issm_slice_chain q) {
   const int64_t hn = (int64_t)q.nheads * q.dstate, sn = (int64_t)h * q.dstate + n;
   const int total = q.nmain + (q.f_tail ? 1 : 0);
   float run = !q.start ? 0.f : q.start_f32 ? ((const float*)q.start)[i] : ldf((const bf16*)q.start + i);
-#pragma unroll 4
-  for (int k = 0; k < total; ++k) {
-    const int s = q.descending ? total - 1 - k : k;
-    const bool tail = s == q.nmain;
-    const int64_t row = tail ? b : b * q.nmain + s, at = row * hpn + e;
-    void* en = tail ? q.enter_tail : q.enter_main;
-    if (q.enter_f32) ((float*)en)[at] = run;
-    else stf((bf16*)en + at, run);
-    run = fmaf(exp2f((tail ? q.s_tail : q.s_main)[row * hn + sn]), run, (tail ? q.f_tail : q.f_main)[at]);
+  for (int k0 = 0; k0 < total; k0 += 8) {                  // eight slices' loads at once: one latency, not eight
+    float local[8], sum[8];
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int c = min(k0 + k, total - 1), s = q.descending ? total - 1 - c : c;
+      const bool tail = s == q.nmain;
+      const int64_t row = tail ? b : b * q.nmain + s;
+      local[k] = (tail ? q.f_tail : q.f_main)[row * hpn + e];
+      sum[k] = (tail ? q.s_tail : q.s_main)[row * hn + sn];
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      if (k0 + k >= total) break;
+      const int s = q.descending ? total - 1 - k0 - k : k0 + k;
+      const bool tail = s == q.nmain;
+      const int64_t at = (tail ? b : b * q.nmain + s) * hpn + e;
+      void* en = tail ? q.enter_tail : q.enter_main;
+      if (q.enter_f32) ((float*)en)[at] = run;
+      else stf((bf16*)en + at, run);
+      run = fmaf(exp2f(sum[k]), run, local[k]);
+    }
   }
   if (q.last) {
     if (q.last_f32) ((float*)q.last)[i] = run;

@@ -973,10 +973,11 @@ bool blk_plan(const issm_params& p, int pass, Plan* out) {
   q.nslice = (nw32 + q.nw - 1) / q.nw;
   q.nblk = (p.seqlen + R - 1) / R;
   // segments only when the streams leave most of the chip idle: the extra states-only walk costs about half a pass.
-  // 148 SMs x 6 warps; a segment keeps at least 4 blocks
+  // 148 SMs x 10 warps, a segment keeps at least 2 blocks: both scan directions of 2 x 1024 points, 8 heads, 256 states float
+  // 1006 us (6 warps, 4 blocks: 1160), 2 x 3000 points 2834 us (3060), 1 x 300 points 379 us (565)
   const long warps = (long)p.batch * p.nheads * q.nslice * q.nw;
-  long want = (148L * 6) / warps;
-  if (want > q.nblk / 4) want = q.nblk / 4;
+  long want = (148L * 10) / warps;
+  if (want > q.nblk / 2) want = q.nblk / 2;
   if (want < 2) want = 1;
   q.seg_blk = (q.nblk + (int)want - 1) / (int)want;
   q.nseg = (q.nblk + q.seg_blk - 1) / q.seg_blk;
